@@ -85,3 +85,24 @@ def test_half_outputs_sharded_upload_and_error_paths():
     b96, w96 = _upload(D.Q4_1, 8, 96, seed=27)
     with pytest.raises(XnqError):
         w96.matmul_t(torch.zeros(1, 96, device=DEV))
+
+
+# around the edges of the kernel's splits: one piece of 32 or one super-block, the k where more warps share a row (64 and 128 pieces) and a
+# ragged last round of pieces; odd row counts; every tile of activation rows (1, 2, 4, 8, 16) with remainders
+@pytest.mark.parametrize("dt", FORMATS)
+@pytest.mark.parametrize("kb", [1, 7, 8, 15, 16, 21])
+def test_matmul_row_and_tile_edges(dt, kb):
+    k = 256 * kb if dt.block_size == 256 else 192 * kb - 64 * (kb == 1)
+    for n, m in ((1, 2), (3, 3), (17, 8), (33, 9), (2, 35)):
+        blocks, w = _upload(dt, n, k, seed=kb + n)
+        x = synth.make_activation(m, k, seed=kb + m)
+        xd = torch.from_numpy(x).to(DEV)
+        got = w.matmul_t(xd)
+        want = O.matmul(int(dt), x, blocks, n)
+        # both sides add at most two rounded f32 terms per 32 elements to a running f32 sum: k / 16 roundings of partial sums that stay
+        # below sum |w| |x| (doubled: the min terms do not cancel in it; the activations' own rounding is common to both sides)
+        dense = np.abs(O.to_float(int(dt), blocks, n * k).reshape(n, k)).astype(np.float64)
+        bound = 4 * (k / 16 + 8) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ dense.T + np.abs(x).max() * dense.max() * 32)
+        assert (np.abs(got.cpu().numpy().astype(np.float64) - want) <= bound).all(), (dt.name, n, k, m)
+        for r in (0, m - 1):   # the sum's order depends on k alone
+            assert torch.equal(w.matmul_t(xd[r:r + 1]), got[r:r + 1])

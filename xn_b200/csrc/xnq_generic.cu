@@ -6,14 +6,10 @@
 // They are therefore kept on the device exactly as in the file (canonical blocks, no re-layout) and served by one plain
 // kernel per operation:
 //   to_float   one thread per element, the reference's arithmetic operation for operation (bit-identical results);
-//   matmul     activations are quantized to the canonical blocks of the format's VecDotType (Q8_0, Q8_1 or Q8_K, by the
-//              same quantizers that xnq_quantize_act exposes, byte-identical to the reference's), then one warp per
-//              weight row, lane l taking blocks l, l + 32, ...: each block's integer sums and its scaling in f32 are
-//              exactly the reference's, the block contributions are added lane-wise and then across the warp (the one
-//              difference from the reference's serial sum; within 2e-3 under its own metric). All activation rows are
-//              served by the same warp in turn, so the weight is read from DRAM once.
-// HBM-bound streaming kernels in the style of the four main formats would be the next step for any of these formats that
-// turns out to matter.
+//   matmul     activations are quantized to the block format of the weight's VecDotType (Q8_0, Q8_1 or Q8_K) as planar codes,
+//              scales and 16-sums, then one kernel unpacks the file's blocks to int8 codes in registers and multiplies them with
+//              dp4a: each block's integer sums are exact, scales are applied in f32 as in the reference, and only the order in
+//              which block contributions are added differs from its serial sum (within 2e-3 under its own metric).
 #include "xnq_common.cuh"
 #include "xnq_quantize_act.cuh"
 #include "xnq_unpack.cuh"
@@ -26,9 +22,6 @@ constexpr int TPB = 256;
 __device__ __forceinline__ uint32_t ld16(const uint8_t *p) { return *reinterpret_cast<const uint16_t *>(p); } // blocks are 2-byte aligned
 __device__ __forceinline__ uint32_t ld32(const uint8_t *p) { return ld16(p) | (ld16(p + 2) << 16); }
 __device__ __forceinline__ float ldh(const uint8_t *p) { return __half2float(__ushort_as_half((unsigned short)ld16(p))); }
-__device__ __forceinline__ float ldf(const uint8_t *p) { return __uint_as_float(ld32(p)); }
-__device__ __forceinline__ int ldi8(const uint8_t *p) { return (int)(int8_t)*p; }
-__device__ __forceinline__ int ldi16(const uint8_t *p) { return (int)(int16_t)ld16(p); }
 
 // 6-bit (scale, min) pair j of the 12 packed bytes of a Q4_K / Q5_K block (utils.rs:53-63)
 __device__ __forceinline__ void scale_min_k4(int j, const uint8_t *q, int &sc, int &mn) {
@@ -151,107 +144,322 @@ __global__ void __launch_bounds__(TPB) quantize_q8_1_kernel(const XT *x, int64_t
   *reinterpret_cast<uint16_t *>(b + 2) = __half_as_ushort(sh);
 }
 
-// ---- dots: one weight block against the matching activation block(s), exactly the reference's arithmetic -------------
-// 32-element formats: a = the activation block (Q8_0 {f16 d; i8 qs[32]} or Q8_1 {f16 d; f16 s; i8 qs[32]})
-__device__ __forceinline__ float dot_q4_1(const uint8_t *w, const uint8_t *a) { // k_quants.rs:328-339
-  int sumi = 0;
+// ---- matmul -----------------------------------------------------------------------------------------------------------
+// A lane takes one 32-element piece of a weight row (a block of the 32-element formats, an eighth of a super-block), turns it
+// into eight words of int8 codes in registers, and multiplies it with up to MT activation rows by dp4a: a weight is loaded and
+// unpacked once for all of a tile's rows, an activation piece is loaded (L1) once for the warp's R weight rows.
+//   codes   element 4 i + b of the piece in byte b of c[i], offsets (-16, -4) already applied
+//   s0, s1  integer scales of the piece's first and second 16 elements (1 where the format has none); m0, m1 the integer mins
+//   d, m    the block's f16 scale and min / min scale
+struct Piece {
+  uint32_t c[8];
+  float d, m;
+  int s0, s1, m0, m1;
+};
+
+__device__ __forceinline__ uint32_t ldw(const uint8_t *p) { return __ldg(reinterpret_cast<const unsigned int *>(p)); }
+__device__ __forceinline__ uint4 ldw4(const uint8_t *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
+__device__ __forceinline__ float h_lo(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w & 0xffffu))); }
+__device__ __forceinline__ float h_hi(uint32_t w) { return __half2float(__ushort_as_half((unsigned short)(w >> 16))); }
+// bits 0..3 of b to bit 0 of bytes 0..3
+__device__ __forceinline__ uint32_t spread4(uint32_t b) { return ((b & 0xfu) * 0x00204081u) & 0x01010101u; }
+// bytewise x - off for bytes below 128
+__device__ __forceinline__ uint32_t sub_bytes(uint32_t x, uint32_t off) { return ((x | 0x80808080u) - off) ^ 0x80808080u; }
+
+// The words a piece is made of, as loaded (all loads of a piece are issued before any of its arithmetic). Blocks of 22 and 110
+// bytes are only 2-byte aligned: the words that cover them are loaded aligned (each holds at least one of the block's bytes, so
+// none lies outside the allocation, whose size is a multiple of 256) and shifted into place.
+template <int DT>
+struct Raw;
+template <>
+struct Raw<XNQ_Q4_1> { // {f16 d; f16 m; u8 qs[16]}
+  uint32_t w[5];
+  __device__ __forceinline__ void load(const uint8_t *row, int j) {
 #pragma unroll
-  for (int j = 0; j < 16; j++) sumi += (w[4 + j] & 0x0F) * ldi8(a + 4 + j) + (w[4 + j] >> 4) * ldi8(a + 4 + j + 16);
-  return __fadd_rn(__fmul_rn(__fmul_rn((float)sumi, ldh(w)), ldh(a)), __fmul_rn(ldh(w + 2), ldh(a + 2)));
-}
-__device__ __forceinline__ float dot_q5_0(const uint8_t *w, const uint8_t *a) { // k_quants.rs:423-436
-  const uint32_t qh = ld32(w + 2);
-  int sumi = 0;
-#pragma unroll
-  for (int j = 0; j < 32; j++) sumi += (code_q5(qh, w + 6, j) - 16) * ldi8(a + 2 + j);
-  return __fmul_rn(__fmul_rn((float)sumi, ldh(w)), ldh(a));
-}
-__device__ __forceinline__ float dot_q5_1(const uint8_t *w, const uint8_t *a) { // k_quants.rs:529-541
-  const uint32_t qh = ld32(w + 4);
-  int sumi = 0;
-#pragma unroll
-  for (int j = 0; j < 32; j++) sumi += code_q5(qh, w + 8, j) * ldi8(a + 4 + j);
-  return __fadd_rn(__fmul_rn(__fmul_rn((float)sumi, ldh(w)), ldh(a)), __fmul_rn(ldh(w + 2), ldh(a + 2)));
-}
-// 256-element formats: a = BlockQ8K {f32 d; i8 qs[256]; i16 bsums[16]}
-__device__ __forceinline__ float dot_q2k(const uint8_t *w, const uint8_t *a) { // k_quants.rs:904-945
-  int summs = 0;
-#pragma unroll
-  for (int j = 0; j < 16; j++) summs += ldi16(a + 260 + 2 * j) * (w[j] >> 4);
-  const float ad = ldf(a), dall = __fmul_rn(ad, ldh(w + 80)), dmin = __fmul_rn(ad, ldh(w + 82));
-  int isum = 0;
-  for (int g = 0; g < 16; g++) { // group g: 16 elements; half = g / 8, shift pair = (g % 8) / 2, part = g % 2
-    const int half = g >> 3, sh = (g & 7) >> 1, part = g & 1;
-    const uint8_t *q2 = w + 16 + 32 * half + 16 * part;
-    const uint8_t *q8 = a + 4 + 128 * half + 32 * sh + 16 * part;
-    int isuml = 0;
-#pragma unroll
-    for (int l = 0; l < 16; l++) isuml += ldi8(q8 + l) * ((q2[l] >> (2 * sh)) & 3);
-    isum += (w[g] & 0xF) * isuml;
+    for (int i = 0; i < 5; i++) w[i] = ldw(row + (int64_t)j * 20 + 4 * i);
   }
-  return __fsub_rn(__fmul_rn(dall, (float)isum), __fmul_rn(dmin, (float)summs));
-}
-__device__ __forceinline__ float dot_q3k(const uint8_t *w, const uint8_t *a) { // k_quants.rs:1087-1176: eight f32 lanes per block, added here
-  int aux32[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int s = 0; s < 16; s++) {
-    const int scale = q3k_scale(w + 96, s) - 32;
+  __device__ __forceinline__ void unpack(int, Piece &p) const {
+    p.d = h_lo(w[0]), p.m = h_hi(w[0]);
 #pragma unroll
-    for (int e = 0; e < 16; e++) aux32[e & 7] += scale * (ldi8(a + 4 + 16 * s + e) * code_q3k(w, 16 * s + e));
+    for (int i = 0; i < 4; i++) p.c[i] = w[1 + i] & 0x0f0f0f0fu, p.c[4 + i] = (w[1 + i] >> 4) & 0x0f0f0f0fu;
   }
-  const float d = __fmul_rn(ldh(w + 108), ldf(a));
-  float t = 0.f;
+};
+template <>
+struct Raw<XNQ_Q5_0> { // {f16 d; u8 qh[4]; u8 qs[16]}, 22 bytes
+  uint32_t w[6];
+  int sh;
+  __device__ __forceinline__ void load(const uint8_t *row, int j) {
+    const uint8_t *b = row + (int64_t)j * 22;
+    const int off = (int)(reinterpret_cast<uintptr_t>(b) & 2);
+    sh = 8 * off;
 #pragma unroll
-  for (int l = 0; l < 8; l++) t = __fadd_rn(t, __fmul_rn(d, (float)aux32[l]));
-  return t;
-}
-__device__ __forceinline__ float dot_q5k(const uint8_t *w, const uint8_t *a) { // k_quants.rs:1540-1604
-  int aux32[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int sumi = 0;
-  for (int s = 0; s < 8; s++) {
-    int sc, mn;
-    scale_min_k4(s, w + 4, sc, mn);
-    sumi += (ldi16(a + 260 + 4 * s) + ldi16(a + 260 + 4 * s + 2)) * mn;
-#pragma unroll
-    for (int e = 0; e < 32; e++) aux32[e & 7] += sc * (ldi8(a + 4 + 32 * s + e) * code_q5k(w, 32 * s + e));
+    for (int i = 0; i < 6; i++) w[i] = ldw(b - off + 4 * i);
   }
-  const float ad = ldf(a), d = __fmul_rn(ldh(w), ad), dmin = __fmul_rn(ldh(w + 2), ad);
-  float t = 0.f;
+  __device__ __forceinline__ void unpack(int, Piece &p) const {
+    uint32_t v[6];
 #pragma unroll
-  for (int l = 0; l < 8; l++) t = __fadd_rn(t, __fmul_rn(d, (float)aux32[l]));
-  return __fsub_rn(t, __fmul_rn(dmin, (float)sumi));
+    for (int i = 0; i < 6; i++) v[i] = __funnelshift_r(w[i], i < 5 ? w[i + 1] : 0u, sh);
+    p.d = h_lo(v[0]), p.m = 0.f;
+    const uint32_t qh = __funnelshift_r(v[0], v[1], 16);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t q = __funnelshift_r(v[1 + i], v[2 + i], 16);
+      p.c[i] = sub_bytes((q & 0x0f0f0f0fu) | (spread4(qh >> (4 * i)) << 4), 0x10101010u);
+      p.c[4 + i] = sub_bytes(((q >> 4) & 0x0f0f0f0fu) | (spread4(qh >> (16 + 4 * i)) << 4), 0x10101010u);
+    }
+  }
+};
+template <>
+struct Raw<XNQ_Q5_1> { // {f16 d; f16 m; u8 qh[4]; u8 qs[16]}
+  uint32_t w[6];
+  __device__ __forceinline__ void load(const uint8_t *row, int j) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) w[i] = ldw(row + (int64_t)j * 24 + 4 * i);
+  }
+  __device__ __forceinline__ void unpack(int, Piece &p) const {
+    p.d = h_lo(w[0]), p.m = h_hi(w[0]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      p.c[i] = (w[2 + i] & 0x0f0f0f0fu) | (spread4(w[1] >> (4 * i)) << 4);
+      p.c[4 + i] = ((w[2 + i] >> 4) & 0x0f0f0f0fu) | (spread4(w[1] >> (16 + 4 * i)) << 4);
+    }
+  }
+};
+template <>
+struct Raw<XNQ_Q2K> { // {u8 scales[16]; u8 qs[64]; f16 d; f16 dmin}, 84 bytes; piece s: bit pair s % 4 of half s / 4
+  uint32_t q[8], sc, dm;
+  __device__ __forceinline__ void load(const uint8_t *row, int j) {
+    const uint8_t *b = row + (int64_t)(j >> 3) * 84;
+    const int s = j & 7;
+#pragma unroll
+    for (int i = 0; i < 8; i++) q[i] = ldw(b + 16 + 32 * (s >> 2) + 4 * i);
+    sc = ldw(b + 4 * (s >> 1));
+    dm = ldw(b + 80);
+  }
+  __device__ __forceinline__ void unpack(int s, Piece &p) const {
+    const uint32_t b2 = sc >> (16 * (s & 1));
+    p.d = h_lo(dm), p.m = h_hi(dm);
+    p.s0 = b2 & 15, p.m0 = (b2 >> 4) & 15, p.s1 = (b2 >> 8) & 15, p.m1 = (b2 >> 12) & 15;
+#pragma unroll
+    for (int i = 0; i < 8; i++) p.c[i] = (q[i] >> (2 * (s & 3))) & 0x03030303u;
+  }
+};
+template <>
+struct Raw<XNQ_Q3K> { // {u8 hmask[32]; u8 qs[64]; u8 scales[12]; f16 d}, 110 bytes
+  uint32_t hm[9], q[9], sc[4];
+  int sh;
+  __device__ __forceinline__ void load(const uint8_t *row, int j) {
+    const uint8_t *b = row + (int64_t)(j >> 3) * 110;
+    const int s = j & 7, off = (int)(reinterpret_cast<uintptr_t>(b) & 2);
+    sh = 8 * off;
+    b -= off;
+#pragma unroll
+    for (int i = 0; i < 9; i++) hm[i] = ldw(b + 4 * i), q[i] = ldw(b + 32 + 32 * (s >> 2) + 4 * i);
+#pragma unroll
+    for (int i = 0; i < 4; i++) sc[i] = ldw(b + 96 + 4 * i);
+  }
+  __device__ __forceinline__ void unpack(int s, Piece &p) const {
+    const uint32_t a0 = __funnelshift_r(sc[0], sc[1], sh), a1 = __funnelshift_r(sc[1], sc[2], sh), tmp = __funnelshift_r(sc[2], sc[3], sh);
+    p.d = h_lo(sc[3] >> sh), p.m = 0.f;
+    const int g = s >> 1; // the word of four scales (k_quants.rs:1122-1127), of which this piece takes two
+    const uint32_t w4 = ((((g & 1) ? a1 : a0) >> (4 * (g >> 1))) & 0x0f0f0f0fu) | (((tmp >> (2 * g)) & 0x03030303u) << 4);
+    const uint32_t b2 = w4 >> (16 * (s & 1));
+    p.s0 = (int)(b2 & 0xffu) - 32, p.s1 = (int)((b2 >> 8) & 0xffu) - 32;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const uint32_t lo = (__funnelshift_r(q[i], q[i + 1], sh) >> (2 * (s & 3))) & 0x03030303u;
+      const uint32_t hi = (__funnelshift_r(hm[i], hm[i + 1], sh) >> s) & 0x01010101u;
+      p.c[i] = sub_bytes(lo | (hi << 2), 0x04040404u);
+    }
+  }
+};
+template <>
+struct Raw<XNQ_Q5K> { // {f16 d; f16 dmin; u8 scales[12]; u8 qh[32]; u8 qs[128]}, 176 = 11 x 16 bytes
+  uint4 hdr, h[2], q[2];
+  __device__ __forceinline__ void load(const uint8_t *row, int j) {
+    const uint8_t *b = row + (int64_t)(j >> 3) * 176;
+    const int s = j & 7;
+    hdr = ldw4(b);
+    h[0] = ldw4(b + 16), h[1] = ldw4(b + 32);
+    q[0] = ldw4(b + 48 + 32 * (s >> 1)), q[1] = ldw4(b + 64 + 32 * (s >> 1));
+  }
+  __device__ __forceinline__ void unpack(int s, Piece &p) const {
+    const K4Scales ks = unpack_k4(hdr.y, hdr.z, hdr.w);
+    p.d = h_lo(hdr.x), p.m = h_hi(hdr.x);
+    p.s0 = (int)k4_byte(ks.sc_lo, ks.sc_hi, s), p.m0 = (int)k4_byte(ks.mn_lo, ks.mn_hi, s);
+    const uint32_t hw[8] = {h[0].x, h[0].y, h[0].z, h[0].w, h[1].x, h[1].y, h[1].z, h[1].w};
+    const uint32_t qw[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
+#pragma unroll
+    for (int i = 0; i < 8; i++) p.c[i] = ((qw[i] >> (4 * (s & 1))) & 0x0f0f0f0fu) | (((hw[i] >> s) & 0x01010101u) << 4);
+  }
+};
+
+// What one piece adds to the dot of a (weight row, activation row) pair: exact integer sums, scaled in f32 as the reference does
+// (k_quants.rs:328-339 Q4_1, 423-436 Q5_0, 529-541 Q5_1, 904-945 Q2_K, 1087-1176 Q3_K, 1540-1604 Q5_K). lo, hi: the row's 32 codes;
+// da: its block scale; b0, b1: the sums of its first and second 16 codes.
+template <int DT>
+__device__ __forceinline__ float piece_dot(const Piece &p, const uint4 &lo, const uint4 &hi, float da, int b0, int b1, float acc) {
+  int t0 = __dp4a((int)p.c[0], (int)lo.x, 0);
+  t0 = __dp4a((int)p.c[1], (int)lo.y, t0);
+  t0 = __dp4a((int)p.c[2], (int)lo.z, t0);
+  t0 = __dp4a((int)p.c[3], (int)lo.w, t0);
+  int t1 = __dp4a((int)p.c[4], (int)hi.x, (DT == XNQ_Q2K || DT == XNQ_Q3K) ? 0 : t0);
+  t1 = __dp4a((int)p.c[5], (int)hi.y, t1);
+  t1 = __dp4a((int)p.c[6], (int)hi.z, t1);
+  t1 = __dp4a((int)p.c[7], (int)hi.w, t1);
+  if (DT == XNQ_Q4_1 || DT == XNQ_Q5_1) { // the block's min times s = f16(f16(sum) * d), as BlockQ8_1 stores it (k_quants.rs:847-873)
+    const float s = __half2float(__float2half_rn(__fmul_rn(__half2float(__float2half_rn((float)(b0 + b1))), da)));
+    return acc + __fadd_rn(__fmul_rn(__fmul_rn((float)t1, p.d), da), __fmul_rn(p.m, s));
+  }
+  if (DT == XNQ_Q5_0) return acc + __fmul_rn(__fmul_rn((float)t1, p.d), da);
+  if (DT == XNQ_Q2K) return acc + __fsub_rn(__fmul_rn(__fmul_rn(da, p.d), (float)(p.s0 * t0 + p.s1 * t1)), __fmul_rn(__fmul_rn(da, p.m), (float)(p.m0 * b0 + p.m1 * b1)));
+  if (DT == XNQ_Q3K) return acc + __fmul_rn(__fmul_rn(p.d, da), (float)(p.s0 * t0 + p.s1 * t1));
+  return acc + __fsub_rn(__fmul_rn(__fmul_rn(p.d, da), (float)(p.s0 * t1)), __fmul_rn(__fmul_rn(p.m, da), (float)(p.m0 * (b0 + b1))));
 }
 
-// One warp per weight row; lane l takes blocks l, l + 32, ...; activation rows in turn.
-template <int DT>
-__global__ void __launch_bounds__(TPB) generic_matmul_kernel(const uint8_t *w, const uint8_t *act, int64_t n, int64_t m, int nblk, int wts, int ats, void *y,
-                                                             int y_dtype, int64_t ldy) {
-  const int64_t row = blockIdx.x * (int64_t)(TPB / 32) + (threadIdx.x >> 5);
-  if (row >= n) return;
-  const int lane = threadIdx.x & 31;
-  const uint8_t *wr = w + row * (int64_t)nblk * wts;
-  for (int64_t r = 0; r < m; r++) {
-    const uint8_t *ar = act + r * (int64_t)nblk * ats;
-    float sum = 0.f;
-    for (int b = lane; b < nblk; b += 32) {
-      const uint8_t *wb = wr + (int64_t)b * wts, *ab = ar + (int64_t)b * ats;
-      float v;
-      if (DT == XNQ_Q4_1) v = dot_q4_1(wb, ab);
-      else if (DT == XNQ_Q5_0) v = dot_q5_0(wb, ab);
-      else if (DT == XNQ_Q5_1) v = dot_q5_1(wb, ab);
-      else if (DT == XNQ_Q2K) v = dot_q2k(wb, ab);
-      else if (DT == XNQ_Q3K) v = dot_q3k(wb, ab);
-      else v = dot_q5k(wb, ab);
-      sum += v;
+// What bounds it: at a few rows the loads a warp keeps in flight against DRAM latency, at many the dp4a rate. A warp owns GR
+// weight rows and every (32 KS)-th group of pieces; KS warps share the rows of a longer k (their sums meet in shared memory), so
+// that a few thousand rows give every SM enough warps. The order of the sum over k depends on k alone: a row's result is the
+// same bits in a batch, alone or in a shard. The weights of the first pieces are requested before the wait for the kernel that
+// quantizes the activations. Measured, Q5_K 4096 x 4096, 7 rows: 381 us a call with one lane per super-block reading single bytes (each
+// code extracted and multiplied by itself, one activation row after the other), 21 us like this, most of it the host's share of the call.
+constexpr int GR = 2;
+__host__ __device__ constexpr int k_splits(int pieces) { return pieces < 64 ? 1 : (pieces < 128 ? 2 : 4); }
+
+template <int DT, int MT>
+__global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *__restrict__ w, ActView act, int64_t n, int64_t row_bytes, void *y, int y_dtype,
+                                                             int64_t ldy) {
+  constexpr int NV = GR * MT;
+  constexpr bool K256 = DT == XNQ_Q2K || DT == XNQ_Q3K || DT == XNQ_Q5K;
+  __shared__ float red[TPB / 32][NV];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int pieces = (int)(act.k / 32), ks_n = k_splits(pieces);
+  const int ks = warp & (ks_n - 1), grp = warp / ks_n;
+  const int64_t row0 = ((int64_t)blockIdx.x * (TPB / 32 / ks_n) + grp) * GR;
+  const int64_t m0 = (int64_t)blockIdx.y * MT;
+  const int rows = (int)min((int64_t)MT, act.m - m0);
+  const int s = lane & 7;
+  const uint8_t *wr[GR];
+#pragma unroll
+  for (int r = 0; r < GR; r++) wr[r] = w + min(row0 + r, n - 1) * row_bytes; // past the last row: a duplicate, never stored
+  Raw<DT> raw[GR];
+  int j = ks * 32 + lane;
+  if (j < pieces) {
+#pragma unroll
+    for (int r = 0; r < GR; r++) raw[r].load(wr[r], j);
+  }
+  pdl_wait();
+  const int nblk_a = K256 ? pieces >> 3 : pieces;
+  const int8_t *aq = act.q + m0 * act.k;
+  const float *ad = act.d + m0 * nblk_a;
+  const int16_t *ab = act.bsum + m0 * (act.k / 16);
+  float acc[NV];
+#pragma unroll
+  for (int i = 0; i < NV; i++) acc[i] = 0.f;
+  while (j < pieces) {
+    Piece p[GR];
+#pragma unroll
+    for (int r = 0; r < GR; r++) raw[r].unpack(s, p[r]);
+    const int jn = j + 32 * ks_n;
+    if (MT < 16 && jn < pieces) { // the next pieces are on their way while these are multiplied (16 rows: no registers left for them)
+#pragma unroll
+      for (int r = 0; r < GR; r++) raw[r].load(wr[r], jn);
     }
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    if (lane == 0) {
-      const int64_t idx = r * ldy + row;
-      if (y_dtype == XNQ_F32) static_cast<float *>(y)[idx] = sum;
-      else if (y_dtype == XNQ_F16) static_cast<__half *>(y)[idx] = __float2half_rn(sum);
-      else static_cast<__nv_bfloat16 *>(y)[idx] = __float2bfloat16_rn(sum);
+    for (int i = 0; i < MT; i++) {
+      if (i < rows) {
+        const uint4 *a = reinterpret_cast<const uint4 *>(aq + (int64_t)i * act.k + (int64_t)j * 32);
+        const uint4 lo = a[0], hi = a[1];
+        const float da = ad[(int64_t)i * nblk_a + (K256 ? j >> 3 : j)];
+        int b0 = 0, b1 = 0;
+        if (DT != XNQ_Q5_0 && DT != XNQ_Q3K) {
+          const uint32_t b = *reinterpret_cast<const uint32_t *>(ab + (int64_t)i * (act.k / 16) + 2 * (int64_t)j);
+          b0 = (int)(int16_t)(b & 0xffffu), b1 = (int)(int16_t)(b >> 16);
+        }
+#pragma unroll
+        for (int r = 0; r < GR; r++) acc[i * GR + r] = piece_dot<DT>(p[r], lo, hi, da, b0, b1, acc[i * GR + r]);
+      }
     }
+    if (MT >= 16 && jn < pieces) {
+#pragma unroll
+      for (int r = 0; r < GR; r++) raw[r].load(wr[r], jn);
+    }
+    j = jn;
   }
+  // sums over the lanes: as long as a thread holds more than one value, each step hands half of them to the partner lane, so NV
+  // values cost NV - 1 exchanges and end up in different lanes (value v in the lanes whose upper bits are v); the additions are
+  // those of the plain xor tree
+  int nv = NV, off = 16;
+#pragma unroll
+  for (int step = 0; step < 5; step++) {
+    if (nv > 1) {
+      nv >>= 1;
+#pragma unroll
+      for (int v = 0; v < NV / 2; v++) {
+        if (v < nv) {
+          const bool up = (lane & off) != 0;
+          const float keep = up ? acc[v + nv] : acc[v], give = up ? acc[v] : acc[v + nv];
+          acc[v] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+      }
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+    }
+    off >>= 1;
+  }
+  constexpr int PER = 32 / NV; // lanes that hold the same value
+  const int v = lane / PER;
+  if (ks_n > 1) {
+    if (lane % PER == 0) red[warp][v] = acc[0];
+    __syncthreads();
+    if (ks > 0) return;
+    for (int i = 1; i < ks_n; i++) acc[0] += red[warp + i][v];
+  }
+  const int i = v / GR;
+  const int64_t row = row0 + v % GR;
+  if (lane % PER == 0 && i < rows && row < n) {
+    const int64_t idx = (m0 + i) * ldy + row;
+    if (y_dtype == XNQ_F32) static_cast<float *>(y)[idx] = acc[0];
+    else if (y_dtype == XNQ_F16) static_cast<__half *>(y)[idx] = __float2half_rn(acc[0]);
+    else static_cast<__nv_bfloat16 *>(y)[idx] = __float2bfloat16_rn(acc[0]);
+  }
+}
+
+template <int DT>
+int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes, void *y, int y_dtype, int64_t ldy, cudaStream_t s) {
+  const int rows_per_cta = TPB / 32 / k_splits((int)(w.k / 32)) * GR;
+  const int mt = act.m >= 9 ? 16 : (act.m >= 5 ? 8 : (act.m >= 3 ? 4 : (int)act.m));
+  // grid.y is limited to 65535 tiles of activation rows
+  const int64_t pass = (int64_t)mt * 65535, nblk_a = w.k / (act.act_dtype == XNQ_Q8_0 ? QK : QK_K);
+  const size_t yes = type_size(y_dtype);
+  for (int64_t r0 = 0; r0 < act.m; r0 += pass) {
+    ActView a = act;
+    a.m = act.m - r0 < pass ? act.m - r0 : pass;
+    a.q += r0 * w.k, a.d += r0 * nblk_a, a.bsum += r0 * (w.k / 16);
+    void *yp = static_cast<char *>(y) + (size_t)r0 * ldy * yes;
+    const dim3 grid((unsigned)((w.n + rows_per_cta - 1) / rows_per_cta), (unsigned)((a.m + mt - 1) / mt));
+    cudaError_t e;
+    switch (mt) {
+      case 1: e = launch_pdl(generic_matmul_kernel<DT, 1>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
+      case 2: e = launch_pdl(generic_matmul_kernel<DT, 2>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
+      case 4: e = launch_pdl(generic_matmul_kernel<DT, 4>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
+      case 8: e = launch_pdl(generic_matmul_kernel<DT, 8>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
+      default: e = launch_pdl(generic_matmul_kernel<DT, 16>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
+    }
+    XNQ_CUDA(e);
+    count_launch();
+  }
+  return XNQ_OK;
+}
+template <int DT>
+int init_matmul_dt() { // kernels are loaded before any stream capture
+  cudaFuncAttributes fa;
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 1>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 2>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 4>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 8>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 16>));
+  return XNQ_OK;
 }
 
 inline unsigned grid_for(int64_t work, int per) { return (unsigned)((work + per - 1) / per); }
@@ -291,36 +499,32 @@ int launch_quantize_q8_1(const void *x, int x_dtype, int64_t m, int64_t k, int64
   return XNQ_OK;
 }
 
-size_t generic_workspace_bytes(const WeightView &w, int64_t m) {
-  const int adt = act_dtype_for(w.dtype);
-  return ((size_t)m * (size_t)(w.k / block_size(adt)) * (size_t)type_size(adt) + 255) & ~(size_t)255;
-}
+// The activations' planar image: codes, block scales, 16-sums. Q8_1 blocks have the codes and the (f16-rounded) scale of Q8_0
+// blocks; the sum they also store follows from the 16-sums.
+static int generic_act_dtype(const WeightView &w) { return act_dtype_for(w.dtype) == XNQ_Q8K ? XNQ_Q8K : XNQ_Q8_0; }
+size_t generic_workspace_bytes(const WeightView &w, int64_t m) { return act_workspace_bytes(m, w.k, generic_act_dtype(w)); }
 
 // y[m, n] = x[m, k] . W^T for a weight held as canonical blocks; workspace: generic_workspace_bytes(w, m)
 int launch_generic_matmul(const WeightView &w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
                           cudaStream_t s) {
-  const int adt = act_dtype_for(w.dtype);
   // the reference's dots of the 32-element formats refuse an odd number of blocks (k_quants.rs:322-325, 413-415, 523-526)
   if (block_size(w.dtype) == 32 && (w.k / 32) % 2) return fail(XNQ_ERR_SHAPE, "matmul_t: k = %lld is not divisible by 64 (an even number of 32-value blocks)", (long long)w.k);
-  int rc = adt == XNQ_Q8_1 ? launch_quantize_q8_1(x, x_dtype, m, w.k, ldx, workspace, s) : launch_quantize_act_blocks(adt, x, x_dtype, m, w.k, ldx, workspace, s);
+  const ActView act = act_view(workspace, m, w.k, generic_act_dtype(w));
+  int rc = launch_quantize_act_planar(act, x, x_dtype, ldx, s);
   if (rc != XNQ_OK) return rc;
-  const int nblk = (int)(w.k / block_size(w.dtype)), wts = type_size(w.dtype), ats = type_size(adt);
-  const unsigned g = grid_for(w.n, TPB / 32);
-  const uint8_t *act = static_cast<const uint8_t *>(workspace);
+  const int64_t row_bytes = w.k / block_size(w.dtype) * type_size(w.dtype);
   profile_mark(s, true);
   switch (w.dtype) {
-    case XNQ_Q4_1: generic_matmul_kernel<XNQ_Q4_1><<<g, TPB, 0, s>>>(w.qs, act, w.n, m, nblk, wts, ats, y, y_dtype, ldy); break;
-    case XNQ_Q5_0: generic_matmul_kernel<XNQ_Q5_0><<<g, TPB, 0, s>>>(w.qs, act, w.n, m, nblk, wts, ats, y, y_dtype, ldy); break;
-    case XNQ_Q5_1: generic_matmul_kernel<XNQ_Q5_1><<<g, TPB, 0, s>>>(w.qs, act, w.n, m, nblk, wts, ats, y, y_dtype, ldy); break;
-    case XNQ_Q2K: generic_matmul_kernel<XNQ_Q2K><<<g, TPB, 0, s>>>(w.qs, act, w.n, m, nblk, wts, ats, y, y_dtype, ldy); break;
-    case XNQ_Q3K: generic_matmul_kernel<XNQ_Q3K><<<g, TPB, 0, s>>>(w.qs, act, w.n, m, nblk, wts, ats, y, y_dtype, ldy); break;
-    case XNQ_Q5K: generic_matmul_kernel<XNQ_Q5K><<<g, TPB, 0, s>>>(w.qs, act, w.n, m, nblk, wts, ats, y, y_dtype, ldy); break;
-    default: return fail(XNQ_ERR_DTYPE, "matmul_t: dtype %d", w.dtype);
+    case XNQ_Q4_1: rc = launch_matmul_dt<XNQ_Q4_1>(w, act, row_bytes, y, y_dtype, ldy, s); break;
+    case XNQ_Q5_0: rc = launch_matmul_dt<XNQ_Q5_0>(w, act, row_bytes, y, y_dtype, ldy, s); break;
+    case XNQ_Q5_1: rc = launch_matmul_dt<XNQ_Q5_1>(w, act, row_bytes, y, y_dtype, ldy, s); break;
+    case XNQ_Q2K: rc = launch_matmul_dt<XNQ_Q2K>(w, act, row_bytes, y, y_dtype, ldy, s); break;
+    case XNQ_Q3K: rc = launch_matmul_dt<XNQ_Q3K>(w, act, row_bytes, y, y_dtype, ldy, s); break;
+    case XNQ_Q5K: rc = launch_matmul_dt<XNQ_Q5K>(w, act, row_bytes, y, y_dtype, ldy, s); break;
+    default: rc = fail(XNQ_ERR_DTYPE, "matmul_t: dtype %d", w.dtype);
   }
   profile_mark(s, false);
-  XNQ_CUDA(cudaGetLastError());
-  count_launch();
-  return XNQ_OK;
+  return rc;
 }
 
 int generic_init(int) { // kernels are loaded before any stream capture
@@ -331,13 +535,13 @@ int generic_init(int) { // kernels are loaded before any stream capture
   XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_q8_1_kernel<float>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_q8_1_kernel<__half>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_q8_1_kernel<__nv_bfloat16>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<XNQ_Q4_1>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<XNQ_Q5_0>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<XNQ_Q5_1>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<XNQ_Q2K>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<XNQ_Q3K>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<XNQ_Q5K>));
-  return XNQ_OK;
+  int rc;
+  if ((rc = init_matmul_dt<XNQ_Q4_1>()) != XNQ_OK) return rc;
+  if ((rc = init_matmul_dt<XNQ_Q5_0>()) != XNQ_OK) return rc;
+  if ((rc = init_matmul_dt<XNQ_Q5_1>()) != XNQ_OK) return rc;
+  if ((rc = init_matmul_dt<XNQ_Q2K>()) != XNQ_OK) return rc;
+  if ((rc = init_matmul_dt<XNQ_Q3K>()) != XNQ_OK) return rc;
+  return init_matmul_dt<XNQ_Q5K>();
 }
 
 } // namespace xnq

@@ -41,6 +41,8 @@ constexpr int TPB = 256;
 template <int ACT, typename XT, int LAYOUT>
 __global__ void __launch_bounds__(TPB) quantize_act_kernel(const XT *__restrict__ x, int64_t m, int64_t k, int64_t ldx,
                                                            uint8_t *__restrict__ blocks, ActView pl) {
+  pdl_launch_dependents(); // the matmul that reads the image may set itself up and request its first weights now
+  pdl_wait();              // x may be the previous kernel's output; the image may still be read by the previous call
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t per_row = k / 8;
   const bool valid = t < m * per_row;
@@ -89,14 +91,11 @@ int launch_typed(const void *x, int x_dtype, int64_t m, int64_t k, int64_t ldx, 
   if (threads == 0) return XNQ_OK;
   const unsigned grid = (unsigned)((threads + TPB - 1) / TPB);
   switch (x_dtype) {
-    case XNQ_F32: quantize_act_kernel<ACT, float, LAYOUT><<<grid, TPB, 0, s>>>(static_cast<const float *>(x), m, k, ldx, blocks, pl); break;
-    case XNQ_F16: quantize_act_kernel<ACT, __half, LAYOUT><<<grid, TPB, 0, s>>>(static_cast<const __half *>(x), m, k, ldx, blocks, pl); break;
-    case XNQ_BF16:
-      quantize_act_kernel<ACT, __nv_bfloat16, LAYOUT><<<grid, TPB, 0, s>>>(static_cast<const __nv_bfloat16 *>(x), m, k, ldx, blocks, pl);
-      break;
+    case XNQ_F32: XNQ_CUDA(launch_pdl(quantize_act_kernel<ACT, float, LAYOUT>, dim3(grid), dim3(TPB), 0, s, static_cast<const float *>(x), m, k, ldx, blocks, pl)); break;
+    case XNQ_F16: XNQ_CUDA(launch_pdl(quantize_act_kernel<ACT, __half, LAYOUT>, dim3(grid), dim3(TPB), 0, s, static_cast<const __half *>(x), m, k, ldx, blocks, pl)); break;
+    case XNQ_BF16: XNQ_CUDA(launch_pdl(quantize_act_kernel<ACT, __nv_bfloat16, LAYOUT>, dim3(grid), dim3(TPB), 0, s, static_cast<const __nv_bfloat16 *>(x), m, k, ldx, blocks, pl)); break;
     default: return fail(XNQ_ERR_DTYPE, "quantize_act: activation dtype %d is not f32/f16/bf16", x_dtype);
   }
-  XNQ_CUDA(cudaGetLastError());
   count_launch();
   return XNQ_OK;
 }
