@@ -3,8 +3,8 @@
 //
 //   D[128 weight rows, mt activation rows] += A[128, 64] . B[mt, 64]^T      per k-step of 64
 //
-//   A  weights of the tile, dequantized by four producer warps (one thread per weight row) from the
-//      quantized blocks straight into the 128-byte-swizzled K-major shared-memory image the MMA reads.
+//   A  weights of the tile, dequantized by sixteen producer warps from the quantized blocks straight into
+//      the 128-byte-swizzled K-major shared-memory image the MMA reads.
 //      Every weight is dequantized once per m-tile (mt up to 256 rows).
 //   B  activations, prepared once per call by prefill_prepare_acts: quantized to Q8_0 / Q8_K exactly
 //      as the reference's quantize_lhs does (k_quants.rs:2015-2026), dequantized, scaled by a power of
@@ -22,9 +22,9 @@
 //
 // k order. A dot product does not care in which order k is visited as long as both operands agree,
 // so within a k-step the 64 elements are stored in the order the nibble unpack produces them
-// (xnq_prefill.cuh: kperm) and the activation image uses the same order; no shuffles are needed.
+// (xnq_prefill_rows.cuh) and the activation image uses the same order; no shuffles are needed.
 //
-// Synchronisation. Per stage: a_full (128 producer arrivals), b_full (bulk-copy transaction bytes),
+// Synchronisation. Per stage: a_full (one arrival per producer warp of the stage), b_full (bulk-copy transaction bytes),
 // empty (tcgen05.commit by the MMA thread). Every wait is bounded; on expiry a status bit is set and
 // every role falls through to the common exit, where tensor memory is released.
 #include <algorithm>
@@ -44,22 +44,16 @@ namespace {
 constexpr int BK = 64;             // k-step (elements) = one 128-byte swizzle row of fp16
 constexpr int TILE_N = 128;        // weight rows per CTA = UMMA M
 constexpr int MAX_MT = 256;        // activation rows per CTA = UMMA N
-constexpr int GROUP = 256;         // one producer group: two threads per weight row
-constexpr int PRODUCERS = 2 * GROUP; // two groups take alternate k-steps, so a warp's per-k-step latency chain is halved
-constexpr int LOADER_WARP = PRODUCERS / 32, MMA_WARP = LOADER_WARP + 1;
-constexpr int NTHREADS = PRODUCERS + 64; // warps 0-15 producers/epilogue, then the loader warp and the MMA warp
-constexpr uint32_t WAIT_LIMIT = 1u << 26; // non-blocking polls (a few ns each): about a second
+constexpr int PRODUCER_WARPS = 16; // four row groups of 32 rows x four warps
+constexpr int LOADER_WARP = PRODUCER_WARPS, MMA_WARP = LOADER_WARP + 1;
+constexpr int NTHREADS = PRODUCER_WARPS * 32 + 64; // warps 0-15 producers, then the loader warp and the MMA warp
+constexpr uint32_t WAIT_LIMIT = 1u << 26; // polls of a flag in global memory
 constexpr int A_STAGE_BYTES = TILE_N * BK * 2; // 16 KB
-#ifndef XNQ_PF_NSTAGES
-#define XNQ_PF_NSTAGES 4
-#endif
-#ifndef XNQ_PF_RAW_DEPTH
-#define XNQ_PF_RAW_DEPTH 2
-#endif
-constexpr int NSTAGES = XNQ_PF_NSTAGES; // even: each producer group owns every other A stage
-        // A stages (16 KB each)
-constexpr int RAW_DEPTH = XNQ_PF_RAW_DEPTH; // own k-steps (every other one) of raw weight bytes a producer thread keeps in flight
-constexpr int RAW_SLOT_MAX = 80;   // largest per-thread slot (Q6_K)
+// A stages. At least as many as a super-step has k-steps: step i then waits for the MMAs of a step of an EARLIER super-step, whose
+// producer (same row group) has already waited for the phase before; with fewer, a warp could test a barrier that is two phases
+// behind, which reads as complete.
+constexpr int MIN_STAGES = 4, MAX_STAGES = 8;
+constexpr int MAX_RAW_SLOTS = 6;   // super-steps of raw weight bytes in shared memory
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -82,21 +76,51 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned int bit) {
-  for (uint32_t i = 0; i < WAIT_LIMIT; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  atomicOr(&g_prefill_status, bit);
-  return false;
+// One wait attempt during which the hardware may keep the thread suspended for up to `ns` nanoseconds (it takes no issue slots).
+__device__ __forceinline__ bool mbar_suspend(uint32_t bar, uint32_t parity, uint32_t ns) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(ns)
+      : "memory");
+  return ok != 0;
 }
-// for waits that are long by design (a drain warp waiting out a whole main loop): poll at a low rate so the
-// poller does not take issue slots from the producer warps of its scheduler
-__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, unsigned int bit) {
-  for (uint32_t i = 0; i < (WAIT_LIMIT >> 4); ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    __nanosleep(200);
+__device__ __forceinline__ unsigned long long wall_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull; // a wait that lasts two seconds is given up
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned int bit) {
+  unsigned long long t0 = 0;
+  for (unsigned int attempt = 1;; attempt++) { // the wall clock is read on every 16th failed attempt only
+    if (mbar_suspend(bar, parity, 1000000u)) return true;
+    if ((attempt & 15u) == 0) {
+      const unsigned long long now = wall_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > WAIT_LIMIT_NS) break;
+    }
   }
   atomicOr(&g_prefill_status, bit);
   return false;
+}
+// by a whole warp that stays converged; the result is the same in all lanes
+__device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity, unsigned int bit) {
+  const bool ok = mbar_wait(bar, parity, bit);
+  return __all_sync(0xffffffffu, ok);
+}
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e != 0;
 }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
@@ -160,9 +184,10 @@ struct PrefillArgs {
   int64_t m, m_pad;
   int ksteps;
   int nstages;            // A (weight) stages
-  int b_stages;           // B (activation) stages: deeper, the bulk copy's L2 latency has to be covered
+  int b_stages;           // B (activation) stages
+  int raw_slots;          // raw super-steps in shared memory, the one being converted included
   uint32_t b_stride;      // bytes between B stages (largest mt of the grid x 128, multiple of 1024)
-  uint32_t b_off, raw_off; // offsets of the B ring and of the producers' raw rings from the aligned base
+  uint32_t b_off, raw_off; // offsets of the B ring and of the raw ring from the aligned base
   float wscale;           // power of two applied to every dequantized weight
   // persistent kernel: tile t = tile_n * tiles_m + tile_m; work unit u = t * ksteps + kt; CTA c takes units
   // [units * c / G, units * (c + 1) / G), or whole tiles when the output cannot be accumulated atomically
@@ -172,14 +197,21 @@ struct PrefillArgs {
   unsigned int *tile_cnt; // [tiles] arrival tickets then [tiles] "first partial stored" flags; zeroed by the prepare kernel
 };
 
-// Dequantize the 64 weights of k-step `kt` of row `row` and store them as 8 swizzled 16-byte chunks.
-// All arithmetic is fp16 on exactly representable integers times an fp16 scale.
 using namespace prefill_rows;
 
-__device__ __forceinline__ void zero_half_row(uint32_t dst_row, int hf) { // chunks 4hf..4hf+3, whatever the swizzle
-  const int sw = (dst_row >> 7) & 7;
-#pragma unroll
-  for (int c = 0; c < 4; c++) sts128(dst_row + (((hf * 4 + c) ^ sw) << 4), 0, 0, 0, 0);
+// waits until at most `pending` of this thread's committed copy groups are still in flight
+__device__ __forceinline__ void cp_async_wait(int pending) {
+  switch (pending) {
+    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+    default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+  }
+}
+
+__device__ __forceinline__ void zero_row(uint32_t dst_row, int sw, int c0, int n) { // chunks c0 .. c0 + n - 1
+  for (int c = c0; c < c0 + n; c++) sts128(dst_row + ((c ^ sw) << 4), 0, 0, 0, 0);
 }
 
 // Writes one 32-column chunk of an accumulator row block: column j of the chunk is activation row
@@ -214,9 +246,13 @@ __device__ __forceinline__ void drain_chunk(const uint32_t (&v)[32], float ru_la
 // theirs atomically after seeing the flag (two to three parts per split tile; f32 output only - other
 // output types get whole tiles). The accumulator is double-buffered in tensor memory (2 x 256 columns)
 // and drained by four dedicated warps, so the drain of one segment overlaps the MMAs of the next.
-// Roles: 16 producer warps in two groups that take alternate k-steps (two threads per weight row, each with a
-// private cp.async ring of raw bytes), one activation-loader warp (one bulk copy per stage), one MMA-issuing
-// warp, eight drain warps. Stage counters run on across segments.
+// Roles: 16 producer warps, one activation-loader warp (one bulk copy per stage), one MMA-issuing warp, eight drain
+// warps. Stage counters run on across segments.
+// Producers: the four warps of a row group (32 weight rows) fetch the group's bytes of a super-step together, several
+// super-steps ahead, and each then converts its own k-step of it (or its half of one), so the k-steps of a super-step are
+// converted side by side and a warp's chain of waits, loads, arithmetic and stores has a super-step's MMAs to run in. One
+// barrier of the row group's four warps per super-step makes the copies visible to all of them and tells that the slot of
+// the previous super-step has been read.
 constexpr int EPI_WARPS = 8; // two per accumulator lane quarter, splitting the columns
 constexpr int EPI_WARP0 = MMA_WARP + 1;
 constexpr int NTHREADS_SK = NTHREADS + EPI_WARPS * 32;
@@ -240,14 +276,14 @@ template <typename RowT>
 __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(PrefillArgs p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  __shared__ __align__(8) uint64_t bars[4 * 8 + 4]; // a_full, a_empty, b_full, b_empty (8 each), acc_full[2], acc_empty[2]
+  __shared__ __align__(8) uint64_t bars[4 * MAX_STAGES + 4]; // a_full, a_empty, b_full, b_empty (8 each), acc_full[2], acc_empty[2]
   __shared__ uint32_t tmem_slot;
   __shared__ unsigned int s_ticket;
   const int S = p.nstages;
   const int SB = p.b_stages;
   const uint32_t a_full = smem_u32(bars), a_empty = a_full + 64, b_full = a_full + 128, b_empty = a_full + 192, acc_full = a_full + 256,
                  acc_empty = a_full + 272;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // so that the compiler knows `warp` to be uniform
   const uint32_t a_ring = smem_base, b_ring = smem_base + p.b_off;
   const int KT = p.ksteps;
 
@@ -267,7 +303,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
-      mbar_init(a_full + 8 * s, GROUP / 32);
+      mbar_init(a_full + 8 * s, PRODUCER_WARPS / RowT::KPS);
       mbar_init(a_empty + 8 * s, 1);
     }
     for (int s = 0; s < SB; s++) {
@@ -287,124 +323,161 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_d = tmem_slot;
+  pdl_launch_dependents();
+  const uint32_t tmem_d = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
-  if (warp < PRODUCERS / 32) {
-    // ---- producers: group g takes this CTA's steps g, g+2, ... -------------------------------------------
-    const int grp = threadIdx.x / GROUP, tg = threadIdx.x % GROUP;
-    const int r = tg & (TILE_N - 1), hf = tg >> 7;
-    const int sw = r & 7;
-    const uint32_t raw_base = smem_base + p.raw_off;
-    Cursor cur = start, pre = start;
-    cur.advance(grp, KT, TM);
-    pre.advance(grp, KT, TM);
+  if (warp < PRODUCER_WARPS) {
+    // ---- producers (nothing here waits for the kernel that prepares the activations: weights are immutable) ----
+    constexpr int KPS = RowT::KPS, NCOPY = (32 * RowT::ITEMS + 127) / 128;
+    const int rg = warp & 3, kg = warp >> 2;
+    const int kk = kg % KPS, hf = kg / KPS; // this warp's k-step of a super-step; which half of it (KPS = 2)
+    const int r = 32 * rg + lane, sw = r & 7;
+    const int t = kg * 32 + lane; // 0..127 in the row group
+    const uint32_t raw = smem_base + p.raw_off + (uint32_t)(rg * 32 * RowT::ROWB);
+    constexpr uint32_t SLOT = TILE_N * RowT::ROWB;
+    const int SPT = (KT + KPS - 1) / KPS; // super-steps per tile
+    const int R = p.raw_slots;
+    // position of the copies in the super-step space
+    int l_n = start.tile_n, l_m = start.tile_m, l_s = start.kt / KPS, l_slot = 0;
+    const int last_kt = nsteps - 1 + start.kt; // counted from the start of the first tile
+    int l_left = nsteps > 0 ? (last_kt / KT) * SPT + (last_kt % KT) / KPS - l_s + 1 : 0; // super-steps still to be copied
+    int left = l_left;
+    Item it[NCOPY]; // this thread's copies; their addresses change with the tile only
+    auto bind = [&]() {
 #pragma unroll
-    for (int j = 0; j < RAW_DEPTH; j++) {
-      if (grp + 2 * j < nsteps) {
-        const int64_t row = (int64_t)pre.tile_n * TILE_N + r;
-        RowT::issue(p.w, row < p.w.n ? row : p.w.n - 1, pre.kt, hf, raw_base + (j * PRODUCERS + threadIdx.x) * RowT::SLOT);
-        pre.advance(2, KT, TM);
+      for (int i = 0; i < NCOPY; i++) {
+        const int item = min(i * 128 + t, 32 * RowT::ITEMS - 1);
+        it[i] = RowT::item(p.w, min((int64_t)l_n * TILE_N + 32 * rg + item / RowT::ITEMS, p.w.n - 1), item % RowT::ITEMS);
+      }
+    };
+    bind();
+    auto issue = [&]() {
+      if (l_left > 0) {
+        l_left--;
+        const uint32_t dst = raw + (uint32_t)l_slot * SLOT;
+#pragma unroll
+        for (int i = 0; i < NCOPY; i++) {
+          const int item = i * 128 + t;
+          if ((32 * RowT::ITEMS) % 128 == 0 || item < 32 * RowT::ITEMS) {
+            const uint32_t off = ((uint32_t)l_s * it[i].mul) & ~15u;
+            cp_async16(dst + (uint32_t)((item / RowT::ITEMS) * RowT::ROWB + (item % RowT::ITEMS) * 16), it[i].p + (off < it[i].lim ? off : 0u), off < it[i].lim ? 16u : 0u);
+          }
+        }
+        if (++l_slot == R) l_slot = 0;
+        if (++l_s == SPT) {
+          l_s = 0;
+          if (++l_m == TM) {
+            l_m = 0, l_n++;
+            bind();
+          }
+        }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    int rs = 0;
+    };
+    for (int j = 0; j < R - 1; j++) issue();
+    int c_n = start.tile_n, c_m = start.tile_m, c_s = start.kt / KPS, c_slot = 0;
+    int base_i = -start.kt; // the CTA's step number of the current tile's first k-step
+    int at = 0, s = 0;      // s = at % S, lap: parity of at / S, of the last step this warp looked at
+    uint32_t lap = 0;
     bool alive = true;
-    for (int i = grp; i < nsteps && alive; i += 2) {
-      const int s = i % S;
-      const uint32_t round = (uint32_t)(i / S);
-      const uint32_t slot = raw_base + (rs * PRODUCERS + threadIdx.x) * RowT::SLOT;
-      asm volatile("cp.async.wait_group %0;" ::"n"(RAW_DEPTH - 1) : "memory");
-      if (i >= S) {
-        int ok = 1;
-        if (lane == 0) ok = mbar_wait(a_empty + 8 * s, (round - 1) & 1, 1u) ? 1 : 0;
-        __syncwarp();
-        alive = __shfl_sync(0xffffffffu, ok, 0) != 0;
+    for (; left > 0; left--) {
+      cp_async_wait(R - 2); // the super-step's copies of this thread have landed
+      asm volatile("bar.sync %0, 128;" ::"r"(2 + rg) : "memory"); // ... and those of the row group's other threads; all have read the previous slot
+      issue();              // into the previous slot
+      const int kt = c_s * KPS + kk, i = base_i + kt;
+      if (alive && kt < KT && i >= 0 && i < nsteps) {
+        for (s += i - at, at = i; s >= S; lap ^= 1u) s -= S;
+        if (i >= S) alive = mbar_wait_uniform(a_empty + 8 * s, lap ^ 1u, 1u); // a warp that gave up still takes part in the barriers
+        if (alive) {
+          const uint32_t dst_row = a_ring + s * A_STAGE_BYTES + r * 128;
+          const uint32_t slot = raw + (uint32_t)c_slot * SLOT + (uint32_t)(lane * RowT::ROWB);
+          if ((int64_t)c_n * TILE_N + r < p.w.n) RowT::store(slot, c_s, kk, hf, p.wscale, dst_row, sw);
+          else zero_row(dst_row, sw, KPS == 2 ? 4 * hf : 0, KPS == 2 ? 4 : 8);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(a_full + 8 * s);
+        }
       }
-      if (!alive) break;
-      const int64_t row = (int64_t)cur.tile_n * TILE_N + r;
-      const uint32_t dst_row = a_ring + s * A_STAGE_BYTES + r * 128;
-      if (row < p.w.n) RowT::store(p.w, slot, cur.kt, hf, p.wscale, dst_row, sw);
-      else zero_half_row(dst_row, hf);
-      if (i + 2 * RAW_DEPTH < nsteps) {
-        const int64_t prow = (int64_t)pre.tile_n * TILE_N + r;
-        RowT::issue(p.w, prow < p.w.n ? prow : p.w.n - 1, pre.kt, hf, slot);
-        pre.advance(2, KT, TM);
+      if (++c_slot == R) c_slot = 0;
+      if (++c_s == SPT) {
+        c_s = 0;
+        base_i += KT;
+        if (++c_m == TM) c_m = 0, c_n++;
       }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(a_full + 8 * s);
-      rs = (rs + 1 == RAW_DEPTH) ? 0 : rs + 1;
-      cur.advance(2, KT, TM);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
   } else if (warp == LOADER_WARP) {
-    // ---- activation loader ------------------------------------------------------------------------------
-    if (lane == 0) {
-      Cursor cur = start;
-      int issued = 0;
-      for (int i = 0; i < nsteps; i++) {
-        const int s = i % SB;
-        const uint32_t round = (uint32_t)(i / SB);
-        if (round > 0 && !mbar_wait(b_empty + 8 * s, (round - 1) & 1, 2u)) break;
-        const int64_t m0 = (int64_t)cur.tile_m * MAX_MT;
-        const uint32_t bytes = (uint32_t)min((int64_t)MAX_MT, p.m_pad - m0) * 128;
-        mbar_expect_tx(b_full + 8 * s, bytes);
-        bulk_g2s(b_ring + s * p.b_stride, p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128, bytes, b_full + 8 * s);
-        issued = i + 1;
-        cur.advance(1, KT, TM);
+    // ---- activation loader: the whole warp runs the loop, one elected lane issues (see the MMA issuer) ----
+    pdl_wait(); // the activation image is the previous kernel's output
+    Cursor cur = start;
+    int sb = 0, issued = 0;
+    uint32_t lap = 0;
+    for (int i = 0; i < nsteps; i++) {
+      if (i >= SB && !mbar_wait_uniform(b_empty + 8 * sb, lap ^ 1u, 2u)) break;
+      const int64_t m0 = (int64_t)cur.tile_m * MAX_MT;
+      const uint32_t bytes = (uint32_t)min((int64_t)MAX_MT, p.m_pad - m0) * 128;
+      if (elect_one()) {
+        mbar_expect_tx(b_full + 8 * sb, bytes);
+        bulk_g2s(b_ring + sb * p.b_stride, p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128, bytes, b_full + 8 * sb);
       }
-      for (int i = max(0, issued - SB); i < issued; i++) mbar_wait(b_full + 8 * (i % SB), (i / SB) & 1, 2u); // nothing in flight at exit
+      __syncwarp();
+      issued = i + 1;
+      cur.advance(1, KT, TM);
+      if (++sb == SB) sb = 0, lap ^= 1u;
     }
+    for (int i = max(0, issued - SB); i < issued; i++) mbar_wait_uniform(b_full + 8 * (i % SB), (i / SB) & 1, 2u); // nothing in flight at exit
   } else if (warp == MMA_WARP) {
-    // ---- MMA issuer -------------------------------------------------------------------------------------
-    if (lane == 0) {
-      Cursor cur = start;
-      bool alive = true, a_ready = false, b_ready = false;
-      int i = 0, s = 0, sb = 0;
-      uint32_t round = 0, bround = 0;
-      for (int seg = 0; i < nsteps && alive; seg++) {
-        const int len = min(KT - cur.kt, nsteps - i);
-        const int buf = seg & 1, use = seg >> 1;
-        if (use > 0) alive = mbar_wait(acc_empty + 8 * buf, (use - 1) & 1, 4u); // the drain of this buffer's previous segment
+    // ---- MMA issuer: the whole warp runs the loop and one elected lane issues. Inside a branch on the lane number the compiler
+    // moves every MMA's descriptors from vector to uniform registers one after the other, which holds the thread for 96 cycles
+    // per MMA; converged, an MMA leaves every 40 (N <= 32), 48 (64), 64 (128) or 128 (256) cycles, the tensor core's own rate. ----
+    Cursor cur = start;
+    bool alive = true, a_ready = false, b_ready = false;
+    int i = 0, s = 0, sb = 0;
+    uint32_t round = 0, bround = 0;
+    for (int seg = 0; i < nsteps && alive; seg++) {
+      const int len = min(KT - cur.kt, nsteps - i);
+      const int buf = seg & 1, use = seg >> 1;
+      if (use > 0) alive = mbar_wait_uniform(acc_empty + 8 * buf, (use - 1) & 1, 4u); // the drain of this buffer's previous segment
+      if (!alive) break;
+      tc_fence_after();
+      const int64_t m0 = (int64_t)cur.tile_m * MAX_MT;
+      const uint32_t idesc = idesc_f16((int)min((int64_t)MAX_MT, p.m_pad - m0));
+      const uint32_t d = tmem_d + (uint32_t)(buf * MAX_MT);
+      for (int j = 0; j < len && alive; j++, i++) {
+        if (!a_ready) alive = mbar_wait_uniform(a_full + 8 * s, round & 1, 4u);
+        if (alive && !b_ready) alive = mbar_wait_uniform(b_full + 8 * sb, bround & 1, 4u);
         if (!alive) break;
         tc_fence_after();
-        const int64_t m0 = (int64_t)cur.tile_m * MAX_MT;
-        const uint32_t idesc = idesc_f16((int)min((int64_t)MAX_MT, p.m_pad - m0));
-        const uint32_t d = tmem_d + (uint32_t)(buf * MAX_MT);
-        for (int j = 0; j < len && alive; j++, i++) {
-          if (!a_ready) alive = mbar_wait(a_full + 8 * s, round & 1, 4u);
-          if (alive && !b_ready) alive = mbar_wait(b_full + 8 * sb, bround & 1, 4u);
-          if (!alive) break;
-          tc_fence_after();
-          const uint64_t adesc = smem_desc_sw128(a_ring + s * A_STAGE_BYTES);
-          const uint64_t bdesc = smem_desc_sw128(b_ring + sb * p.b_stride);
-          const int cs = s, csb = sb;
-          if (++s == S) {
-            s = 0;
-            round++;
-          }
-          if (++sb == SB) {
-            sb = 0;
-            bround++;
-          }
-          // probe the next step's barriers now: the test's latency hides behind the issue of this step's MMAs
-          a_ready = i + 1 < nsteps && mbar_try_wait(a_full + 8 * s, round & 1);
-          b_ready = i + 1 < nsteps && mbar_try_wait(b_full + 8 * sb, bround & 1);
+        const uint64_t adesc = smem_desc_sw128(a_ring + s * A_STAGE_BYTES);
+        const uint64_t bdesc = smem_desc_sw128(b_ring + sb * p.b_stride);
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < BK / 16; ks++) umma_f16(d, adesc + (uint64_t)(ks * 2), bdesc + (uint64_t)(ks * 2), idesc, (j | ks) ? 1u : 0u);
-          umma_commit(a_empty + 8 * cs);
-          umma_commit(b_empty + 8 * csb);
+          umma_commit(a_empty + 8 * s);
+          umma_commit(b_empty + 8 * sb);
+          if (j == len - 1) umma_commit(acc_full + 8 * buf);
         }
-        if (alive) umma_commit(acc_full + 8 * buf);
-        cur.advance(len, KT, TM);
+        __syncwarp();
+        if (++s == S) {
+          s = 0;
+          round++;
+        }
+        if (++sb == SB) {
+          sb = 0;
+          bround++;
+        }
+        // probe the next step's barriers while this step's MMAs run
+        a_ready = i + 1 < nsteps && __all_sync(0xffffffffu, mbar_try_wait(a_full + 8 * s, round & 1));
+        b_ready = i + 1 < nsteps && __all_sync(0xffffffffu, mbar_try_wait(b_full + 8 * sb, bround & 1));
       }
+      cur.advance(len, KT, TM);
     }
   } else {
     // ---- drain: four warps, warp q reads accumulator lanes 32q.. (weight rows), all columns -----------------
     const int q = warp & 3; // tensor-memory lanes a warp may read are fixed by its index modulo 4
     const int half = (warp - EPI_WARP0) >> 2; // which half of the 32-column chunks this warp takes
-    const int et = threadIdx.x - EPI_WARP0 * 32; // 0..127
+    const int et = threadIdx.x - EPI_WARP0 * 32; // 0..255
+    pdl_wait(); // the previous kernel writes the row factors and zeroes the tiles' tickets
     Cursor cur = start;
     bool alive = true;
     int i = 0;
@@ -419,7 +492,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       // one thread waits for the accumulator and, for a tile shared with other CTAs, settles who stores and
       // who adds; the four warps then act on the same answers
       if (et == 0) {
-        unsigned int t = mbar_wait_relaxed(acc_full + 8 * buf, use & 1, 8u) ? 0u : 0x80000000u;
+        unsigned int t = mbar_wait(acc_full + 8 * buf, use & 1, 8u) ? 0u : 0x80000000u;
         if (!whole && t == 0) {
           t = atomicAdd(p.tile_cnt + tile, 1u);
           if (t > 0) { // wait (bounded) until the first finisher's stores are visible
@@ -482,17 +555,11 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
 }
 
 // ---- activation image -----------------------------------------------------------------------------------
-// position of source element e (0..63) of a k-step inside the stored k-step, per weight format
-__device__ __forceinline__ int kpos_q4_0(int e) { // stored chunk (b*4 + wi) holds [j, j+2, j+16, j+18, j+1, j+3, j+17, j+19] + 32b, j = 4wi
-  const int b = e >> 5, x = e & 31, hi = x >> 4, y = x & 15, wi = y >> 2, t = y & 3;
-  const int slot = (t & 1) * 4 + hi * 2 + (t >> 1);
-  return (b * 4 + wi) * 8 + slot;
-}
-__device__ __forceinline__ int kpos_q4k(int e) { // stored chunk wi holds [l, l+2, 32+l, 32+l+2, l+1, l+3, 32+l+1, 32+l+3], l = 4wi
-  const int hi = e >> 5, y = e & 31, wi = y >> 2, t = y & 3;
-  const int slot = (t & 1) * 4 + hi * 2 + (t >> 1);
-  return wi * 8 + slot;
-}
+// Stored order inside a k-step: Q8_0 and Q6_K natural. Q4_0 and Q4_K store pairs of 4-element runs that lie 16 (Q4_0) or 32
+// (Q4_K) elements apart as one 8-element chunk [j, j+2, f+j, f+j+2, j+1, j+3, f+j+1, f+j+3], f = 16 or 32: the order the nibble
+// unpack produces. A thread holds 8 consecutive elements (two such runs) and its partner, 2 or 4 lanes away, the other two.
+__device__ __forceinline__ int kpair_shift(int wdtype) { return wdtype == XNQ_Q4_0 ? 2 : (wdtype == XNQ_Q4K ? 4 : 0); }
+__device__ __forceinline__ uint32_t pack_h2(__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); }
 
 // One CTA per activation row: Q8 quantize (the reference's activation blocks), dequantize, scale the row
 // by a power of two so its largest magnitude lands in [2^11, 2^12), store fp16 into the swizzled image.
@@ -501,6 +568,8 @@ __global__ void __launch_bounds__(256) prefill_prepare_acts(const XT *__restrict
                                                             int wdtype, float wscale, uint8_t *__restrict__ xh, float *__restrict__ row_unscale,
                                                             unsigned int *__restrict__ tile_cnt, int tile_words) {
   __shared__ float red[8];
+  pdl_launch_dependents(); // the matmul kernel may set itself up and request its first weights now
+  pdl_wait();              // x may be the previous kernel's output; the scratch may still be read by the previous call
   const int64_t row = blockIdx.x;
   if (blockIdx.x == 0) // the persistent kernel's per-tile tickets and flags start every call at zero
     for (int i = threadIdx.x; i < tile_words; i += blockDim.x) tile_cnt[i] = 0;
@@ -550,19 +619,28 @@ __global__ void __launch_bounds__(256) prefill_prepare_acts(const XT *__restrict
       for (int i = 0; i < 8; i++) v[i] = 0.f;
     }
     const Quant8 q = ACT == XNQ_Q8_0 ? quantize8_q8_0(v, lane) : quantize8_q8k(v, lane);
-    if (t >= per_row) continue;
     const float ds = q.d * rscale; // exact unless it leaves the normal range
-    const int64_t kt = t >> 3;
-    __half *dst = img + (kt * m_pad + row) * 64;
-    const int sw = (int)(row & 7);
+    __half h[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const int code = (int)(int8_t)(((i < 4 ? q.lo : q.hi) >> (8 * (i & 3))) & 0xff);
-      const int esrc = (int)((t & 7) * 8 + i);
-      const int pos = wdtype == XNQ_Q4_0 ? kpos_q4_0(esrc) : (wdtype == XNQ_Q4K ? kpos_q4k(esrc) : esrc);
-      const int chunk = pos >> 3;
-      dst[((chunk ^ sw) << 3) + (pos & 7)] = __float2half_rn(valid ? (float)code * ds : 0.f);
+      h[i] = __float2half_rn(valid ? (float)code * ds : 0.f);
     }
+    const int ps = kpair_shift(wdtype);
+    uint4 out;
+    int chunk = (int)(t & 7);
+    if (ps == 0) {
+      out = make_uint4(pack_h2(h[0], h[1]), pack_h2(h[2], h[3]), pack_h2(h[4], h[5]), pack_h2(h[6], h[7]));
+    } else { // runs A (elements 0..3) and B (4..7): the lower thread of a pair stores both threads' runs A, the upper one their runs B
+      const bool upper = (t & ps) != 0;
+      const uint32_t a02 = pack_h2(h[0], h[2]), a13 = pack_h2(h[1], h[3]), b02 = pack_h2(h[4], h[6]), b13 = pack_h2(h[5], h[7]);
+      const uint32_t g0 = __shfl_xor_sync(0xffffffffu, upper ? a02 : b02, ps), g1 = __shfl_xor_sync(0xffffffffu, upper ? a13 : b13, ps);
+      out = upper ? make_uint4(g0, b02, g1, b13) : make_uint4(a02, g0, a13, g1);
+      // Q4_0: block b = t >> 2, run pair (t & 1); Q4_K: run pair (t & 3)
+      chunk = ps == 2 ? ((chunk >> 2) * 4 + (chunk & 1) * 2 + (upper ? 1 : 0)) : ((chunk & 3) * 2 + (upper ? 1 : 0));
+    }
+    if (t >= per_row) continue;
+    *reinterpret_cast<uint4 *>(img + ((t >> 3) * m_pad + row) * 64 + ((chunk ^ (int)(row & 7)) << 3)) = out;
   }
 }
 
@@ -570,12 +648,12 @@ int g_num_sms = 0;
 
 template <typename RowT>
 int launch_persistent_fmt(const PrefillArgs &a, unsigned ctas, size_t smem, cudaStream_t s) {
-  prefill_persistent_kernel<RowT><<<ctas, NTHREADS_SK, smem, s>>>(a);
-  XNQ_CUDA(cudaGetLastError());
+  XNQ_CUDA(launch_pdl(prefill_persistent_kernel<RowT>, dim3(ctas), dim3(NTHREADS_SK), smem, s, a));
   count_launch();
   return XNQ_OK;
 }
 
+static_assert(RowQ4_0::ROWB == RowQ4K::ROWB && RowQ8_0::ROWB == RowQ4K::ROWB, "the raw ring's plan assumes one slot size for these");
 constexpr size_t PREFILL_SMEM = 226 * 1024; // everything an SM offers minus the static barriers and a reserve
 
 } // namespace
@@ -602,8 +680,8 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   uint8_t *xh = reinterpret_cast<uint8_t *>(tile_cnt) + cnt_bytes;
   const int act = act_dtype_for(w.dtype);
 #define XNQ_PREP(ACT, XT)                                                                                                   \
-  prefill_prepare_acts<ACT, XT><<<(unsigned)m_pad, 256, 0, s>>>(static_cast<const XT *>(x), m, k, ldx, m_pad, ksteps, w.dtype, wscale, xh, \
-                                                                row_unscale, tile_cnt, (int)(cnt_bytes / 4))
+  XNQ_CUDA(launch_pdl(prefill_prepare_acts<ACT, XT>, dim3((unsigned)m_pad), dim3(256), 0, s, static_cast<const XT *>(x), m, k, ldx, m_pad, ksteps, \
+                      w.dtype, wscale, xh, row_unscale, tile_cnt, (int)(cnt_bytes / 4)))
   if (act == XNQ_Q8_0) {
     if (x_dtype == XNQ_F32) XNQ_PREP(XNQ_Q8_0, float);
     else if (x_dtype == XNQ_F16) XNQ_PREP(XNQ_Q8_0, __half);
@@ -614,7 +692,6 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
     else XNQ_PREP(XNQ_Q8K, __nv_bfloat16);
   }
 #undef XNQ_PREP
-  XNQ_CUDA(cudaGetLastError());
   count_launch();
 
   PrefillArgs a{};
@@ -627,16 +704,22 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   a.m = m;
   a.m_pad = m_pad;
   a.ksteps = ksteps;
-  a.nstages = NSTAGES;
-  // shared-memory plan: A ring | B ring (as deep as fits, at most 8) | raw rings
-  const int slot = w.dtype == XNQ_Q6K ? 80 : 48;
+  // Shared-memory plan: A ring | B ring | raw ring. At 256 activation rows there is room for four weight and three activation stages
+  // beside two or three raw slots; narrower tiles take up to eight of each, so that a producer warp can be a whole super-step ahead of
+  // the MMAs, and what is left goes to the raw ring (it covers the memory latency of the weights).
+  const uint32_t slot = TILE_N * (w.dtype == XNQ_Q6K ? RowQ6K::ROWB : RowQ4K::ROWB);
   const uint32_t mt_max = (uint32_t)std::min<int64_t>(MAX_MT, m_pad);
   a.b_stride = (mt_max * 128 + 1023) & ~1023u;
-  const size_t raw_bytes = (size_t)RAW_DEPTH * PRODUCERS * slot;
-  const size_t fixed = (size_t)NSTAGES * A_STAGE_BYTES + raw_bytes + 1024; // + alignment slack
-  a.b_stages = (int)std::min<size_t>(8, (PREFILL_SMEM - fixed) / a.b_stride);
-  if (a.b_stages < 2) return fail(XNQ_ERR_SIZE, "prefill: shared-memory plan does not fit");
-  a.b_off = NSTAGES * A_STAGE_BYTES;
+  const size_t budget = PREFILL_SMEM - 1024; // alignment slack
+  a.nstages = MIN_STAGES, a.b_stages = 3;
+  for (int st = MAX_STAGES; st >= MIN_STAGES; st--)
+    if ((size_t)st * (A_STAGE_BYTES + a.b_stride) + 3 * slot <= budget) {
+      a.nstages = a.b_stages = st;
+      break;
+    }
+  if ((size_t)a.nstages * A_STAGE_BYTES + (size_t)a.b_stages * a.b_stride + 2 * slot > budget) return fail(XNQ_ERR_SIZE, "prefill: shared-memory plan does not fit");
+  a.raw_slots = (int)std::min<size_t>(MAX_RAW_SLOTS, (budget - (size_t)a.nstages * A_STAGE_BYTES - (size_t)a.b_stages * a.b_stride) / slot);
+  a.b_off = a.nstages * A_STAGE_BYTES;
   a.raw_off = a.b_off + a.b_stages * a.b_stride;
   a.wscale = wscale;
   const dim3 grid((unsigned)((w.n + TILE_N - 1) / TILE_N), (unsigned)((m_pad + MAX_MT - 1) / MAX_MT));

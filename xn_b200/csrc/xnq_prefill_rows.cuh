@@ -1,16 +1,15 @@
-// Per-format weight producers of the prefill kernel: two threads own one weight row of the tile.
+// Per-format weight producers of the prefill kernel.
 //
-// A k-step of a row is handled in two halves that are several k-steps apart in time:
-//   issue()  cp.async copies of the row's raw quantized bytes for that k-step into a slot of the
-//            thread's PRIVATE shared-memory ring (no other thread reads it, so no barrier is needed:
-//            cp.async.wait_group orders the copies before the same thread's loads);
-//   store()  read the slot, dequantize to fp16 and write the 8 swizzled 16-byte chunks of the row into
-//            the A stage the tensor core reads.
-// Keeping DEPTH k-steps of copies in flight per thread hides the HBM latency without holding the bytes
-// in registers. Slot sizes are odd multiples of 16 bytes, so a quarter-warp's 128-bit reads of eight
-// neighbouring slots fall into eight different bank groups.
+// The weight rows of a tile are fetched and dequantized in row groups of 32 rows. A row group's bytes of one super-step (256 k,
+// Q8_0: 128 k) are one slot of a shared-memory ring: ROWB bytes per row, an odd multiple of 16, so that a quarter warp's 128-bit
+// reads of eight neighbouring rows fall into eight different bank groups.
+//   item()   one of the ITEMS 16-byte copies that make up a row's super-step: where it comes from and how that moves with the
+//            super-step. Consecutive threads take consecutive copies, so that a copy instruction of a warp touches four to six runs
+//            of memory (one thread per row would touch 32).
+//   store()  reads the row's bytes of one 64-wide k-step (or of half of it) from the slot, dequantizes to fp16 and writes the
+//            swizzled 16-byte chunks of the row into the A stage the tensor core reads.
 //
-// Stored k order inside a k-step (the activation image uses the same one, see kpos_* in xnq_prefill.cu):
+// Stored k order inside a k-step (the activation image uses the same one, see kpair_shift in xnq_prefill.cu):
 //   Q8_0, Q6_K  natural
 //   Q4_0        chunk 4b + wi = elements [j, j+2, j+16, j+18, j+1, j+3, j+17, j+19] + 32b, j = 4wi
 //   Q4_K        chunk wi      = elements [l, l+2, 32+l, 32+l+2, l+1, l+3, 32+l+1, 32+l+3], l = 4wi
@@ -22,11 +21,9 @@
 namespace xnq {
 namespace prefill_rows {
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+// bytes 0: zeros are written and nothing is read
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
@@ -49,52 +46,54 @@ __device__ __forceinline__ __half2 scaled_half2(uint32_t f16_bits, float wscale)
   return __float2half2_rn(__half2float(__ushort_as_half((unsigned short)f16_bits)) * wscale);
 }
 
-// Two threads share a weight row: thread half hf (0/1) produces chunks 4*hf .. 4*hf+3 of the k-step.
+// A copy's bytes of super-step ss are at p + ((ss * mul) & ~15); from lim on there is nothing (zeros are stored).
+struct Item {
+  const uint8_t *p;
+  uint32_t mul, lim;
+};
+constexpr uint32_t NO_LIMIT = 0xffffffffu;
+
+// KPS k-steps per super-step. KPS = 4: one thread converts a row's whole k-step; KPS = 2: two threads, half hf (32 elements) each.
 // All shared-memory reads of a call are issued before any arithmetic.
 
-struct RowQ4_0 { // half = one 32-element block
-  static constexpr int SLOT = 48; // 16 nibble bytes | f16 scale pair | pad   (odd multiple of 16)
-  __device__ static __forceinline__ void issue(const WeightView &w, int64_t row, int kt, int hf, uint32_t slot) {
-    const int64_t nblk = w.k / QK;
-    const int64_t b = min((int64_t)kt * 2 + hf, nblk - 1); // odd block count: the missing block is zeroed in store()
-    cp_async16(slot, w.qs + (row * nblk + b) * 16);
-    cp_async4(slot + 16, w.d + row * w.dstride + (b & ~(int64_t)1));
+struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
+  static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
+  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { // scales beyond the last block are zero
+    if (c < 8) return Item{w.qs + row * (w.k / 2) + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k / 2 - 16 * c)};
+    return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 16u, NO_LIMIT};
   }
-  __device__ static __forceinline__ void store(const WeightView &w, uint32_t slot, int kt, int hf, float wscale, uint32_t dst_row, int sw) {
-    const uint4 q = lds128(slot);
-    const uint32_t dd = lds32(slot + 16);
-    const bool ok = (int64_t)kt * 2 + hf < w.k / QK;
-    const __half2 d2 = ok ? scaled_half2(hf ? (dd >> 16) : (dd & 0xffffu), wscale) : __float2half2_rn(0.f);
+  __device__ static __forceinline__ void store(uint32_t slot, int, int kk, int, float wscale, uint32_t dst_row, int sw) {
+    const uint4 q[2] = {lds128(slot + 32 * kk), lds128(slot + 32 * kk + 16)};
+    const uint32_t dd = lds32(slot + 128 + 4 * kk);
     const __half2 off = h2_from_bits(0x64086408u); // 1032 = 1024 + 8
-    const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int wi = 0; wi < 4; wi++) {
-      uint32_t o[4];
+    for (int b = 0; b < 2; b++) {
+      const __half2 d2 = scaled_half2(b ? (dd >> 16) : (dd & 0xffffu), wscale);
+      const uint32_t wd[4] = {q[b].x, q[b].y, q[b].z, q[b].w};
 #pragma unroll
-      for (int p = 0; p < 4; p++) { // nibble pairs (p, p+4) of the word
-        const __half2 v = h2_from_bits(((wd[wi] >> (4 * p)) & 0x000f000fu) | 0x64006400u);
-        o[p] = bits_from_h2(__hmul2(__hsub2(v, off), d2));
+      for (int wi = 0; wi < 4; wi++) {
+        uint32_t o[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) { // nibble pairs (p, p+4) of the word
+          const __half2 v = h2_from_bits(((wd[wi] >> (4 * p)) & 0x000f000fu) | 0x64006400u);
+          o[p] = bits_from_h2(__hmul2(__hsub2(v, off), d2));
+        }
+        sts128(dst_row + (((b * 4 + wi) ^ sw) << 4), o[0], o[1], o[2], o[3]);
       }
-      sts128(dst_row + (((hf * 4 + wi) ^ sw) << 4), o[0], o[1], o[2], o[3]);
     }
   }
 };
 
-struct RowQ8_0 { // half = one 32-element block
-  static constexpr int SLOT = 48; // 32 codes | f16 scale pair | pad
-  __device__ static __forceinline__ void issue(const WeightView &w, int64_t row, int kt, int hf, uint32_t slot) {
-    const int64_t nblk = w.k / QK;
-    const int64_t b = min((int64_t)kt * 2 + hf, nblk - 1);
-    const uint8_t *r = w.qs + row * w.k + b * 32;
-    cp_async16(slot, r);
-    cp_async16(slot + 16, r + 16);
-    cp_async4(slot + 32, w.d + row * w.dstride + (b & ~(int64_t)1));
+struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighbour
+  static constexpr int KPS = 2, ROWB = 144, ITEMS = 9;
+  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) {
+    if (c < 8) return Item{w.qs + row * w.k + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k - 16 * c)};
+    return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 8u, NO_LIMIT};
   }
-  __device__ static __forceinline__ void store(const WeightView &w, uint32_t slot, int kt, int hf, float wscale, uint32_t dst_row, int sw) {
-    const uint4 q[2] = {lds128(slot), lds128(slot + 16)};
-    const uint32_t dd = lds32(slot + 32);
-    const bool ok = (int64_t)kt * 2 + hf < w.k / QK;
-    const __half2 d2 = ok ? scaled_half2(hf ? (dd >> 16) : (dd & 0xffffu), wscale) : __float2half2_rn(0.f);
+  __device__ static __forceinline__ void store(uint32_t slot, int ss, int kk, int hf, float wscale, uint32_t dst_row, int sw) { // half = one block
+    const uint4 q[2] = {lds128(slot + 64 * kk + 32 * hf), lds128(slot + 64 * kk + 32 * hf + 16)};
+    const uint32_t dd = lds32(slot + 128 + 8 * (ss & 1) + 4 * kk);
+    const __half2 d2 = scaled_half2(hf ? (dd >> 16) : (dd & 0xffffu), wscale);
     const __half2 off = h2_from_bits(0x64806480u); // 1152 = 1024 + 128
 #pragma unroll
     for (int c = 0; c < 4; c++) { // chunk = 8 codes
@@ -112,17 +111,11 @@ struct RowQ8_0 { // half = one 32-element block
   }
 };
 
-struct RowQ4K { // half = 16 of the 32 nibble bytes of the k-step's group (words 4*hf .. 4*hf+3)
-  static constexpr int SLOT = 48; // header | 16 nibble bytes | pad
-  __device__ static __forceinline__ void issue(const WeightView &w, int64_t row, int kt, int hf, uint32_t slot) {
-    const int64_t nsb = w.k / QK_K;
-    const uint8_t *blk = w.qs + (row * nsb + (kt >> 2)) * 144;
-    cp_async16(slot, blk);
-    cp_async16(slot + 16, blk + 16 + 32 * (kt & 3) + 16 * hf);
-  }
-  __device__ static __forceinline__ void store(const WeightView &, uint32_t slot, int kt, int hf, float wscale, uint32_t dst_row, int sw) {
-    const int g = kt & 3;
-    const uint4 hdr = lds128(slot), q = lds128(slot + 16);
+struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
+  static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
+  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { return Item{w.qs + row * (w.k / QK_K) * 144 + 16 * c, 144u, NO_LIMIT}; }
+  __device__ static __forceinline__ void store(uint32_t slot, int, int g, int, float wscale, uint32_t dst_row, int sw) {
+    const uint4 hdr = lds128(slot), q[2] = {lds128(slot + 16 + 32 * g), lds128(slot + 32 + 32 * g)};
     const __half2 dm = *reinterpret_cast<const __half2 *>(&hdr.x);
     const uint32_t f = k4_field(hdr.y, hdr.z, hdr.w, g);
     const float d = __low2float(dm) * wscale, mn = __high2float(dm) * wscale;
@@ -130,58 +123,58 @@ struct RowQ4K { // half = 16 of the 32 nibble bytes of the k-step's group (words
     const __half2 a_lo = __float2half2_rn(d * (float)(f & 63)), a_hi = __float2half2_rn(d * (float)((f >> 6) & 63));
     const __half2 b_lo = __float2half2_rn(-mn * (float)((f >> 12) & 63)), b_hi = __float2half2_rn(-mn * (float)(f >> 18));
     const __half2 k1024 = h2_from_bits(0x64006400u);
-    const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int wi = 0; wi < 4; wi++) {
+    for (int wi = 0; wi < 8; wi++) {
+      const uint4 &v = q[wi >> 2];
+      const uint32_t wd = (wi & 3) == 0 ? v.x : ((wi & 3) == 1 ? v.y : ((wi & 3) == 2 ? v.z : v.w));
       uint32_t o[4];
 #pragma unroll
       for (int p = 0; p < 4; p++) { // pairs: p=0 (l, l+2) low, p=1 (32+l, 32+l+2) high, p=2 (l+1, l+3) low, p=3 high
-        const __half2 c = __hsub2(h2_from_bits(((wd[wi] >> (4 * p)) & 0x000f000fu) | 0x64006400u), k1024);
+        const __half2 c = __hsub2(h2_from_bits(((wd >> (4 * p)) & 0x000f000fu) | 0x64006400u), k1024);
         o[p] = bits_from_h2((p & 1) ? __hfma2(c, a_hi, b_hi) : __hfma2(c, a_lo, b_lo));
       }
-      sts128(dst_row + (((hf * 4 + wi) ^ sw) << 4), o[0], o[1], o[2], o[3]);
+      sts128(dst_row + ((wi ^ sw) << 4), o[0], o[1], o[2], o[3]);
     }
   }
 };
 
-struct RowQ6K { // half = one 32-element group: hf = 0 takes the nibbles of ql[l], hf = 1 those of ql[l + 32]
-  static constexpr int SLOT = 80; // 32 ql bytes | 32 qh bytes | 4 scales | f16 d pair | pad
-  __device__ static __forceinline__ void issue(const WeightView &w, int64_t row, int kt, int hf, uint32_t slot) {
-    const int64_t nsb = w.k / QK_K;
-    const int sb = kt >> 2, s = kt & 3, h = s >> 1, hi_pair = s & 1;
-    const int64_t blk = row * nsb + sb;
-    cp_async16(slot, w.qs + blk * 128 + 64 * h + 32 * hf);
-    cp_async16(slot + 16, w.qs + blk * 128 + 64 * h + 32 * hf + 16);
-    cp_async16(slot + 32, w.qh + blk * 64 + 32 * h);
-    cp_async16(slot + 48, w.qh + blk * 64 + 32 * h + 16);
-    cp_async4(slot + 64, w.sc + blk * 16 + 8 * h + 4 * hi_pair);
-    cp_async4(slot + 68, w.d + row * w.dstride + (sb & ~1));
+struct RowQ6K { // 128 ql bytes | 64 qh bytes | 16 scales | the f16 d of eight super-blocks
+  static constexpr int KPS = 4, ROWB = 240, ITEMS = 14;
+  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) {
+    const int64_t blk = row * (w.k / QK_K);
+    if (c < 8) return Item{w.qs + blk * 128 + 16 * c, 128u, NO_LIMIT};
+    if (c < 12) return Item{w.qh + blk * 64 + 16 * (c - 8), 64u, NO_LIMIT};
+    if (c == 12) return Item{reinterpret_cast<const uint8_t *>(w.sc + blk * 16), 16u, NO_LIMIT};
+    return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 2u, NO_LIMIT};
   }
-  __device__ static __forceinline__ void store(const WeightView &, uint32_t slot, int kt, int hf, float wscale, uint32_t dst_row, int sw) {
-    const int sb = kt >> 2, hi_pair = kt & 1;
-    const uint4 ql[2] = {lds128(slot), lds128(slot + 16)};
-    const uint4 qh[2] = {lds128(slot + 32), lds128(slot + 48)};
-    const uint32_t sc4 = lds32(slot + 64), dd = lds32(slot + 68);
-    const float d = __half2float(__ushort_as_half((unsigned short)((sb & 1) ? (dd >> 16) : (dd & 0xffffu)))) * wscale;
+  // k-step kk = 2 h + hi_pair of the super-block: group 0 takes ql[l] of half h, group 1 ql[l + 32], both the low (hi_pair 0) or high nibbles
+  __device__ static __forceinline__ void store(uint32_t slot, int ss, int kk, int, float wscale, uint32_t dst_row, int sw) {
+    const int h = kk >> 1, sh = 4 * (kk & 1);
+    const uint4 qh[2] = {lds128(slot + 128 + 32 * h), lds128(slot + 144 + 32 * h)};
+    const uint32_t sc4 = lds32(slot + 192 + 8 * h + 4 * (kk & 1)), dd = lds32(slot + 208 + 4 * ((ss >> 1) & 3));
+    const float d = __half2float(__ushort_as_half((unsigned short)((ss & 1) ? (dd >> 16) : (dd & 0xffffu)))) * wscale;
     const __half2 off = h2_from_bits(0x64206420u); // 1056 = 1024 + 32
-    const int sh = 4 * hi_pair;       // low or high nibble of ql, and which half of qh's four bit pairs
-    const int hsh = sh + 2 * hf;      // bit position of this group's two high bits inside a qh byte
 #pragma unroll
-    for (int c = 0; c < 4; c++) { // chunk of 8 elements l = 8c .. 8c+7
-      const uint32_t lw[2] = {(c & 1) ? ql[c >> 1].z : ql[c >> 1].x, (c & 1) ? ql[c >> 1].w : ql[c >> 1].y};
-      const uint32_t hw[2] = {(c & 1) ? qh[c >> 1].z : qh[c >> 1].x, (c & 1) ? qh[c >> 1].w : qh[c >> 1].y};
-      const int8_t sc = (int8_t)((sc4 >> (8 * (2 * hf + (c >> 1)))) & 0xff);
-      const __half2 s2 = __float2half2_rn(d * (float)sc);
-      uint32_t o[4];
+    for (int hf = 0; hf < 2; hf++) {
+      const uint4 ql[2] = {lds128(slot + 64 * h + 32 * hf), lds128(slot + 64 * h + 32 * hf + 16)};
+      const int hsh = sh + 2 * hf; // bit position of this group's two high bits inside a qh byte
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const uint32_t code = ((lw[j] >> sh) & 0x0f0f0f0fu) | (((hw[j] >> hsh) << 4) & 0x30303030u);
-        const __half2 lo = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4140));
-        const __half2 hi = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4342));
-        o[2 * j] = bits_from_h2(__hmul2(__hsub2(lo, off), s2));
-        o[2 * j + 1] = bits_from_h2(__hmul2(__hsub2(hi, off), s2));
+      for (int c = 0; c < 4; c++) { // chunk of 8 elements l = 8c .. 8c+7
+        const uint32_t lw[2] = {(c & 1) ? ql[c >> 1].z : ql[c >> 1].x, (c & 1) ? ql[c >> 1].w : ql[c >> 1].y};
+        const uint32_t hw[2] = {(c & 1) ? qh[c >> 1].z : qh[c >> 1].x, (c & 1) ? qh[c >> 1].w : qh[c >> 1].y};
+        const int8_t sc = (int8_t)((sc4 >> (8 * (2 * hf + (c >> 1)))) & 0xff);
+        const __half2 s2 = __float2half2_rn(d * (float)sc);
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const uint32_t code = ((lw[j] >> sh) & 0x0f0f0f0fu) | (((hw[j] >> hsh) << 4) & 0x30303030u);
+          const __half2 lo = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4140));
+          const __half2 hi = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4342));
+          o[2 * j] = bits_from_h2(__hmul2(__hsub2(lo, off), s2));
+          o[2 * j + 1] = bits_from_h2(__hmul2(__hsub2(hi, off), s2));
+        }
+        sts128(dst_row + (((hf * 4 + c) ^ sw) << 4), o[0], o[1], o[2], o[3]);
       }
-      sts128(dst_row + (((hf * 4 + c) ^ sw) << 4), o[0], o[1], o[2], o[3]);
     }
   }
 };
