@@ -427,30 +427,29 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     }
     for (int i = max(0, issued - SB); i < issued; i++) mbar_wait_uniform(b_full + 8 * (i % SB), (i / SB) & 1, 2u); // nothing in flight at exit
   } else if (warp == MMA_WARP) {
-    // ---- MMA issuer: the whole warp runs the loop and one elected lane issues. Inside a branch on the lane number the compiler
-    // moves every MMA's descriptors from vector to uniform registers one after the other, which holds the thread for 96 cycles
-    // per MMA; converged, an MMA leaves every 40 (N <= 32), 48 (64), 64 (128) or 128 (256) cycles, the tensor core's own rate. ----
+    // ---- MMA issuer: the whole warp runs the loop and one elected lane issues. Everything that decides a loop's course or a
+    // descriptor is a function of launch parameters and counters (a wait that gave up only makes the rest of the loop idle), so
+    // that the compiler can keep the descriptors in uniform registers: moving them there from vector registers, one after the
+    // other, holds a thread for 96 cycles per MMA, while the tensor core takes one every 40 (N <= 32), 48 (64), 64 (128) or
+    // 128 (256) cycles. ----
     Cursor cur = start;
-    bool alive = true, a_ready = false, b_ready = false;
+    bool alive = true;
     int i = 0, s = 0, sb = 0;
     uint32_t round = 0, bround = 0;
-    for (int seg = 0; i < nsteps && alive; seg++) {
+    for (int seg = 0; i < nsteps; seg++) {
       const int len = min(KT - cur.kt, nsteps - i);
       const int buf = seg & 1, use = seg >> 1;
-      if (use > 0) alive = mbar_wait_uniform(acc_empty + 8 * buf, (use - 1) & 1, 4u); // the drain of this buffer's previous segment
-      if (!alive) break;
-      tc_fence_after();
-      const int64_t m0 = (int64_t)cur.tile_m * MAX_MT;
-      const uint32_t idesc = idesc_f16((int)min((int64_t)MAX_MT, p.m_pad - m0));
+      if (use > 0 && alive) alive = mbar_wait(acc_empty + 8 * buf, (use - 1) & 1, 4u); // the drain of this buffer's previous segment
+      const uint32_t idesc = idesc_f16(min(MAX_MT, (int)p.m_pad - cur.tile_m * MAX_MT));
       const uint32_t d = tmem_d + (uint32_t)(buf * MAX_MT);
-      for (int j = 0; j < len && alive; j++, i++) {
-        if (!a_ready) alive = mbar_wait_uniform(a_full + 8 * s, round & 1, 4u);
-        if (alive && !b_ready) alive = mbar_wait_uniform(b_full + 8 * sb, bround & 1, 4u);
-        if (!alive) break;
+      for (int j = 0; j < len; j++) {
+        if (alive) alive = mbar_wait(a_full + 8 * s, round & 1, 4u);
+        if (alive) alive = mbar_wait(b_full + 8 * sb, bround & 1, 4u);
         tc_fence_after();
+        __syncwarp();
         const uint64_t adesc = smem_desc_sw128(a_ring + s * A_STAGE_BYTES);
         const uint64_t bdesc = smem_desc_sw128(b_ring + sb * p.b_stride);
-        if (elect_one()) {
+        if (elect_one() && alive) {
 #pragma unroll
           for (int ks = 0; ks < BK / 16; ks++) umma_f16(d, adesc + (uint64_t)(ks * 2), bdesc + (uint64_t)(ks * 2), idesc, (j | ks) ? 1u : 0u);
           umma_commit(a_empty + 8 * s);
@@ -466,10 +465,8 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
           sb = 0;
           bround++;
         }
-        // probe the next step's barriers while this step's MMAs run
-        a_ready = i + 1 < nsteps && __all_sync(0xffffffffu, mbar_try_wait(a_full + 8 * s, round & 1));
-        b_ready = i + 1 < nsteps && __all_sync(0xffffffffu, mbar_try_wait(b_full + 8 * sb, bround & 1));
       }
+      i += len;
       cur.advance(len, KT, TM);
     }
   } else {
@@ -653,6 +650,7 @@ int launch_persistent_fmt(const PrefillArgs &a, unsigned ctas, size_t smem, cuda
   return XNQ_OK;
 }
 
+constexpr size_t SM_SMEM = 228 * 1024, MAX_SPREAD = 200 * 1024;
 static_assert(RowQ4_0::ROWB == RowQ4K::ROWB && RowQ8_0::ROWB == RowQ4K::ROWB, "the raw ring's plan assumes one slot size for these");
 constexpr size_t PREFILL_SMEM = 226 * 1024; // everything an SM offers minus the static barriers and a reserve
 
@@ -679,8 +677,12 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   const size_t cnt_bytes = tile_words(m_pad, w.n);
   uint8_t *xh = reinterpret_cast<uint8_t *>(tile_cnt) + cnt_bytes;
   const int act = act_dtype_for(w.dtype);
+  // The rows' CTAs are started while the previous kernel drains, and the first SM that is free would take eight of them (10 us for
+  // 32 rows instead of 3); unused shared memory keeps them apart: at most ceil(rows / SMs) to an SM.
+  const size_t spread = std::min<size_t>(MAX_SPREAD, (SM_SMEM / (size_t)((m_pad + g_num_sms - 1) / g_num_sms)) / 2048 * 1024);
+  // (each CTA also takes 1 KB of its own)
 #define XNQ_PREP(ACT, XT)                                                                                                   \
-  XNQ_CUDA(launch_pdl(prefill_prepare_acts<ACT, XT>, dim3((unsigned)m_pad), dim3(256), 0, s, static_cast<const XT *>(x), m, k, ldx, m_pad, ksteps, \
+  XNQ_CUDA(launch_pdl(prefill_prepare_acts<ACT, XT>, dim3((unsigned)m_pad), dim3(256), spread, s, static_cast<const XT *>(x), m, k, ldx, m_pad, ksteps, \
                       w.dtype, wscale, xh, row_unscale, tile_cnt, (int)(cnt_bytes / 4)))
   if (act == XNQ_Q8_0) {
     if (x_dtype == XNQ_F32) XNQ_PREP(XNQ_Q8_0, float);
@@ -752,6 +754,14 @@ int prefill_init(int device) {
   XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowQ8_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
   XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowQ4K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
   XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowQ6K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
+#define XNQ_PREP_INIT(ACT, XT) XNQ_CUDA(cudaFuncSetAttribute(prefill_prepare_acts<ACT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SPREAD))
+  XNQ_PREP_INIT(XNQ_Q8_0, float);
+  XNQ_PREP_INIT(XNQ_Q8_0, __half);
+  XNQ_PREP_INIT(XNQ_Q8_0, __nv_bfloat16);
+  XNQ_PREP_INIT(XNQ_Q8K, float);
+  XNQ_PREP_INIT(XNQ_Q8K, __half);
+  XNQ_PREP_INIT(XNQ_Q8K, __nv_bfloat16);
+#undef XNQ_PREP_INIT
   unsigned int zero = 0;
   XNQ_CUDA(cudaMemcpyToSymbol(g_prefill_status, &zero, sizeof(zero)));
   return XNQ_OK;
