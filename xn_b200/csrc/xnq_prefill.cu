@@ -3,9 +3,11 @@
 //
 //   D[128 weight rows, mt activation rows] += A[128, 64] . B[mt, 64]^T      per k-step of 64
 //
-//   A  weights of the tile, dequantized by sixteen producer warps from the quantized blocks straight into
-//      the 128-byte-swizzled K-major shared-memory image the MMA reads.
-//      Every weight is dequantized once per m-tile (mt up to 256 rows).
+//   A  weights of the tile, dequantized by sixteen producer warps from the quantized blocks into tensor
+//      memory, from where the MMA reads them (a lane is a weight row, a column two values). In shared
+//      memory, as they were before, they cost a write and a read of 16 KB per k-step, and with 256
+//      activation rows the shared memory's 128 bytes a cycle were what bounded the kernel (105 KB and
+//      850 cycles a k-step; now 73 KB). Every weight is dequantized once per m-tile (mt up to 256 rows).
 //   B  activations, prepared once per call by prefill_prepare_acts: quantized to Q8_0 / Q8_K exactly
 //      as the reference's quantize_lhs does (k_quants.rs:2015-2026), dequantized, scaled by a power of
 //      two per row and stored as fp16 in the same swizzled image, so that one 1-D bulk-async copy
@@ -24,9 +26,9 @@
 // so within a k-step the 64 elements are stored in the order the nibble unpack produces them
 // (xnq_prefill_rows.cuh) and the activation image uses the same order; no shuffles are needed.
 //
-// Synchronisation. Per stage: a_full (one arrival per producer warp of the stage), b_full (bulk-copy transaction bytes),
-// empty (tcgen05.commit by the MMA thread). Every wait is bounded; on expiry a status bit is set and
-// every role falls through to the common exit, where tensor memory is released.
+// Synchronisation. Per stage: full (one arrival per producer warp of the stage and one of the loader, whose
+// bulk copy adds its transaction bytes) and empty (tcgen05.commit by the MMA warp). Every wait is bounded; on
+// expiry a status bit is set and every role falls through to the common exit, where tensor memory is released.
 #include <algorithm>
 #include <cstring>
 
@@ -48,8 +50,9 @@ constexpr int PRODUCER_WARPS = 16; // four row groups of 32 rows x four warps
 constexpr int LOADER_WARP = PRODUCER_WARPS, MMA_WARP = LOADER_WARP + 1;
 constexpr int NTHREADS = PRODUCER_WARPS * 32 + 64; // warps 0-15 producers, then the loader warp and the MMA warp
 constexpr uint32_t WAIT_LIMIT = 1u << 26; // polls of a flag in global memory
-constexpr int A_STAGE_BYTES = TILE_N * BK * 2; // 16 KB
-// A stages. At least as many as a super-step has k-steps: step i then waits for the MMAs of a step of an EARLIER super-step, whose
+constexpr int A_COLS = BK / 2;     // tensor-memory columns of a stage's weights
+constexpr int A_COL0 = 256;        // they start behind the accumulators: one of 256 columns or two of 128
+// Stages. At least as many as a super-step has k-steps: step i then waits for the MMAs of a step of an EARLIER super-step, whose
 // producer (same row group) has already waited for the phase before; with fewer, a warp could test a barrier that is two phases
 // behind, which reads as complete.
 constexpr int MIN_STAGES = 4, MAX_STAGES = 8;
@@ -138,12 +141,13 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// A from tensor memory, B from shared memory
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // arrives on the mbarrier once every MMA issued so far by this thread has finished reading smem / writing tmem
@@ -162,6 +166,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
+      "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major, 128-byte-swizzled operand tile: rows of 128 bytes, 8-row groups 1024 bytes apart.
@@ -183,11 +195,11 @@ struct PrefillArgs {
   int64_t ldy;
   int64_t m, m_pad;
   int ksteps;
-  int nstages;            // A (weight) stages
-  int b_stages;           // B (activation) stages
+  int nstages;            // stages: weights in tensor memory, activations in shared memory
+  int acc_bufs;           // accumulators: 1 of 256 columns, 2 of 128 (tiles of up to 128 activation rows)
   int raw_slots;          // raw super-steps in shared memory, the one being converted included
   uint32_t b_stride;      // bytes between B stages (largest mt of the grid x 128, multiple of 1024)
-  uint32_t b_off, raw_off; // offsets of the B ring and of the raw ring from the aligned base
+  uint32_t raw_off;       // offset of the raw ring behind the B ring
   float wscale;           // power of two applied to every dequantized weight
   // persistent kernel: tile t = tile_n * tiles_m + tile_m; work unit u = t * ksteps + kt; CTA c takes units
   // [units * c / G, units * (c + 1) / G), or whole tiles when the output cannot be accumulated atomically
@@ -208,10 +220,6 @@ __device__ __forceinline__ void cp_async_wait(int pending) {
     case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
     default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
   }
-}
-
-__device__ __forceinline__ void zero_row(uint32_t dst_row, int sw, int c0, int n) { // chunks c0 .. c0 + n - 1
-  for (int c = c0; c < c0 + n; c++) sts128(dst_row + ((c ^ sw) << 4), 0, 0, 0, 0);
 }
 
 // Writes one 32-column chunk of an accumulator row block: column j of the chunk is activation row
@@ -244,8 +252,8 @@ __device__ __forceinline__ void drain_chunk(const uint32_t (&v)[32], float ru_la
 // together whatever the tile count, and a tile whose k-steps are split between CTAs is summed in
 // global memory: the first CTA to finish its part stores it and raises the tile's flag, the others add
 // theirs atomically after seeing the flag (two to three parts per split tile; f32 output only - other
-// output types get whole tiles). The accumulator is double-buffered in tensor memory (2 x 256 columns)
-// and drained by four dedicated warps, so the drain of one segment overlaps the MMAs of the next.
+// output types get whole tiles). Tiles of up to 128 activation rows have two accumulators, so the drain of one
+// segment overlaps the MMAs of the next; wider ones have one, and the producers fill the stages meanwhile.
 // Roles: 16 producer warps, one activation-loader warp (one bulk copy per stage), one MMA-issuing warp, eight drain
 // warps. Stage counters run on across segments.
 // Producers: the four warps of a row group (32 weight rows) fetch the group's bytes of a super-step together, several
@@ -276,15 +284,14 @@ template <typename RowT>
 __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(PrefillArgs p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  __shared__ __align__(8) uint64_t bars[4 * MAX_STAGES + 4]; // a_full, a_empty, b_full, b_empty (8 each), acc_full[2], acc_empty[2]
+  __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 4]; // full, empty (8 each), acc_full[2], acc_empty[2]
   __shared__ uint32_t tmem_slot;
   __shared__ unsigned int s_ticket;
   const int S = p.nstages;
-  const int SB = p.b_stages;
-  const uint32_t a_full = smem_u32(bars), a_empty = a_full + 64, b_full = a_full + 128, b_empty = a_full + 192, acc_full = a_full + 256,
-                 acc_empty = a_full + 272;
+  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, acc_full = empty + 8 * MAX_STAGES, acc_empty = acc_full + 16;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // so that the compiler knows `warp` to be uniform
-  const uint32_t a_ring = smem_base, b_ring = smem_base + p.b_off;
+  const uint32_t b_ring = smem_base;
+  const int NACC = p.acc_bufs;
   const int KT = p.ksteps;
 
   // this CTA's range of work units
@@ -303,12 +310,8 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
-      mbar_init(a_full + 8 * s, PRODUCER_WARPS / RowT::KPS);
-      mbar_init(a_empty + 8 * s, 1);
-    }
-    for (int s = 0; s < SB; s++) {
-      mbar_init(b_full + 8 * s, 1);
-      mbar_init(b_empty + 8 * s, 1);
+      mbar_init(full + 8 * s, PRODUCER_WARPS / RowT::KPS + 1);
+      mbar_init(empty + 8 * s, 1);
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(acc_full + 8 * b, 1);
@@ -317,7 +320,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == LOADER_WARP) {
-    tmem_alloc(smem_u32(&tmem_slot), 2 * MAX_MT);
+    tmem_alloc(smem_u32(&tmem_slot), 512);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     constexpr int KPS = RowT::KPS, NCOPY = (32 * RowT::ITEMS + 127) / 128;
     const int rg = warp & 3, kg = warp >> 2;
     const int kk = kg % KPS, hf = kg / KPS; // this warp's k-step of a super-step; which half of it (KPS = 2)
-    const int r = 32 * rg + lane, sw = r & 7;
+    const int r = 32 * rg + lane;
     const int t = kg * 32 + lane; // 0..127 in the row group
     const uint32_t raw = smem_base + p.raw_off + (uint32_t)(rg * 32 * RowT::ROWB);
     constexpr uint32_t SLOT = TILE_N * RowT::ROWB;
@@ -387,15 +390,25 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       const int kt = c_s * KPS + kk, i = base_i + kt;
       if (alive && kt < KT && i >= 0 && i < nsteps) {
         for (s += i - at, at = i; s >= S; lap ^= 1u) s -= S;
-        if (i >= S) alive = mbar_wait_uniform(a_empty + 8 * s, lap ^ 1u, 1u); // a warp that gave up still takes part in the barriers
+        if (i >= S) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 1u); // a warp that gave up still takes part in the barriers
         if (alive) {
-          const uint32_t dst_row = a_ring + s * A_STAGE_BYTES + r * 128;
+          tc_fence_after();
           const uint32_t slot = raw + (uint32_t)c_slot * SLOT + (uint32_t)(lane * RowT::ROWB);
-          if ((int64_t)c_n * TILE_N + r < p.w.n) RowT::store(slot, c_s, kk, hf, p.wscale, dst_row, sw);
-          else zero_row(dst_row, sw, KPS == 2 ? 4 * hf : 0, KPS == 2 ? 4 : 8);
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          const uint32_t dst = tmem_d + ((uint32_t)(32 * rg) << 16) + (uint32_t)(A_COL0 + s * A_COLS);
+          const bool in_w = (int64_t)c_n * TILE_N + r < p.w.n;
+#pragma unroll
+          for (int h = 0; h < KPS / 2; h++) {
+            const int half = KPS == 2 ? hf : h;
+            uint32_t o[16];
+            RowT::half(slot, c_s, kk, half, p.wscale, o);
+#pragma unroll
+            for (int e = 0; e < 16; e++) o[e] = in_w ? o[e] : 0u;
+            tmem_st16(dst + 16 * half, o);
+          }
+          tmem_st_wait();
+          tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(a_full + 8 * s);
+          if (lane == 0) mbar_arrive(full + 8 * s);
         }
       }
       if (++c_slot == R) c_slot = 0;
@@ -410,22 +423,22 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     // ---- activation loader: the whole warp runs the loop, one elected lane issues (see the MMA issuer) ----
     pdl_wait(); // the activation image is the previous kernel's output
     Cursor cur = start;
-    int sb = 0, issued = 0;
+    int s = 0, issued = 0;
     uint32_t lap = 0;
     for (int i = 0; i < nsteps; i++) {
-      if (i >= SB && !mbar_wait_uniform(b_empty + 8 * sb, lap ^ 1u, 2u)) break;
+      if (i >= S && !mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 2u)) break;
       const int64_t m0 = (int64_t)cur.tile_m * MAX_MT;
       const uint32_t bytes = (uint32_t)min((int64_t)MAX_MT, p.m_pad - m0) * 128;
       if (elect_one()) {
-        mbar_expect_tx(b_full + 8 * sb, bytes);
-        bulk_g2s(b_ring + sb * p.b_stride, p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128, bytes, b_full + 8 * sb);
+        mbar_expect_tx(full + 8 * s, bytes);
+        bulk_g2s(b_ring + s * p.b_stride, p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128, bytes, full + 8 * s);
       }
       __syncwarp();
       issued = i + 1;
       cur.advance(1, KT, TM);
-      if (++sb == SB) sb = 0, lap ^= 1u;
+      if (++s == S) s = 0, lap ^= 1u;
     }
-    for (int i = max(0, issued - SB); i < issued; i++) mbar_wait_uniform(b_full + 8 * (i % SB), (i / SB) & 1, 2u); // nothing in flight at exit
+    for (int i = max(0, issued - S); i < issued; i++) mbar_wait_uniform(full + 8 * (i % S), (i / S) & 1, 2u); // nothing in flight at exit
   } else if (warp == MMA_WARP) {
     // ---- MMA issuer: the whole warp runs the loop and one elected lane issues. Everything that decides a loop's course or a
     // descriptor is a function of launch parameters and counters (a wait that gave up only makes the rest of the loop idle), so
@@ -434,36 +447,30 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     // 128 (256) cycles. ----
     Cursor cur = start;
     bool alive = true;
-    int i = 0, s = 0, sb = 0;
-    uint32_t round = 0, bround = 0;
+    int i = 0, s = 0;
+    uint32_t round = 0;
     for (int seg = 0; i < nsteps; seg++) {
       const int len = min(KT - cur.kt, nsteps - i);
-      const int buf = seg & 1, use = seg >> 1;
+      const int buf = NACC == 2 ? seg & 1 : 0, use = NACC == 2 ? seg >> 1 : seg;
       if (use > 0 && alive) alive = mbar_wait(acc_empty + 8 * buf, (use - 1) & 1, 4u); // the drain of this buffer's previous segment
       const uint32_t idesc = idesc_f16(min(MAX_MT, (int)p.m_pad - cur.tile_m * MAX_MT));
-      const uint32_t d = tmem_d + (uint32_t)(buf * MAX_MT);
+      const uint32_t d = tmem_d + (uint32_t)(buf * 128);
       for (int j = 0; j < len; j++) {
-        if (alive) alive = mbar_wait(a_full + 8 * s, round & 1, 4u);
-        if (alive) alive = mbar_wait(b_full + 8 * sb, bround & 1, 4u);
+        if (alive) alive = mbar_wait(full + 8 * s, round & 1, 4u);
         tc_fence_after();
         __syncwarp();
-        const uint64_t adesc = smem_desc_sw128(a_ring + s * A_STAGE_BYTES);
-        const uint64_t bdesc = smem_desc_sw128(b_ring + sb * p.b_stride);
+        const uint32_t a = tmem_d + (uint32_t)(A_COL0 + s * A_COLS);
+        const uint64_t bdesc = smem_desc_sw128(b_ring + s * p.b_stride);
         if (elect_one() && alive) {
 #pragma unroll
-          for (int ks = 0; ks < BK / 16; ks++) umma_f16(d, adesc + (uint64_t)(ks * 2), bdesc + (uint64_t)(ks * 2), idesc, (j | ks) ? 1u : 0u);
-          umma_commit(a_empty + 8 * s);
-          umma_commit(b_empty + 8 * sb);
+          for (int ks = 0; ks < BK / 16; ks++) umma_f16(d, a + (uint32_t)(ks * 8), bdesc + (uint64_t)(ks * 2), idesc, (j | ks) ? 1u : 0u);
+          umma_commit(empty + 8 * s);
           if (j == len - 1) umma_commit(acc_full + 8 * buf);
         }
         __syncwarp();
         if (++s == S) {
           s = 0;
           round++;
-        }
-        if (++sb == SB) {
-          sb = 0;
-          bround++;
         }
       }
       i += len;
@@ -481,7 +488,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     for (int seg = 0; i < nsteps && alive; seg++) {
       const int len = min(KT - cur.kt, nsteps - i);
       const bool whole = cur.kt == 0 && len == KT;
-      const int buf = seg & 1, use = seg >> 1;
+      const int buf = NACC == 2 ? seg & 1 : 0, use = NACC == 2 ? seg >> 1 : seg;
       const int tile_n = cur.tile_n, tile_m = cur.tile_m, tile = cur.tile(TM);
       const int64_t row = (int64_t)tile_n * TILE_N + 32 * q + lane;
       const int64_t m0 = (int64_t)tile_m * MAX_MT;
@@ -513,7 +520,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); // s_ticket may be rewritten from here on
       if (alive) {
         tc_fence_after();
-        const uint32_t lane_addr = tmem_d + (uint32_t)(buf * MAX_MT) + ((uint32_t)(32 * q) << 16);
+        const uint32_t lane_addr = tmem_d + (uint32_t)(buf * 128) + ((uint32_t)(32 * q) << 16);
         for (int c0 = 32 * half; c0 < mt; c0 += 32 * (EPI_WARPS / 4)) {
           uint32_t v[32];
           tmem_ld32(lane_addr + c0, v);
@@ -548,7 +555,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
 
   tc_fence_before();
   __syncthreads();
-  if (warp == LOADER_WARP) tmem_dealloc(tmem_d, 2 * MAX_MT);
+  if (warp == LOADER_WARP) tmem_dealloc(tmem_d, 512);
 }
 
 // ---- activation image -----------------------------------------------------------------------------------
@@ -706,23 +713,18 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   a.m = m;
   a.m_pad = m_pad;
   a.ksteps = ksteps;
-  // Shared-memory plan: A ring | B ring | raw ring. At 256 activation rows there is room for four weight and three activation stages
-  // beside two or three raw slots; narrower tiles take up to eight of each, so that a producer warp can be a whole super-step ahead of
-  // the MMAs, and what is left goes to the raw ring (it covers the memory latency of the weights).
+  // Shared-memory plan: B ring | raw ring. With up to eight stages a producer warp can be a whole super-step ahead of the MMAs; what is
+  // left goes to the raw ring (it covers the memory latency of the weights). At 256 activation rows that is five stages and three
+  // raw slots (two for Q6_K).
   const uint32_t slot = TILE_N * (w.dtype == XNQ_Q6K ? RowQ6K::ROWB : RowQ4K::ROWB);
   const uint32_t mt_max = (uint32_t)std::min<int64_t>(MAX_MT, m_pad);
   a.b_stride = (mt_max * 128 + 1023) & ~1023u;
   const size_t budget = PREFILL_SMEM - 1024; // alignment slack
-  a.nstages = MIN_STAGES, a.b_stages = 3;
-  for (int st = MAX_STAGES; st >= MIN_STAGES; st--)
-    if ((size_t)st * (A_STAGE_BYTES + a.b_stride) + 3 * slot <= budget) {
-      a.nstages = a.b_stages = st;
-      break;
-    }
-  if ((size_t)a.nstages * A_STAGE_BYTES + (size_t)a.b_stages * a.b_stride + 2 * slot > budget) return fail(XNQ_ERR_SIZE, "prefill: shared-memory plan does not fit");
-  a.raw_slots = (int)std::min<size_t>(MAX_RAW_SLOTS, (budget - (size_t)a.nstages * A_STAGE_BYTES - (size_t)a.b_stages * a.b_stride) / slot);
-  a.b_off = a.nstages * A_STAGE_BYTES;
-  a.raw_off = a.b_off + a.b_stages * a.b_stride;
+  a.nstages = (int)std::min<size_t>(MAX_STAGES, (budget - 2 * slot) / a.b_stride);
+  if (a.nstages < MIN_STAGES) return fail(XNQ_ERR_SIZE, "prefill: shared-memory plan does not fit");
+  a.raw_slots = (int)std::min<size_t>(MAX_RAW_SLOTS, (budget - (size_t)a.nstages * a.b_stride) / slot);
+  a.raw_off = a.nstages * a.b_stride;
+  a.acc_bufs = m_pad <= 128 ? 2 : 1;
   a.wscale = wscale;
   const dim3 grid((unsigned)((w.n + TILE_N - 1) / TILE_N), (unsigned)((m_pad + MAX_MT - 1) / MAX_MT));
   a.tiles_n = (int)grid.x;

@@ -6,8 +6,8 @@
 //   item()   one of the ITEMS 16-byte copies that make up a row's super-step: where it comes from and how that moves with the
 //            super-step. Consecutive threads take consecutive copies, so that a copy instruction of a warp touches four to six runs
 //            of memory (one thread per row would touch 32).
-//   store()  reads the row's bytes of one 64-wide k-step (or of half of it) from the slot, dequantizes to fp16 and writes the
-//            swizzled 16-byte chunks of the row into the A stage the tensor core reads.
+//   half()   reads the row's bytes of half a 64-wide k-step from the slot and dequantizes them to fp16: the 16 packed pairs that go
+//            to the row's lane of tensor memory, where the MMA reads its weight operand.
 //
 // Stored k order inside a k-step (the activation image uses the same one, see kpair_shift in xnq_prefill.cu):
 //   Q8_0, Q6_K  natural
@@ -35,9 +35,6 @@ __device__ __forceinline__ uint32_t lds32(uint32_t a) {
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
 }
-__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 // 0x6400 is 1024.0 in fp16 and its ulp is 1: OR-ing an integer 0..1023 into the low bits gives 1024 + i exactly.
 __device__ __forceinline__ __half2 h2_from_bits(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
 __device__ __forceinline__ uint32_t bits_from_h2(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
@@ -53,8 +50,7 @@ struct Item {
 };
 constexpr uint32_t NO_LIMIT = 0xffffffffu;
 
-// KPS k-steps per super-step. KPS = 4: one thread converts a row's whole k-step; KPS = 2: two threads, half hf (32 elements) each.
-// All shared-memory reads of a call are issued before any arithmetic.
+// KPS k-steps per super-step ss. KPS = 4: one thread converts both halves of a row's k-step kk; KPS = 2: two threads, a half each.
 
 struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
   static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
@@ -62,25 +58,17 @@ struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
     if (c < 8) return Item{w.qs + row * (w.k / 2) + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k / 2 - 16 * c)};
     return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 16u, NO_LIMIT};
   }
-  __device__ static __forceinline__ void store(uint32_t slot, int, int kk, int, float wscale, uint32_t dst_row, int sw) {
-    const uint4 q[2] = {lds128(slot + 32 * kk), lds128(slot + 32 * kk + 16)};
+  __device__ static __forceinline__ void half(uint32_t slot, int, int kk, int hf, float wscale, uint32_t (&o)[16]) { // half = one block
+    const uint4 q = lds128(slot + 32 * kk + 16 * hf);
     const uint32_t dd = lds32(slot + 128 + 4 * kk);
     const __half2 off = h2_from_bits(0x64086408u); // 1032 = 1024 + 8
+    const __half2 d2 = scaled_half2(hf ? (dd >> 16) : (dd & 0xffffu), wscale);
+    const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
-      const __half2 d2 = scaled_half2(b ? (dd >> 16) : (dd & 0xffffu), wscale);
-      const uint32_t wd[4] = {q[b].x, q[b].y, q[b].z, q[b].w};
+    for (int wi = 0; wi < 4; wi++)
 #pragma unroll
-      for (int wi = 0; wi < 4; wi++) {
-        uint32_t o[4];
-#pragma unroll
-        for (int p = 0; p < 4; p++) { // nibble pairs (p, p+4) of the word
-          const __half2 v = h2_from_bits(((wd[wi] >> (4 * p)) & 0x000f000fu) | 0x64006400u);
-          o[p] = bits_from_h2(__hmul2(__hsub2(v, off), d2));
-        }
-        sts128(dst_row + (((b * 4 + wi) ^ sw) << 4), o[0], o[1], o[2], o[3]);
-      }
-    }
+      for (int p = 0; p < 4; p++) // nibble pairs (p, p+4) of the word
+        o[4 * wi + p] = bits_from_h2(__hmul2(__hsub2(h2_from_bits(((wd[wi] >> (4 * p)) & 0x000f000fu) | 0x64006400u), off), d2));
   }
 };
 
@@ -90,7 +78,7 @@ struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighb
     if (c < 8) return Item{w.qs + row * w.k + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k - 16 * c)};
     return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 8u, NO_LIMIT};
   }
-  __device__ static __forceinline__ void store(uint32_t slot, int ss, int kk, int hf, float wscale, uint32_t dst_row, int sw) { // half = one block
+  __device__ static __forceinline__ void half(uint32_t slot, int ss, int kk, int hf, float wscale, uint32_t (&o)[16]) { // half = one block
     const uint4 q[2] = {lds128(slot + 64 * kk + 32 * hf), lds128(slot + 64 * kk + 32 * hf + 16)};
     const uint32_t dd = lds32(slot + 128 + 8 * (ss & 1) + 4 * kk);
     const __half2 d2 = scaled_half2(hf ? (dd >> 16) : (dd & 0xffffu), wscale);
@@ -98,15 +86,13 @@ struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighb
 #pragma unroll
     for (int c = 0; c < 4; c++) { // chunk = 8 codes
       const uint32_t ww[2] = {((c & 1) ? q[c >> 1].z : q[c >> 1].x) ^ 0x80808080u, ((c & 1) ? q[c >> 1].w : q[c >> 1].y) ^ 0x80808080u};
-      uint32_t o[4];
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const __half2 lo = h2_from_bits(__byte_perm(ww[j], 0x64646464u, 0x4140)); // bytes 0,1 -> 1024 + (b + 128)
         const __half2 hi = h2_from_bits(__byte_perm(ww[j], 0x64646464u, 0x4342)); // bytes 2,3
-        o[2 * j] = bits_from_h2(__hmul2(__hsub2(lo, off), d2));
-        o[2 * j + 1] = bits_from_h2(__hmul2(__hsub2(hi, off), d2));
+        o[4 * c + 2 * j] = bits_from_h2(__hmul2(__hsub2(lo, off), d2));
+        o[4 * c + 2 * j + 1] = bits_from_h2(__hmul2(__hsub2(hi, off), d2));
       }
-      sts128(dst_row + (((hf * 4 + c) ^ sw) << 4), o[0], o[1], o[2], o[3]);
     }
   }
 };
@@ -114,8 +100,8 @@ struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighb
 struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
   static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
   __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { return Item{w.qs + row * (w.k / QK_K) * 144 + 16 * c, 144u, NO_LIMIT}; }
-  __device__ static __forceinline__ void store(uint32_t slot, int, int g, int, float wscale, uint32_t dst_row, int sw) {
-    const uint4 hdr = lds128(slot), q[2] = {lds128(slot + 16 + 32 * g), lds128(slot + 32 + 32 * g)};
+  __device__ static __forceinline__ void half(uint32_t slot, int, int g, int hf, float wscale, uint32_t (&o)[16]) { // half = words 4 hf .. of the group
+    const uint4 hdr = lds128(slot), q = lds128(slot + 16 + 32 * g + 16 * hf);
     const __half2 dm = *reinterpret_cast<const __half2 *>(&hdr.x);
     const uint32_t f = k4_field(hdr.y, hdr.z, hdr.w, g);
     const float d = __low2float(dm) * wscale, mn = __high2float(dm) * wscale;
@@ -123,18 +109,14 @@ struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
     const __half2 a_lo = __float2half2_rn(d * (float)(f & 63)), a_hi = __float2half2_rn(d * (float)((f >> 6) & 63));
     const __half2 b_lo = __float2half2_rn(-mn * (float)((f >> 12) & 63)), b_hi = __float2half2_rn(-mn * (float)(f >> 18));
     const __half2 k1024 = h2_from_bits(0x64006400u);
+    const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int wi = 0; wi < 8; wi++) {
-      const uint4 &v = q[wi >> 2];
-      const uint32_t wd = (wi & 3) == 0 ? v.x : ((wi & 3) == 1 ? v.y : ((wi & 3) == 2 ? v.z : v.w));
-      uint32_t o[4];
+    for (int wi = 0; wi < 4; wi++)
 #pragma unroll
       for (int p = 0; p < 4; p++) { // pairs: p=0 (l, l+2) low, p=1 (32+l, 32+l+2) high, p=2 (l+1, l+3) low, p=3 high
-        const __half2 c = __hsub2(h2_from_bits(((wd >> (4 * p)) & 0x000f000fu) | 0x64006400u), k1024);
-        o[p] = bits_from_h2((p & 1) ? __hfma2(c, a_hi, b_hi) : __hfma2(c, a_lo, b_lo));
+        const __half2 c = __hsub2(h2_from_bits(((wd[wi] >> (4 * p)) & 0x000f000fu) | 0x64006400u), k1024);
+        o[4 * wi + p] = bits_from_h2((p & 1) ? __hfma2(c, a_hi, b_hi) : __hfma2(c, a_lo, b_lo));
       }
-      sts128(dst_row + ((wi ^ sw) << 4), o[0], o[1], o[2], o[3]);
-    }
   }
 };
 
@@ -148,32 +130,27 @@ struct RowQ6K { // 128 ql bytes | 64 qh bytes | 16 scales | the f16 d of eight s
     return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 2u, NO_LIMIT};
   }
   // k-step kk = 2 h + hi_pair of the super-block: group 0 takes ql[l] of half h, group 1 ql[l + 32], both the low (hi_pair 0) or high nibbles
-  __device__ static __forceinline__ void store(uint32_t slot, int ss, int kk, int, float wscale, uint32_t dst_row, int sw) {
+  __device__ static __forceinline__ void half(uint32_t slot, int ss, int kk, int hf, float wscale, uint32_t (&o)[16]) {
     const int h = kk >> 1, sh = 4 * (kk & 1);
     const uint4 qh[2] = {lds128(slot + 128 + 32 * h), lds128(slot + 144 + 32 * h)};
+    const uint4 ql[2] = {lds128(slot + 64 * h + 32 * hf), lds128(slot + 64 * h + 32 * hf + 16)};
     const uint32_t sc4 = lds32(slot + 192 + 8 * h + 4 * (kk & 1)), dd = lds32(slot + 208 + 4 * ((ss >> 1) & 3));
     const float d = __half2float(__ushort_as_half((unsigned short)((ss & 1) ? (dd >> 16) : (dd & 0xffffu)))) * wscale;
     const __half2 off = h2_from_bits(0x64206420u); // 1056 = 1024 + 32
+    const int hsh = sh + 2 * hf; // bit position of this group's two high bits inside a qh byte
 #pragma unroll
-    for (int hf = 0; hf < 2; hf++) {
-      const uint4 ql[2] = {lds128(slot + 64 * h + 32 * hf), lds128(slot + 64 * h + 32 * hf + 16)};
-      const int hsh = sh + 2 * hf; // bit position of this group's two high bits inside a qh byte
+    for (int c = 0; c < 4; c++) { // chunk of 8 elements l = 8c .. 8c+7
+      const uint32_t lw[2] = {(c & 1) ? ql[c >> 1].z : ql[c >> 1].x, (c & 1) ? ql[c >> 1].w : ql[c >> 1].y};
+      const uint32_t hw[2] = {(c & 1) ? qh[c >> 1].z : qh[c >> 1].x, (c & 1) ? qh[c >> 1].w : qh[c >> 1].y};
+      const int8_t sc = (int8_t)((sc4 >> (8 * (2 * hf + (c >> 1)))) & 0xff);
+      const __half2 s2 = __float2half2_rn(d * (float)sc);
 #pragma unroll
-      for (int c = 0; c < 4; c++) { // chunk of 8 elements l = 8c .. 8c+7
-        const uint32_t lw[2] = {(c & 1) ? ql[c >> 1].z : ql[c >> 1].x, (c & 1) ? ql[c >> 1].w : ql[c >> 1].y};
-        const uint32_t hw[2] = {(c & 1) ? qh[c >> 1].z : qh[c >> 1].x, (c & 1) ? qh[c >> 1].w : qh[c >> 1].y};
-        const int8_t sc = (int8_t)((sc4 >> (8 * (2 * hf + (c >> 1)))) & 0xff);
-        const __half2 s2 = __float2half2_rn(d * (float)sc);
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-          const uint32_t code = ((lw[j] >> sh) & 0x0f0f0f0fu) | (((hw[j] >> hsh) << 4) & 0x30303030u);
-          const __half2 lo = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4140));
-          const __half2 hi = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4342));
-          o[2 * j] = bits_from_h2(__hmul2(__hsub2(lo, off), s2));
-          o[2 * j + 1] = bits_from_h2(__hmul2(__hsub2(hi, off), s2));
-        }
-        sts128(dst_row + (((hf * 4 + c) ^ sw) << 4), o[0], o[1], o[2], o[3]);
+      for (int j = 0; j < 2; j++) {
+        const uint32_t code = ((lw[j] >> sh) & 0x0f0f0f0fu) | (((hw[j] >> hsh) << 4) & 0x30303030u);
+        const __half2 lo = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4140));
+        const __half2 hi = h2_from_bits(__byte_perm(code, 0x64646464u, 0x4342));
+        o[4 * c + 2 * j] = bits_from_h2(__hmul2(__hsub2(lo, off), s2));
+        o[4 * c + 2 * j + 1] = bits_from_h2(__hmul2(__hsub2(hi, off), s2));
       }
     }
   }
