@@ -54,22 +54,6 @@
 namespace xnq {
 
 __device__ unsigned int g_imma_status; // sticky: 1 producer, 2 converter, 4 mma, 8 drain wait expired
-#ifdef XNQ_DEV_TRACE
-__device__ long long g_imma_trace[32]; // development builds only: cycles block 0's roles spend in each wait
-__device__ long long g_imma_tl[8 * 64];  // development builds only: block 0's per-unit time line (clock64), 8 points x 64 units
-#define XNQ_TL(pt, i) do { if (blockIdx.x == 0 && (i) < 64) g_imma_tl[(pt) * 64 + (i)] = clock64(); } while (0)
-#define XNQ_GT(i) do { if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) { unsigned long long g_; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g_)); g_imma_trace[i] = (long long)g_; } } while (0)
-#define XNQ_TACC(i) do { const long long t1_ = clock64(); tacc[i] += t1_ - t0_; t0_ = t1_; } while (0)
-#define XNQ_TDECL long long tacc[6] = {0, 0, 0, 0, 0, 0}; long long t0_ = clock64()
-#define XNQ_TDUMP(base, cond) do { if ((cond) && blockIdx.x == 0) for (int i_ = 0; i_ < 6; i_++) g_imma_trace[(base) + i_] = tacc[i_]; } while (0)
-#else
-#define XNQ_GT(i) do { } while (0)
-#define XNQ_TL(pt, i) do { } while (0)
-#define XNQ_TACC(i) do { } while (0)
-#define XNQ_TDECL do { } while (0)
-#define XNQ_TDUMP(base, cond) do { } while (0)
-#endif
-
 namespace {
 
 constexpr int TILE_N = 128;         // weight rows per tile = UMMA M
@@ -78,11 +62,11 @@ constexpr int CONV_WARPS = 8, DRAIN_WARPS = 16;
 constexpr int ACT_PRODUCER_WARP = 0, MMA_WARP = 1, CONV_WARP0 = 3, DRAIN_WARP0 = CONV_WARP0 + CONV_WARPS; // MMA issuers: warps 1 and 2
 constexpr int NTHREADS = (DRAIN_WARP0 + DRAIN_WARPS) * 32; // 864
 constexpr int A_STAGE_BYTES = TILE_N * 128; // one 128-k half step of int8 codes
-constexpr int MAX_A_STAGES = 8, SIDE_STAGES = 8, MAX_RAW_STAGES = 8; // side stages are small (scale bytes and records of one step): enough of them that
+constexpr int SIDE_STAGES = 8, MAX_RAW_STAGES = 8, MAX_B_STAGES = 8; // side stages are small (scale bytes and records of one step): enough of them that
                                                                    // the converters, which fill them, never wait for the drain, which frees them
 constexpr int HDR_BYTES = TILE_N * 16;      // per 256-k step: 16 bytes of scale data per weight row
 constexpr int TMEM_COLS = 512;              // all of the SM's tensor memory: 512 / (4 slices x NP) accumulator buffers, at most 8
-constexpr size_t IMMA_SMEM = 226 * 1024;
+constexpr size_t IMMA_SMEM = 226 * 1024, MAX_SPREAD = 120 * 1024;
 constexpr uint32_t PF_CHUNK = 16384;              // bytes per L2 prefetch request
 constexpr size_t PF_MAX_BYTES = 80ull << 20;      // larger weights are not prefetched whole: they would push each other out of L2
 
@@ -146,13 +130,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
   atomicOr(&g_imma_status, bit);
   return false;
 }
-// bounded wait of a whole warp: lane 0 polls (32 lanes polling one word keep the shared-memory pipe busy for
-// nothing), the other lanes park on the warp barrier
+// bounded wait of a whole warp (one instruction per attempt for all lanes); the result is the same in all lanes
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, unsigned int bit) {
-  int ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, bit) ? 1 : 0;
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+  const bool ok = mbar_wait(bar, parity, bit);
+  return __all_sync(0xffffffffu, ok);
+}
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e != 0;
 }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
@@ -338,47 +329,46 @@ struct ConvQ4K { // 128 code bytes per row and step: four 32-byte chunks; chunk 
   }
 };
 
-// ---- drain: scale the four slices of a half step and add them to the running sums ----------------------------
+// ---- drain: scale the eight slices of a step and add them to the running sums --------------------------------
 // hdr: the row's 16 scale bytes of the 256-k step; meta: shared address of the step's per-activation-row records
-// (32 bytes each); v[j][c]: slice j (block 4h + j of the step), column c of this thread; c0: first column.
+// (32 bytes each); v[j][c]: slice j (block j of the step), column c of this thread; c0: first column.
 //   Q4_0 / Q8_0  hdr = eight f16 block scales; record = eight f32 activation block scales
 //   Q4_K         hdr = f16 d, f16 dmin, four 24-bit fields sc[2g] | sc[2g+1] << 6 | mn[2g] << 12 | mn[2g+1] << 18;
-//                record = {lo(h=0), hi(h=0), lo(h=1), hi(h=1), f32 d, 0, 0, 0}: the four sub-blocks' 32-sums of the
-//                activation codes, s = 128 * hi + lo with lo in 0..127 (one byte each)
+//                record = {lo(h=0), hi(h=0), lo(h=1), hi(h=1), f32 d, 0, 0, 0}: the 32-sums of the activation codes of
+//                each half's four sub-blocks, s = 128 * hi + lo with lo in 0..127 (one byte each)
 template <int CH>
 struct DrainBlockScaled {
-  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int h, int c0, const uint32_t (&v)[4][CH], float *acc) {
-    const uint32_t w0 = h ? hdr.z : hdr.x, w1 = h ? hdr.w : hdr.y;
-    const __half2 h0 = *reinterpret_cast<const __half2 *>(&w0), h1 = *reinterpret_cast<const __half2 *>(&w1);
-    const float dw[4] = {__low2float(h0), __high2float(h0), __low2float(h1), __high2float(h1)};
+  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int c0, const uint32_t (&v)[8][CH], float *acc) {
+    const uint32_t w[4] = {hdr.x, hdr.y, hdr.z, hdr.w};
 #pragma unroll
     for (int c = 0; c < CH; c++) {
-      const uint4 da = lds128(meta + (uint32_t)(c0 + c) * 32 + 16 * h);
-      acc[c] += (float)(int)v[0][c] * (dw[0] * __uint_as_float(da.x));
-      acc[c] += (float)(int)v[1][c] * (dw[1] * __uint_as_float(da.y));
-      acc[c] += (float)(int)v[2][c] * (dw[2] * __uint_as_float(da.z));
-      acc[c] += (float)(int)v[3][c] * (dw[3] * __uint_as_float(da.w));
+      const uint4 a = lds128(meta + (uint32_t)(c0 + c) * 32), b = lds128(meta + (uint32_t)(c0 + c) * 32 + 16);
+      const uint32_t da[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const __half2 h = *reinterpret_cast<const __half2 *>(&w[j >> 1]);
+        acc[c] += (float)(int)v[j][c] * (((j & 1) ? __high2float(h) : __low2float(h)) * __uint_as_float(da[j]));
+      }
     }
   }
 };
 template <int CH>
-struct DrainQ4K {
-  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int h, int c0, const uint32_t (&v)[4][CH], float *acc) {
+struct DrainQ4K { // integer sums over the whole super-block, scaled once, as the CPU code does
+  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int c0, const uint32_t (&v)[8][CH], float *acc) {
     const __half2 dm = *reinterpret_cast<const __half2 *>(&hdr.x);
     const float d = __low2float(dm), dmin = __high2float(dm);
-    // fields 2h and 2h + 1: bits [48h, 48h + 48) of the 96-bit field array in hdr.y, hdr.z, hdr.w
-    const uint32_t lo32 = h ? __funnelshift_r(hdr.z, hdr.w, 16) : hdr.y;
-    const uint32_t hi16 = h ? (hdr.w >> 16) : (hdr.z & 0xffffu);
-    const uint32_t f0 = lo32 & 0xffffffu, f1 = __funnelshift_r(lo32, hi16, 24) & 0xffffffu;
-    const int sc0 = f0 & 63, sc1 = (f0 >> 6) & 63, sc2 = f1 & 63, sc3 = (f1 >> 6) & 63;
-    const uint32_t mins = ((f0 >> 12) & 63) | (((f0 >> 18) & 63) << 8) | (((f1 >> 12) & 63) << 16) | (((f1 >> 18) & 63) << 24);
+    const uint32_t F[4] = {hdr.y & 0xffffffu, __funnelshift_r(hdr.y, hdr.z, 24) & 0xffffffu, __funnelshift_r(hdr.z, hdr.w, 16) & 0xffffffu, hdr.w >> 8};
+    const uint32_t mins0 = ((F[0] >> 12) & 63u) | (((F[0] >> 18) & 63u) << 8) | (((F[1] >> 12) & 63u) << 16) | (((F[1] >> 18) & 63u) << 24);
+    const uint32_t mins1 = ((F[2] >> 12) & 63u) | (((F[2] >> 18) & 63u) << 8) | (((F[3] >> 12) & 63u) << 16) | (((F[3] >> 18) & 63u) << 24);
 #pragma unroll
     for (int c = 0; c < CH; c++) {
       const uint32_t rec = meta + (uint32_t)(c0 + c) * 32;
-      const uint2 bs = lds64(rec + 8 * h);
+      const uint4 bs = lds128(rec);
       const float da = __uint_as_float(lds32(rec + 16));
-      const int isum = sc0 * (int)v[0][c] + sc1 * (int)v[1][c] + sc2 * (int)v[2][c] + sc3 * (int)v[3][c];
-      const int msum = dp4a_uu(mins, bs.x, 0) + dp4a_us(mins, bs.y, 0) * 128;
+      int isum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; j++) isum += (int)((F[j >> 1] >> (6 * (j & 1))) & 63u) * (int)v[j][c];
+      const int msum = dp4a_uu(mins0, bs.x, dp4a_uu(mins1, bs.z, 0)) + 128 * dp4a_us(mins0, bs.y, dp4a_us(mins1, bs.w, 0));
       acc[c] += da * (d * (float)isum - dmin * (float)msum);
     }
   }
@@ -386,25 +376,20 @@ struct DrainQ4K {
 
 template <typename Conv, template <int> class Drain, int NP>
 __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant__ ImmaArgs p) {
-  // Drain warps per half-step group: eight, two per accumulator lane quarter, splitting the columns. (Four per group with 16
-  // activation rows, which halves the fixed cost per step, was no faster: each warp's chain of loads from tensor memory and
-  // arithmetic per half step then takes longer than the MMAs of a step.)
-  constexpr int DWG = 8;
-  constexpr int NPT = NP / (DWG / 4); // columns per drain thread
-  constexpr int CH = NPT > 16 ? 4 : (NPT > 8 ? 8 : NPT); // columns read back at a time: what the register budget holds next to the sums
+  constexpr int NPT = NP / (DRAIN_WARPS / 4); // columns per drain thread: four warps per accumulator lane quarter split them
+  constexpr int CH = 4;                       // columns read back at a time, all eight slices of a step: what the register budget holds
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand stages need 1024-byte alignment
-  constexpr int NBUF = TMEM_COLS / (4 * NP) > 8 ? 8 : TMEM_COLS / (4 * NP); // accumulator buffers (even: buffer parity = half step parity)
+  constexpr int NBUF = TMEM_COLS / (8 * NP) > 4 ? 8 : TMEM_COLS / (8 * NP) * 2; // accumulator buffers (even: buffer parity = half step parity)
   constexpr int BUF_COLS = 4 * NP;
-  // barriers: b_full [4], side_full/side_empty [8], a_full/mma_done [8], acc_empty [8]
-  __shared__ __align__(8) uint64_t bars[44];
+  // barriers: b_full/b_empty [8], side_full/side_empty [8], a_full/mma_done [8], acc_empty [8]
+  __shared__ __align__(8) uint64_t bars[56];
   __shared__ uint32_t tmem_slot;
   __shared__ unsigned int s_ticket;
-  const uint32_t b_full = smem_u32(bars), side_full = b_full + 32, side_empty = b_full + 96, a_full = b_full + 160, mma_done = b_full + 224,
-                 acc_empty = b_full + 288;
-  XNQ_GT(26);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int RS = p.raw_stages, BS = p.b_stages, AS = p.a_stages;
+  const uint32_t b_full = smem_u32(bars), b_empty = b_full + 64, side_full = b_full + 128, side_empty = b_full + 192, a_full = b_full + 256,
+                 mma_done = b_full + 320, acc_empty = b_full + 384;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // so that the compiler knows `warp` to be uniform
+  const int RS = p.raw_stages, BS = p.b_stages, AS = p.a_stages, AP = AS / 2; // AP: operand stages in whole steps
   const int NB = min(NBUF, AS); // accumulator buffers in use: a drain group waiting on mma_done must not be lapped by the MMA thread,
                                 // which can run ahead by NB half steps, so the ring of mma_done barriers (AS) is at least that long
   const int KT = p.nsteps;
@@ -414,13 +399,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 8; s++) {
-      mbar_init(a_full + 8 * s, CONV_WARPS / 2); // the four converter warps of the step's group (one barrier per step: entries 0 .. BS - 1)
+      mbar_init(a_full + 8 * s, CONV_WARPS / 2); // the four converter warps of the step's group (one barrier per step: entries 0 .. AP - 1)
       mbar_init(mma_done + 8 * s, 1);            // the half step's MMAs have read their operands and written their slices
-      mbar_init(acc_empty + 8 * s, DWG);
+      mbar_init(acc_empty + 8 * s, DRAIN_WARPS);
       mbar_init(side_full + 8 * s, 1 + CONV_WARPS / 2); // the producer's transaction + the four converter warps that copy the scale bytes
-      mbar_init(side_empty + 8 * s, 2 * DWG);
+      mbar_init(side_empty + 8 * s, DRAIN_WARPS);
+      mbar_init(b_full + 8 * s, 1);
+      mbar_init(b_empty + 8 * s, 2); // both half steps' MMAs
     }
-    for (int s = 0; s < 4; s++) mbar_init(b_full + 8 * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == MMA_WARP) { // one warp owns the tensor-memory allocation
@@ -431,81 +417,71 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
   __syncthreads();
   tc_fence_after();
   pdl_launch_dependents(); // the next kernel in the stream may be set up while this one runs
-  const uint32_t tmem_d = tmem_slot;
+  const uint32_t tmem_d = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
   if (warp == ACT_PRODUCER_WARP) {
-    // ---- activation producer: per 256-k step the activations' operand image and their records ----
-    if (lane == 0) {
-      // A 256-k step of a tile is 128 separate runs of 144 to 256 bytes, 2 to 4 KB apart. So that DRAM is read in long
-      // contiguous runs all the same, the weight is asked into L2 whole when the kernel starts, every CTA asking for its
-      // share of the bytes (not of the work: any CTA's copies then hit in L2, or go to DRAM when they are early).
+    // ---- activation producer: per 256-k step the activations' operand image and their records. The whole warp runs the loop and
+    // one elected lane issues (see the MMA issuers). ----
+    // A 256-k step of a tile is 128 separate runs of 144 to 256 bytes, 2 to 4 KB apart. So that DRAM is read in long
+    // contiguous runs all the same, the weight is asked into L2 whole when the kernel starts, every CTA asking for its
+    // share of the bytes (not of the work: any CTA's copies then hit in L2, or go to DRAM when they are early).
+    if (elect_one()) {
       for (int st = 0; st < p.nstreams; st++) {
         const unsigned long long o0 = p.pf_share[st] * blockIdx.x, o1 = min(o0 + p.pf_share[st], p.pf_bytes[st]);
         for (unsigned long long o = o0; o < o1; o += PF_CHUNK) bulk_prefetch_l2(p.pf_base[st] + o, (uint32_t)min((unsigned long long)PF_CHUNK, o1 - o));
       }
-      pdl_wait();
-      bool alive = true;
-      int kt = kt0, bs = 0;
-      uint32_t b_ph = 0; // (i / BS) & 1
-      for (int i = 0; i < nunits && alive; i++) {
-        const int ss = i % SIDE_STAGES;
-        // the B stage of step i - BS is free once that step's second half has been multiplied: BS = AS / 2, so this is
-        // the barrier of half step 2 i + 1 one phase back (a second commit per step cost the issuing thread over a
-        // thousand cycles)
-        if (i >= BS) alive = mbar_wait(mma_done + 8 * (2 * bs), b_ph ^ 1u, 1u) && mbar_wait(mma_done + 8 * (2 * bs + 1), b_ph ^ 1u, 1u);
-        if (alive && i >= SIDE_STAGES) alive = mbar_wait(side_empty + 8 * ss, ((i / SIDE_STAGES) - 1) & 1, 1u);
-        if (!alive) break;
+    }
+    __syncwarp();
+    pdl_wait();
+    bool alive = true;
+    int kt = kt0, bs = 0;
+    uint32_t b_ph = 0; // (i / BS) & 1
+    for (int i = 0; i < nunits; i++) {
+      const int ss = i % SIDE_STAGES;
+      if (alive && i >= BS) alive = mbar_wait(b_empty + 8 * bs, b_ph ^ 1u, 1u);
+      if (alive && i >= SIDE_STAGES) alive = mbar_wait(side_empty + 8 * ss, ((i / SIDE_STAGES) - 1) & 1, 1u);
+      __syncwarp();
+      if (elect_one() && alive) {
         mbar_expect_tx(b_full + 8 * bs, p.b_stage_bytes);
         mbar_expect_tx(side_full + 8 * ss, (uint32_t)NP * 32u);
         bulk_g2s(base + p.b_off + bs * p.b_stage_bytes, p.bimg + ((size_t)kt * 2) * (NP * 128), p.b_stage_bytes, b_full + 8 * bs);
         bulk_g2s(base + p.side_off + ss * p.side_stage_bytes + HDR_BYTES, p.meta + (size_t)kt * (NP * 32), (uint32_t)NP * 32u, side_full + 8 * ss);
-        XNQ_TL(1, i);
-        if (++kt == KT) kt = 0;
-        if (++bs == BS) bs = 0, b_ph ^= 1u;
       }
+      __syncwarp();
+      if (++kt == KT) kt = 0;
+      if (++bs == BS) bs = 0, b_ph ^= 1u;
     }
   } else if (warp == MMA_WARP || warp == MMA_WARP + 1) {
-    // ---- MMA issuers: one thread per half step. A tcgen05.mma of this shape keeps the thread that issues it busy for about
-    // 134 cycles, but two threads issuing into different accumulator slices get twice the rate (measured up to N = 64), so
-    // the two halves of a step are issued by two warps, each with its own commit. ----
-    const int hh = warp - MMA_WARP;
-    if (lane == 0) {
-      const uint32_t idesc = idesc_i8(NP);
-      bool alive = true;
-      XNQ_TDECL;
-      int bs = 0, nb = 0; // i % BS, i % (NB / 2): AS and NB are even, so half step j = 2 i + h uses A stage 2 bs + h and buffer 2 nb + h
-      uint32_t b_ph = 0, acc_ph = 0; // (i / BS) & 1 = (j / AS) & 1, (j / NB) & 1
-      for (int i = 0; i < nunits && alive; i++) {
-        XNQ_TACC(0);
-        alive = mbar_wait(b_full + 8 * bs, b_ph, 4u);
-        XNQ_TACC(1);
-        if (alive) alive = mbar_wait(a_full + 8 * bs, b_ph, 4u); // both halves of the step's operand image
-        XNQ_TACC(2);
-        {
-          const int h = hh;
-          const int sa = 2 * bs + h, buf = 2 * nb + h;
-          XNQ_TACC(0);
-          if (alive && 2 * i >= NB) alive = mbar_wait(acc_empty + 8 * buf, acc_ph ^ 1u, 4u); // the drain of the buffer's previous half step
-          XNQ_TACC(3);
-          if (!alive) break;
-          if (h == 0) XNQ_TL(4, i);
-          tc_fence_after();
-          const uint64_t adesc = smem_desc_sw128(base + p.a_off + sa * A_STAGE_BYTES);
-          const uint64_t bdesc = smem_desc_sw128(base + p.b_off + bs * p.b_stage_bytes + h * (NP * 128));
+    // ---- MMA issuers: one warp per half step. The whole warp runs the loop and one elected lane issues; everything that decides the
+    // loop's course or a descriptor is a function of launch parameters and counters (a wait that gave up only makes the rest of the
+    // loop idle), so the compiler keeps the descriptors in uniform registers. In a branch on the lane number they were moved there
+    // from vector registers, one after the other, which held the thread for 96 cycles per MMA; the tensor core takes one every 40
+    // (NP <= 32) or 48 (NP = 64) cycles. ----
+    const int h = warp - MMA_WARP;
+    const uint32_t idesc = idesc_i8(NP);
+    bool alive = true;
+    int ap = 0, bs = 0, nb = 0; // i % AP, i % BS, i % (NB / 2): half step j = 2 i + h uses A stage 2 ap + h and buffer 2 nb + h
+    uint32_t a_ph = 0, b_ph = 0, acc_ph = 0; // the parities of the laps
+    for (int i = 0; i < nunits; i++) {
+      const int sa = 2 * ap + h, buf = 2 * nb + h;
+      if (alive) alive = mbar_wait(b_full + 8 * bs, b_ph, 4u);
+      if (alive) alive = mbar_wait(a_full + 8 * ap, a_ph, 4u); // both halves of the step's operand image
+      if (alive && 2 * i >= NB) alive = mbar_wait(acc_empty + 8 * buf, acc_ph ^ 1u, 4u); // the drain of the buffer's previous half step
+      tc_fence_after();
+      __syncwarp();
+      const uint64_t adesc = smem_desc_sw128(base + p.a_off + sa * A_STAGE_BYTES);
+      const uint64_t bdesc = smem_desc_sw128(base + p.b_off + bs * p.b_stage_bytes + h * (NP * 128));
+      if (elect_one() && alive) {
 #pragma unroll
-          for (int q = 0; q < 4; q++) // K = 32 per instruction: advance 32 bytes inside the swizzle row; slice q of the buffer
-            umma_i8(tmem_d + (uint32_t)(buf * BUF_COLS + q * NP), adesc + (uint64_t)(q * 2), bdesc + (uint64_t)(q * 2), idesc);
-          XNQ_TACC(4);
-          // the arrival serves the drain (the slices are written) and, together with the other half's, the converters and the
-          // activation producer (the stages are free)
-          umma_commit(mma_done + 8 * sa);
-          XNQ_TACC(5);
-          if (h == 1) XNQ_TL(5, i);
-        }
-        if (++bs == BS) bs = 0, b_ph ^= 1u;
-        if (2 * ++nb == NB) nb = 0, acc_ph ^= 1u;
+        for (int q = 0; q < 4; q++) // K = 32 per instruction: advance 32 bytes inside the swizzle row; slice q of the buffer
+          umma_i8(tmem_d + (uint32_t)(buf * BUF_COLS + q * NP), adesc + (uint64_t)(q * 2), bdesc + (uint64_t)(q * 2), idesc);
+        umma_commit(mma_done + 8 * sa); // serves the drain (the slices are written) and, with the other half's, the converters (the stages are free)
+        umma_commit(b_empty + 8 * bs);
       }
-      XNQ_TDUMP(6, hh == 0);
+      __syncwarp();
+      if (++ap == AP) ap = 0, a_ph ^= 1u;
+      if (++bs == BS) bs = 0, b_ph ^= 1u;
+      if (2 * ++nb == NB) nb = 0, acc_ph ^= 1u;
     }
   } else if (warp < DRAIN_WARP0) {
     // ---- converters: group g (four warps, one thread per weight row) produces the steps i = g, g + 2, ... of this CTA: a
@@ -548,29 +524,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
       cp_async_commit();
     }
     bool alive = true;
-    XNQ_TDECL;
-    int rs = 0, bs = g % BS;
-    uint32_t a_ph = (uint32_t)(g / BS) & 1u; // (i / BS) & 1
+    int rs = 0, bs = g % AP;
+    uint32_t a_ph = (uint32_t)(g / AP) & 1u; // (i / AP) & 1
     for (int i = g; i < nunits && alive; i += 2) {
       const int ss = i % SIDE_STAGES;
-      XNQ_TACC(0);
       cp_async_wait(D - 1); // one group per step and lane, committed in step order: step i's has landed
       __syncwarp();         // ... for every lane of the warp
-      XNQ_TACC(1);
-      if (threadIdx.x == CONV_WARP0 * 32) XNQ_TL(2, i);
       const uint32_t slot = slot0 + (uint32_t)rs * SLOT;
       { // hand the row's 16 scale bytes to the drain
         if (i >= SIDE_STAGES) alive = mbar_wait_warp(side_empty + 8 * ss, ((i / SIDE_STAGES) - 1) & 1, 2u);
-        XNQ_TACC(2);
         if (!alive) break;
         const uint4 hv = lds128(slot + 32 * STEP + lane * 16);
         sts128(base + p.side_off + ss * p.side_stage_bytes + (uint32_t)r * 16, hv);
         __syncwarp();
         if (lane == 0) mbar_arrive(side_full + 8 * ss);
       }
-      XNQ_TACC(0);
-      if (i >= BS) alive = mbar_wait_warp(mma_done + 8 * (2 * bs), a_ph ^ 1u, 2u) && mbar_wait_warp(mma_done + 8 * (2 * bs + 1), a_ph ^ 1u, 2u); // both halves of the stage have been multiplied
-      XNQ_TACC(3);
+      if (i >= AP) alive = mbar_wait_warp(mma_done + 8 * (2 * bs), a_ph ^ 1u, 2u) && mbar_wait_warp(mma_done + 8 * (2 * bs + 1), a_ph ^ 1u, 2u); // both halves of the stage have been multiplied
       if (!alive) break;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
@@ -589,87 +558,62 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
       if (lane == 0) mbar_arrive(a_full + 8 * bs);
       if (l_i < nunits) issue(); // into the slot just read
       cp_async_commit();
-      if (threadIdx.x == CONV_WARP0 * 32) XNQ_TL(3, i);
       if (++rs == D) rs = 0;
       for (int t = 0; t < 2; t++)
-        if (++bs == BS) bs = 0, a_ph ^= 1u;
+        if (++bs == AP) bs = 0, a_ph ^= 1u;
     }
     cp_async_wait(0); // nothing may be in flight into this CTA's shared memory when it exits
-    XNQ_TDUMP(12, threadIdx.x == CONV_WARP0 * 32);
-  } else if (warp - DRAIN_WARP0 < 2 * DWG) {
-    // ---- drain: group h (DWG warps) owns half step h of every 256-k step and the accumulator buffers of its parity. Warp
-    // quarter q reads accumulator lanes 32q.. (weight rows); with eight warps per group the two warps of a quarter split the
-    // columns. Each group keeps its own f32 sums; at the end of a segment group 1 hands its sums to group 0 through scratch
-    // memory. ----
+  } else {
+    // ---- drain: warp quarter q reads accumulator lanes 32q.. (weight rows), four warps of a quarter split the columns; every warp
+    // takes both half steps of every step and keeps f32 sums in registers. (Two groups of eight warps that took one half step each had
+    // twice the columns per thread: at 64 rows they read them back four at a time, eight trips to tensor memory of 550 cycles per
+    // half step; twice the integer-to-float conversions; and the groups' sums had to meet in memory at the end of a tile.) ----
     const int dwi = warp - DRAIN_WARP0;
-    const int q = warp & 3, h = dwi / DWG, cg = (dwi % DWG) >> 2;
-    const int c0 = cg * NPT;
+    const int q = warp & 3, c0 = (dwi >> 2) * NPT;
     const int et = threadIdx.x - DRAIN_WARP0 * 32; // 0..511
     pdl_wait(); // the kernel that prepares the activations also zeroes the tiles' tickets
-#ifdef XNQ_DEV_TRACE
-    if (blockIdx.x == 0 && threadIdx.x == DRAIN_WARP0 * 32) { unsigned long long g_; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g_)); g_imma_trace[28] = (long long)g_; }
-#endif
     bool alive = true;
     int tile = tile0, kt = kt0;
     float acc[NPT];
 #pragma unroll
     for (int c = 0; c < NPT; c++) acc[c] = 0.f;
     int seg_kt0 = kt0; // first step of the current segment inside its tile
-    float *pair = p.pair_scratch + (size_t)blockIdx.x * NP * TILE_N; // group 1 -> group 0
-    XNQ_TDECL;
-    int bs = 0, nb = 0;  // i % BS, i % (NB / 2)
-    uint32_t a_ph = 0;   // (i / BS) & 1
+    int ap = 0, nb = 0;  // i % AP, i % (NB / 2)
+    uint32_t a_ph = 0;   // (i / AP) & 1
     for (int i = 0; i < nunits; i++) {
       const int ss = i % SIDE_STAGES;
-      const int sa = 2 * bs + h, buf = 2 * nb + h;
-      XNQ_TACC(0);
       if (alive) alive = mbar_wait_warp(side_full + 8 * ss, (i / SIDE_STAGES) & 1, 8u);
-      XNQ_TACC(1);
       const uint32_t side = base + p.side_off + ss * p.side_stage_bytes;
       uint4 hdr = make_uint4(0, 0, 0, 0);
       if (alive) hdr = lds128(side + (uint32_t)(32 * q + lane) * 16);
-      if (alive) alive = mbar_wait_warp(mma_done + 8 * sa, a_ph, 8u);
-      XNQ_TACC(2);
-      if (threadIdx.x == DRAIN_WARP0 * 32) XNQ_TL(6, i);
+      if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap), a_ph, 8u);
+      if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap + 1), a_ph, 8u);
       if (alive) {
         tc_fence_after();
-        const uint32_t taddr = tmem_d + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BUF_COLS + c0);
+        const uint32_t taddr = tmem_d + ((uint32_t)(32 * q) << 16) + (uint32_t)(2 * nb * BUF_COLS + c0); // the halves' buffers are neighbours
 #pragma unroll
-        for (int ch = 0; ch < NPT / CH; ch++) { // eight columns at a time keeps the slices' values within the register budget
-          uint32_t v[4][CH];
+        for (int ch = 0; ch < NPT / CH; ch++) {
+          uint32_t v[8][CH];
 #pragma unroll
-          for (int s = 0; s < 4; s++) tmem_ld<CH>(taddr + (uint32_t)(s * NP + ch * CH), v[s]);
+          for (int j = 0; j < 8; j++) tmem_ld<CH>(taddr + (uint32_t)(j * NP + ch * CH), v[j]);
           tmem_ld_wait();
-          XNQ_TACC(3);
-          if (ch == NPT / CH - 1) { // every value of the buffer this warp needs is in registers: it may be overwritten
+          if (ch == NPT / CH - 1) { // every value of the buffers this warp needs is in registers: they may be overwritten
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty + 8 * buf);
+            if (lane == 0) mbar_arrive(acc_empty + 8 * (2 * nb)), mbar_arrive(acc_empty + 8 * (2 * nb + 1));
           }
-          Drain<CH>::run(hdr, side + HDR_BYTES, h, c0 + ch * CH, v, acc + ch * CH);
+          Drain<CH>::run(hdr, side + HDR_BYTES, c0 + ch * CH, v, acc + ch * CH);
         }
       }
       __syncwarp();
       if (alive && lane == 0) mbar_arrive(side_empty + 8 * ss);
-      if (threadIdx.x == DRAIN_WARP0 * 32) XNQ_TL(7, i);
       // ---- end of a segment (the tile's last step, or this CTA's last unit): store or hand over the sums ----
       const bool tile_end = kt == KT - 1, range_end = i == nunits - 1;
       if (tile_end || range_end) {
         const int64_t row = (int64_t)tile * TILE_N + 32 * q + lane;
-        // group 1's sums (the odd half steps) join group 0's (the even ones): always even + odd, whatever the timing
-        if (h == 1) {
-#pragma unroll
-          for (int c = 0; c < NPT; c++) pair[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
-          __threadfence_block();
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(2 * DWG * 32) : "memory");
-        if (h == 0) {
-#pragma unroll
-          for (int c = 0; c < NPT; c++) acc[c] += pair[(size_t)(c0 + c) * TILE_N + 32 * q + lane];
-        }
         const bool whole = seg_kt0 == 0 && tile_end;
         if (whole) {
-          if (h == 0 && alive && row < p.w.n) {
+          if (alive && row < p.w.n) {
 #pragma unroll
             for (int c = 0; c < NPT; c++) {
               const int64_t col = c0 + c;
@@ -681,25 +625,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
               }
             }
           }
-          asm volatile("bar.sync 1, %0;" ::"n"(2 * DWG * 32) : "memory"); // group 0 has read the scratch: it may be rewritten
         } else {
           // this CTA's first segment (it starts where the CTA's range starts) uses scratch slot 2c, a later one 2c + 1
           const int seg_u0 = tile * KT + seg_kt0;
           float *mine = p.partials + ((size_t)2 * blockIdx.x + (seg_u0 == u0 ? 0 : 1)) * NP * TILE_N;
-          if (h == 0) {
 #pragma unroll
-            for (int c = 0; c < NPT; c++) mine[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
-            __threadfence();
-          }
-          asm volatile("bar.sync 1, %0;" ::"n"(2 * DWG * 32) : "memory");
+          for (int c = 0; c < NPT; c++) mine[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
+          __threadfence();
+          asm volatile("bar.sync 1, %0;" ::"n"(DRAIN_WARPS * 32) : "memory");
           if (et == 0) s_ticket = atomicAdd(p.tile_cnt + tile, 1u);
-          asm volatile("bar.sync 1, %0;" ::"n"(2 * DWG * 32) : "memory");
+          asm volatile("bar.sync 1, %0;" ::"n"(DRAIN_WARPS * 32) : "memory");
           const unsigned int ticket = s_ticket;
-          asm volatile("bar.sync 1, %0;" ::"n"(2 * DWG * 32) : "memory"); // s_ticket may be rewritten from here on
+          asm volatile("bar.sync 1, %0;" ::"n"(DRAIN_WARPS * 32) : "memory"); // s_ticket may be rewritten from here on
           const int t_u0 = tile * KT, t_u1 = t_u0 + KT;
           const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u1 - 1, p.units_q, p.units_r);
           if (et == 0 && (int)ticket == c_last - c_first) p.tile_cnt[tile] = 0u; // every part has its ticket: the word is zero again for the next call
-          if (h == 0 && (int)ticket == c_last - c_first) { // the last part to arrive adds all parts in k order
+          if ((int)ticket == c_last - c_first) { // the last part to arrive adds all parts in k order
             __threadfence();
             float (&sum)[NPT] = acc; // the segment's own sums are in its scratch slot by now
 #pragma unroll
@@ -732,18 +673,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
         kt = 0;
         tile++;
       }
-      if (++bs == BS) bs = 0, a_ph ^= 1u;
+      if (++ap == AP) ap = 0, a_ph ^= 1u;
       if (2 * ++nb == NB) nb = 0;
     }
-    XNQ_TDUMP(18, threadIdx.x == DRAIN_WARP0 * 32);
   }
 
   tc_fence_before();
   __syncthreads();
-#ifdef XNQ_DEV_TRACE
-  if (blockIdx.x == 0 && threadIdx.x == 0) g_imma_trace[30] = nunits;
-  XNQ_GT(27);
-#endif
   if (warp == MMA_WARP) tmem_dealloc(tmem_d, TMEM_COLS);
 }
 
@@ -810,7 +746,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1) imma_q4k_fold_kernel(const __gr
   // One commit per issuer and step, on the step's accumulator buffer (acc_full, all four issuers): it tells the drain that the
   // slices are written and the converters that the operand stages of that step have been read. A barrier per operand stage
   // would be lapped: the issuers may run NBUF steps ahead of the drain, and a waiter that misses two phases waits for ever.
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int D = p.raw_stages; // raw slots per converter warp
   const int KT = p.nsteps;
   const int u0 = cta_first_unit((int)blockIdx.x, p.units_q, p.units_r);
@@ -838,7 +774,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1) imma_q4k_fold_kernel(const __gr
   __syncthreads();
   tc_fence_after();
   pdl_launch_dependents();
-  const uint32_t tmem_d = tmem_slot;
+  const uint32_t tmem_d = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
   if (warp == F_ACT_WARP) {
     // ---- activation producer ----
@@ -865,25 +801,29 @@ __global__ void __launch_bounds__(F_NTHREADS, 1) imma_q4k_fold_kernel(const __gr
   } else if (warp < F_CONV_WARP0) {
     // ---- MMA issuers: plane pl (0: q_lo sc, 1: q_hi sc) of half step h ----
     const int pl = (warp - F_MMA_WARP0) >> 1, h = (warp - F_MMA_WARP0) & 1;
-    if (lane == 0) {
-      const uint32_t idesc = idesc_u8s8(NP);
-      RingPos rp{0, 0}; // step i in the drain-freed ring
-      uint32_t acc_ph = 0;
-      for (int i = 0; i < nunits; i++) {
-        const int buf = i & (NBUF - 1), st = 2 * (i & 1) + h; // half step j = 2 i + h uses operand stage j % 4
-        if (!mbar_wait(b_full + 8 * rp.idx, rp.ph, 4u)) break;
-        if (!mbar_wait(a_full + 8 * st, (uint32_t)(i >> 1) & 1u, 4u)) break;
-        if (i >= NBUF && !mbar_wait(acc_empty + 8 * buf, acc_ph ^ 1u, 4u)) break; // the drain of the buffer's previous step
-        tc_fence_after();
-        const uint64_t adesc = smem_desc_sw128(base + p.a_off + st * F_A_STAGE_BYTES + pl * A_STAGE_BYTES);
-        const uint64_t bdesc = smem_desc_sw128(base + p.b_off + rp.idx * p.b_stage_bytes + h * (NP * 128));
-        const uint32_t dcol = tmem_d + (uint32_t)(buf * BUF_COLS + (pl * 2 + h) * NP);
+    // (the whole warp runs the loop, as in the kernel above)
+    const uint32_t idesc = idesc_u8s8(NP);
+    bool alive = true;
+    RingPos rp{0, 0}; // step i in the drain-freed ring
+    uint32_t acc_ph = 0;
+    for (int i = 0; i < nunits; i++) {
+      const int buf = i & (NBUF - 1), st = 2 * (i & 1) + h; // half step j = 2 i + h uses operand stage j % 4
+      if (alive) alive = mbar_wait(b_full + 8 * rp.idx, rp.ph, 4u);
+      if (alive) alive = mbar_wait(a_full + 8 * st, (uint32_t)(i >> 1) & 1u, 4u);
+      if (alive && i >= NBUF) alive = mbar_wait(acc_empty + 8 * buf, acc_ph ^ 1u, 4u); // the drain of the buffer's previous step
+      tc_fence_after();
+      __syncwarp();
+      const uint64_t adesc = smem_desc_sw128(base + p.a_off + st * F_A_STAGE_BYTES + pl * A_STAGE_BYTES);
+      const uint64_t bdesc = smem_desc_sw128(base + p.b_off + rp.idx * p.b_stage_bytes + h * (NP * 128));
+      const uint32_t dcol = tmem_d + (uint32_t)(buf * BUF_COLS + (pl * 2 + h) * NP);
+      if (elect_one() && alive) {
 #pragma unroll
         for (int q = 0; q < 4; q++) umma_i8_acc(dcol, adesc + (uint64_t)(q * 2), bdesc + (uint64_t)(q * 2), idesc, q > 0 ? 1u : 0u);
         umma_commit(acc_full + 8 * buf);
-        rp.advance(1, F_RING);
-        if (buf == NBUF - 1) acc_ph ^= 1u;
       }
+      __syncwarp();
+      rp.advance(1, F_RING);
+      if (buf == NBUF - 1) acc_ph ^= 1u;
     }
   } else if (warp < F_DRAIN_WARP0) {
     // ---- converters: group h (four warps, one thread per weight row) writes both planes of half step h of every step ----
@@ -1115,7 +1055,6 @@ __global__ void __launch_bounds__(256) imma_prepare(const XT *__restrict__ x, co
                                                     uint8_t *__restrict__ bimg, uint8_t *__restrict__ meta, unsigned int *__restrict__ tile_cnt, int tiles) {
   pdl_launch_dependents(); // the matmul kernel may start its set-up and its weight loads now
   pdl_wait();              // x may be the previous kernel's output; the scratch may still be read by the previous call
-  XNQ_GT(24);
   const int row = blockIdx.x;
   if (blockIdx.x == 0 && blockIdx.y == 0)
     for (int i = threadIdx.x; i < tiles; i += blockDim.x) tile_cnt[i] = 0;
@@ -1178,7 +1117,6 @@ __global__ void __launch_bounds__(256) imma_prepare(const XT *__restrict__ x, co
       }
     }
   }
-  XNQ_GT(25);
 }
 
 int g_sms = 0;
@@ -1188,9 +1126,9 @@ struct Plan {
   int NP, nsteps, tiles, grid;
   size_t bimg_bytes, meta_bytes, cnt_bytes, part_bytes, pair_bytes;
 };
-Plan plan_for(int64_t m, int64_t k, int64_t n) {
+Plan plan_for(int64_t m, int64_t k, int64_t n, bool operand = false) { // operand images have their own row counts (operand_np)
   Plan pl{};
-  pl.NP = m <= 16 ? 16 : (m <= 32 ? 32 : 64);
+  pl.NP = operand ? operand_np(m) : (int)((m + 15) / 16 * 16);
   pl.nsteps = (int)((k + 255) / 256);
   pl.tiles = (int)((n + TILE_N - 1) / TILE_N);
   const long long units = (long long)pl.tiles * pl.nsteps;
@@ -1220,6 +1158,7 @@ int launch_np(const ImmaArgs &a, int NP, unsigned grid, cudaStream_t s) {
   cfg.numAttrs = 1;
   if (NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 16>, a));
   else if (NP == 32) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 32>, a));
+  else if (NP == 48) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 48>, a));
   else XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 64>, a));
   count_launch();
   return XNQ_OK;
@@ -1229,6 +1168,7 @@ template <typename Conv, template <int> class Drain>
 int init_np() {
   XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+  XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 48>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   return XNQ_OK;
 }
@@ -1244,7 +1184,7 @@ bool imma_supported(const WeightView &w, int64_t m) {
 
 // scratch of one call: the activations' operand image and records, the split tiles' tickets and partial sums
 size_t imma_workspace_bytes(int64_t m, int64_t k, int64_t n) {
-  const Plan pl = plan_for(std::min<int64_t>(m, MAX_NP), k, n);
+  const Plan pl = plan_for(std::min<int64_t>(m, MAX_NP), k, n, true); // an operand image may have more rows than the float form
   return pl.bimg_bytes + pl.meta_bytes + pl.cnt_bytes + pl.part_bytes + pl.pair_bytes + 256;
 }
 
@@ -1263,7 +1203,7 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
   if (operand && (act != XNQ_Q8K || k % 256 || m > pass_rows)) return fail(XNQ_ERR_UNSUPPORTED, "imma: an operand image serves Q8_K activations of one pass (m = %lld)", (long long)m);
   for (int64_t r0 = 0; r0 < m; r0 += pass_rows) { // passes of at most 64 (32) activation rows
     const int64_t rows = std::min<int64_t>(pass_rows, m - r0);
-    const Plan pl = plan_for(rows, k, w.n);
+    const Plan pl = plan_for(rows, k, w.n, operand);
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     uint8_t *bimg = ws;
     uint8_t *meta = bimg + pl.bimg_bytes;
@@ -1285,8 +1225,12 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
       const int blk = act == XNQ_Q8_0 ? QK : QK_K;
       iq = av.q + r0 * k, id = av.d + r0 * (k / blk), ib = av.bsum + r0 * (k / 16);
     }
+    // The CTAs are started while the previous kernel drains, and the first SM that is free would take eight of them (3.9 us instead of
+    // 1.3): unused shared memory keeps them apart.
+    const dim3 prep_grid((unsigned)pl.NP, (unsigned)std::min<int64_t>(16, (k + 2047) / 2048));
+    const size_t spread = MAX_SPREAD / ((prep_grid.x * prep_grid.y + 147) / 148) / 1024 * 1024;
 #define XNQ_IMMA_PREP(ACT, XT)                                                                                                          \
-  XNQ_CUDA(launch_pdl(imma_prepare<ACT, XT>, dim3((unsigned)pl.NP, (unsigned)std::min<int64_t>(16, (k + 2047) / 2048)), dim3(256), 0, s,     \
+  XNQ_CUDA(launch_pdl(imma_prepare<ACT, XT>, prep_grid, dim3(256), spread, s,     \
                       iq ? nullptr : static_cast<const XT *>(x) + r0 * ldx, iq, id, ib, rows, k, ldx, pl.NP, pl.nsteps, bimg, meta, cnt, pl.tiles))
     if (operand) {
       // nothing to prepare
@@ -1338,9 +1282,6 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
       for (int st = 0; st < 2; st++) {
         a.pf_base[st] = st < a.nstreams ? a.src[st] : nullptr;
         a.pf_bytes[st] = st < a.nstreams && total <= PF_MAX_BYTES ? (unsigned long long)(((size_t)a.row_bytes[st] * (size_t)w.n) & ~(size_t)15) : 0ull;
-#ifdef XNQ_DEV_TRACE
-        if (const char *e = getenv("XNQ_IMMA_PF")) if (atoi(e) == 0) a.pf_bytes[st] = 0;
-#endif
         a.pf_share[st] = ((a.pf_bytes[st] / (unsigned)pl.grid) + PF_CHUNK - 1) & ~(unsigned long long)(PF_CHUNK - 1);
       }
     }
@@ -1379,19 +1320,19 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     // goes to raw stages, which hide the memory latency.
     const size_t budget = IMMA_SMEM - 1024; // 1024: alignment slack of the base
     a.a_stages = 0;
-    int as_order[3] = {6, 4, 8};
-#ifdef XNQ_DEV_TRACE
-    if (const char *e = getenv("XNQ_IMMA_AS")) as_order[0] = atoi(e);
-#endif
+    static constexpr int as_order[3] = {6, 4, 8};
     for (int ai = 0; ai < 3 && !a.a_stages; ai++) {
       const int as = as_order[ai];
-      for (int rs = MAX_RAW_STAGES; rs >= 2 && !a.a_stages; rs -= 2) // even: the two converter groups own half of the slots each
-        if ((size_t)as * A_STAGE_BYTES + (size_t)(as / 2) * a.b_stage_bytes + (size_t)SIDE_STAGES * a.side_stage_bytes + (size_t)rs * a.raw_stage_bytes + 256 <= budget &&
-            (rs >= 4 || as == 4))
-          a.a_stages = as, a.raw_stages = rs;
+      for (int rs = MAX_RAW_STAGES; rs >= 2 && !a.a_stages; rs -= 2) { // even: the two converter groups own half of the slots each
+        const size_t fixed = (size_t)as * A_STAGE_BYTES + (size_t)SIDE_STAGES * a.side_stage_bytes + (size_t)rs * a.raw_stage_bytes + 256;
+        if (rs < 4 && as != 4) continue;
+        // The activations' copies queue behind the weights': with three stages of a step each a step took the 4500 cycles of their
+        // latency divided by three
+        const int bs = fixed >= budget ? 0 : (int)std::min<size_t>(MAX_B_STAGES, (budget - fixed) / a.b_stage_bytes);
+        if (bs >= (pl.NP <= 32 && ai == 0 ? 5 : 2)) a.a_stages = as, a.raw_stages = rs, a.b_stages = bs;
+      }
     }
     if (!a.a_stages) return fail(XNQ_ERR_SIZE, "imma: shared-memory plan does not fit");
-    a.b_stages = a.a_stages / 2;
     a.a_off = 0;
     a.b_off = (uint32_t)a.a_stages * A_STAGE_BYTES;
     a.side_off = a.b_off + a.b_stages * a.b_stage_bytes;
@@ -1416,15 +1357,19 @@ int imma_init(int device) {
   XNQ_CUDA(cudaFuncSetAttribute(imma_q4k_fold_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   if ((rc = init_np<ConvQ8_0, DrainBlockScaled>()) != XNQ_OK) return rc;
   if ((rc = init_np<ConvQ4_0, DrainBlockScaled>()) != XNQ_OK) return rc;
+#define XNQ_IMMA_PREP_INIT(ACT, XT) XNQ_CUDA(cudaFuncSetAttribute(imma_prepare<ACT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SPREAD))
+  XNQ_IMMA_PREP_INIT(XNQ_Q8_0, float);
+  XNQ_IMMA_PREP_INIT(XNQ_Q8_0, __half);
+  XNQ_IMMA_PREP_INIT(XNQ_Q8_0, __nv_bfloat16);
+  XNQ_IMMA_PREP_INIT(XNQ_Q8K, float);
+  XNQ_IMMA_PREP_INIT(XNQ_Q8K, __half);
+  XNQ_IMMA_PREP_INIT(XNQ_Q8K, __nv_bfloat16);
+#undef XNQ_IMMA_PREP_INIT
   unsigned int zero = 0;
   XNQ_CUDA(cudaMemcpyToSymbol(g_imma_status, &zero, sizeof(zero)));
   return XNQ_OK;
 }
 
-#ifdef XNQ_DEV_TRACE
-extern "C" int xnq_dev_imma_trace(long long *out) { return cudaMemcpyFromSymbol(out, g_imma_trace, sizeof(long long) * 32) == cudaSuccess ? 0 : -6; }
-extern "C" int xnq_dev_imma_timeline(long long *out) { return cudaMemcpyFromSymbol(out, g_imma_tl, sizeof(long long) * 8 * 64) == cudaSuccess ? 0 : -6; }
-#endif
 
 void imma_set_fold(int on) { g_fold.store(on); }
 
