@@ -26,6 +26,8 @@ from .dtypes import GgmlDType
 
 _TORCH_TO_XNQ = {torch.float32: GgmlDType.F32, torch.float16: GgmlDType.F16, torch.bfloat16: GgmlDType.BF16}
 
+_XNQ_IDS = {t: int(d) for t, d in _TORCH_TO_XNQ.items()}
+
 
 def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
@@ -96,7 +98,7 @@ class QCudaTensor:
         check(_lib.lib().xnq_weight_info(self._h, dt, nt, nl, r0, k, nb))
         self._dtype = GgmlDType(dt.value)
         self.n_total, self.n, self.row0, self.k, self.device_bytes = nt.value, nl.value, r0.value, k.value, nb.value
-        self._ws: Optional[torch.Tensor] = None
+        self._ws_need: tuple[int, int] = (-1, 0)
 
     # -- construction ---------------------------------------------------------------------------
     @classmethod
@@ -192,7 +194,10 @@ class QCudaTensor:
         """Scratch for ``m`` activation rows. All weights of a device share one buffer (the reference's device
         has a single stream, cuda_backend/mod.rs:141-167, so calls never overlap); it only ever grows, and
         outgrown buffers stay alive because a captured graph may still point at them."""
-        need = _lib.lib().xnq_matmul_workspace_bytes(self._h, m)
+        last = self._ws_need   # (rows, bytes) of the size asked for last: a program calls a linear with the same few row counts
+        if last[0] != m:
+            last = self._ws_need = (m, _lib.lib().xnq_matmul_workspace_bytes(self._h, m))
+        need = last[1]
         pool = _workspaces.setdefault(self.device.index or 0, [])
         if not pool or pool[-1].numel() < need:
             pool.append(torch.empty(max(need, 256), dtype=torch.uint8, device=self.device))
@@ -242,25 +247,39 @@ class QCudaTensor:
                                               ctypes.c_void_p(ws.data_ptr()) if ws is not None else None, ws.numel() if ws is not None else 0,
                                               _stream_ptr(self.device)))
             return out
-        if lhs.shape[-1] != self.k:
-            raise ValueError(f"cuda quantized matmul: input {tuple(lhs.shape)} does not match weight (n={self.n}, k={self.k})")
-        if lhs.dtype not in _TORCH_TO_XNQ:
+        k, n, device = self.k, self.n, self.device
+        shape = lhs.shape
+        if shape[-1] != k:
+            raise ValueError(f"cuda quantized matmul: input {tuple(shape)} does not match weight (n={n}, k={k})")
+        x_dtype = _XNQ_IDS.get(lhs.dtype)
+        if x_dtype is None:
             raise ValueError(f"cuda quantized matmul: unsupported activation dtype {lhs.dtype}")
-        if lhs.device != self.device:
-            raise ValueError(f"cuda quantized matmul: input on {lhs.device}, weight on {self.device}")
-        x = lhs.reshape(-1, self.k)
-        if x.stride(-1) != 1 or (x.shape[0] > 1 and x.stride(0) < self.k):
+        if lhs.device != device:
+            raise ValueError(f"cuda quantized matmul: input on {lhs.device}, weight on {device}")
+        x = lhs if lhs.dim() == 2 else lhs.reshape(-1, k)
+        m, ldx = x.shape[0], x.stride(0)
+        if x.stride(1) != 1 or (m > 1 and ldx < k):
             x = x.contiguous()
-        m = x.shape[0]
-        ldx = x.stride(0) if m > 1 else self.k
+            ldx = k
+        if m <= 1:
+            ldx = k
         if out is None:
-            out = torch.empty(lhs.shape[:-1] + (self.n,), dtype=lhs.dtype, device=self.device)
-        y = out.view(-1, self.n)
+            out = torch.empty(shape[:-1] + (n,), dtype=lhs.dtype, device=device)
+            y, y_dtype, ldy = out, x_dtype, n
+        else:
+            y = out.view(-1, n)
+            y_dtype, ldy = int(_TORCH_TO_XNQ[y.dtype]), y.stride(0) if m > 1 else n
         ws = self.workspace(m)
-        with torch.cuda.device(self.device):
-            check(_lib.lib().xnq_matmul_t(self._h, ctypes.c_void_p(x.data_ptr()), int(_TORCH_TO_XNQ[x.dtype]), m, ldx,
-                                          ctypes.c_void_p(y.data_ptr()), int(_TORCH_TO_XNQ[y.dtype]), y.stride(0) if m > 1 else self.n,
-                                          ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(self.device)))
+        # The call launches on the current device: it is switched only where that is another one (the guard and the Stream object
+        # take several times as long as the call).
+        index = device.index
+        if index is not None and index == torch.cuda.current_device():
+            check(_lib.lib().xnq_matmul_t(self._h, x.data_ptr(), x_dtype, m, ldx, y.data_ptr(), y_dtype, ldy, ws.data_ptr(), ws.numel(),
+                                          torch._C._cuda_getCurrentRawStream(index)))
+        else:
+            with torch.cuda.device(device):
+                check(_lib.lib().xnq_matmul_t(self._h, x.data_ptr(), x_dtype, m, ldx, y.data_ptr(), y_dtype, ldy, ws.data_ptr(), ws.numel(),
+                                              _stream_ptr(device)))
         return out
 
     def forward_host(self, x: np.ndarray, bias: Optional[np.ndarray] = None, out: Optional[np.ndarray] = None) -> np.ndarray:
@@ -307,7 +326,7 @@ class QCudaLinear:
         if xs.dim() < 2:
             raise ValueError(f"input tensor has only one dimension {tuple(xs.shape)}")  # mod.rs:363-365
         out = self.weight.matmul_t(xs)
-        return out if self.bias is None else out + self.bias.to(out.dtype)  # broadcast_add, q8.rs:172-175
+        return out if self.bias is None else out.add_(self.bias.to(out.dtype))  # broadcast_add, q8.rs:172-175
 
     __call__ = forward
 
