@@ -29,7 +29,14 @@ static std::atomic<int> g_opt_gather_cta_fence{1};
 static std::atomic<int> g_opt_host_direct_y{1};
 static std::atomic<int> g_opt_matvec_mma{1};
 static std::atomic<int> g_opt_imma{1};
-static bool use_imma(const xnq_weight *w, int64_t m) { return m >= 2 && m <= IMMA_MAX_M && g_opt_imma.load(std::memory_order_relaxed) && imma_supported(w->v, m); }
+// The integer tensor-core kernel, except up to four rows of Q4_0 / Q8_0 that the dp4a kernel can stage at once: it streams the weight
+// without the operand image and its hand-overs (Q4_0 4096 x 4096, 2 rows: 8.1 us against 12.5; Q8_0 11008 x 4096, 2 rows: 17.0 against
+// 21.1; 4096 x 4096, 3 rows: 11.0 against 13.2). Q4_K stays on one kernel from two rows on, so that operand images and float rows give
+// the same bits.
+static bool use_imma(const xnq_weight *w, int64_t m) {
+  if (m < 2 || m > IMMA_MAX_M || !g_opt_imma.load(std::memory_order_relaxed) || !imma_supported(w->v, m)) return false;
+  return m > 4 || w->v.dtype == XNQ_Q4K || matvec_rows_per_pass(w->v.dtype, w->v.k) < m;
+}
 // Small batches: the integer-MMA kernel where it serves the weight and wins (Q4_K, five rows and up), else the
 // dp4a kernel. Returns the rows per launch.
 int64_t small_batch_pass(const xnq_weight *w, int64_t m, int y_dtype, bool *use_mma) {
@@ -129,8 +136,8 @@ static int matmul_from_operand(const xnq_weight *w, const void *image, int64_t m
   if (!image || !y) return fail(XNQ_ERR_NULL, "matmul_t: image or y is NULL");
   if (!aligned(image, 256)) return fail(XNQ_ERR_ALIGN, "matmul_t: the operand image must be 256-byte aligned");
   if (!aligned(y, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "matmul_t: y is not aligned to its element size");
-  if (act_dtype_for(w->v.dtype) != XNQ_Q8K || !is_fast_dtype(w->v.dtype) || !use_imma(w, m))
-    return fail(XNQ_ERR_UNSUPPORTED, "matmul_t: an operand image serves 2..%lld rows on weights of the integer tensor-core kernel with Q8_K activations (dtype %d, m = %lld)",
+  if (w->v.dtype != XNQ_Q4K || !use_imma(w, m))
+    return fail(XNQ_ERR_UNSUPPORTED, "matmul_t: an operand image serves 2..%lld rows on Q4_K weights (dtype %d, m = %lld)",
                 (long long)IMMA_MAX_M, w->v.dtype, (long long)m);
   if (!workspace || !aligned(workspace, 256) || ws_bytes < imma_workspace_bytes(m, k, n))
     return fail(XNQ_ERR_SIZE, "matmul_t: the workspace (256-byte aligned, %zu bytes) is needed for the partial sums", imma_workspace_bytes(m, k, n));
@@ -554,7 +561,7 @@ size_t xnq_matmul_workspace_bytes(const xnq_weight *w, int64_t max_m) {
   if (is_generic_dtype(w->v.dtype)) return generic_workspace_bytes(w->v, max_m);
   const int64_t rows = max_m < MATVEC_MAX_M ? max_m : MATVEC_MAX_M;
   size_t decode = act_workspace_bytes(rows, w->v.k, act_dtype_for(w->v.dtype));
-  if (max_m >= 2 && imma_supported(w->v, 2)) decode = std::max(decode, imma_workspace_bytes(std::min<int64_t>(max_m, IMMA_MAX_M), w->v.k, w->v.n));
+  if (max_m >= 2 && imma_supported(w->v, w->v.dtype == XNQ_Q6K ? MATVEC_MAX_M : 2)) decode = std::max(decode, imma_workspace_bytes(std::min<int64_t>(max_m, IMMA_MAX_M), w->v.k, w->v.n));
   if (max_m <= MATVEC_MAX_M) return decode;
   const size_t prefill = prefill_workspace_bytes(max_m, w->v.k, w->v.n); // m > 16 runs on the tensor cores
   return prefill > decode ? prefill : decode;

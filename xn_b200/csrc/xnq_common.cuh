@@ -319,13 +319,13 @@ int matvec_tma_init(int device);
 int matvec_status(unsigned int *bits);
 int matvec_check_record(unsigned long long out[8]);
 
-// xnq_imma.cu  (2 <= m: tcgen05 kind::i8, exact integer block sums; Q4_0 / Q8_0 / Q4_K)
+// xnq_imma.cu  (2 <= m <= 64: tcgen05 kind::i8, exact integer block sums; Q4_0 / Q8_0 / Q4_K, and Q6_K from 6 to 16 rows)
 bool imma_supported(const WeightView &w, int64_t m);
 size_t imma_workspace_bytes(int64_t m, int64_t k, int64_t n);
 int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
                 cudaStream_t s);
 int imma_init(int device);
-void imma_set_fold(int mode); // Q4_K kernel with the sub-block scales folded into the weight operand: 0 never, 1 where it is faster (17..32 rows), 2 always
+void imma_set_fold(int mode); // Q4_K kernel with the sub-block scales folded into the weight operand: 2 always, else never
 int imma_status(unsigned int *bits);
 int decoder_ops_init();
 int decoder_status(unsigned int *bits); // 1 rope/store, 2 attention: a position outside [0, max_seq)

@@ -12,6 +12,10 @@
 // dp4a), f16 block scale times f16-rounded activation scale for Q4_0 / Q8_0. Nothing is rounded before the
 // f32 scaling, so results stay within the f32-accumulate bound (2e-3) at every batch size served.
 //
+// Q6_K (6 to 16 rows) has a scale per 16 elements, half an MMA's K. Its activation operand holds every row twice, once with the
+// upper and once with the lower 16 of each 32 codes zeroed, so that one MMA yields both 16-sums; the drain multiplies the sixteen sums
+// of a super-block with the int8 scales, adds them as integers and scales once, as the CPU code does (k_quants.rs:1743-1799).
+//
 // Roles of the 27 warps of a CTA (one CTA per SM, persistent):
 //   producer (1)    one thread requests, per 256-k step, the 1-D bulk copies of the quantized activations (already in
 //                   the MMA's shared-memory layout) and of their per-block metadata into rings of stages guarded by
@@ -57,6 +61,9 @@ __device__ unsigned int g_imma_status; // sticky: 1 producer, 2 converter, 4 mma
 namespace {
 
 constexpr int TILE_N = 128;         // weight rows per tile = UMMA M
+// Q6_K: below six rows the dp4a kernel is as fast or faster (4096 x 4096, 5 rows: 12.3 us against 13.5; 8 rows: 13.7 against 13.5, and on
+// 32000 x 4096 62 against 48), above 16 the fp16 kernel is (32000 x 4096, 24 rows: 59 us here, 55 there).
+constexpr int64_t Q6K_MIN_M = 6, Q6K_MAX_M = 16;
 constexpr int MAX_NP = 64;          // activation rows per pass = UMMA N (multiple of 16)
 constexpr int CONV_WARPS = 8, DRAIN_WARPS = 16;
 constexpr int ACT_PRODUCER_WARP = 0, MMA_WARP = 1, CONV_WARP0 = 3, DRAIN_WARP0 = CONV_WARP0 + CONV_WARPS; // MMA issuers: warps 1 and 2
@@ -299,7 +306,8 @@ __device__ __forceinline__ uint4 raw_chunk(uint32_t row, int key, int c) {
   return lds128(row + (uint32_t)((c ^ (key & (STEP / 16 - 1))) << 4));
 }
 struct ConvQ8_0 { // 256 code bytes per row and step
-  static constexpr int STEP = 256;
+  static constexpr int STEP = 256, HI = 0; // HI: bytes per row and step of a second code stream
+  static constexpr bool PAIRED = false;    // two operand columns per activation row
   __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; i++) out[i] = raw_chunk<STEP>(row, key, 8 * h + 4 * p + i);
@@ -308,7 +316,8 @@ struct ConvQ8_0 { // 256 code bytes per row and step
 __device__ __forceinline__ uint32_t nib_lo_s8(uint32_t w) { return (((w & 0x0f0f0f0fu) | 0x80808080u) - 0x08080808u) ^ 0x80808080u; } // code - 8 per byte
 __device__ __forceinline__ uint32_t nib_hi_s8(uint32_t w) { return ((((w >> 4) & 0x0f0f0f0fu) | 0x80808080u) - 0x08080808u) ^ 0x80808080u; }
 struct ConvQ4_0 { // eight blocks of 16 nibble bytes per row and step; element j < 16 low nibble of byte j, j >= 16 high nibble of byte j - 16
-  static constexpr int STEP = 128;
+  static constexpr int STEP = 128, HI = 0;
+  static constexpr bool PAIRED = false;
   __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
 #pragma unroll
     for (int bb = 0; bb < 2; bb++) {
@@ -319,13 +328,33 @@ struct ConvQ4_0 { // eight blocks of 16 nibble bytes per row and step; element j
   }
 };
 struct ConvQ4K { // 128 code bytes per row and step: four 32-byte chunks; chunk c = sub-block 2c in the low nibbles, 2c+1 in the high ones
-  static constexpr int STEP = 128;
+  static constexpr int STEP = 128, HI = 0;
+  static constexpr bool PAIRED = false;
   __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
     const uint4 a = raw_chunk<STEP>(row, key, 2 * (2 * h + p)), b = raw_chunk<STEP>(row, key, 2 * (2 * h + p) + 1);
     out[0] = make_uint4(a.x & 0x0f0f0f0fu, a.y & 0x0f0f0f0fu, a.z & 0x0f0f0f0fu, a.w & 0x0f0f0f0fu);
     out[1] = make_uint4(b.x & 0x0f0f0f0fu, b.y & 0x0f0f0f0fu, b.z & 0x0f0f0f0fu, b.w & 0x0f0f0f0fu);
     out[2] = make_uint4((a.x >> 4) & 0x0f0f0f0fu, (a.y >> 4) & 0x0f0f0f0fu, (a.z >> 4) & 0x0f0f0f0fu, (a.w >> 4) & 0x0f0f0f0fu);
     out[3] = make_uint4((b.x >> 4) & 0x0f0f0f0fu, (b.y >> 4) & 0x0f0f0f0fu, (b.z >> 4) & 0x0f0f0f0fu, (b.w >> 4) & 0x0f0f0f0fu);
+  }
+};
+
+__device__ __forceinline__ uint32_t q6_code(uint32_t ql, int sh, uint32_t qh, int hsh) { // four 6-bit codes - 32 as int8
+  const uint32_t c = ((ql >> sh) & 0x0f0f0f0fu) | (((qh >> hsh) & 0x03030303u) << 4);
+  return ((c | 0x80808080u) - 0x20202020u) ^ 0x80808080u;
+}
+struct ConvQ6K { // 128 ql bytes and 64 qh bytes per row and step. 64 k number 2 h + p: the two 32-element groups 2 p, 2 p + 1 of half h
+  static constexpr int STEP = 128, HI = 64;
+  static constexpr bool PAIRED = true;
+  // row / hi: the row's 128 and 64 bytes in the slot
+  __device__ static __forceinline__ void run(uint32_t row, uint32_t hi, int key, int h, int p, uint4 (&out)[4]) {
+#pragma unroll
+    for (int half = 0; half < 2; half++) { // elements 0..15 and 16..31 of the groups
+      const uint4 a = raw_chunk<STEP>(row, key, 4 * h + half), b = raw_chunk<STEP>(row, key, 4 * h + 2 + half), q = raw_chunk<HI>(hi, key, 2 * h + half);
+      const int sh = 4 * p, h0 = 4 * p, h1 = 4 * p + 2; // groups 0, 1: low nibbles of ql[l], ql[l + 32]; groups 2, 3: the high nibbles
+      out[half] = make_uint4(q6_code(a.x, sh, q.x, h0), q6_code(a.y, sh, q.y, h0), q6_code(a.z, sh, q.z, h0), q6_code(a.w, sh, q.w, h0));
+      out[2 + half] = make_uint4(q6_code(b.x, sh, q.x, h1), q6_code(b.y, sh, q.y, h1), q6_code(b.z, sh, q.z, h1), q6_code(b.w, sh, q.w, h1));
+    }
   }
 };
 
@@ -374,9 +403,24 @@ struct DrainQ4K { // integer sums over the whole super-block, scaled once, as th
   }
 };
 
+// Q6_K, the four slices of half step h: v[2 j + u][c] is the sum of the u-th 16 elements of block j. hdr: the row's sixteen int8 scales.
+template <int CH>
+__device__ __forceinline__ void q6k_sums(const uint4 &hdr, int h, const uint32_t (&v)[8][CH], int (&isum)[CH]) {
+  const uint32_t w[2] = {h ? hdr.z : hdr.x, h ? hdr.w : hdr.y};
+#pragma unroll
+  for (int c = 0; c < CH; c++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) isum[c] += (int)(int8_t)((w[j >> 2] >> (8 * (j & 3))) & 0xffu) * (int)v[j][c];
+}
+template <int CH>
+struct DrainQ6K { // (the paired form has its own drain, by half steps)
+  __device__ static __forceinline__ void run(const uint4 &, uint32_t, int, const uint32_t (&)[8][CH], float *) {}
+};
+
 template <typename Conv, template <int> class Drain, int NP>
 __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant__ ImmaArgs p) {
-  constexpr int NPT = NP / (DRAIN_WARPS / 4); // columns per drain thread: four warps per accumulator lane quarter split them
+  constexpr int ROWS = Conv::PAIRED ? NP / 2 : NP; // activation rows of the operand; NP: its columns
+  constexpr int NPT = ROWS / (DRAIN_WARPS / 4); // rows per drain thread: four warps per accumulator lane quarter split them
   constexpr int CH = 4;                       // columns read back at a time, all eight slices of a step: what the register budget holds
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand stages need 1024-byte alignment
@@ -487,7 +531,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
     // ---- converters: group g (four warps, one thread per weight row) produces the steps i = g, g + 2, ... of this CTA: a
     // step's chain of waits, loads, stores and fences has the time of two steps' MMAs to run in ----
     constexpr int STEP = Conv::STEP, CPR = STEP / 16, RPI = 32 / CPR; // code bytes per row and step; 16-byte chunks per row; rows per copy instruction
-    constexpr uint32_t SLOT = 32 * STEP + 512;                          // a warp's slot: its rows' code bytes, then 16 scale bytes per row
+    constexpr uint32_t SIDE = 32 * (STEP + Conv::HI), SLOT = SIDE + 512 + (Conv::PAIRED ? 512 : 0); // a warp's slot: its rows' code bytes, then 16 scale bytes per row (Q6_K: and 16 that hold d)
     const int cw = warp - CONV_WARP0;
     const int r0 = (cw & 3) * 32, r = r0 + lane, g = cw >> 2;
     const int sw = r & 7;
@@ -509,11 +553,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
         const bool ok = grow < n;
         cp_async16(dst + (uint32_t)(rw * STEP + ((c ^ (rw & (CPR - 1))) << 4)), p.src[0] + (size_t)(ok ? grow : n - 1) * p.row_bytes[0] + in_row, ok ? bytes : 0u);
       }
-      { // the rows' 16 scale bytes of the step: the head of the Q4_K super-block, or eight f16 block scales
+      if constexpr (Conv::HI > 0) { // Q6_K: the qh bytes, then the 16 bytes that hold the super-block's f16 d
+        constexpr int HPR = Conv::HI / 16;
+#pragma unroll
+        for (int q = 0; q < HPR; q++) {
+          const int rw = q * (32 / HPR) + lane / HPR, hc = lane % HPR;
+          const int64_t grow = min((int64_t)l_tile * TILE_N + r0 + rw, n - 1);
+          cp_async16(dst + 32 * STEP + (uint32_t)(rw * Conv::HI + ((hc ^ (rw & (HPR - 1))) << 4)), p.w.qh + (size_t)grow * (p.row_bytes[0] / 2) + (uint32_t)l_kt * Conv::HI + hc * 16, 16u);
+        }
+        const int64_t grow = min((int64_t)l_tile * TILE_N + r, n - 1);
+        cp_async16(dst + SIDE + 512 + lane * 16, p.w.d + grow * p.w.dstride + (l_kt & ~7), 16u);
+      }
+      { // the rows' 16 scale bytes of the step: the head of the Q4_K super-block, eight f16 block scales, or the sixteen int8 scales of Q6_K
         const int st = p.nstreams - 1;
         const int64_t grow = (int64_t)l_tile * TILE_N + r;
         const bool ok = grow < n && (uint32_t)l_kt * p.step_bytes[st] + 16 <= p.row_bytes[st];
-        cp_async16(dst + 32 * STEP + lane * 16, p.src[st] + (size_t)(grow < n ? grow : n - 1) * p.row_bytes[st] + (ok ? (size_t)l_kt * p.step_bytes[st] : 0), ok ? 16u : 0u);
+        cp_async16(dst + SIDE + lane * 16, p.src[st] + (size_t)(grow < n ? grow : n - 1) * p.row_bytes[st] + (ok ? (size_t)l_kt * p.step_bytes[st] : 0), ok ? 16u : 0u);
       }
       l_i += 2, l_kt += 2;
       while (l_kt >= KT) l_kt -= KT, l_tile++;
@@ -534,7 +589,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
       { // hand the row's 16 scale bytes to the drain
         if (i >= SIDE_STAGES) alive = mbar_wait_warp(side_empty + 8 * ss, ((i / SIDE_STAGES) - 1) & 1, 2u);
         if (!alive) break;
-        const uint4 hv = lds128(slot + 32 * STEP + lane * 16);
+        const uint4 hv = lds128(slot + SIDE + lane * 16);
+        if constexpr (Conv::PAIRED) { // the super-block's d, widened, behind the records
+          const int sb = (kt0 + i) % KT;
+          const uint32_t dd = lds32(slot + SIDE + 512 + lane * 16 + 4 * ((sb >> 1) & 3));
+          const float d = __half2float(__ushort_as_half((unsigned short)((sb & 1) ? (dd >> 16) : (dd & 0xffffu))));
+          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + p.side_off + ss * p.side_stage_bytes + HDR_BYTES + (uint32_t)(NP * 32) + (uint32_t)r * 4), "f"(d) : "memory");
+        }
         sts128(base + p.side_off + ss * p.side_stage_bytes + (uint32_t)r * 16, hv);
         __syncwarp();
         if (lane == 0) mbar_arrive(side_full + 8 * ss);
@@ -544,8 +605,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         uint4 lo[4], hi[4];
-        Conv::run(slot + (uint32_t)lane * STEP, lane, h, 0, lo);
-        Conv::run(slot + (uint32_t)lane * STEP, lane, h, 1, hi);
+        if constexpr (Conv::HI > 0) {
+          Conv::run(slot + (uint32_t)lane * STEP, slot + 32 * STEP + (uint32_t)(lane * Conv::HI), lane, h, 0, lo);
+          Conv::run(slot + (uint32_t)lane * STEP, slot + 32 * STEP + (uint32_t)(lane * Conv::HI), lane, h, 1, hi);
+        } else {
+          Conv::run(slot + (uint32_t)lane * STEP, lane, h, 0, lo);
+          Conv::run(slot + (uint32_t)lane * STEP, lane, h, 1, hi);
+        }
         const uint32_t dst_row = base + p.a_off + (2 * bs + h) * A_STAGE_BYTES + (uint32_t)r * 128;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
@@ -585,7 +651,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
       if (alive) alive = mbar_wait_warp(side_full + 8 * ss, (i / SIDE_STAGES) & 1, 8u);
       const uint32_t side = base + p.side_off + ss * p.side_stage_bytes;
       uint4 hdr = make_uint4(0, 0, 0, 0);
+      float dw = 0.f;
       if (alive) hdr = lds128(side + (uint32_t)(32 * q + lane) * 16);
+      if (Conv::PAIRED && alive) dw = __uint_as_float(lds32(side + HDR_BYTES + (uint32_t)(NP * 32 + (32 * q + lane) * 4)));
       if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap), a_ph, 8u);
       if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap + 1), a_ph, 8u);
       if (alive) {
@@ -594,15 +662,28 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
 #pragma unroll
         for (int ch = 0; ch < NPT / CH; ch++) {
           uint32_t v[8][CH];
+          if constexpr (Conv::PAIRED) {
+            int isum[CH] = {};
 #pragma unroll
-          for (int j = 0; j < 8; j++) tmem_ld<CH>(taddr + (uint32_t)(j * NP + ch * CH), v[j]);
-          tmem_ld_wait();
+            for (int h = 0; h < 2; h++) {
+#pragma unroll
+              for (int j = 0; j < 8; j++) tmem_ld<CH>(taddr + (uint32_t)(h * BUF_COLS + (j >> 1) * NP + (j & 1) * ROWS + ch * CH), v[j]);
+              tmem_ld_wait();
+              q6k_sums<CH>(hdr, h, v, isum);
+            }
+#pragma unroll
+            for (int c = 0; c < CH; c++) acc[ch * CH + c] += (dw * __uint_as_float(lds32(side + HDR_BYTES + (uint32_t)(c0 + ch * CH + c) * 32 + 16))) * (float)isum[c];
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) tmem_ld<CH>(taddr + (uint32_t)(j * NP + ch * CH), v[j]);
+            tmem_ld_wait();
+          }
           if (ch == NPT / CH - 1) { // every value of the buffers this warp needs is in registers: they may be overwritten
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + 8 * (2 * nb)), mbar_arrive(acc_empty + 8 * (2 * nb + 1));
           }
-          Drain<CH>::run(hdr, side + HDR_BYTES, c0 + ch * CH, v, acc + ch * CH);
+          if constexpr (!Conv::PAIRED) Drain<CH>::run(hdr, side + HDR_BYTES, c0 + ch * CH, v, acc + ch * CH);
         }
       }
       __syncwarp();
@@ -628,7 +709,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
         } else {
           // this CTA's first segment (it starts where the CTA's range starts) uses scratch slot 2c, a later one 2c + 1
           const int seg_u0 = tile * KT + seg_kt0;
-          float *mine = p.partials + ((size_t)2 * blockIdx.x + (seg_u0 == u0 ? 0 : 1)) * NP * TILE_N;
+          float *mine = p.partials + ((size_t)2 * blockIdx.x + (seg_u0 == u0 ? 0 : 1)) * ROWS * TILE_N;
 #pragma unroll
           for (int c = 0; c < NPT; c++) mine[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
           __threadfence();
@@ -647,7 +728,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
             for (int c = 0; c < NPT; c++) sum[c] = 0.f;
             for (int cc = c_first; cc <= c_last; cc++) {
               const int cu0 = cta_first_unit(cc, p.units_q, p.units_r);
-              const float *part = p.partials + ((size_t)2 * cc + (cu0 >= t_u0 ? 0 : 1)) * NP * TILE_N;
+              const float *part = p.partials + ((size_t)2 * cc + (cu0 >= t_u0 ? 0 : 1)) * ROWS * TILE_N;
 #pragma unroll
               for (int c = 0; c < NPT; c++) sum[c] += __ldcg(part + (size_t)(c0 + c) * TILE_N + 32 * q + lane);
             }
@@ -1052,7 +1133,7 @@ __global__ void __launch_bounds__(F_NTHREADS, 1) imma_q4k_fold_kernel(const __gr
 template <int ACT, typename XT>
 __global__ void __launch_bounds__(256) imma_prepare(const XT *__restrict__ x, const int8_t *__restrict__ img_q, const float *__restrict__ img_d,
                                                     const int16_t *__restrict__ img_b, int64_t m, int64_t k, int64_t ldx, int NP, int nsteps,
-                                                    uint8_t *__restrict__ bimg, uint8_t *__restrict__ meta, unsigned int *__restrict__ tile_cnt, int tiles) {
+                                                    uint8_t *__restrict__ bimg, uint8_t *__restrict__ meta, unsigned int *__restrict__ tile_cnt, int tiles, int paired) {
   pdl_launch_dependents(); // the matmul kernel may start its set-up and its weight loads now
   pdl_wait();              // x may be the previous kernel's output; the scratch may still be read by the previous call
   const int row = blockIdx.x;
@@ -1090,7 +1171,13 @@ __global__ void __launch_bounds__(256) imma_prepare(const XT *__restrict__ x, co
       const int64_t hs = k8 >> 7;
       const int chunk = (int)((k8 & 127) >> 4);
       uint8_t *dst = bimg + (size_t)hs * (NP * 128) + (size_t)(row >> 3) * 1024 + (size_t)(row & 7) * 128 + (size_t)((chunk ^ (row & 7)) << 4) + (k8 & 8);
-      *reinterpret_cast<uint2 *>(dst) = make_uint2(lo, hi);
+      if (paired) { // column `row` holds the first 16 of every 32 elements, column NP / 2 + row (a multiple of 8 further on) the others
+        uint8_t *dst2 = dst + (size_t)(NP / 2 >> 3) * 1024;
+        *reinterpret_cast<uint2 *>((chunk & 1) ? dst2 : dst) = make_uint2(lo, hi);
+        *reinterpret_cast<uint2 *>((chunk & 1) ? dst : dst2) = make_uint2(0u, 0u);
+      } else {
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(lo, hi);
+      }
       uint32_t *rec = reinterpret_cast<uint32_t *>(meta + ((size_t)(k8 >> 8) * NP + row) * 32);
       if (ACT == XNQ_Q8_0) {
         if ((lane & 3) == 0) rec[(k8 & 255) >> 5] = __float_as_uint(d); // eight f32 block scales (0 beyond k)
@@ -1120,15 +1207,16 @@ __global__ void __launch_bounds__(256) imma_prepare(const XT *__restrict__ x, co
 }
 
 int g_sms = 0;
-std::atomic<int> g_fold{1}; // Q4_K, imma_q4k_fold_kernel: 0 never, 1 for the batch sizes it is faster at, 2 whenever the weight is Q4_K
+std::atomic<int> g_fold{0}; // Q4_K, imma_q4k_fold_kernel: 2 whenever the weight is Q4_K, else never
 
 struct Plan {
   int NP, nsteps, tiles, grid;
   size_t bimg_bytes, meta_bytes, cnt_bytes, part_bytes, pair_bytes;
 };
-Plan plan_for(int64_t m, int64_t k, int64_t n, bool operand = false) { // operand images have their own row counts (operand_np)
+// operand images have their own row counts (operand_np); paired: two operand columns per row
+Plan plan_for(int64_t m, int64_t k, int64_t n, bool operand, bool paired) {
   Plan pl{};
-  pl.NP = operand ? operand_np(m) : (int)((m + 15) / 16 * 16);
+  pl.NP = operand ? operand_np(m) : (int)((m + 15) / 16 * 16) * (paired ? 2 : 1);
   pl.nsteps = (int)((k + 255) / 256);
   pl.tiles = (int)((n + TILE_N - 1) / TILE_N);
   const long long units = (long long)pl.tiles * pl.nsteps;
@@ -1156,7 +1244,9 @@ int launch_np(const ImmaArgs &a, int NP, unsigned grid, cudaStream_t s) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 16>, a));
+  if constexpr (Conv::PAIRED) { // 16 rows, 32 columns
+    XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 32>, a));
+  } else if (NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 16>, a));
   else if (NP == 32) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 32>, a));
   else if (NP == 48) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 48>, a));
   else XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 64>, a));
@@ -1166,10 +1256,12 @@ int launch_np(const ImmaArgs &a, int NP, unsigned grid, cudaStream_t s) {
 
 template <typename Conv, template <int> class Drain>
 int init_np() {
-  XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+  if constexpr (!Conv::PAIRED) {
+    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 48>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+  }
   XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 48>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   return XNQ_OK;
 }
 
@@ -1177,14 +1269,19 @@ int init_np() {
 
 bool imma_supported(const WeightView &w, int64_t m) {
   if (g_sms <= 0 || m < 1 || w.n < 1) return false;
-  if (w.dtype != XNQ_Q4_0 && w.dtype != XNQ_Q8_0 && w.dtype != XNQ_Q4K) return false;
+  if (w.dtype == XNQ_Q6K) {
+    if (m < Q6K_MIN_M || m > Q6K_MAX_M) return false;
+  } else if (w.dtype != XNQ_Q4_0 && w.dtype != XNQ_Q8_0 && w.dtype != XNQ_Q4K) {
+    return false;
+  }
   if (((w.n + TILE_N - 1) / TILE_N) * ((w.k + 255) / 256) >= (1ll << 30)) return false; // the (tile, step) space is indexed with 32-bit integers
   return true;
 }
 
 // scratch of one call: the activations' operand image and records, the split tiles' tickets and partial sums
 size_t imma_workspace_bytes(int64_t m, int64_t k, int64_t n) {
-  const Plan pl = plan_for(std::min<int64_t>(m, MAX_NP), k, n, true); // an operand image may have more rows than the float form
+  // the widest operand any form of these rows takes: two columns per row up to 16 rows (Q6_K), an operand image's count above
+  const Plan pl = m <= Q6K_MAX_M ? plan_for(m, k, n, false, true) : plan_for(std::min<int64_t>(m, MAX_NP), k, n, true, false);
   return pl.bimg_bytes + pl.meta_bytes + pl.cnt_bytes + pl.part_bytes + pl.pair_bytes + 256;
 }
 
@@ -1194,16 +1291,18 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
   const int64_t k = w.k;
   const int act = act_dtype_for(w.dtype);
   const size_t yes = type_size(y_dtype);
-  // Q4_K: sub-block scales folded into the weight operand. Measured on the 14336 x 4096 weight: as fast as the per-block
-  // kernel up to 16 rows, 8 % faster for 17..32, slower beyond (it runs in passes of 32 rows), so by default it takes 17..32.
+  // Q4_K with the sub-block scales folded into the weight operand is kept behind the option: it needs half the slices to drain but
+  // twice the MMAs, and since the per-block kernel issues its MMAs at the tensor core's rate that is nowhere faster (14336 x 4096,
+  // 32 rows: 28.7 us against 26.4; 4096 x 4096: 22.4 against 14.7).
   const int fold_opt = g_fold.load(std::memory_order_relaxed);
-  const bool fold = w.dtype == XNQ_Q4K && (fold_opt == 2 || (fold_opt == 1 && m > 16 && m <= 32)) && !(x_dtype == XNQ_ACT_OPERAND && m > 32); // an operand image is one pass
+  const bool fold = w.dtype == XNQ_Q4K && fold_opt == 2 && !(x_dtype == XNQ_ACT_OPERAND && m > 32); // an operand image is one pass
+  const bool paired = w.dtype == XNQ_Q6K;
   const int64_t pass_rows = fold ? 32 : MAX_NP;
   const bool operand = x_dtype == XNQ_ACT_OPERAND; // the activations arrive in the kernel's own layout, with their ticket words: no activation kernel
-  if (operand && (act != XNQ_Q8K || k % 256 || m > pass_rows)) return fail(XNQ_ERR_UNSUPPORTED, "imma: an operand image serves Q8_K activations of one pass (m = %lld)", (long long)m);
+  if (operand && (w.dtype != XNQ_Q4K || k % 256 || m > pass_rows)) return fail(XNQ_ERR_UNSUPPORTED, "imma: an operand image serves Q8_K activations of one pass (m = %lld)", (long long)m);
   for (int64_t r0 = 0; r0 < m; r0 += pass_rows) { // passes of at most 64 (32) activation rows
     const int64_t rows = std::min<int64_t>(pass_rows, m - r0);
-    const Plan pl = plan_for(rows, k, w.n, operand);
+    const Plan pl = plan_for(rows, k, w.n, operand, paired);
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     uint8_t *bimg = ws;
     uint8_t *meta = bimg + pl.bimg_bytes;
@@ -1227,11 +1326,11 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     }
     // The CTAs are started while the previous kernel drains, and the first SM that is free would take eight of them (3.9 us instead of
     // 1.3): unused shared memory keeps them apart.
-    const dim3 prep_grid((unsigned)pl.NP, (unsigned)std::min<int64_t>(16, (k + 2047) / 2048));
+    const dim3 prep_grid((unsigned)(paired ? pl.NP / 2 : pl.NP), (unsigned)std::min<int64_t>(16, (k + 2047) / 2048));
     const size_t spread = MAX_SPREAD / ((prep_grid.x * prep_grid.y + 147) / 148) / 1024 * 1024;
 #define XNQ_IMMA_PREP(ACT, XT)                                                                                                          \
   XNQ_CUDA(launch_pdl(imma_prepare<ACT, XT>, prep_grid, dim3(256), spread, s,     \
-                      iq ? nullptr : static_cast<const XT *>(x) + r0 * ldx, iq, id, ib, rows, k, ldx, pl.NP, pl.nsteps, bimg, meta, cnt, pl.tiles))
+                      iq ? nullptr : static_cast<const XT *>(x) + r0 * ldx, iq, id, ib, rows, k, ldx, pl.NP, pl.nsteps, bimg, meta, cnt, pl.tiles, paired ? 1 : 0))
     if (operand) {
       // nothing to prepare
     } else if (act == XNQ_Q8_0) {
@@ -1274,6 +1373,10 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
         a.nstreams = 2, a.src[0] = w.qs, a.row_bytes[0] = (uint32_t)(k / 2), a.step_bytes[0] = 128, a.code_off = 0, step_code = ConvQ4_0::STEP;
         a.src[1] = reinterpret_cast<const uint8_t *>(w.d), a.row_bytes[1] = (uint32_t)(w.dstride * 2), a.step_bytes[1] = 16;
         break;
+      case XNQ_Q6K: // a row's qh bytes are half its ql bytes; they and d are addressed from the weight itself
+        a.nstreams = 2, a.src[0] = w.qs, a.row_bytes[0] = (uint32_t)(k / 2), a.step_bytes[0] = 128, a.code_off = 0, step_code = ConvQ6K::STEP + ConvQ6K::HI + 16;
+        a.src[1] = reinterpret_cast<const uint8_t *>(w.sc), a.row_bytes[1] = (uint32_t)(k / 16), a.step_bytes[1] = 16;
+        break;
       default: return fail(XNQ_ERR_DTYPE, "imma: dtype %d", w.dtype);
     }
     {
@@ -1314,7 +1417,7 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     }
     a.raw_stage_bytes = (uint32_t)(CONV_WARPS / 2) * (32u * (uint32_t)step_code + 512u); // a step in flight: four warp slots of the rows' code bytes and 16 scale bytes per row
     a.b_stage_bytes = (uint32_t)pl.NP * 256;
-    a.side_stage_bytes = HDR_BYTES + (uint32_t)pl.NP * 32;
+    a.side_stage_bytes = HDR_BYTES + (uint32_t)pl.NP * 32 + (paired ? TILE_N * 4 : 0);
     // shared-memory plan: A stages (half steps) | B stages (half as many whole steps) | side stages | raw stages. The MMA
     // issuer bounds a step, so the converters and the drain need little slack (six half steps of operand image); what remains
     // goes to raw stages, which hide the memory latency.
@@ -1340,6 +1443,7 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     profile_mark(s, true);
     if (w.dtype == XNQ_Q4K) rc = launch_np<ConvQ4K, DrainQ4K>(a, pl.NP, (unsigned)pl.grid, s);
     else if (w.dtype == XNQ_Q8_0) rc = launch_np<ConvQ8_0, DrainBlockScaled>(a, pl.NP, (unsigned)pl.grid, s);
+    else if (w.dtype == XNQ_Q6K) rc = launch_np<ConvQ6K, DrainQ6K>(a, pl.NP, (unsigned)pl.grid, s);
     else rc = launch_np<ConvQ4_0, DrainBlockScaled>(a, pl.NP, (unsigned)pl.grid, s);
     profile_mark(s, false);
     if (rc != XNQ_OK) return rc;
@@ -1356,6 +1460,7 @@ int imma_init(int device) {
   XNQ_CUDA(cudaFuncSetAttribute(imma_q4k_fold_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   XNQ_CUDA(cudaFuncSetAttribute(imma_q4k_fold_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   if ((rc = init_np<ConvQ8_0, DrainBlockScaled>()) != XNQ_OK) return rc;
+  if ((rc = init_np<ConvQ6K, DrainQ6K>()) != XNQ_OK) return rc;
   if ((rc = init_np<ConvQ4_0, DrainBlockScaled>()) != XNQ_OK) return rc;
 #define XNQ_IMMA_PREP_INIT(ACT, XT) XNQ_CUDA(cudaFuncSetAttribute(imma_prepare<ACT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SPREAD))
   XNQ_IMMA_PREP_INIT(XNQ_Q8_0, float);
