@@ -288,6 +288,10 @@ int xnq_swiglu(const float *gate_up, float *out, void *act_image, int act_dtype,
 int xnq_rope_kv_store(const float *qkv, const float *cos_table, const float *sin_table, const long long *pos_dev,
                       float *q_out, void *k_cache, void *v_cache, int64_t batch, int heads, int kv_heads,
                       int head_dim, int64_t max_seq, void *stream);
+/* The same for a whole prompt at positions 0 .. seq - 1 of every sequence: qkv[batch, seq, (heads + 2 kv_heads) * head_dim] f32,
+ * q_out[batch, heads, seq, head_dim] bf16. seq <= max_seq, head_dim a multiple of 8. */
+int xnq_rope_kv_store_prompt(const float *qkv, const float *cos_table, const float *sin_table, void *q_out, void *k_cache, void *v_cache,
+                             int64_t batch, int64_t seq, int heads, int kv_heads, int head_dim, int64_t max_seq, void *stream);
 /* Single-query attention over cache positions 0..*pos_dev: out[batch, heads, head_dim] =
  * softmax(q k^T / sqrt(head_dim)) v with heads / kv_heads query heads per KV head. head_dim 128. The
  * sequence is split over several CTAs per head; `workspace` (xnq_attn_decode_workspace_bytes, zeroed

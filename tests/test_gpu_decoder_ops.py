@@ -232,3 +232,29 @@ def test_activation_images_equal_the_in_call_quantizer():
                 assert torch.equal(w.matmul_t(img3), w.matmul_t(h)), (dt.name, k, m, "swiglu")
     with pytest.raises(ValueError):
         w.matmul_t(ops.ActImage.for_weight(D.Q8_0, 1, 14336, DEV))   # a Q8_0 image does not fit a Q4_K weight
+
+
+@pytest.mark.parametrize("B,S,H,KV,hd", [(1, 1, 4, 4, 128), (2, 17, 4, 2, 128), (1, 256, 8, 1, 128), (3, 5, 6, 2, 64), (1, 7, 2, 1, 8)])
+def test_prompt_rope_and_cache_store_are_the_torch_operations_bits(B, S, H, KV, hd):
+    """q, the rotated k and the plain v of a prompt equal separate rounded operations bit for bit; cache rows past it are untouched."""
+    from xn_b200 import decoder_ops as ops
+    max_seq = 256
+    g = torch.Generator(device="cpu"); g.manual_seed(100 * S + H)
+    qkv = torch.randn(B, S, (H + 2 * KV) * hd, generator=g).to(DEV)
+    ang = torch.arange(max_seq, dtype=torch.float32)[:, None] / 10000.0 ** (torch.arange(0, hd, 2, dtype=torch.float32) / hd)[None]
+    cos, sin = ang.cos().to(DEV), ang.sin().to(DEV)
+    kc = torch.full((B, KV, max_seq, hd), 7.0, dtype=torch.bfloat16, device=DEV)
+    vc = kc.clone()
+    got = ops.rope_kv_store_prompt(qkv, cos, sin, kc, vc, H, KV)
+    q, k, v = qkv.split([H * hd, KV * hd, KV * hd], dim=-1)
+
+    def rot(t, heads):
+        t = t.view(B, S, heads, hd)
+        x1, x2 = t[..., :hd // 2], t[..., hd // 2:]
+        c, s = cos[:S, None], sin[:S, None]
+        return torch.cat([x1 * c - x2 * s, x2 * c + x1 * s], -1).to(torch.bfloat16).transpose(1, 2)
+    assert torch.equal(got, rot(q, H)) and torch.equal(kc[:, :, :S], rot(k, KV))
+    assert torch.equal(vc[:, :, :S], v.view(B, S, KV, hd).to(torch.bfloat16).transpose(1, 2))
+    assert bool((kc[:, :, S:] == 7).all()) and bool((vc[:, :, S:] == 7).all())
+    with pytest.raises(ValueError):
+        ops.rope_kv_store_prompt(qkv[..., :-hd].contiguous(), cos, sin, kc, vc, H, KV)

@@ -183,3 +183,20 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
         _lib.check(L.xnq_attn_decode(_p(q), _p(k_cache), _p(v_cache), _p(pos), _p(out), B, heads, kv_heads, hd, max_seq, _p(ws), ws.numel(),
                                      _stream_ptr(q.device)))
     return out
+
+
+def rope_kv_store_prompt(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, heads: int, kv_heads: int) -> torch.Tensor:
+    """A whole prompt at positions 0 .. S - 1: rotate q and k, store k and v (bf16) into the caches ``[B, kv_heads, max_seq, hd]``.
+    ``qkv`` is ``[B, S, (heads + 2 kv_heads) * hd]``; returns q as ``[B, heads, S, hd]`` bf16 (xnq_rope_kv_store_prompt)."""
+    _f32c(qkv, cos, sin)
+    B, S, width = qkv.shape
+    Bc, kvc, max_seq, hd = k_cache.shape
+    if k_cache.dtype is not torch.bfloat16 or not k_cache.is_contiguous() or v_cache.dtype is not torch.bfloat16 or not v_cache.is_contiguous() or v_cache.shape != k_cache.shape:
+        raise ValueError("rope_kv_store_prompt: caches must be contiguous bf16 [B, kv_heads, max_seq, hd]")
+    if Bc != B or kvc != kv_heads or width != (heads + 2 * kv_heads) * hd or min(cos.shape[0], sin.shape[0]) < S or cos.shape[1] != hd // 2 or sin.shape[1] != hd // 2:
+        raise ValueError(f"rope_kv_store_prompt: qkv {tuple(qkv.shape)} does not fit caches {tuple(k_cache.shape)}")
+    q = torch.empty((B, heads, S, hd), dtype=torch.bfloat16, device=qkv.device)
+    with torch.cuda.device(qkv.device):
+        _lib.check(_lib.lib().xnq_rope_kv_store_prompt(_p(qkv), _p(cos), _p(sin), _p(q), _p(k_cache), _p(v_cache), B, S, heads, kv_heads, hd, max_seq,
+                                                       _stream_ptr(qkv.device)))
+    return q

@@ -16,7 +16,7 @@ Tensor parallelism over ``world`` ranks (one process per GPU):
     its summand into every rank's buffer; the next residual-add + RMSNorm adds the summands;
   * the LM head is N-sharded and its output columns are gathered the same way.
 
-Prefill runs RMSNorm, RoPE and attention as torch ops. A decode step uses the library's fused operators
+Prefill runs RMSNorm and attention as torch ops (its RoPE + KV-cache store and SwiGLU are the library's). A decode step uses the library's fused operators
 between the linears (residual-add + RMSNorm, RoPE + KV-cache store, single-query attention, SwiGLU), so
 one layer is ten launches and the whole step is one CUDA graph.
 """
@@ -228,11 +228,27 @@ class QLlama:
         x1, x2 = x[..., : x.shape[-1] // 2], x[..., x.shape[-1] // 2:]
         return torch.cat([x1 * cos - x2 * sin, x2 * cos + x1 * sin], dim=-1)
 
-    def _block(self, L: _Layer, x: torch.Tensor, pos_idx: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
-        """x [B, S, d]; pos_idx [S] int64 positions of these tokens; mask broadcastable to [B, H, S, max_seq]."""
-        c, hd = self.cfg, self.cfg.head_dim
+    def _block(self, L: _Layer, x: torch.Tensor, pos_idx: torch.Tensor, mask: torch.Tensor, prompt: bool) -> torch.Tensor:
+        """x [B, S, d]; pos_idx [S] int64 positions of these tokens; mask broadcastable to [B, H, S, max_seq]. ``prompt``: the
+        positions are 0 .. S - 1."""
         B, S, _ = x.shape
         qkv = L.wqkv.matmul_t(self._rms(x, L.norm1))
+        if prompt and self.cfg.head_dim % 8 == 0:
+            q = ops.rope_kv_store_prompt(qkv, self.cos, self.sin, L.k_cache, L.v_cache, self.hl, self.kvl)
+        else:
+            q = self._rope_store(L, qkv, pos_idx)
+        a = F.scaled_dot_product_attention(q, L.k_cache, L.v_cache, attn_mask=mask, enable_gqa=True)
+        a = a.transpose(1, 2).reshape(B, S, self.hl * self.cfg.head_dim).float()
+        x = x + self._sum_parts(self._linear_parts(L.wo, a))
+        f = self.cfg.ffn // self.world
+        gu = L.wgu.matmul_t(self._rms(x, L.norm2)).view(B * S, 2 * f)
+        h = ops.swiglu(gu, torch.empty((B * S, f), device=self.device)).view(B, S, f)
+        return x + self._sum_parts(self._linear_parts(L.wdown, h))
+
+    def _rope_store(self, L: _Layer, qkv: torch.Tensor, pos_idx: torch.Tensor) -> torch.Tensor:
+        """q and k rotated at ``pos_idx``, k and v stored into the caches at these positions; returns q [B, H, S, hd] bf16."""
+        hd = self.cfg.head_dim
+        B, S, _ = qkv.shape
         q, k, v = qkv.split([self.hl * hd, self.kvl * hd, self.kvl * hd], dim=-1)
         q = q.view(B, S, self.hl, hd).transpose(1, 2)
         k = k.view(B, S, self.kvl, hd).transpose(1, 2)
@@ -241,22 +257,16 @@ class QLlama:
         q, k = self._rope(q, cos, sin), self._rope(k, cos, sin)
         L.k_cache.index_copy_(2, pos_idx, k.to(torch.bfloat16))
         L.v_cache.index_copy_(2, pos_idx, v.to(torch.bfloat16))
-        a = F.scaled_dot_product_attention(q.to(torch.bfloat16), L.k_cache, L.v_cache, attn_mask=mask, enable_gqa=True)
-        a = a.transpose(1, 2).reshape(B, S, self.hl * hd).float()
-        x = x + self._sum_parts(self._linear_parts(L.wo, a))
-        gu = L.wgu.matmul_t(self._rms(x, L.norm2))
-        g, u = gu.split(c.ffn // self.world, dim=-1)
-        x = x + self._sum_parts(self._linear_parts(L.wdown, F.silu(g) * u))
-        return x
+        return q.to(torch.bfloat16)
 
-    def _forward(self, tokens: torch.Tensor, pos_idx: torch.Tensor) -> torch.Tensor:
-        """tokens [B, S] -> logits of the last position [B, vocab]."""
+    def _forward(self, tokens: torch.Tensor, pos_idx: torch.Tensor, prompt: bool = False) -> torch.Tensor:
+        """tokens [B, S] -> logits of the last position [B, vocab]. ``prompt``: the positions are 0 .. S - 1."""
         self._gather_idx = 0
         ar = torch.arange(self.max_seq, device=self.device)
         mask = (ar[None, :] <= pos_idx[:, None])[None, None]  # [1, 1, S, max_seq]: causal over the cache
         x = self.embed.index_select(0, tokens.reshape(-1)).view(*tokens.shape, -1).float()
         for L in self.layers:
-            x = self._block(L, x, pos_idx, mask)
+            x = self._block(L, x, pos_idx, mask, prompt)
         x = self._rms(x[:, -1:, :], self.norm)
         logits = self._linear_gathered(self.lm_head, x).view(tokens.shape[0], -1)
         return logits if self.pg is None else logits.clone()   # out of the exchange slot before it is reused
@@ -315,8 +325,9 @@ class QLlama:
     def prefill(self, prompt: torch.Tensor) -> torch.Tensor:
         """prompt [B, S] token ids; fills the cache, sets the decode position, returns the last logits."""
         B, S = prompt.shape
-        pos_idx = torch.arange(S, device=self.device)
-        logits = self._forward(prompt, pos_idx)
+        if S > self.max_seq:
+            raise ValueError(f"a prompt of {S} tokens does not fit the cache of {self.max_seq} positions")
+        logits = self._forward(prompt, torch.arange(S, device=self.device), prompt=S > 0)
         self.pos.fill_(S)
         self.tokens.copy_(logits.argmax(-1))
         return logits
