@@ -229,9 +229,6 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float *gu, float *out
 // step's first kernel, and everything behind it may rely on the previous step's stores (position, tokens, cache rows) being complete.
 __global__ void __launch_bounds__(256) embed_rows_kernel(const __nv_bfloat16 *table, const long long *tokens, float *x, int d, long long vocab);
 
-// tokens[row] = index of the first largest logit of the row (torch.argmax's rule), then *pos += 1 (one thread). One CTA per row.
-__global__ void __launch_bounds__(256) argmax_advance_kernel(const float *logits, long long n, long long *tokens, long long *pos);
-
 __device__ unsigned int g_decoder_status; // sticky: 1 rope/store, 2 attention saw a position outside [0, max_seq), 4 an embedding token outside the table
 
 __global__ void __launch_bounds__(256) embed_rows_kernel(const __nv_bfloat16 *table, const long long *tokens, float *x, int d, long long vocab) {
@@ -252,18 +249,37 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const __nv_bfloat16 *ta
   }
 }
 
-__global__ void __launch_bounds__(256) argmax_advance_kernel(const float *logits, long long n, long long *tokens, long long *pos) {
-  __shared__ float s_v[8];
-  __shared__ long long s_i[8];
+// tokens[row] = index of the first largest logit of the row (torch.argmax's rule), then *pos += 1 (one thread). One CTA per row.
+constexpr int ARGMAX_THREADS = 1024;
+__global__ void __launch_bounds__(ARGMAX_THREADS) argmax_advance_kernel(const float *logits, long long n, long long *tokens, long long *pos) {
+  __shared__ float s_v[ARGMAX_THREADS / 32];
+  __shared__ long long s_i[ARGMAX_THREADS / 32];
   pdl_launch_dependents();
   pdl_wait(); // the logits are the previous kernel's output
   const float *row = logits + (long long)blockIdx.x * n;
   float best = -INFINITY;
   long long bi = n; // no candidate yet
-  for (long long i = threadIdx.x; i < n; i += 256) {
-    const float v = row[i];
+  auto see = [&](float v, long long i) {
     if (v > best || (v == best && i < bi)) best = v, bi = i;
+  };
+  // One CTA reads the row, so it is bound by the loads in flight: eight 16-byte loads per thread and round (32000 logits in one round
+  // of 1024 threads; 256 threads with one 4-byte load at a time took 12 us, now 5).
+  constexpr int U = 8;
+  const long long n4 = (reinterpret_cast<uintptr_t>(row) & 15) == 0 ? n / 4 : 0;
+  for (long long base = threadIdx.x; base < n4; base += U * ARGMAX_THREADS) {
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long i = base + u * ARGMAX_THREADS;
+      v[u] = *reinterpret_cast<const float4 *>(row + 4 * (i < n4 ? i : base)); // past the end: the first one again, which changes nothing
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long i = 4 * (base + u * ARGMAX_THREADS < n4 ? base + u * ARGMAX_THREADS : base);
+      see(v[u].x, i), see(v[u].y, i + 1), see(v[u].z, i + 2), see(v[u].w, i + 3);
+    }
   }
+  for (long long i = 4 * n4 + threadIdx.x; i < n; i += ARGMAX_THREADS) see(row[i], i);
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, off);
@@ -273,11 +289,18 @@ __global__ void __launch_bounds__(256) argmax_advance_kernel(const float *logits
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) s_v[warp] = best, s_i[warp] = bi;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; w++)
-      if (s_v[w] > best || (s_v[w] == best && s_i[w] < bi)) best = s_v[w], bi = s_i[w];
-    tokens[blockIdx.x] = bi < n ? bi : 0; // a row of -inf / NaN only: token 0
-    if (blockIdx.x == 0 && pos) *pos += 1;
+  if (warp == 0) {
+    best = s_v[lane], bi = s_i[lane]; // as many warps as lanes
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, off);
+      const long long oi = __shfl_xor_sync(0xffffffffu, bi, off);
+      if (ov > best || (ov == best && oi < bi)) best = ov, bi = oi;
+    }
+    if (lane == 0) {
+      tokens[blockIdx.x] = bi < n ? bi : 0; // a row of NaN only: token 0
+      if (blockIdx.x == 0 && pos) *pos += 1;
+    }
   }
 }
 
@@ -670,7 +693,7 @@ int xnq_argmax_advance(const float *logits, int64_t rows, int64_t n, long long *
   if (!logits || !tokens) return fail(XNQ_ERR_NULL, "argmax_advance: NULL argument");
   if (rows < 0 || n < 1) return fail(XNQ_ERR_SHAPE, "argmax_advance: rows = %lld, n = %lld", (long long)rows, (long long)n);
   if (rows == 0) return XNQ_OK;
-  XNQ_CUDA(launch_pdl(argmax_advance_kernel, dim3((unsigned)rows), dim3(256), 0, static_cast<cudaStream_t>(stream), logits, (long long)n, tokens, pos));
+  XNQ_CUDA(launch_pdl(argmax_advance_kernel, dim3((unsigned)rows), dim3(ARGMAX_THREADS), 0, static_cast<cudaStream_t>(stream), logits, (long long)n, tokens, pos));
   count_launch();
   return XNQ_OK;
 }
