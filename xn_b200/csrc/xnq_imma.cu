@@ -16,7 +16,7 @@
 // upper and once with the lower 16 of each 32 codes zeroed, so that one MMA yields both 16-sums; the drain multiplies the sixteen sums
 // of a super-block with the int8 scales, adds them as integers and scales once, as the CPU code does (k_quants.rs:1743-1799).
 //
-// Roles of the 27 warps of a CTA (one CTA per SM, persistent):
+// Roles of the 19 or 27 warps of a CTA (one CTA per SM, persistent):
 //   producer (1)    one thread requests, per 256-k step, the 1-D bulk copies of the quantized activations (already in
 //                   the MMA's shared-memory layout) and of their per-block metadata into rings of stages guarded by
 //                   mbarriers; when the kernel starts it also asks for the CTA's share of the weight's bytes to be
@@ -31,14 +31,9 @@
 //                   a box took 5000 to 7000 cycles to arrive, with or without the bytes in L2, about 17 cycles per box
 //                   row, which held the whole kernel at a third of the memory's rate. One bulk copy per row before
 //                   that: the copy engine takes some 60 ns per copy whatever its size.)
-//   MMA issuers (2) one thread per half step issues its four K = 32 MMAs into accumulator buffer h and commits them; an
-//                   MMA of this shape keeps its issuing thread busy for about 134 cycles whatever M (64 / 128) and
-//                   N <= 128 are, while two issuing threads reach twice the rate (measured), so the halves of a step
-//                   are issued by two warps;
-//   drain (16)      two groups of eight warps; group h owns accumulator buffer h: reads its slices back with
-//                   tcgen05.ld, scales, and keeps f32 sums in registers across the k steps of a tile; two warps
-//                   per accumulator lane quarter split the columns. At the end of a segment the odd half steps'
-//                   sums are added to the even ones' (always in that order).
+//   MMA issuers (2) one warp per half step issues its four K = 32 MMAs into accumulator buffer h and commits them;
+//   drain (16, or 8 with 16 activation rows) read the slices of a step back with tcgen05.ld, scale, and keep f32 sums in registers
+//                   across the k steps of a tile; the warps of an accumulator lane quarter split the columns.
 //
 // Work is the flattened (tile of 128 weight rows, 256-k step) space, cut into equal contiguous ranges, one
 // per CTA, so all SMs finish together however few tiles there are. A tile whose steps are split between
@@ -67,7 +62,6 @@ constexpr int64_t Q6K_MIN_M = 6, Q6K_MAX_M = 16;
 constexpr int MAX_NP = 64;          // activation rows per pass = UMMA N (multiple of 16)
 constexpr int CONV_WARPS = 8, DRAIN_WARPS = 16;
 constexpr int ACT_PRODUCER_WARP = 0, MMA_WARP = 1, CONV_WARP0 = 3, DRAIN_WARP0 = CONV_WARP0 + CONV_WARPS; // MMA issuers: warps 1 and 2
-constexpr int NTHREADS = (DRAIN_WARP0 + DRAIN_WARPS) * 32; // 864
 constexpr int A_STAGE_BYTES = TILE_N * 128; // one 128-k half step of int8 codes
 constexpr int SIDE_STAGES = 8, MAX_RAW_STAGES = 8, MAX_B_STAGES = 8; // side stages are small (scale bytes and records of one step): enough of them that
                                                                    // the converters, which fill them, never wait for the drain, which frees them
@@ -182,11 +176,6 @@ __device__ __forceinline__ void cp_async_wait(int pending) {
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ uint2 lds64(uint32_t a) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
   return v;
 }
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
@@ -417,11 +406,17 @@ struct DrainQ6K { // (the paired form has its own drain, by half steps)
   __device__ static __forceinline__ void run(const uint4 &, uint32_t, int, const uint32_t (&)[8][CH], float *) {}
 };
 
+// Drain warps: a warp's waits and its decoding of the row's scales cost as much as four columns' arithmetic; with 16 rows eight warps of
+// eight columns each do better than sixteen of four (Q6_K 32000 x 4096, 16 rows: 48.5 -> 46.4 us; Q8_0 11008 x 4096, 8 rows: 21.7 -> 20.9).
+__host__ __device__ constexpr int drain_warps(int rows) { return rows == 16 ? 8 : DRAIN_WARPS; }
+__host__ __device__ constexpr int imma_threads(int rows) { return (DRAIN_WARP0 + drain_warps(rows)) * 32; }
+
 template <typename Conv, template <int> class Drain, int NP>
-__global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant__ ImmaArgs p) {
+__global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) imma_kernel(const __grid_constant__ ImmaArgs p) {
   constexpr int ROWS = Conv::PAIRED ? NP / 2 : NP; // activation rows of the operand; NP: its columns
-  constexpr int NPT = ROWS / (DRAIN_WARPS / 4); // rows per drain thread: four warps per accumulator lane quarter split them
-  constexpr int CH = 4;                       // columns read back at a time, all eight slices of a step: what the register budget holds
+  constexpr int DW = drain_warps(ROWS);
+  constexpr int NPT = ROWS / (DW / 4); // rows per drain thread: the warps of an accumulator lane quarter split them
+  constexpr int CH = DW == 8 ? 8 : 4;  // columns read back at a time, all eight slices of a step: what the register budget holds
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand stages need 1024-byte alignment
   constexpr int NBUF = TMEM_COLS / (8 * NP) > 4 ? 8 : TMEM_COLS / (8 * NP) * 2; // accumulator buffers (even: buffer parity = half step parity)
@@ -445,9 +440,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
     for (int s = 0; s < 8; s++) {
       mbar_init(a_full + 8 * s, CONV_WARPS / 2); // the four converter warps of the step's group (one barrier per step: entries 0 .. AP - 1)
       mbar_init(mma_done + 8 * s, 1);            // the half step's MMAs have read their operands and written their slices
-      mbar_init(acc_empty + 8 * s, DRAIN_WARPS);
+      mbar_init(acc_empty + 8 * s, DW);
       mbar_init(side_full + 8 * s, 1 + CONV_WARPS / 2); // the producer's transaction + the four converter warps that copy the scale bytes
-      mbar_init(side_empty + 8 * s, DRAIN_WARPS);
+      mbar_init(side_empty + 8 * s, DW);
       mbar_init(b_full + 8 * s, 1);
       mbar_init(b_empty + 8 * s, 2); // both half steps' MMAs
     }
@@ -630,7 +625,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
     }
     cp_async_wait(0); // nothing may be in flight into this CTA's shared memory when it exits
   } else {
-    // ---- drain: warp quarter q reads accumulator lanes 32q.. (weight rows), four warps of a quarter split the columns; every warp
+    // ---- drain: warp quarter q reads accumulator lanes 32q.. (weight rows), the warps of a quarter split the columns; every warp
     // takes both half steps of every step and keeps f32 sums in registers. (Two groups of eight warps that took one half step each had
     // twice the columns per thread: at 64 rows they read them back four at a time, eight trips to tensor memory of 550 cycles per
     // half step; twice the integer-to-float conversions; and the groups' sums had to meet in memory at the end of a tile.) ----
@@ -713,11 +708,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) imma_kernel(const __grid_constant
 #pragma unroll
           for (int c = 0; c < NPT; c++) mine[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
           __threadfence();
-          asm volatile("bar.sync 1, %0;" ::"n"(DRAIN_WARPS * 32) : "memory");
+          asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
           if (et == 0) s_ticket = atomicAdd(p.tile_cnt + tile, 1u);
-          asm volatile("bar.sync 1, %0;" ::"n"(DRAIN_WARPS * 32) : "memory");
+          asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
           const unsigned int ticket = s_ticket;
-          asm volatile("bar.sync 1, %0;" ::"n"(DRAIN_WARPS * 32) : "memory"); // s_ticket may be rewritten from here on
+          asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory"); // s_ticket may be rewritten from here on
           const int t_u0 = tile * KT, t_u1 = t_u0 + KT;
           const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u1 - 1, p.units_q, p.units_r);
           if (et == 0 && (int)ticket == c_last - c_first) p.tile_cnt[tile] = 0u; // every part has its ticket: the word is zero again for the next call
@@ -1236,7 +1231,7 @@ int launch_np(const ImmaArgs &a, int NP, unsigned grid, cudaStream_t s) {
   // its weight loads are issued before griddepcontrol.wait
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(NTHREADS);
+  cfg.blockDim = dim3((unsigned)imma_threads(Conv::PAIRED ? NP / 2 : NP));
   cfg.dynamicSmemBytes = IMMA_SMEM;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
