@@ -132,3 +132,42 @@ def test_prefill_device_status_is_clean(Q):
     bits = ctypes.c_uint(123)
     _lib.check(_lib.lib().xnq_device_status(ctypes.byref(bits)))
     assert bits.value == 0, f"device status bits {bits.value:#x}"
+
+
+def _f32_bound(O, dt, w, x, n, k):
+    """What exact block sums that are scaled and added in f32 may differ by: at most two rounded terms per 32 elements on each side, of
+    partial sums that stay below sum |w| |x| (doubled for min terms that do not cancel in it)."""
+    dense = np.abs(O.to_float(int(dt), w, n * k).reshape(n, k)).astype(np.float64)
+    return 4 * (k / 16 + 8) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ dense.T + np.abs(x).max() * dense.max() * 32)
+
+
+# the integer kernel around its operand row counts (16, 32, 48, 64) and the row counts where other kernels take over, over one step,
+# a partial step, more steps than its rings have stages, and rows of a last tile
+@pytest.mark.parametrize("dt", WEIGHT_TYPES)
+@pytest.mark.parametrize("m", [4, 5, 6, 16, 17, 32, 33, 48, 49, 64])
+def test_integer_kernel_row_and_step_edges(Q, O, dt, m):
+    if dt is D.Q6K and m > 16:
+        pytest.skip("more than 16 rows of Q6_K run on fp16 operands")
+    for n, k in ((3, 256), (130, 256 * 5), (129, 256 * 13)) if dt.block_size == 256 else ((3, 32), (130, 1312), (129, 3360)):
+        w = synth.make_weight(dt, n, k, seed=m + n)
+        x = synth.make_activation(m, k, seed=m + k)
+        t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+        got = t.matmul_t(torch.from_numpy(x).to(DEV)).cpu().numpy().astype(np.float64)
+        assert (np.abs(got - O.matmul(int(dt), x, w, n)) <= _f32_bound(O, dt, w, x, n, k)).all(), (dt.name, m, n, k)
+
+
+# the fp16 kernel: one and two accumulators, tiles that end with 1 and 16 rows, k-steps that do not fill a super-step or a stage ring,
+# output types that are stored whole, a weight of less than a tile and one row more than a tile
+@pytest.mark.parametrize("dt", WEIGHT_TYPES)
+@pytest.mark.parametrize("m", [65, 128, 129, 257, 513])
+def test_fp16_kernel_tile_and_step_edges(Q, O, dt, m):
+    for n, k in ((3, 256), (129, 256 * 5)) if dt.block_size == 256 else ((3, 32), (129, 96), (40, 1312)):
+        w = synth.make_weight(dt, n, k, seed=m + n)
+        x = synth.make_activation(m, k, seed=m + k)
+        t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+        xd = torch.from_numpy(x).to(DEV)
+        want = O.matmul(int(dt), x, w, n)
+        got = t.matmul_t(xd)
+        _check(got.cpu().numpy(), want, f"{dt.name} m={m} n={n} k={k}")
+        half = t.matmul_t(xd, out=torch.empty(m, n, dtype=torch.float16, device=DEV))
+        assert torch.allclose(half.float(), got, rtol=2.0 ** -10, atol=1e-4 * float(got.abs().max()))   # rounded once; parts of a split tile may meet in another order
