@@ -68,17 +68,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 // One wait attempt during which the hardware may keep the thread suspended for up to `ns` nanoseconds (it takes no issue slots).
 __device__ __forceinline__ bool mbar_suspend(uint32_t bar, uint32_t parity, uint32_t ns) {
   uint32_t ok;
@@ -334,7 +323,6 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     constexpr int KPS = RowT::KPS, NCOPY = (32 * RowT::ITEMS + 127) / 128;
     const int rg = warp & 3, kg = warp >> 2;
     const int kk = kg % KPS, hf = kg / KPS; // this warp's k-step of a super-step; which half of it (KPS = 2)
-    const int r = 32 * rg + lane;
     const int t = kg * 32 + lane; // 0..127 in the row group
     const uint32_t raw = smem_base + p.raw_off + (uint32_t)(rg * 32 * RowT::ROWB);
     constexpr uint32_t SLOT = TILE_N * RowT::ROWB;
@@ -378,7 +366,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     for (int j = 0; j < R - 1; j++) issue();
-    int c_n = start.tile_n, c_m = start.tile_m, c_s = start.kt / KPS, c_slot = 0;
+    int c_s = start.kt / KPS, c_slot = 0;
     int base_i = -start.kt; // the CTA's step number of the current tile's first k-step
     int at = 0, s = 0;      // s = at % S, lap: parity of at / S, of the last step this warp looked at
     uint32_t lap = 0;
@@ -395,14 +383,12 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
           tc_fence_after();
           const uint32_t slot = raw + (uint32_t)c_slot * SLOT + (uint32_t)(lane * RowT::ROWB);
           const uint32_t dst = tmem_d + ((uint32_t)(32 * rg) << 16) + (uint32_t)(A_COL0 + s * A_COLS);
-          const bool in_w = (int64_t)c_n * TILE_N + r < p.w.n;
+          const typename RowT::Head head = RowT::head(slot, c_s, kk, p.wscale);
 #pragma unroll
           for (int h = 0; h < KPS / 2; h++) {
             const int half = KPS == 2 ? hf : h;
             uint32_t o[16];
-            RowT::half(slot, c_s, kk, half, p.wscale, o);
-#pragma unroll
-            for (int e = 0; e < 16; e++) o[e] = in_w ? o[e] : 0u;
+            RowT::half(head, slot, kk, half, o); // a lane past the weight's last row repeats that row and is not stored
             tmem_st16(dst + 16 * half, o);
           }
           tmem_st_wait();
@@ -415,7 +401,6 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       if (++c_s == SPT) {
         c_s = 0;
         base_i += KT;
-        if (++c_m == TM) c_m = 0, c_n++;
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");

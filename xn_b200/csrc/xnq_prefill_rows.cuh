@@ -6,8 +6,9 @@
 //   item()   one of the ITEMS 16-byte copies that make up a row's super-step: where it comes from and how that moves with the
 //            super-step. Consecutive threads take consecutive copies, so that a copy instruction of a warp touches four to six runs
 //            of memory (one thread per row would touch 32).
-//   half()   reads the row's bytes of half a 64-wide k-step from the slot and dequantizes them to fp16: the 16 packed pairs that go
-//            to the row's lane of tensor memory, where the MMA reads its weight operand.
+//   head()   what the two halves of a row's 64-wide k-step share (scales, high bits)
+//   half()   reads the row's bytes of half a k-step from the slot and dequantizes them to fp16: the 16 packed pairs that go to the
+//            row's lane of tensor memory, where the MMA reads its weight operand.
 //
 // Stored k order inside a k-step (the activation image uses the same one, see kpair_shift in xnq_prefill.cu):
 //   Q8_0, Q6_K  natural
@@ -58,11 +59,15 @@ struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
     if (c < 8) return Item{w.qs + row * (w.k / 2) + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k / 2 - 16 * c)};
     return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 16u, NO_LIMIT};
   }
-  __device__ static __forceinline__ void half(uint32_t slot, int, int kk, int hf, float wscale, uint32_t (&o)[16]) { // half = one block
+  struct Head {
+    uint32_t dd;
+    float wscale;
+  };
+  __device__ static __forceinline__ Head head(uint32_t slot, int, int kk, float wscale) { return Head{lds32(slot + 128 + 4 * kk), wscale}; }
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int kk, int hf, uint32_t (&o)[16]) { // half = one block
     const uint4 q = lds128(slot + 32 * kk + 16 * hf);
-    const uint32_t dd = lds32(slot + 128 + 4 * kk);
     const __half2 off = h2_from_bits(0x64086408u); // 1032 = 1024 + 8
-    const __half2 d2 = scaled_half2(hf ? (dd >> 16) : (dd & 0xffffu), wscale);
+    const __half2 d2 = scaled_half2(hf ? (hd.dd >> 16) : (hd.dd & 0xffffu), hd.wscale);
     const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int wi = 0; wi < 4; wi++)
@@ -78,10 +83,11 @@ struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighb
     if (c < 8) return Item{w.qs + row * w.k + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k - 16 * c)};
     return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 8u, NO_LIMIT};
   }
-  __device__ static __forceinline__ void half(uint32_t slot, int ss, int kk, int hf, float wscale, uint32_t (&o)[16]) { // half = one block
+  using Head = RowQ4_0::Head;
+  __device__ static __forceinline__ Head head(uint32_t slot, int ss, int kk, float wscale) { return Head{lds32(slot + 128 + 8 * (ss & 1) + 4 * kk), wscale}; }
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int kk, int hf, uint32_t (&o)[16]) { // half = one block
     const uint4 q[2] = {lds128(slot + 64 * kk + 32 * hf), lds128(slot + 64 * kk + 32 * hf + 16)};
-    const uint32_t dd = lds32(slot + 128 + 8 * (ss & 1) + 4 * kk);
-    const __half2 d2 = scaled_half2(hf ? (dd >> 16) : (dd & 0xffffu), wscale);
+    const __half2 d2 = scaled_half2(hf ? (hd.dd >> 16) : (hd.dd & 0xffffu), hd.wscale);
     const __half2 off = h2_from_bits(0x64806480u); // 1152 = 1024 + 128
 #pragma unroll
     for (int c = 0; c < 4; c++) { // chunk = 8 codes
@@ -100,14 +106,20 @@ struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighb
 struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
   static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
   __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { return Item{w.qs + row * (w.k / QK_K) * 144 + 16 * c, 144u, NO_LIMIT}; }
-  __device__ static __forceinline__ void half(uint32_t slot, int, int g, int hf, float wscale, uint32_t (&o)[16]) { // half = words 4 hf .. of the group
-    const uint4 hdr = lds128(slot), q = lds128(slot + 16 + 32 * g + 16 * hf);
+  struct Head {
+    __half2 a_lo, a_hi, b_lo, b_hi;
+  };
+  // value = (d*sc) * code - (dmin*m): low nibbles are sub-block 2g, high nibbles sub-block 2g+1
+  __device__ static __forceinline__ Head head(uint32_t slot, int, int g, float wscale) {
+    const uint4 hdr = lds128(slot);
     const __half2 dm = *reinterpret_cast<const __half2 *>(&hdr.x);
     const uint32_t f = k4_field(hdr.y, hdr.z, hdr.w, g);
     const float d = __low2float(dm) * wscale, mn = __high2float(dm) * wscale;
-    // value = (d*sc) * code - (dmin*m): low nibbles are sub-block 2g, high nibbles sub-block 2g+1
-    const __half2 a_lo = __float2half2_rn(d * (float)(f & 63)), a_hi = __float2half2_rn(d * (float)((f >> 6) & 63));
-    const __half2 b_lo = __float2half2_rn(-mn * (float)((f >> 12) & 63)), b_hi = __float2half2_rn(-mn * (float)(f >> 18));
+    return Head{__float2half2_rn(d * (float)(f & 63)), __float2half2_rn(d * (float)((f >> 6) & 63)), __float2half2_rn(-mn * (float)((f >> 12) & 63)),
+                __float2half2_rn(-mn * (float)(f >> 18))};
+  }
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int g, int hf, uint32_t (&o)[16]) { // half = words 4 hf .. of the group
+    const uint4 q = lds128(slot + 16 + 32 * g + 16 * hf);
     const __half2 k1024 = h2_from_bits(0x64006400u);
     const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -115,7 +127,7 @@ struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
 #pragma unroll
       for (int p = 0; p < 4; p++) { // pairs: p=0 (l, l+2) low, p=1 (32+l, 32+l+2) high, p=2 (l+1, l+3) low, p=3 high
         const __half2 c = __hsub2(h2_from_bits(((wd[wi] >> (4 * p)) & 0x000f000fu) | 0x64006400u), k1024);
-        o[4 * wi + p] = bits_from_h2((p & 1) ? __hfma2(c, a_hi, b_hi) : __hfma2(c, a_lo, b_lo));
+        o[4 * wi + p] = bits_from_h2((p & 1) ? __hfma2(c, hd.a_hi, hd.b_hi) : __hfma2(c, hd.a_lo, hd.b_lo));
       }
   }
 };
@@ -130,20 +142,32 @@ struct RowQ6K { // 128 ql bytes | 64 qh bytes | 16 scales | the f16 d of eight s
     return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 2u, NO_LIMIT};
   }
   // k-step kk = 2 h + hi_pair of the super-block: group 0 takes ql[l] of half h, group 1 ql[l + 32], both the low (hi_pair 0) or high nibbles
-  __device__ static __forceinline__ void half(uint32_t slot, int ss, int kk, int hf, float wscale, uint32_t (&o)[16]) {
+  struct Head {
+    uint4 qh[2];
+    uint32_t sc4;
+    float d;
+  };
+  __device__ static __forceinline__ Head head(uint32_t slot, int ss, int kk, float wscale) {
+    const int h = kk >> 1;
+    Head hd;
+    hd.qh[0] = lds128(slot + 128 + 32 * h), hd.qh[1] = lds128(slot + 144 + 32 * h);
+    hd.sc4 = lds32(slot + 192 + 8 * h + 4 * (kk & 1));
+    const uint32_t dd = lds32(slot + 208 + 4 * ((ss >> 1) & 3));
+    hd.d = __half2float(__ushort_as_half((unsigned short)((ss & 1) ? (dd >> 16) : (dd & 0xffffu)))) * wscale;
+    return hd;
+  }
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int kk, int hf, uint32_t (&o)[16]) {
     const int h = kk >> 1, sh = 4 * (kk & 1);
-    const uint4 qh[2] = {lds128(slot + 128 + 32 * h), lds128(slot + 144 + 32 * h)};
+    const uint4 (&qh)[2] = hd.qh;
     const uint4 ql[2] = {lds128(slot + 64 * h + 32 * hf), lds128(slot + 64 * h + 32 * hf + 16)};
-    const uint32_t sc4 = lds32(slot + 192 + 8 * h + 4 * (kk & 1)), dd = lds32(slot + 208 + 4 * ((ss >> 1) & 3));
-    const float d = __half2float(__ushort_as_half((unsigned short)((ss & 1) ? (dd >> 16) : (dd & 0xffffu)))) * wscale;
     const __half2 off = h2_from_bits(0x64206420u); // 1056 = 1024 + 32
     const int hsh = sh + 2 * hf; // bit position of this group's two high bits inside a qh byte
 #pragma unroll
     for (int c = 0; c < 4; c++) { // chunk of 8 elements l = 8c .. 8c+7
       const uint32_t lw[2] = {(c & 1) ? ql[c >> 1].z : ql[c >> 1].x, (c & 1) ? ql[c >> 1].w : ql[c >> 1].y};
       const uint32_t hw[2] = {(c & 1) ? qh[c >> 1].z : qh[c >> 1].x, (c & 1) ? qh[c >> 1].w : qh[c >> 1].y};
-      const int8_t sc = (int8_t)((sc4 >> (8 * (2 * hf + (c >> 1)))) & 0xff);
-      const __half2 s2 = __float2half2_rn(d * (float)sc);
+      const int8_t sc = (int8_t)((hd.sc4 >> (8 * (2 * hf + (c >> 1)))) & 0xff);
+      const __half2 s2 = __float2half2_rn(hd.d * (float)sc);
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const uint32_t code = ((lw[j] >> sh) & 0x0f0f0f0fu) | (((hw[j] >> hsh) << 4) & 0x30303030u);
