@@ -66,15 +66,22 @@ __device__ __forceinline__ float rms_apply(float v, float r, float g) { return _
 // v + 0.5 share a binade whose ulp divides 0.5, or the sum lands just ABOVE a power of two, so the
 // addition never rounds up across an integer; the one exception, |v| just under 0.5 (the sum would
 // round to 1), is caught by the guard. cvt.rzi of NaN is 0 and of +-inf saturates, as `as` does.
-__device__ __forceinline__ int round_away_sat_i8(float v) {
+__device__ __forceinline__ int round_away(float v) { // before the saturation
   const int r = __float2int_rz(v + copysignf(0.5f, v));
-  return fabsf(v) < 0.5f ? 0 : max(-128, min(127, r));
+  return fabsf(v) < 0.5f ? 0 : r;
 }
+__device__ __forceinline__ int round_away_sat_i8(float v) { return max(-128, min(127, round_away(v))); }
 
-__device__ __forceinline__ void pack8(const int q[8], Quant8 &o) {
-  o.lo = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
-  o.hi = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
-  int s = q[0] + q[1] + q[2] + q[3] + q[4] + q[5] + q[6] + q[7];
+// two integers saturated to int8 in the lower half (lo in byte 0), the lower half of `upper` above them
+__device__ __forceinline__ uint32_t pack_sat_i8(int lo, int hi, uint32_t upper) {
+  uint32_t d;
+  asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(upper));
+  return d;
+}
+__device__ __forceinline__ void pack8(const int q[8], Quant8 &o) { // saturates, as the reference's `as i8` does
+  o.lo = pack_sat_i8(q[0], q[1], pack_sat_i8(q[2], q[3], 0u));
+  o.hi = pack_sat_i8(q[4], q[5], pack_sat_i8(q[6], q[7], 0u));
+  int s = __dp4a((int)o.lo, 0x01010101, __dp4a((int)o.hi, 0x01010101, 0));
   s += __shfl_xor_sync(0xffffffffu, s, 1);
   o.sum16 = s;
 }
@@ -90,7 +97,7 @@ __device__ __forceinline__ Quant8 quantize8_q8_0(const float v[8], int /*lane*/)
   const float id = d != 0.f ? __fdiv_rn(1.0f, d) : 0.f;
   int q[8];
 #pragma unroll
-  for (int i = 0; i < 8; i++) q[i] = round_away_sat_i8(__fmul_rn(v[i], id));
+  for (int i = 0; i < 8; i++) q[i] = round_away(__fmul_rn(v[i], id));
   Quant8 o;
   pack8(q, o);
   o.d_unrounded = d;
@@ -100,28 +107,16 @@ __device__ __forceinline__ Quant8 quantize8_q8_0(const float v[8], int /*lane*/)
 
 // One Q8_K block = the whole warp (256 elements). `max` is the FIRST element of largest magnitude,
 // sign kept (the reference scans with a strict `<`).
-__device__ __forceinline__ Quant8 quantize8_q8k(const float v[8], int lane) {
-  float amax = 0.f, mx = 0.f;
-  int idx = lane * 8;
+__device__ __forceinline__ Quant8 quantize8_q8k(const float v[8], int /*lane*/) {
+  float amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const float a = fabsf(v[i]);
-    if (amax < a) {
-      amax = a;
-      mx = v[i];
-      idx = lane * 8 + i;
-    }
-  }
+  for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i])); // a NaN operand is ignored, as in the reference's comparison
+  amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax))); // magnitudes order like their bits
+  float mx = v[7]; // the lane's first element of that magnitude, if it has one
 #pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    const float oa = __shfl_xor_sync(0xffffffffu, amax, off);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-    if (oa > amax || (oa == amax && oi < idx)) {
-      amax = oa;
-      idx = oi;
-    }
-  }
-  mx = __shfl_sync(0xffffffffu, mx, idx >> 3); // the winning lane's own first-largest element is element idx
+  for (int i = 6; i >= 0; i--) mx = fabsf(v[i]) == amax ? v[i] : mx;
+  const unsigned int have = __ballot_sync(0xffffffffu, fabsf(mx) == amax);
+  mx = __shfl_sync(0xffffffffu, mx, __ffs(have) - 1);
   Quant8 o;
   int q[8];
   if (amax == 0.f) {
@@ -133,7 +128,7 @@ __device__ __forceinline__ Quant8 quantize8_q8k(const float v[8], int lane) {
   }
   const float iscale = __fdiv_rn(-128.f, mx);
 #pragma unroll
-  for (int i = 0; i < 8; i++) q[i] = min(127, round_away_sat_i8(__fmul_rn(iscale, v[i])));
+  for (int i = 0; i < 8; i++) q[i] = round_away(__fmul_rn(iscale, v[i]));
   pack8(q, o);
   o.d = o.d_unrounded = __fdiv_rn(1.0f, iscale);
   return o;
