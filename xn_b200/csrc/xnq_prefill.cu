@@ -342,16 +342,19 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       }
     };
     bind();
+    uint32_t to[NCOPY]; // where they go in a slot
+#pragma unroll
+    for (int i = 0; i < NCOPY; i++) to[i] = raw + (uint32_t)(((i * 128 + t) / RowT::ITEMS) * RowT::ROWB + ((i * 128 + t) % RowT::ITEMS) * 16);
     auto issue = [&]() {
       if (l_left > 0) {
         l_left--;
-        const uint32_t dst = raw + (uint32_t)l_slot * SLOT;
+        const uint32_t slot = (uint32_t)l_slot * SLOT;
 #pragma unroll
         for (int i = 0; i < NCOPY; i++) {
-          const int item = i * 128 + t;
-          if ((32 * RowT::ITEMS) % 128 == 0 || item < 32 * RowT::ITEMS) {
+          if ((32 * RowT::ITEMS) % 128 == 0 || i * 128 + t < 32 * RowT::ITEMS) {
             const uint32_t off = ((uint32_t)l_s * it[i].mul) & ~15u;
-            cp_async16(dst + (uint32_t)((item / RowT::ITEMS) * RowT::ROWB + (item % RowT::ITEMS) * 16), it[i].p + (off < it[i].lim ? off : 0u), off < it[i].lim ? 16u : 0u);
+            if (RowT::LIMITED) cp_async16(to[i] + slot, it[i].p + (off < it[i].lim ? off : 0u), off < it[i].lim ? 16u : 0u);
+            else cp_async16(to[i] + slot, it[i].p + off, 16u);
           }
         }
         if (++l_slot == R) l_slot = 0;

@@ -54,6 +54,7 @@ constexpr uint32_t NO_LIMIT = 0xffffffffu;
 // KPS k-steps per super-step ss. KPS = 4: one thread converts both halves of a row's k-step kk; KPS = 2: two threads, a half each.
 
 struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
+  static constexpr bool LIMITED = true; // rows may end inside a super-step
   static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
   __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { // scales beyond the last block are zero
     if (c < 8) return Item{w.qs + row * (w.k / 2) + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k / 2 - 16 * c)};
@@ -78,6 +79,7 @@ struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
 };
 
 struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighbour
+  static constexpr bool LIMITED = true;
   static constexpr int KPS = 2, ROWB = 144, ITEMS = 9;
   __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) {
     if (c < 8) return Item{w.qs + row * w.k + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k - 16 * c)};
@@ -104,6 +106,7 @@ struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighb
 };
 
 struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
+  static constexpr bool LIMITED = false;
   static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
   __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { return Item{w.qs + row * (w.k / QK_K) * 144 + 16 * c, 144u, NO_LIMIT}; }
   struct Head {
@@ -133,6 +136,7 @@ struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
 };
 
 struct RowQ6K { // 128 ql bytes | 64 qh bytes | 16 scales | the f16 d of eight super-blocks
+  static constexpr bool LIMITED = false;
   static constexpr int KPS = 4, ROWB = 240, ITEMS = 14;
   __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) {
     const int64_t blk = row * (w.k / QK_K);
