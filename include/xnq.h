@@ -272,6 +272,10 @@ int xnq_comm_free(xnq_comm *c);
  * image (act_dtype XNQ_Q8_0 or XNQ_Q8K) of the normalized rows: exactly what quantizing `out` would give. */
 int xnq_add_rmsnorm(float *x, const float *delta, int delta_parts, const float *weight, float eps, float *out,
                     void *act_image, int act_dtype, int64_t rows, int64_t d, void *stream);
+/* RMSNorm of many rows around a mean that the caller forms: x[n] += delta[n] (delta may be NULL) and square[n] = x * x in one pass;
+ * then out[rows, d] = (x * rsqrt(mean[row] + eps)) * weight[d]. Every operation is rounded separately. n and d multiples of 4. */
+int xnq_add_square(float *x, const float *delta, float *square, int64_t n, void *stream);
+int xnq_norm_scale(const float *x, const float *mean, const float *weight, float eps, float *out, int64_t rows, int64_t d, void *stream);
 /* The two ends of a decode step (llama.rs:300-320, the embedding lookup and the greedy choice of the next token).
  * xnq_embed_rows: x[rows, d] (f32) = table[tokens[r], :] of a bf16 table [vocab, d]; a token outside the table gives zeros
  * and sets status bit 26. It is launched as a plain kernel, never programmatically overlapped: as the first kernel of a

@@ -258,3 +258,15 @@ def test_prompt_rope_and_cache_store_are_the_torch_operations_bits(B, S, H, KV, 
     assert bool((kc[:, :, S:] == 7).all()) and bool((vc[:, :, S:] == 7).all())
     with pytest.raises(ValueError):
         ops.rope_kv_store_prompt(qkv[..., :-hd].contiguous(), cos, sin, kc, vc, H, KV)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 4), (2, 17, 516), (1, 40, 4096), (300, 1024)])
+@pytest.mark.parametrize("with_delta", [True, False])
+def test_add_rmsnorm_rows_is_the_torch_operations_bits(shape, with_delta):
+    from xn_b200 import decoder_ops as ops
+    g = torch.Generator(device="cpu"); g.manual_seed(sum(shape))
+    x, delta, w = (torch.randn(s, generator=g).to(DEV) for s in (shape, shape, shape[-1:]))
+    want_x = x + delta if with_delta else x.clone()
+    want = want_x * torch.rsqrt(want_x.pow(2).mean(-1, keepdim=True) + 1e-5) * w
+    got = ops.add_rmsnorm_rows(x, delta if with_delta else None, w, 1e-5)
+    assert torch.equal(x, want_x) and torch.equal(got, want)

@@ -84,6 +84,8 @@ def lib() -> ctypes.CDLL:
     L.xnq_attn_decode.argtypes = [vp, vp, vp, vp, vp, i64, ci, ci, ci, i64, vp, sz, vp]
     L.xnq_rope_attn_decode.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, ci, ci, ci, i64, vp, sz, vp]
     L.xnq_rope_kv_store_prompt.argtypes = [vp, vp, vp, vp, vp, vp, i64, i64, ci, ci, ci, i64, vp]
+    L.xnq_add_square.argtypes = [vp, vp, vp, i64, vp]
+    L.xnq_norm_scale.argtypes = [vp, vp, vp, fp, vp, i64, i64, vp]
     L.xnq_device_status.argtypes = [ctypes.POINTER(ctypes.c_uint)]
     L.xnq_device_check_record.argtypes = [ctypes.POINTER(ctypes.c_ulonglong)]
     L.xnq_set_option.argtypes = [ctypes.c_char_p, ci]

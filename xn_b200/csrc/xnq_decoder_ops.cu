@@ -224,6 +224,32 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const float *gu, float *out
   }
 }
 
+// The passes of a prompt's RMSNorm around the mean of squares, 16 bytes per thread; bound by their 16 and 8 bytes per value. As separate
+// operations (add, square, add eps, rsqrt, two products) they were six passes.
+__global__ void __launch_bounds__(256) add_square_kernel(float4 *x, const float4 *delta, float4 *square, int64_t n4) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x;
+  if (i >= n4) return;
+  float4 v = x[i];
+  if (delta) {
+    const float4 a = delta[i];
+    v = make_float4(__fadd_rn(v.x, a.x), __fadd_rn(v.y, a.y), __fadd_rn(v.z, a.z), __fadd_rn(v.w, a.w));
+    x[i] = v;
+  }
+  square[i] = make_float4(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y), __fmul_rn(v.z, v.z), __fmul_rn(v.w, v.w));
+}
+__global__ void __launch_bounds__(256) norm_scale_kernel(const float *x, const float *mean, const float *w, float eps, float *out, int d) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t row = blockIdx.x;
+  const float r = rsqrtf(__fadd_rn(mean[row], eps));
+  for (int i = threadIdx.x * 4; i < d; i += 1024) {
+    const float4 v = *reinterpret_cast<const float4 *>(x + row * d + i), g = *reinterpret_cast<const float4 *>(w + i);
+    *reinterpret_cast<float4 *>(out + row * d + i) = make_float4(rms_apply(v.x, r, g.x), rms_apply(v.y, r, g.y), rms_apply(v.z, r, g.z), rms_apply(v.w, r, g.w));
+  }
+}
+
 // x[row, :] = table[tokens[row], :] widened to f32 (bf16 table). One CTA per row, 8 elements per thread and pass. A token outside
 // [0, vocab) gives a row of zeros and sets status bit 4. Launched as a plain (not programmatically dependent) kernel: it is the
 // step's first kernel, and everything behind it may rely on the previous step's stores (position, tokens, cache rows) being complete.
@@ -672,6 +698,29 @@ int xnq_rope_kv_store_prompt(const float *qkv, const float *cos_table, const flo
   XNQ_CUDA(launch_pdl(rope_store_prompt_kernel, dim3((unsigned)seq, (unsigned)batch), dim3(256), 0, static_cast<cudaStream_t>(stream), qkv, cos_table, sin_table,
                       static_cast<__nv_bfloat16 *>(q_out), static_cast<__nv_bfloat16 *>(k_cache), static_cast<__nv_bfloat16 *>(v_cache), (int)seq, heads, kv_heads, head_dim,
                       (int)max_seq));
+  count_launch();
+  return XNQ_OK;
+}
+
+int xnq_add_square(float *x, const float *delta, float *square, int64_t n, void *stream) {
+  clear_error();
+  if (!x || !square) return fail(XNQ_ERR_NULL, "add_square: NULL argument");
+  if (n < 0 || n % 4 || n / 1024 >= INT32_MAX) return fail(XNQ_ERR_SHAPE, "add_square: n = %lld (a multiple of 4)", (long long)n);
+  if (((uintptr_t)x | (uintptr_t)delta | (uintptr_t)square) & 15) return fail(XNQ_ERR_ALIGN, "add_square: pointers must be 16-byte aligned");
+  if (n == 0) return XNQ_OK;
+  XNQ_CUDA(launch_pdl(add_square_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, static_cast<cudaStream_t>(stream), reinterpret_cast<float4 *>(x),
+                      reinterpret_cast<const float4 *>(delta), reinterpret_cast<float4 *>(square), n / 4));
+  count_launch();
+  return XNQ_OK;
+}
+
+int xnq_norm_scale(const float *x, const float *mean, const float *weight, float eps, float *out, int64_t rows, int64_t d, void *stream) {
+  clear_error();
+  if (!x || !mean || !weight || !out) return fail(XNQ_ERR_NULL, "norm_scale: NULL argument");
+  if (rows < 0 || rows > INT32_MAX || d <= 0 || d % 4 || d > INT32_MAX / 2) return fail(XNQ_ERR_SHAPE, "norm_scale: rows = %lld, d = %lld (a multiple of 4)", (long long)rows, (long long)d);
+  if (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out) & 15) return fail(XNQ_ERR_ALIGN, "norm_scale: pointers must be 16-byte aligned");
+  if (rows == 0) return XNQ_OK;
+  XNQ_CUDA(launch_pdl(norm_scale_kernel, dim3((unsigned)rows), dim3(256), 0, static_cast<cudaStream_t>(stream), x, mean, weight, eps, out, (int)d));
   count_launch();
   return XNQ_OK;
 }

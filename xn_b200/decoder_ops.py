@@ -200,3 +200,19 @@ def rope_kv_store_prompt(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor
         _lib.check(_lib.lib().xnq_rope_kv_store_prompt(_p(qkv), _p(cos), _p(sin), _p(q), _p(k_cache), _p(v_cache), B, S, heads, kv_heads, hd, max_seq,
                                                        _stream_ptr(qkv.device)))
     return q
+
+
+def add_rmsnorm_rows(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor, eps: float) -> torch.Tensor:
+    """In place ``x += delta`` (skipped when None), returns ``x * rsqrt(mean(x^2) + eps) * weight`` over the last dimension: the
+    values of the separate torch operations bit for bit, in three launches (xnq_add_square, torch's mean, xnq_norm_scale). For many
+    rows; :func:`add_rmsnorm` is one launch but forms the mean in its own order."""
+    _f32c(x, delta, weight)
+    d = x.shape[-1]
+    if weight.numel() != d or (delta is not None and delta.numel() != x.numel()):
+        raise ValueError(f"add_rmsnorm_rows: x {tuple(x.shape)}, weight {tuple(weight.shape)}, delta {None if delta is None else tuple(delta.shape)}")
+    out = torch.empty_like(x)   # the squares, then the result
+    with torch.cuda.device(x.device):
+        _lib.check(_lib.lib().xnq_add_square(_p(x), _p(delta), _p(out), x.numel(), _stream_ptr(x.device)))
+        mean = out.mean(-1)
+        _lib.check(_lib.lib().xnq_norm_scale(_p(x), _p(mean), _p(weight), eps, _p(out), x.numel() // d, d, _stream_ptr(x.device)))
+    return out

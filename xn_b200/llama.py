@@ -16,7 +16,7 @@ Tensor parallelism over ``world`` ranks (one process per GPU):
     its summand into every rank's buffer; the next residual-add + RMSNorm adds the summands;
   * the LM head is N-sharded and its output columns are gathered the same way.
 
-Prefill runs RMSNorm and attention as torch ops (its RoPE + KV-cache store and SwiGLU are the library's). A decode step uses the library's fused operators
+Prefill runs attention and the mean of its RMSNorms as torch ops, the rest as the library's operators. A decode step uses the library's fused operators
 between the linears (residual-add + RMSNorm, RoPE + KV-cache store, single-query attention, SwiGLU), so
 one layer is ten launches and the whole step is one CUDA graph.
 """
@@ -228,22 +228,26 @@ class QLlama:
         x1, x2 = x[..., : x.shape[-1] // 2], x[..., x.shape[-1] // 2:]
         return torch.cat([x1 * cos - x2 * sin, x2 * cos + x1 * sin], dim=-1)
 
-    def _block(self, L: _Layer, x: torch.Tensor, pos_idx: torch.Tensor, mask: torch.Tensor, prompt: bool) -> torch.Tensor:
-        """x [B, S, d]; pos_idx [S] int64 positions of these tokens; mask broadcastable to [B, H, S, max_seq]. ``prompt``: the
-        positions are 0 .. S - 1."""
+    def _block(self, L: _Layer, x: torch.Tensor, delta: Optional[torch.Tensor], pos_idx: torch.Tensor, mask: torch.Tensor, prompt: bool) -> torch.Tensor:
+        """x [B, S, d], to which ``delta`` is added first (in place); pos_idx [S] int64 positions of these tokens; mask broadcastable
+        to [B, H, S, max_seq]. ``prompt``: the positions are 0 .. S - 1. Returns what is still to be added to x."""
         B, S, _ = x.shape
-        qkv = L.wqkv.matmul_t(self._rms(x, L.norm1))
+        eps = self.cfg.rms_eps
+        qkv = L.wqkv.matmul_t(ops.add_rmsnorm_rows(x, delta, L.norm1, eps))
         if prompt and self.cfg.head_dim % 8 == 0:
             q = ops.rope_kv_store_prompt(qkv, self.cos, self.sin, L.k_cache, L.v_cache, self.hl, self.kvl)
         else:
             q = self._rope_store(L, qkv, pos_idx)
         a = F.scaled_dot_product_attention(q, L.k_cache, L.v_cache, attn_mask=mask, enable_gqa=True)
-        a = a.transpose(1, 2).reshape(B, S, self.hl * self.cfg.head_dim).float()
-        x = x + self._sum_parts(self._linear_parts(L.wo, a))
+        a = a.transpose(1, 2).reshape(B, S, self.hl * self.cfg.head_dim)
+        if self.pg is None:   # the linear takes the bf16 rows as they are
+            o = L.wo.matmul_t(a, out=torch.empty_like(x))
+        else:
+            o = self._sum_parts(self._linear_parts(L.wo, a.float()))
         f = self.cfg.ffn // self.world
-        gu = L.wgu.matmul_t(self._rms(x, L.norm2)).view(B * S, 2 * f)
+        gu = L.wgu.matmul_t(ops.add_rmsnorm_rows(x, o, L.norm2, eps)).view(B * S, 2 * f)
         h = ops.swiglu(gu, torch.empty((B * S, f), device=self.device)).view(B, S, f)
-        return x + self._sum_parts(self._linear_parts(L.wdown, h))
+        return self._sum_parts(self._linear_parts(L.wdown, h))
 
     def _rope_store(self, L: _Layer, qkv: torch.Tensor, pos_idx: torch.Tensor) -> torch.Tensor:
         """q and k rotated at ``pos_idx``, k and v stored into the caches at these positions; returns q [B, H, S, hd] bf16."""
@@ -265,9 +269,10 @@ class QLlama:
         ar = torch.arange(self.max_seq, device=self.device)
         mask = (ar[None, :] <= pos_idx[:, None])[None, None]  # [1, 1, S, max_seq]: causal over the cache
         x = self.embed.index_select(0, tokens.reshape(-1)).view(*tokens.shape, -1).float()
+        delta = None
         for L in self.layers:
-            x = self._block(L, x, pos_idx, mask, prompt)
-        x = self._rms(x[:, -1:, :], self.norm)
+            delta = self._block(L, x, delta, pos_idx, mask, prompt)
+        x = self._rms(x[:, -1:, :] + delta[:, -1:, :], self.norm)
         logits = self._linear_gathered(self.lm_head, x).view(tokens.shape[0], -1)
         return logits if self.pg is None else logits.clone()   # out of the exchange slot before it is reused
 
