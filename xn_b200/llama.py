@@ -230,7 +230,7 @@ class QLlama:
 
     def _block(self, L: _Layer, x: torch.Tensor, delta: Optional[torch.Tensor], pos_idx: torch.Tensor, mask: torch.Tensor, prompt: bool) -> torch.Tensor:
         """x [B, S, d], to which ``delta`` is added first (in place); pos_idx [S] int64 positions of these tokens; mask broadcastable
-        to [B, H, S, max_seq]. ``prompt``: the positions are 0 .. S - 1. Returns what is still to be added to x."""
+        to [B, H, S, the leading cache positions attended to]. ``prompt``: the positions are 0 .. S - 1. Returns what is still to be added to x."""
         B, S, _ = x.shape
         eps = self.cfg.rms_eps
         qkv = L.wqkv.matmul_t(ops.add_rmsnorm_rows(x, delta, L.norm1, eps))
@@ -238,7 +238,8 @@ class QLlama:
             q = ops.rope_kv_store_prompt(qkv, self.cos, self.sin, L.k_cache, L.v_cache, self.hl, self.kvl)
         else:
             q = self._rope_store(L, qkv, pos_idx)
-        a = F.scaled_dot_product_attention(q, L.k_cache, L.v_cache, attn_mask=mask, enable_gqa=True)
+        kv = mask.shape[-1]
+        a = F.scaled_dot_product_attention(q, L.k_cache[:, :, :kv], L.v_cache[:, :, :kv], attn_mask=mask, enable_gqa=True)
         a = a.transpose(1, 2).reshape(B, S, self.hl * self.cfg.head_dim)
         if self.pg is None:   # the linear takes the bf16 rows as they are
             o = L.wo.matmul_t(a, out=torch.empty_like(x))
@@ -266,8 +267,10 @@ class QLlama:
     def _forward(self, tokens: torch.Tensor, pos_idx: torch.Tensor, prompt: bool = False) -> torch.Tensor:
         """tokens [B, S] -> logits of the last position [B, vocab]. ``prompt``: the positions are 0 .. S - 1."""
         self._gather_idx = 0
-        ar = torch.arange(self.max_seq, device=self.device)
-        mask = (ar[None, :] <= pos_idx[:, None])[None, None]  # [1, 1, S, max_seq]: causal over the cache
+        # a prompt attends to its own positions; whole tiles of the cache, so that the attention sees the same alignment whatever S is
+        kv = min(self.max_seq, (tokens.shape[1] + 63) // 64 * 64) if prompt else self.max_seq
+        ar = torch.arange(kv, device=self.device)
+        mask = (ar[None, :] <= pos_idx[:, None])[None, None]  # [1, 1, S, kv]: causal over the cache
         x = self.embed.index_select(0, tokens.reshape(-1)).view(*tokens.shape, -1).float()
         delta = None
         for L in self.layers:
