@@ -677,8 +677,12 @@ int xnq_linear_forward_host(xnq_weight *w, const float *x_host, int64_t m, const
   // saves the device-to-host copy and its launch; anything else goes through the staging buffer. The
   // activations are always copied in: every CTA reads all of x, which must not cross the host link 148 times.
   float *y_direct = nullptr;
-  // (not where the small-batch kernel splits k between CTAs that add into y atomically: that needs device memory)
-  if (!bias_host && m <= MATVEC_MAX_M && !(m >= 5 && matvec_mma_accumulates_in_y(w->v, m)) && g_opt_host_direct_y.load(std::memory_order_relaxed)) {
+  // Not with two rows or more on the dp4a kernels: they store a few neighbouring values of a row at a time, and the host link takes
+  // those one by one (Q4_0 14336 x 4096, 4 rows: 112 us against 58 with the copy; Q6_K 4096 x 4096, 2 rows: 49 against 43). The integer
+  // tensor-core kernel stores runs of 128 values (same weight, 5 rows: 55 against 63), the generic one runs of a CTA (Q5_K, 4 rows: 59
+  // against 71).
+  const bool long_runs = m == 1 || is_generic_dtype(w->v.dtype) || use_imma(w, m);
+  if (!bias_host && m <= MATVEC_MAX_M && long_runs && g_opt_host_direct_y.load(std::memory_order_relaxed)) {
     cudaPointerAttributes attr;
     if (cudaPointerGetAttributes(&attr, y_host) == cudaSuccess && attr.type == cudaMemoryTypeHost && attr.devicePointer &&
         (reinterpret_cast<uintptr_t>(attr.devicePointer) & 15) == 0)

@@ -282,7 +282,6 @@ int64_t matvec_rows_per_pass(int wdtype, int64_t k);
 // xnq_matvec_mma.cu  (5 <= m <= 16, Q4_K: integer tensor-core MMAs)
 int64_t matvec_mma_rows_per_pass(const WeightView &w, int y_dtype); // 0: not served
 int launch_matvec_mma(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s);
-bool matvec_mma_accumulates_in_y(const WeightView &w, int64_t m); // k split between CTAs that add into y atomically
 int matvec_mma_init(int device);
 // rows per launch of the small-batch path that xnq_matmul_t takes for this weight, and which kernel that is
 int64_t small_batch_pass(const xnq_weight *w, int64_t m, int y_dtype, bool *use_mma);

@@ -674,7 +674,8 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   const int act = act_dtype_for(w.dtype);
   // The rows' CTAs are started while the previous kernel drains, and the first SM that is free would take eight of them (10 us for
   // 32 rows instead of 3); unused shared memory keeps them apart: at most ceil(rows / SMs) to an SM.
-  const size_t spread = std::min<size_t>(MAX_SPREAD, (SM_SMEM / (size_t)((m_pad + g_num_sms - 1) / g_num_sms)) / 2048 * 1024);
+  const int64_t sms = g_num_sms > 0 ? g_num_sms : 148;
+  const size_t spread = std::min<size_t>(MAX_SPREAD, (SM_SMEM / (size_t)((m_pad + sms - 1) / sms)) / 2048 * 1024);
   // (each CTA also takes 1 KB of its own)
 #define XNQ_PREP(ACT, XT)                                                                                                   \
   XNQ_CUDA(launch_pdl(prefill_prepare_acts<ACT, XT>, dim3((unsigned)m_pad), dim3(256), spread, s, static_cast<const XT *>(x), m, k, ldx, m_pad, ksteps, \
