@@ -50,7 +50,7 @@ WORKLOADS = {
     # prefill (m > 16): the tensor-core kernel; roofline is reported against the dense bf16/fp16 tensor peak
     "C2_q8_0_11008x4096_m128": (D.Q8_0, 11008, 4096, 128),
     "C2_q8_0_11008x4096_m512": (D.Q8_0, 11008, 4096, 512),
-    "C3_q4k_14336x4096_m32": (D.Q4K, 14336, 4096, 32),   # the folded-scale variant of the integer tensor-core kernel (17..32 rows)
+    "C3_q4k_14336x4096_m32": (D.Q4K, 14336, 4096, 32),
     "C3_q4k_14336x4096_m64": (D.Q4K, 14336, 4096, 64),
     "C3_q4k_14336x4096_m512": (D.Q4K, 14336, 4096, 512),
 }
@@ -258,7 +258,7 @@ def _graph_us(torch, dev, fn, calls: int, reps: int) -> float:
 EXTRA_MATMULS = [
     ("C1_q4_0_4096x4096", D.Q4_0, 4096, 4096, (1,)),
     ("C2_q8_0_11008x4096", D.Q8_0, 11008, 4096, (1, 16, 128, 512)),
-    ("C3_q4k_14336x4096", D.Q4K, 14336, 4096, (4, 16, 32, 64, 512)),   # 32: the folded-scale variant of the integer kernel
+    ("C3_q4k_14336x4096", D.Q4K, 14336, 4096, (4, 16, 32, 64, 512)),
     ("C4_q6k_128256x4096", D.Q6K, 128256, 4096, (1, 16, 32)),          # 16: the dp4a small-batch kernel
 ]
 

@@ -325,12 +325,9 @@ def test_tma_ring_decode_kernel_matches_oracle_and_plain_kernel(Q, O, dt, n, k):
 
 @pytest.mark.parametrize("m", [2, 8, 16, 17, 32, 33, 48, 64])
 @pytest.mark.parametrize("n,k", [(128, 256), (200, 1024), (1000, 4096), (300, 11008)])
-def test_q4k_small_batch_folded_scales_match_oracle_and_per_block_kernel(Q, O, m, n, k):
-    """Q4_K small batches run with the sub-block scales folded into the weight operand (two unsigned planes,
-    one drain per 256 block; option 2 forces it for every batch size, the default takes it for 17..32 rows)
-    or, with the option 0, with one accumulator slice per 32 elements. Both are
-    exact integer sums followed by the same f32 scaling, so both must meet the reference's bound against the
-    oracle, and each other up to f32 summation order."""
+def test_q4k_small_batches_match_oracle_whatever_imma_fold(Q, O, m, n, k):
+    """Q4_K batches of 2..64 rows meet the reference's bound against the oracle. The option imma_fold chose a second kernel that is
+    gone: its values are still accepted and change nothing."""
     from xn_b200 import _lib
     L = _lib.lib()
     dt = D.Q4K
@@ -339,16 +336,11 @@ def test_q4k_small_batch_folded_scales_match_oracle_and_per_block_kernel(Q, O, m
     x = _tricky(m, k, 50 + m)
     xd = torch.from_numpy(x).to(DEV)
     want = O.matmul(int(dt), x, w, n)
-    try:
-        _lib.check(L.xnq_set_option(b"imma_fold", 2))
-        got_fold = t.matmul_t(xd).cpu().numpy()
-        _lib.check(L.xnq_set_option(b"imma_fold", 0))
-        got_blk = t.matmul_t(xd).cpu().numpy()
-    finally:
-        _lib.check(L.xnq_set_option(b"imma_fold", 1))
-    assert_close_ref(got_fold, want, TOL_F32, f"fold m={m} n={n} k={k}")
-    assert_close_ref(got_blk, want, TOL_F32, f"per-block m={m} n={n} k={k}")
-    assert_close_ref(got_fold, got_blk, 5e-4, "fold vs per-block")
+    got = t.matmul_t(xd).cpu().numpy()
+    assert_close_ref(got, want, TOL_F32, f"m={m} n={n} k={k}")
+    for value in (2, 1, 0):
+        _lib.check(L.xnq_set_option(b"imma_fold", value))
+        assert np.array_equal(t.matmul_t(xd).cpu().numpy(), got), value
 
 
 def test_zz_device_status_is_clean(Q):

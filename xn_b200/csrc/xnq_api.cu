@@ -282,10 +282,7 @@ int xnq_set_option(const char *name, int value) {
     g_opt_matvec_tma.store(value != 0);
     return XNQ_OK;
   }
-  if (std::strcmp(name, "imma_fold") == 0) {
-    imma_set_fold(value);
-    return XNQ_OK;
-  }
+  if (std::strcmp(name, "imma_fold") == 0) return XNQ_OK; // chose a kernel that is no longer there
   if (std::strcmp(name, "imma") == 0) {
     g_opt_imma.store(value);
     return XNQ_OK;

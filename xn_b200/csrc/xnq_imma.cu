@@ -43,9 +43,6 @@
 // Every wait is bounded; on expiry a status bit is set and the roles fall through to the common exit, where
 // tensor memory is released.
 #include <algorithm>
-#include <atomic>
-#include <cstdlib>
-#include <cstring>
 
 #include "xnq_common.cuh"
 #include "xnq_quantize_act.cuh"
@@ -263,7 +260,6 @@ struct ImmaArgs {
                         // no thread divides 64-bit numbers before its first copy
   unsigned int *tile_cnt; // [tiles] arrival tickets of split tiles, zeroed by the prepare kernel
   float *partials;        // [2 * grid][NP][128] partial sums of split tiles
-  float *pair_scratch;    // [grid][NP][128]: the odd half steps' sums on their way to the even ones'
   // raw weight bytes: stream 0 holds the codes (Q4_K: the whole 144-byte super-blocks), stream 1 the f16 block scales of Q4_0 / Q8_0
   const uint8_t *src[2];
   int nstreams;
@@ -294,9 +290,15 @@ template <int STEP>
 __device__ __forceinline__ uint4 raw_chunk(uint32_t row, int key, int c) {
   return lds128(row + (uint32_t)((c ^ (key & (STEP / 16 - 1))) << 4));
 }
+template <int CH>
+struct DrainBlockScaled;
+template <int CH>
+struct DrainQ4K;
 struct ConvQ8_0 { // 256 code bytes per row and step
   static constexpr int STEP = 256, HI = 0; // HI: bytes per row and step of a second code stream
   static constexpr bool PAIRED = false;    // two operand columns per activation row
+  template <int CH>
+  using Drain = DrainBlockScaled<CH>;
   __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; i++) out[i] = raw_chunk<STEP>(row, key, 8 * h + 4 * p + i);
@@ -307,6 +309,8 @@ __device__ __forceinline__ uint32_t nib_hi_s8(uint32_t w) { return ((((w >> 4) &
 struct ConvQ4_0 { // eight blocks of 16 nibble bytes per row and step; element j < 16 low nibble of byte j, j >= 16 high nibble of byte j - 16
   static constexpr int STEP = 128, HI = 0;
   static constexpr bool PAIRED = false;
+  template <int CH>
+  using Drain = DrainBlockScaled<CH>;
   __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
 #pragma unroll
     for (int bb = 0; bb < 2; bb++) {
@@ -319,6 +323,8 @@ struct ConvQ4_0 { // eight blocks of 16 nibble bytes per row and step; element j
 struct ConvQ4K { // 128 code bytes per row and step: four 32-byte chunks; chunk c = sub-block 2c in the low nibbles, 2c+1 in the high ones
   static constexpr int STEP = 128, HI = 0;
   static constexpr bool PAIRED = false;
+  template <int CH>
+  using Drain = DrainQ4K<CH>;
   __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
     const uint4 a = raw_chunk<STEP>(row, key, 2 * (2 * h + p)), b = raw_chunk<STEP>(row, key, 2 * (2 * h + p) + 1);
     out[0] = make_uint4(a.x & 0x0f0f0f0fu, a.y & 0x0f0f0f0fu, a.z & 0x0f0f0f0fu, a.w & 0x0f0f0f0fu);
@@ -401,17 +407,13 @@ __device__ __forceinline__ void q6k_sums(const uint4 &hdr, int h, const uint32_t
 #pragma unroll
     for (int j = 0; j < 8; j++) isum[c] += (int)(int8_t)((w[j >> 2] >> (8 * (j & 3))) & 0xffu) * (int)v[j][c];
 }
-template <int CH>
-struct DrainQ6K { // (the paired form has its own drain, by half steps)
-  __device__ static __forceinline__ void run(const uint4 &, uint32_t, int, const uint32_t (&)[8][CH], float *) {}
-};
 
 // Drain warps: a warp's waits and its decoding of the row's scales cost as much as four columns' arithmetic; with 16 rows eight warps of
 // eight columns each do better than sixteen of four (Q6_K 32000 x 4096, 16 rows: 48.5 -> 46.4 us; Q8_0 11008 x 4096, 8 rows: 21.7 -> 20.9).
 __host__ __device__ constexpr int drain_warps(int rows) { return rows == 16 ? 8 : DRAIN_WARPS; }
 __host__ __device__ constexpr int imma_threads(int rows) { return (DRAIN_WARP0 + drain_warps(rows)) * 32; }
 
-template <typename Conv, template <int> class Drain, int NP>
+template <typename Conv, int NP>
 __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) imma_kernel(const __grid_constant__ ImmaArgs p) {
   constexpr int ROWS = Conv::PAIRED ? NP / 2 : NP; // activation rows of the operand; NP: its columns
   constexpr int DW = drain_warps(ROWS);
@@ -678,7 +680,7 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + 8 * (2 * nb)), mbar_arrive(acc_empty + 8 * (2 * nb + 1));
           }
-          if constexpr (!Conv::PAIRED) Drain<CH>::run(hdr, side + HDR_BYTES, c0 + ch * CH, v, acc + ch * CH);
+          if constexpr (!Conv::PAIRED) Conv::template Drain<CH>::run(hdr, side + HDR_BYTES, c0 + ch * CH, v, acc + ch * CH);
         }
       }
       __syncwarp();
@@ -757,369 +759,6 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
   tc_fence_before();
   __syncthreads();
   if (warp == MMA_WARP) tmem_dealloc(tmem_d, TMEM_COLS);
-}
-
-// =====================================================================================================================
-// Q4_K with the sub-block scales folded into the weight operand.
-//
-// The kernel above drains one accumulator slice per 32-element block, because a block's scale cannot be applied on the
-// tensor core. For Q4_K the scales are small integers: a code q (0..15) times its 6-bit sub-block scale sc (0..63) is an
-// integer below 1024, and written as q = 4 q_hi + q_lo (two bits each) both q_lo sc and q_hi sc fit one unsigned byte
-// (<= 189). So the converters write TWO operand planes, P_lo = q_lo sc and P_hi = q_hi sc (one packed multiply per four
-// codes, no carries between bytes), the MMAs ACCUMULATE over the four sub-blocks of a half step,
-//     D_lo = sum_i P_lo[r, i] a[c, i],  D_hi likewise,    sum_g sc_g sum_{i in g} q_i a_i = 4 D_hi + D_lo   (exact integers),
-// and the drain applies d, d_min and the activation scale once per 256-element block, as the CPU code does
-// (k_quants.rs:1380-1410). Per 256-k step that is 16 MMAs instead of 8, issued by four threads (plane x half step; an
-// MMA of this shape costs its issuing thread 134 cycles but several threads issue concurrently), and 4 accumulator
-// slices to drain instead of 8, with the integer scale multiplies gone from the drain, which is what bounded the kernel
-// above (instruction issue). 21 warps: activation producer, 4 MMA issuers, 8 converter warps (group h converts half h of
-// every step into a ring of four half-step stages), 8 drain warps (two groups that take alternate steps; a thread owns
-// one weight row and all NP activation columns). NP is 16 or 32; larger batches run in passes of 32 rows.
-// =====================================================================================================================
-constexpr int F_ISSUERS = 4, F_CONV_WARPS = 8, F_DRAIN_WARPS = 8;
-constexpr int F_ACT_WARP = 0, F_MMA_WARP0 = 1, F_CONV_WARP0 = F_MMA_WARP0 + F_ISSUERS, F_DRAIN_WARP0 = F_CONV_WARP0 + F_CONV_WARPS;
-constexpr int F_NTHREADS = (F_DRAIN_WARP0 + F_DRAIN_WARPS) * 32; // 672
-constexpr int F_RING = 3;                         // stages of the rings that are freed by the drain (activation operand, scale bytes and records)
-constexpr int F_ASTAGES = 4;                      // half-step stages of the weight operand (two steps), two planes each
-constexpr int F_A_STAGE_BYTES = 2 * A_STAGE_BYTES; // plane lo, plane hi
-constexpr uint32_t F_SLOT = 32 * 64 + 512;        // a converter warp's raw slot: 64 code bytes of the half step per row, then the rows' 16 header bytes
-
-// kind::i8 with an UNSIGNED A operand (the scaled codes reach 189) and a signed B operand
-__device__ __forceinline__ uint32_t idesc_u8s8(int umma_n) {
-  return (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(umma_n >> 3) << 17) | ((uint32_t)(TILE_N >> 4) << 24);
-}
-__device__ __forceinline__ void umma_i8_acc(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// a ring position: index in 0..n-1 and the parity of the lap, advanced without a division
-struct RingPos {
-  int idx;
-  uint32_t ph;
-  __device__ __forceinline__ void advance(int by, int n) {
-    idx += by;
-    if (idx >= n) idx -= n, ph ^= 1u;
-  }
-};
-
-template <int NP>
-__global__ void __launch_bounds__(F_NTHREADS, 1) imma_q4k_fold_kernel(const __grid_constant__ ImmaArgs p) {
-  constexpr int NBUF = TMEM_COLS / (4 * NP) > 8 ? 8 : TMEM_COLS / (4 * NP); // accumulator buffers of one step (four slices): 8 or 4, a power of two
-  constexpr int BUF_COLS = 4 * NP;
-  constexpr int CH = 8; // columns read back at a time
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  // barriers: b_full, side_full, side_empty [F_RING]; a_full [F_ASTAGES]; acc_full, acc_empty [8] (NBUF of them in use)
-  __shared__ __align__(8) uint64_t bars[3 * F_RING + F_ASTAGES + 16];
-  __shared__ uint32_t tmem_slot;
-  __shared__ unsigned int s_ticket;
-  const uint32_t b_full = smem_u32(bars), side_full = b_full + 8 * F_RING, side_empty = side_full + 8 * F_RING, a_full = side_empty + 8 * F_RING,
-                 acc_full = a_full + 8 * F_ASTAGES, acc_empty = acc_full + 64;
-  // One commit per issuer and step, on the step's accumulator buffer (acc_full, all four issuers): it tells the drain that the
-  // slices are written and the converters that the operand stages of that step have been read. A barrier per operand stage
-  // would be lapped: the issuers may run NBUF steps ahead of the drain, and a waiter that misses two phases waits for ever.
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int D = p.raw_stages; // raw slots per converter warp
-  const int KT = p.nsteps;
-  const int u0 = cta_first_unit((int)blockIdx.x, p.units_q, p.units_r);
-  const int nunits = p.units_q + ((int)blockIdx.x < p.units_r ? 1 : 0);
-  const int tile0 = u0 / KT, kt0 = u0 - tile0 * KT;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < F_RING; s++) {
-      mbar_init(b_full + 8 * s, 1);
-      mbar_init(side_full + 8 * s, 1 + F_CONV_WARPS / 2); // the producer's transaction + the four converter warps of half 0, which copy the header bytes
-      mbar_init(side_empty + 8 * s, F_DRAIN_WARPS / 2);   // the step's drain group
-    }
-    for (int s = 0; s < F_ASTAGES; s++) mbar_init(a_full + 8 * s, F_CONV_WARPS / 2); // the four converter warps of the half step
-    for (int s = 0; s < 8; s++) {
-      mbar_init(acc_full + 8 * s, F_ISSUERS);
-      mbar_init(acc_empty + 8 * s, F_DRAIN_WARPS / 2);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == F_MMA_WARP0) {
-    tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  pdl_launch_dependents();
-  const uint32_t tmem_d = __shfl_sync(0xffffffffu, tmem_slot, 0);
-
-  if (warp == F_ACT_WARP) {
-    // ---- activation producer ----
-    if (lane == 0) {
-      for (int st = 0; st < p.nstreams; st++) { // the CTA's share of the weight's bytes into L2, in long contiguous runs
-        const unsigned long long o0 = p.pf_share[st] * blockIdx.x, o1 = min(o0 + p.pf_share[st], p.pf_bytes[st]);
-        for (unsigned long long o = o0; o < o1; o += PF_CHUNK) bulk_prefetch_l2(p.pf_base[st] + o, (uint32_t)min((unsigned long long)PF_CHUNK, o1 - o));
-      }
-      pdl_wait();
-      int kt = kt0;
-      RingPos rp{0, 0};
-      for (int i = 0; i < nunits; i++) {
-        // the stage was last used by step i - 3; it is free once that step's drain group has read its records, which also
-        // means the step's MMAs have read the activation operand
-        if (i >= F_RING && !mbar_wait(side_empty + 8 * rp.idx, rp.ph ^ 1u, 1u)) break;
-        mbar_expect_tx(b_full + 8 * rp.idx, p.b_stage_bytes);
-        mbar_expect_tx(side_full + 8 * rp.idx, (uint32_t)NP * 32u);
-        bulk_g2s(base + p.b_off + rp.idx * p.b_stage_bytes, p.bimg + ((size_t)kt * 2) * (NP * 128), p.b_stage_bytes, b_full + 8 * rp.idx);
-        bulk_g2s(base + p.side_off + rp.idx * p.side_stage_bytes + HDR_BYTES, p.meta + (size_t)kt * (NP * 32), (uint32_t)NP * 32u, side_full + 8 * rp.idx);
-        if (++kt == KT) kt = 0;
-        rp.advance(1, F_RING);
-      }
-    }
-  } else if (warp < F_CONV_WARP0) {
-    // ---- MMA issuers: plane pl (0: q_lo sc, 1: q_hi sc) of half step h ----
-    const int pl = (warp - F_MMA_WARP0) >> 1, h = (warp - F_MMA_WARP0) & 1;
-    // (the whole warp runs the loop, as in the kernel above)
-    const uint32_t idesc = idesc_u8s8(NP);
-    bool alive = true;
-    RingPos rp{0, 0}; // step i in the drain-freed ring
-    uint32_t acc_ph = 0;
-    for (int i = 0; i < nunits; i++) {
-      const int buf = i & (NBUF - 1), st = 2 * (i & 1) + h; // half step j = 2 i + h uses operand stage j % 4
-      if (alive) alive = mbar_wait(b_full + 8 * rp.idx, rp.ph, 4u);
-      if (alive) alive = mbar_wait(a_full + 8 * st, (uint32_t)(i >> 1) & 1u, 4u);
-      if (alive && i >= NBUF) alive = mbar_wait(acc_empty + 8 * buf, acc_ph ^ 1u, 4u); // the drain of the buffer's previous step
-      tc_fence_after();
-      __syncwarp();
-      const uint64_t adesc = smem_desc_sw128(base + p.a_off + st * F_A_STAGE_BYTES + pl * A_STAGE_BYTES);
-      const uint64_t bdesc = smem_desc_sw128(base + p.b_off + rp.idx * p.b_stage_bytes + h * (NP * 128));
-      const uint32_t dcol = tmem_d + (uint32_t)(buf * BUF_COLS + (pl * 2 + h) * NP);
-      if (elect_one() && alive) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) umma_i8_acc(dcol, adesc + (uint64_t)(q * 2), bdesc + (uint64_t)(q * 2), idesc, q > 0 ? 1u : 0u);
-        umma_commit(acc_full + 8 * buf);
-      }
-      __syncwarp();
-      rp.advance(1, F_RING);
-      if (buf == NBUF - 1) acc_ph ^= 1u;
-    }
-  } else if (warp < F_DRAIN_WARP0) {
-    // ---- converters: group h (four warps, one thread per weight row) writes both planes of half step h of every step ----
-    const int cw = warp - F_CONV_WARP0;
-    const int r0 = (cw & 3) * 32, r = r0 + lane, h = cw >> 2;
-    const int sw = r & 7;
-    const uint32_t slot0 = base + p.raw_off0 + (uint32_t)(cw * D) * F_SLOT;
-    const int64_t n = p.w.n;
-    int l_i = 0, l_tile = tile0, l_kt = kt0, l_s = 0;
-    auto issue = [&]() { // lane l copies chunk l % 4 of row q * 8 + l / 4 in instruction q; then its own row's header
-      const uint32_t dst = slot0 + (uint32_t)l_s * F_SLOT;
-      const int c = lane & 3;
-      const uint32_t in_row = (uint32_t)l_kt * 144u + 16u + (uint32_t)(h * 64 + c * 16);
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int rw = q * 8 + (lane >> 2);
-        const int64_t grow = (int64_t)l_tile * TILE_N + r0 + rw;
-        const bool ok = grow < n;
-        cp_async16(dst + (uint32_t)(rw * 64 + ((c ^ (rw & 3)) << 4)), p.src[0] + (size_t)(ok ? grow : n - 1) * p.row_bytes[0] + in_row, ok ? 16u : 0u);
-      }
-      const int64_t grow = (int64_t)l_tile * TILE_N + r;
-      cp_async16(dst + 2048 + lane * 16, p.src[0] + (size_t)(grow < n ? grow : n - 1) * p.row_bytes[0] + (size_t)l_kt * 144u, grow < n ? 16u : 0u);
-      l_i++;
-      if (++l_kt == KT) l_kt = 0, l_tile++;
-      if (++l_s == D) l_s = 0;
-    };
-    for (int u = 0; u < D; u++) {
-      if (l_i < nunits) issue();
-      cp_async_commit();
-    }
-    bool alive = true;
-    int rs = 0;
-    RingPos rp{0, 0};
-    for (int i = 0; i < nunits && alive; i++) {
-      const int st = 2 * (i & 1) + h;
-      cp_async_wait(D - 1);
-      __syncwarp();
-      const uint32_t slot = slot0 + (uint32_t)rs * F_SLOT;
-      const uint4 hdr = lds128(slot + 2048 + lane * 16);
-      if (h == 0) { // hand the row's header on to the drain
-        if (i >= F_RING) alive = mbar_wait_warp(side_empty + 8 * rp.idx, rp.ph ^ 1u, 2u);
-        if (!alive) break;
-        sts128(base + p.side_off + rp.idx * p.side_stage_bytes + (uint32_t)r * 16, hdr);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(side_full + 8 * rp.idx);
-      }
-      // the stage's previous half step belongs to step i - 2: all of that step's MMAs have been committed
-      if (i >= 2) alive = mbar_wait_warp(acc_full + 8 * ((i - 2) & (NBUF - 1)), (uint32_t)((i - 2) / NBUF) & 1u, 2u);
-      if (!alive) break;
-      // the four sub-block scales of this half step: fields 2h and 2h + 1 of the repacked header
-      const uint32_t lo32 = h ? __funnelshift_r(hdr.z, hdr.w, 16) : hdr.y;
-      const uint32_t hi16 = h ? (hdr.w >> 16) : (hdr.z & 0xffffu);
-      const uint32_t f0 = lo32 & 0xffffffu, f1 = __funnelshift_r(lo32, hi16, 24) & 0xffffffu;
-      const uint32_t sc[4] = {f0 & 63u, (f0 >> 6) & 63u, f1 & 63u, (f1 >> 6) & 63u};
-      const uint32_t row = slot + (uint32_t)lane * 64;
-      const uint4 raw[4] = {raw_chunk<64>(row, lane, 0), raw_chunk<64>(row, lane, 1), raw_chunk<64>(row, lane, 2), raw_chunk<64>(row, lane, 3)};
-      const uint32_t a_stage = base + p.a_off + st * F_A_STAGE_BYTES + (uint32_t)r * 128;
-#pragma unroll
-      for (int pl = 0; pl < 2; pl++) {
-#pragma unroll
-        for (int pair = 0; pair < 2; pair++) { // 32-byte chunk `pair` of the half step: sub-blocks 2 pair (low nibbles) and 2 pair + 1 (high nibbles)
-#pragma unroll
-          for (int nib = 0; nib < 2; nib++) {
-            const int sh = 4 * nib + 2 * pl;
-            const uint32_t m = sc[2 * pair + nib];
-#pragma unroll
-            for (int half16 = 0; half16 < 2; half16++) { // the chunk's first and second 16 bytes: elements 0..15 and 16..31 of the sub-block
-              const uint4 w = raw[2 * pair + half16];
-              const uint4 o = make_uint4(((w.x >> sh) & 0x03030303u) * m, ((w.y >> sh) & 0x03030303u) * m, ((w.z >> sh) & 0x03030303u) * m,
-                                         ((w.w >> sh) & 0x03030303u) * m);
-              const int chunk = (2 * pair + nib) * 2 + half16; // 16-byte chunk of the 128-byte operand row
-              sts128(a_stage + pl * A_STAGE_BYTES + (uint32_t)((chunk ^ sw) << 4), o);
-            }
-          }
-        }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(a_full + 8 * st);
-      if (l_i < nunits) issue();
-      cp_async_commit();
-      if (++rs == D) rs = 0;
-      rp.advance(1, F_RING);
-    }
-    cp_async_wait(0);
-  } else {
-    // ---- drain: group dg (four warps, a thread per weight row, all NP columns) takes the steps i = dg, dg + 2, ... ----
-    const int dwi = warp - F_DRAIN_WARP0;
-    const int q = warp & 3, dg = dwi >> 2;
-    const int et = threadIdx.x - F_DRAIN_WARP0 * 32; // 0..255
-    pdl_wait(); // the kernel that prepares the activations also zeroes the tiles' tickets
-    bool alive = true;
-    int tile = tile0, kt = kt0;
-    float acc[NP];
-#pragma unroll
-    for (int c = 0; c < NP; c++) acc[c] = 0.f;
-    int seg_kt0 = kt0;
-    float *pair = p.pair_scratch + (size_t)blockIdx.x * NP * TILE_N;
-    RingPos rp{0, 0};
-    for (int i = 0; i < nunits; i++) {
-      const int buf = i & (NBUF - 1);
-      if ((i & 1) == dg) {
-        if (alive) alive = mbar_wait_warp(side_full + 8 * rp.idx, rp.ph, 8u);
-        const uint32_t side = base + p.side_off + rp.idx * p.side_stage_bytes;
-        uint4 hdr = make_uint4(0, 0, 0, 0);
-        if (alive) hdr = lds128(side + (uint32_t)(32 * q + lane) * 16);
-        if (alive) alive = mbar_wait_warp(acc_full + 8 * buf, (uint32_t)(i / NBUF) & 1u, 8u);
-        if (alive) {
-          tc_fence_after();
-          const __half2 dm = *reinterpret_cast<const __half2 *>(&hdr.x);
-          const float d = __low2float(dm), dmin = __high2float(dm);
-          // the eight 6-bit mins as bytes: fields F0..F3 hold mn[2g] at bit 12 and mn[2g+1] at bit 18
-          const uint32_t F0 = hdr.y & 0xffffffu, F1 = __funnelshift_r(hdr.y, hdr.z, 24) & 0xffffffu, F2 = __funnelshift_r(hdr.z, hdr.w, 16) & 0xffffffu, F3 = hdr.w >> 8;
-          const uint32_t mins0 = ((F0 >> 12) & 63u) | (((F0 >> 18) & 63u) << 8) | (((F1 >> 12) & 63u) << 16) | (((F1 >> 18) & 63u) << 24);
-          const uint32_t mins1 = ((F2 >> 12) & 63u) | (((F2 >> 18) & 63u) << 8) | (((F3 >> 12) & 63u) << 16) | (((F3 >> 18) & 63u) << 24);
-          const uint32_t taddr = tmem_d + ((uint32_t)(32 * q) << 16) + (uint32_t)(buf * BUF_COLS);
-#pragma unroll
-          for (int ch = 0; ch < NP / CH; ch++) {
-            uint32_t v[4][CH]; // slices: plane lo half 0, lo half 1, hi half 0, hi half 1
-#pragma unroll
-            for (int sl = 0; sl < 4; sl++) tmem_ld<CH>(taddr + (uint32_t)(sl * NP + ch * CH), v[sl]);
-            tmem_ld_wait();
-            if (ch == NP / CH - 1) { // every value of the buffer is in registers: it may be overwritten
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(acc_empty + 8 * buf);
-            }
-#pragma unroll
-            for (int c = 0; c < CH; c++) {
-              const uint32_t rec = side + HDR_BYTES + (uint32_t)(ch * CH + c) * 32;
-              const uint4 bs = lds128(rec); // {lo bytes half 0, hi bytes half 0, lo bytes half 1, hi bytes half 1} of the activations' 32-sums
-              const float da = __uint_as_float(lds32(rec + 16));
-              const int isum = 4 * ((int)v[2][c] + (int)v[3][c]) + ((int)v[0][c] + (int)v[1][c]);
-              const int msum = dp4a_uu(mins0, bs.x, dp4a_uu(mins1, bs.z, 0)) + 128 * dp4a_us(mins0, bs.y, dp4a_us(mins1, bs.w, 0));
-              acc[ch * CH + c] += da * (d * (float)isum - dmin * (float)msum);
-            }
-          }
-        }
-        __syncwarp();
-        if (alive && lane == 0) mbar_arrive(side_empty + 8 * rp.idx);
-      }
-      // ---- end of a segment (the tile's last step, or this CTA's last unit): store or hand over the sums ----
-      const bool tile_end = kt == KT - 1, range_end = i == nunits - 1;
-      if (tile_end || range_end) {
-        const int64_t row = (int64_t)tile * TILE_N + 32 * q + lane;
-        if (dg == 1) { // the odd steps' sums join the even ones': always even + odd, whatever the timing
-#pragma unroll
-          for (int c = 0; c < NP; c++) pair[(size_t)c * TILE_N + 32 * q + lane] = acc[c];
-          __threadfence_block();
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(F_DRAIN_WARPS * 32) : "memory");
-        if (dg == 0) {
-#pragma unroll
-          for (int c = 0; c < NP; c++) acc[c] += pair[(size_t)c * TILE_N + 32 * q + lane];
-        }
-        const bool whole = seg_kt0 == 0 && tile_end;
-        if (whole) {
-          if (dg == 0 && alive && row < p.w.n) {
-#pragma unroll
-            for (int c = 0; c < NP; c++) {
-              if (c < p.m) {
-                const int64_t idx = (int64_t)c * p.ldy + row;
-                if (p.y_dtype == XNQ_F32) static_cast<float *>(p.y)[idx] = acc[c];
-                else if (p.y_dtype == XNQ_F16) static_cast<__half *>(p.y)[idx] = __float2half_rn(acc[c]);
-                else static_cast<__nv_bfloat16 *>(p.y)[idx] = __float2bfloat16_rn(acc[c]);
-              }
-            }
-          }
-          asm volatile("bar.sync 1, %0;" ::"n"(F_DRAIN_WARPS * 32) : "memory"); // group 0 has read the scratch: it may be rewritten
-        } else {
-          const int seg_u0 = tile * KT + seg_kt0;
-          float *mine = p.partials + ((size_t)2 * blockIdx.x + (seg_u0 == u0 ? 0 : 1)) * NP * TILE_N;
-          if (dg == 0) {
-#pragma unroll
-            for (int c = 0; c < NP; c++) mine[(size_t)c * TILE_N + 32 * q + lane] = acc[c];
-            __threadfence();
-          }
-          asm volatile("bar.sync 1, %0;" ::"n"(F_DRAIN_WARPS * 32) : "memory");
-          if (et == 0) s_ticket = atomicAdd(p.tile_cnt + tile, 1u);
-          asm volatile("bar.sync 1, %0;" ::"n"(F_DRAIN_WARPS * 32) : "memory");
-          const unsigned int ticket = s_ticket;
-          asm volatile("bar.sync 1, %0;" ::"n"(F_DRAIN_WARPS * 32) : "memory");
-          const int t_u0 = tile * KT, t_u1 = t_u0 + KT;
-          const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u1 - 1, p.units_q, p.units_r);
-          if (et == 0 && (int)ticket == c_last - c_first) p.tile_cnt[tile] = 0u; // every part has its ticket: the word is zero again for the next call
-          if (dg == 0 && (int)ticket == c_last - c_first) { // the last part to arrive adds all parts in k order
-            __threadfence();
-#pragma unroll
-            for (int c = 0; c < NP; c++) acc[c] = 0.f;
-            for (int cc = c_first; cc <= c_last; cc++) {
-              const int cu0 = cta_first_unit(cc, p.units_q, p.units_r);
-              const float *part = p.partials + ((size_t)2 * cc + (cu0 >= t_u0 ? 0 : 1)) * NP * TILE_N;
-#pragma unroll
-              for (int c = 0; c < NP; c++) acc[c] += __ldcg(part + (size_t)c * TILE_N + 32 * q + lane);
-            }
-            if (row < p.w.n) {
-#pragma unroll
-              for (int c = 0; c < NP; c++) {
-                if (c < p.m) {
-                  const int64_t idx = (int64_t)c * p.ldy + row;
-                  if (p.y_dtype == XNQ_F32) static_cast<float *>(p.y)[idx] = acc[c];
-                  else if (p.y_dtype == XNQ_F16) static_cast<__half *>(p.y)[idx] = __float2half_rn(acc[c]);
-                  else static_cast<__nv_bfloat16 *>(p.y)[idx] = __float2bfloat16_rn(acc[c]);
-                }
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < NP; c++) acc[c] = 0.f;
-        seg_kt0 = 0;
-      }
-      if (++kt == KT) kt = 0, tile++;
-      rp.advance(1, F_RING);
-    }
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  if (warp == F_MMA_WARP0) tmem_dealloc(tmem_d, TMEM_COLS);
 }
 
 // ---- activations: quantize (or take an activation image), lay out as the MMA's B operand, write the records ----
@@ -1202,11 +841,10 @@ __global__ void __launch_bounds__(256) imma_prepare(const XT *__restrict__ x, co
 }
 
 int g_sms = 0;
-std::atomic<int> g_fold{0}; // Q4_K, imma_q4k_fold_kernel: 2 whenever the weight is Q4_K, else never
 
 struct Plan {
   int NP, nsteps, tiles, grid;
-  size_t bimg_bytes, meta_bytes, cnt_bytes, part_bytes, pair_bytes;
+  size_t bimg_bytes, meta_bytes, cnt_bytes, part_bytes;
 };
 // operand images have their own row counts (operand_np); paired: two operand columns per row
 Plan plan_for(int64_t m, int64_t k, int64_t n, bool operand, bool paired) {
@@ -1221,11 +859,10 @@ Plan plan_for(int64_t m, int64_t k, int64_t n, bool operand, bool paired) {
   pl.meta_bytes = up((size_t)pl.nsteps * pl.NP * 32);
   pl.cnt_bytes = up((size_t)pl.tiles * 4);
   pl.part_bytes = up((size_t)2 * (g_sms > 0 ? g_sms : 148) * pl.NP * TILE_N * 4);
-  pl.pair_bytes = up((size_t)(g_sms > 0 ? g_sms : 148) * pl.NP * TILE_N * 4);
   return pl;
 }
 
-template <typename Conv, template <int> class Drain>
+template <typename Conv>
 int launch_np(const ImmaArgs &a, int NP, unsigned grid, cudaStream_t s) {
   // programmatic stream serialization: the kernel starts while the one that prepares the activations still runs; only
   // its weight loads are issued before griddepcontrol.wait
@@ -1240,23 +877,23 @@ int launch_np(const ImmaArgs &a, int NP, unsigned grid, cudaStream_t s) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if constexpr (Conv::PAIRED) { // 16 rows, 32 columns
-    XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 32>, a));
-  } else if (NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 16>, a));
-  else if (NP == 32) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 32>, a));
-  else if (NP == 48) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 48>, a));
-  else XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, Drain, 64>, a));
+    XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 32>, a));
+  } else if (NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 16>, a));
+  else if (NP == 32) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 32>, a));
+  else if (NP == 48) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 48>, a));
+  else XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 64>, a));
   count_launch();
   return XNQ_OK;
 }
 
-template <typename Conv, template <int> class Drain>
+template <typename Conv>
 int init_np() {
   if constexpr (!Conv::PAIRED) {
-    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
-    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
-    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 48>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+    XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, 48>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   }
-  XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, Drain, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
+  XNQ_CUDA(cudaFuncSetAttribute(imma_kernel<Conv, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
   return XNQ_OK;
 }
 
@@ -1277,7 +914,7 @@ bool imma_supported(const WeightView &w, int64_t m) {
 size_t imma_workspace_bytes(int64_t m, int64_t k, int64_t n) {
   // the widest operand any form of these rows takes: two columns per row up to 16 rows (Q6_K), an operand image's count above
   const Plan pl = m <= Q6K_MAX_M ? plan_for(m, k, n, false, true) : plan_for(std::min<int64_t>(m, MAX_NP), k, n, true, false);
-  return pl.bimg_bytes + pl.meta_bytes + pl.cnt_bytes + pl.part_bytes + pl.pair_bytes + 256;
+  return pl.bimg_bytes + pl.meta_bytes + pl.cnt_bytes + pl.part_bytes + 256;
 }
 
 // x: float activations [m, k] (x_dtype F32 / F16 / BF16, row stride ldx) or an activation image (XNQ_ACT_IMAGE) of m rows.
@@ -1286,17 +923,11 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
   const int64_t k = w.k;
   const int act = act_dtype_for(w.dtype);
   const size_t yes = type_size(y_dtype);
-  // Q4_K with the sub-block scales folded into the weight operand is kept behind the option: it needs half the slices to drain but
-  // twice the MMAs, and since the per-block kernel issues its MMAs at the tensor core's rate that is nowhere faster (14336 x 4096,
-  // 32 rows: 28.7 us against 26.4; 4096 x 4096: 22.4 against 14.7).
-  const int fold_opt = g_fold.load(std::memory_order_relaxed);
-  const bool fold = w.dtype == XNQ_Q4K && fold_opt == 2 && !(x_dtype == XNQ_ACT_OPERAND && m > 32); // an operand image is one pass
   const bool paired = w.dtype == XNQ_Q6K;
-  const int64_t pass_rows = fold ? 32 : MAX_NP;
   const bool operand = x_dtype == XNQ_ACT_OPERAND; // the activations arrive in the kernel's own layout, with their ticket words: no activation kernel
-  if (operand && (w.dtype != XNQ_Q4K || k % 256 || m > pass_rows)) return fail(XNQ_ERR_UNSUPPORTED, "imma: an operand image serves Q8_K activations of one pass (m = %lld)", (long long)m);
-  for (int64_t r0 = 0; r0 < m; r0 += pass_rows) { // passes of at most 64 (32) activation rows
-    const int64_t rows = std::min<int64_t>(pass_rows, m - r0);
+  if (operand && (w.dtype != XNQ_Q4K || k % 256 || m > MAX_NP)) return fail(XNQ_ERR_UNSUPPORTED, "imma: an operand image serves Q8_K activations of one pass (m = %lld)", (long long)m);
+  for (int64_t r0 = 0; r0 < m; r0 += MAX_NP) { // passes of at most 64 activation rows
+    const int64_t rows = std::min<int64_t>(MAX_NP, m - r0);
     const Plan pl = plan_for(rows, k, w.n, operand, paired);
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     uint8_t *bimg = ws;
@@ -1354,7 +985,6 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     a.units_q = a.units / pl.grid, a.units_r = a.units % pl.grid;
     a.tile_cnt = cnt;
     a.partials = partials;
-    a.pair_scratch = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(partials) + pl.part_bytes);
     int rc, step_code; // step_code: code bytes per row and step
     switch (w.dtype) {
       case XNQ_Q4K:
@@ -1383,33 +1013,6 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
         a.pf_share[st] = ((a.pf_bytes[st] / (unsigned)pl.grid) + PF_CHUNK - 1) & ~(unsigned long long)(PF_CHUNK - 1);
       }
     }
-    if (fold) {
-      a.b_stage_bytes = (uint32_t)pl.NP * 256;
-      a.side_stage_bytes = HDR_BYTES + (uint32_t)pl.NP * 32;
-      a.a_off = 0;
-      a.b_off = (uint32_t)F_ASTAGES * F_A_STAGE_BYTES;
-      a.side_off = a.b_off + F_RING * a.b_stage_bytes;
-      a.raw_off0 = (a.side_off + F_RING * a.side_stage_bytes + 127) & ~127u;
-      const size_t left = IMMA_SMEM - 1024 - a.raw_off0;
-      a.raw_stages = (int)std::min<size_t>(6, left / ((size_t)F_CONV_WARPS * F_SLOT)); // raw slots per converter warp
-      if (a.raw_stages < 2) return fail(XNQ_ERR_SIZE, "imma: shared-memory plan does not fit");
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3((unsigned)pl.grid);
-      cfg.blockDim = dim3(F_NTHREADS);
-      cfg.dynamicSmemBytes = IMMA_SMEM;
-      cfg.stream = s;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      profile_mark(s, true);
-      if (pl.NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_q4k_fold_kernel<16>, a));
-      else XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_q4k_fold_kernel<32>, a));
-      count_launch();
-      profile_mark(s, false);
-      continue;
-    }
     a.raw_stage_bytes = (uint32_t)(CONV_WARPS / 2) * (32u * (uint32_t)step_code + 512u); // a step in flight: four warp slots of the rows' code bytes and 16 scale bytes per row
     a.b_stage_bytes = (uint32_t)pl.NP * 256;
     a.side_stage_bytes = HDR_BYTES + (uint32_t)pl.NP * 32 + (paired ? TILE_N * 4 : 0);
@@ -1436,10 +1039,10 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     a.side_off = a.b_off + a.b_stages * a.b_stage_bytes;
     a.raw_off0 = (a.side_off + SIDE_STAGES * a.side_stage_bytes + 127) & ~127u;
     profile_mark(s, true);
-    if (w.dtype == XNQ_Q4K) rc = launch_np<ConvQ4K, DrainQ4K>(a, pl.NP, (unsigned)pl.grid, s);
-    else if (w.dtype == XNQ_Q8_0) rc = launch_np<ConvQ8_0, DrainBlockScaled>(a, pl.NP, (unsigned)pl.grid, s);
-    else if (w.dtype == XNQ_Q6K) rc = launch_np<ConvQ6K, DrainQ6K>(a, pl.NP, (unsigned)pl.grid, s);
-    else rc = launch_np<ConvQ4_0, DrainBlockScaled>(a, pl.NP, (unsigned)pl.grid, s);
+    if (w.dtype == XNQ_Q4K) rc = launch_np<ConvQ4K>(a, pl.NP, (unsigned)pl.grid, s);
+    else if (w.dtype == XNQ_Q8_0) rc = launch_np<ConvQ8_0>(a, pl.NP, (unsigned)pl.grid, s);
+    else if (w.dtype == XNQ_Q6K) rc = launch_np<ConvQ6K>(a, pl.NP, (unsigned)pl.grid, s);
+    else rc = launch_np<ConvQ4_0>(a, pl.NP, (unsigned)pl.grid, s);
     profile_mark(s, false);
     if (rc != XNQ_OK) return rc;
   }
@@ -1451,12 +1054,10 @@ int imma_init(int device) {
   XNQ_CUDA(cudaGetDeviceProperties(&prop, device));
   g_sms = prop.multiProcessorCount;
   int rc;
-  if ((rc = init_np<ConvQ4K, DrainQ4K>()) != XNQ_OK) return rc;
-  XNQ_CUDA(cudaFuncSetAttribute(imma_q4k_fold_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(imma_q4k_fold_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IMMA_SMEM));
-  if ((rc = init_np<ConvQ8_0, DrainBlockScaled>()) != XNQ_OK) return rc;
-  if ((rc = init_np<ConvQ6K, DrainQ6K>()) != XNQ_OK) return rc;
-  if ((rc = init_np<ConvQ4_0, DrainBlockScaled>()) != XNQ_OK) return rc;
+  if ((rc = init_np<ConvQ4K>()) != XNQ_OK) return rc;
+  if ((rc = init_np<ConvQ8_0>()) != XNQ_OK) return rc;
+  if ((rc = init_np<ConvQ6K>()) != XNQ_OK) return rc;
+  if ((rc = init_np<ConvQ4_0>()) != XNQ_OK) return rc;
 #define XNQ_IMMA_PREP_INIT(ACT, XT) XNQ_CUDA(cudaFuncSetAttribute(imma_prepare<ACT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SPREAD))
   XNQ_IMMA_PREP_INIT(XNQ_Q8_0, float);
   XNQ_IMMA_PREP_INIT(XNQ_Q8_0, __half);
@@ -1469,9 +1070,6 @@ int imma_init(int device) {
   XNQ_CUDA(cudaMemcpyToSymbol(g_imma_status, &zero, sizeof(zero)));
   return XNQ_OK;
 }
-
-
-void imma_set_fold(int on) { g_fold.store(on); }
 
 int imma_status(unsigned int *bits) {
   XNQ_CUDA(cudaMemcpyFromSymbol(bits, g_imma_status, sizeof(*bits)));
