@@ -148,14 +148,15 @@ int xnq_quantize_weight(int ggml_dtype, const float *x_dev, int64_t n, int64_t k
 int xnq_quantize_act(int act_dtype, const void *x, int x_dtype, int64_t m, int64_t k, int64_t ldx,
                      void *dst_blocks, void *stream);
 
-/* Scratch bytes xnq_matmul_t needs for up to max_m activation rows against this weight. */
+/* Scratch bytes of xnq_matmul_t for up to max_m activation rows against this weight. (Less is refused, but for Q6_K at 6..16 rows:
+ * xnq_act_image_bytes(XNQ_Q8K, m, k) bytes are enough there for the kernel that needs no partial sums, which is slower.) */
 size_t xnq_matmul_workspace_bytes(const xnq_weight *w, int64_t max_m);
 
 /* y[m, n_local] = x[m, k] . W^T, the quantized matmul of k_quants::matmul (k_quants.rs:1997-2011)
  * = QTensor::matmul_t (quantized/mod.rs:334-339) = Q8Tensor::matmul_t (q8.rs:116-157):
  * activations are quantized to the weight format's VecDotType exactly as the CPU path does, dots
- * use exact integer block sums and f32 accumulation (m <= 16), or tensor-core MMA on the
- * dequantized operands (m > 16).
+ * use exact integer block sums and f32 accumulation (m <= 64; Q6_K: m <= 16; Q4_1, Q5_0, Q5_1, Q2_K, Q3_K
+ * and Q5_K: any m), or tensor-core MMA on the dequantized operands.
  *   x, y: device memory, x_dtype / y_dtype in {F32, F16, BF16}; ldx, ldy in elements;
  *   x rows 16-byte aligned; workspace 256-byte aligned, ws_bytes >= xnq_matmul_workspace_bytes.
  * Enqueues on `stream` only; allocates nothing. */

@@ -139,8 +139,8 @@ static int matmul_from_operand(const xnq_weight *w, const void *image, int64_t m
   if (w->v.dtype != XNQ_Q4K || !use_imma(w, m))
     return fail(XNQ_ERR_UNSUPPORTED, "matmul_t: an operand image serves 2..%lld rows on Q4_K weights (dtype %d, m = %lld)",
                 (long long)IMMA_MAX_M, w->v.dtype, (long long)m);
-  if (!workspace || !aligned(workspace, 256) || ws_bytes < imma_workspace_bytes(m, k, n))
-    return fail(XNQ_ERR_SIZE, "matmul_t: the workspace (256-byte aligned, %zu bytes) is needed for the partial sums", imma_workspace_bytes(m, k, n));
+  if (!workspace || !aligned(workspace, 256) || ws_bytes < imma_workspace_bytes(w->v, m))
+    return fail(XNQ_ERR_SIZE, "matmul_t: the workspace (256-byte aligned, %zu bytes) is needed for the partial sums", imma_workspace_bytes(w->v, m));
   return launch_imma(w->v, image, XNQ_ACT_OPERAND, m, k, y, y_dtype, ldy, workspace, s);
 }
 
@@ -157,7 +157,7 @@ static int matmul_from_image(const xnq_weight *w, const void *image, int64_t m, 
   const int adt = act_dtype_for(w->v.dtype);
   int rc;
   // two rows and up: the integer tensor-core kernel, where the caller gave it its scratch (it re-lays the image out)
-  if (use_imma(w, m) && workspace && aligned(workspace, 256) && ws_bytes >= imma_workspace_bytes(m, k, n))
+  if (use_imma(w, m) && workspace && aligned(workspace, 256) && ws_bytes >= imma_workspace_bytes(w->v, m))
     return launch_imma(w->v, image, XNQ_ACT_IMAGE, m, k, y, y_dtype, ldy, workspace, s);
   if (matvec_tma_enabled() && matvec_tma_supported(w->v, m)) {
     profile_mark(s, true);
@@ -553,15 +553,21 @@ int xnq_matvec_normed(const xnq_weight *w, const float *x_in, const float *delta
   return rc;
 }
 
+// Scratch without which a call of up to max_m rows is refused. Q6_K at 6..16 rows: the dp4a kernel's few KB; the integer tensor-core
+// kernel, which those rows run on where the caller has brought its scratch as well, came later than programs that size their own.
+static size_t least_workspace_bytes(const xnq_weight *w, int64_t max_m) {
+  if (is_generic_dtype(w->v.dtype)) return generic_workspace_bytes(w->v, max_m);
+  size_t need = act_workspace_bytes(std::min<int64_t>(max_m, MATVEC_MAX_M), w->v.k, act_dtype_for(w->v.dtype));
+  if (w->v.dtype != XNQ_Q6K && max_m >= 2 && imma_supported(w->v, 2)) need = std::max(need, imma_workspace_bytes(w->v, std::min<int64_t>(max_m, IMMA_MAX_M)));
+  if (max_m > MATVEC_MAX_M) need = std::max(need, prefill_workspace_bytes(max_m, w->v.k, w->v.n));
+  return need;
+}
+
 size_t xnq_matmul_workspace_bytes(const xnq_weight *w, int64_t max_m) {
   if (!w || max_m <= 0) return 0;
-  if (is_generic_dtype(w->v.dtype)) return generic_workspace_bytes(w->v, max_m);
-  const int64_t rows = max_m < MATVEC_MAX_M ? max_m : MATVEC_MAX_M;
-  size_t decode = act_workspace_bytes(rows, w->v.k, act_dtype_for(w->v.dtype));
-  if (max_m >= 2 && imma_supported(w->v, w->v.dtype == XNQ_Q6K ? MATVEC_MAX_M : 2)) decode = std::max(decode, imma_workspace_bytes(std::min<int64_t>(max_m, IMMA_MAX_M), w->v.k, w->v.n));
-  if (max_m <= MATVEC_MAX_M) return decode;
-  const size_t prefill = prefill_workspace_bytes(max_m, w->v.k, w->v.n); // m > 16 runs on the tensor cores
-  return prefill > decode ? prefill : decode;
+  const size_t need = least_workspace_bytes(w, max_m);
+  const int64_t q6k_rows = std::min<int64_t>(max_m, IMMA_Q6K_MAX_M);
+  return w->v.dtype == XNQ_Q6K && imma_supported(w->v, q6k_rows) ? std::max(need, imma_workspace_bytes(w->v, q6k_rows)) : need;
 }
 
 int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
@@ -579,7 +585,7 @@ int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int
   if (m == 0 || n == 0) return XNQ_OK;
   if (!y) return fail(XNQ_ERR_NULL, "matmul_t: y is NULL");
   if (!aligned(y, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "matmul_t: y is not aligned to its element size");
-  const size_t need = xnq_matmul_workspace_bytes(w, m);
+  const size_t need = least_workspace_bytes(w, m);
   if (!workspace) return fail(XNQ_ERR_NULL, "matmul_t: workspace is NULL (need %zu bytes)", need);
   if (!aligned(workspace, 256)) return fail(XNQ_ERR_ALIGN, "matmul_t: workspace must be 256-byte aligned");
   if (ws_bytes < need) return fail(XNQ_ERR_SIZE, "matmul_t: workspace has %zu bytes, m = %lld needs %zu", ws_bytes, (long long)m, need);
@@ -601,7 +607,8 @@ int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int
     profile_mark(s, false);
     return rc;
   }
-  if (use_imma(w, m)) return launch_imma(w->v, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s); // exact integer dots on the tensor cores
+  if (use_imma(w, m) && ws_bytes >= imma_workspace_bytes(w->v, m)) // exact integer dots on the tensor cores
+    return launch_imma(w->v, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s);
   if (m > MATVEC_MAX_M) return launch_prefill(w->v, w->wscale, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s);
   bool use_mma = false;
   const int64_t pass = small_batch_pass(w, m, y_dtype, &use_mma);

@@ -320,7 +320,7 @@ int matvec_check_record(unsigned long long out[8]);
 
 // xnq_imma.cu  (2 <= m <= 64: tcgen05 kind::i8, exact integer block sums; Q4_0 / Q8_0 / Q4_K, and Q6_K from 6 to 16 rows)
 bool imma_supported(const WeightView &w, int64_t m);
-size_t imma_workspace_bytes(int64_t m, int64_t k, int64_t n);
+size_t imma_workspace_bytes(const WeightView &w, int64_t m);
 int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
                 cudaStream_t s);
 int imma_init(int device);
@@ -337,6 +337,9 @@ constexpr int OPERAND_MAX_TILES = 1024;
 __host__ __device__ inline int operand_np(int64_t m) { return m <= 16 ? 16 : (m <= 32 ? 32 : 64); }
 __host__ __device__ inline size_t operand_bimg_bytes(int np, int64_t k) { return (size_t)(k / 256) * np * 256; }
 __host__ __device__ inline size_t operand_image_bytes(int64_t m, int64_t k) { return OPERAND_TICKET_BYTES + (size_t)(k / 256) * operand_np(m) * 288; }
+// Q6_K: below six rows the dp4a kernel is as fast or faster (4096 x 4096, 5 rows: 12.3 us against 13.5; 8 rows: 13.7 against 13.5, and on
+// 32000 x 4096 62 against 48), above 16 the fp16 kernel is (32000 x 4096, 24 rows: 59 us on the integer kernel, 55 on that one).
+constexpr int64_t IMMA_Q6K_MIN_M = 6, IMMA_Q6K_MAX_M = 16;
 constexpr int64_t IMMA_MAX_M = 64; // batches up to here take the integer tensor-core kernel; larger ones the fp16 one
 
 // xnq_prefill.cu  (m > 64, and Q6_K above 16 rows: tcgen05 / TMEM contraction on fp16 operands)

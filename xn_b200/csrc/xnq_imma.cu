@@ -53,9 +53,6 @@ __device__ unsigned int g_imma_status; // sticky: 1 producer, 2 converter, 4 mma
 namespace {
 
 constexpr int TILE_N = 128;         // weight rows per tile = UMMA M
-// Q6_K: below six rows the dp4a kernel is as fast or faster (4096 x 4096, 5 rows: 12.3 us against 13.5; 8 rows: 13.7 against 13.5, and on
-// 32000 x 4096 62 against 48), above 16 the fp16 kernel is (32000 x 4096, 24 rows: 59 us here, 55 there).
-constexpr int64_t Q6K_MIN_M = 6, Q6K_MAX_M = 16;
 constexpr int MAX_NP = 64;          // activation rows per pass = UMMA N (multiple of 16)
 constexpr int CONV_WARPS = 8, DRAIN_WARPS = 16;
 constexpr int ACT_PRODUCER_WARP = 0, MMA_WARP = 1, CONV_WARP0 = 3, DRAIN_WARP0 = CONV_WARP0 + CONV_WARPS; // MMA issuers: warps 1 and 2
@@ -259,7 +256,7 @@ struct ImmaArgs {
   int units_q, units_r; // CTA c works on units [c * units_q + min(c, units_r), + units_q + (c < units_r)): set at launch, so that
                         // no thread divides 64-bit numbers before its first copy
   unsigned int *tile_cnt; // [tiles] arrival tickets of split tiles, zeroed by the prepare kernel
-  float *partials;        // [2 * grid][NP][128] partial sums of split tiles
+  float *partials;        // [2 * grid][activation rows of the operand][128] partial sums of split tiles
   // raw weight bytes: stream 0 holds the codes (Q4_K: the whole 144-byte super-blocks), stream 1 the f16 block scales of Q4_0 / Q8_0
   const uint8_t *src[2];
   int nstreams;
@@ -858,7 +855,7 @@ Plan plan_for(int64_t m, int64_t k, int64_t n, bool operand, bool paired) {
   pl.bimg_bytes = up((size_t)pl.nsteps * 2 * pl.NP * 128);
   pl.meta_bytes = up((size_t)pl.nsteps * pl.NP * 32);
   pl.cnt_bytes = up((size_t)pl.tiles * 4);
-  pl.part_bytes = up((size_t)2 * (g_sms > 0 ? g_sms : 148) * pl.NP * TILE_N * 4);
+  pl.part_bytes = up((size_t)2 * (g_sms > 0 ? g_sms : 148) * (paired ? pl.NP / 2 : pl.NP) * TILE_N * 4);
   return pl;
 }
 
@@ -902,7 +899,7 @@ int init_np() {
 bool imma_supported(const WeightView &w, int64_t m) {
   if (g_sms <= 0 || m < 1 || w.n < 1) return false;
   if (w.dtype == XNQ_Q6K) {
-    if (m < Q6K_MIN_M || m > Q6K_MAX_M) return false;
+    if (m < IMMA_Q6K_MIN_M || m > IMMA_Q6K_MAX_M) return false;
   } else if (w.dtype != XNQ_Q4_0 && w.dtype != XNQ_Q8_0 && w.dtype != XNQ_Q4K) {
     return false;
   }
@@ -910,10 +907,9 @@ bool imma_supported(const WeightView &w, int64_t m) {
   return true;
 }
 
-// scratch of one call: the activations' operand image and records, the split tiles' tickets and partial sums
-size_t imma_workspace_bytes(int64_t m, int64_t k, int64_t n) {
-  // the widest operand any form of these rows takes: two columns per row up to 16 rows (Q6_K), an operand image's count above
-  const Plan pl = m <= Q6K_MAX_M ? plan_for(m, k, n, false, true) : plan_for(std::min<int64_t>(m, MAX_NP), k, n, true, false);
+// scratch of one call of m rows: the activations' operand image and records, the split tiles' tickets and partial sums. Grows with m.
+size_t imma_workspace_bytes(const WeightView &w, int64_t m) {
+  const Plan pl = plan_for(std::min<int64_t>(m, MAX_NP), w.k, w.n, w.dtype == XNQ_Q4K, w.dtype == XNQ_Q6K); // Q4_K: an operand image's columns are the most
   return pl.bimg_bytes + pl.meta_bytes + pl.cnt_bytes + pl.part_bytes + 256;
 }
 
