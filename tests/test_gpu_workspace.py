@@ -22,6 +22,9 @@ def _up(v):
 
 def earlier_answer(dt, m, k, n):
     """What xnq_matmul_workspace_bytes answered for m rows when the integer tensor-core kernel came in."""
+    if dt not in (D.Q4_0, D.Q8_0, D.Q4K, D.Q6K):   # the canonical activation blocks
+        block, size = {D.Q4_1: (32, 36), D.Q5_0: (32, 34), D.Q5_1: (32, 36)}.get(dt, (256, 292))
+        return _up(m * (k // block) * size)
     rows, block = min(m, 16), 32 if dt in (D.Q4_0, D.Q8_0) else 256
     need = _up(rows * k) + _up(rows * (k // block) * 4) + _up(rows * (k // 16) * 2)
     if dt is not D.Q6K and m >= 2:
@@ -36,7 +39,7 @@ def earlier_answer(dt, m, k, n):
 
 
 @pytest.mark.parametrize("m", [1, 2, 5, 6, 11, 16, 17, 33, 48, 64, 65])
-@pytest.mark.parametrize("dt", [D.Q4_0, D.Q8_0, D.Q4K, D.Q6K], ids=lambda d: d.name)
+@pytest.mark.parametrize("dt", [D.Q4_0, D.Q8_0, D.Q4K, D.Q6K, D.Q4_1, D.Q5_0, D.Q5_1, D.Q2K, D.Q3K, D.Q5K], ids=lambda d: d.name)
 def test_a_workspace_of_the_earlier_size_is_accepted_and_not_overrun(O, dt, m):
     from xn_b200 import _lib
     from xn_b200 import quantized as Q
@@ -55,13 +58,13 @@ def test_a_workspace_of_the_earlier_size_is_accepted_and_not_overrun(O, dt, m):
     _lib.check(L.xnq_matmul_t(w._h, p(xd), int(D.F32), m, k, p(y), int(D.F32), n, p(buf), size, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     assert bool((buf[size:] == 0xA5).all())
     want = O.matmul(int(dt), x, blocks, n)
-    if m <= (16 if dt is D.Q6K else 64):
+    if m <= (16 if dt is D.Q6K else 64) or dt not in (D.Q4_0, D.Q8_0, D.Q4K, D.Q6K):
         assert_close_ref(y.cpu().numpy(), want, 2e-3, f"{dt.name} m={m}")
     else:   # fp16 operands: 5e-3 of the outputs' rms
         assert np.abs(y.cpu().numpy() - want).max() <= 5e-3 * np.sqrt((want.astype(np.float64) ** 2).mean())
 
 
-@pytest.mark.parametrize("dt", [D.Q4_0, D.Q8_0, D.Q4K, D.Q6K], ids=lambda d: d.name)
+@pytest.mark.parametrize("dt", [D.Q4_0, D.Q8_0, D.Q4K, D.Q6K, D.Q5_0, D.Q5K], ids=lambda d: d.name)
 def test_the_answer_for_more_rows_serves_fewer(dt):
     from xn_b200 import _lib
     from xn_b200 import quantized as Q

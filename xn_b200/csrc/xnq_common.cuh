@@ -267,6 +267,7 @@ int layout_init(int device);
 int launch_quantize_act_blocks(int act_dtype, const void *x, int x_dtype, int64_t m, int64_t k, int64_t ldx,
                                void *dst_blocks, cudaStream_t s);
 int launch_quantize_act_planar(const ActView &a, const void *x, int x_dtype, int64_t ldx, cudaStream_t s);
+int launch_quantize_act_f16_scales(const ActView &a, const void *x, int x_dtype, int64_t ldx, cudaStream_t s); // Q8_0 codes; a.d and a.bsum hold __half
 int quantize_init(int device);
 
 // xnq_quantize_weight.cu: dense f32 [n, k] on the device -> canonical GGUF blocks on the device

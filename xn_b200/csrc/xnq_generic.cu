@@ -10,6 +10,8 @@
 //              scales and 16-sums, then one kernel unpacks the file's blocks to int8 codes in registers and multiplies them with
 //              dp4a: each block's integer sums are exact, scales are applied in f32 as in the reference, and only the order in
 //              which block contributions are added differs from its serial sum (within 2e-3 under its own metric).
+#include <algorithm>
+
 #include "xnq_common.cuh"
 #include "xnq_quantize_act.cuh"
 #include "xnq_unpack.cuh"
@@ -296,9 +298,9 @@ struct Raw<XNQ_Q5K> { // {f16 d; f16 dmin; u8 scales[12]; u8 qh[32]; u8 qs[128]}
 
 // What one piece adds to the dot of a (weight row, activation row) pair: exact integer sums, scaled in f32 as the reference does
 // (k_quants.rs:328-339 Q4_1, 423-436 Q5_0, 529-541 Q5_1, 904-945 Q2_K, 1087-1176 Q3_K, 1540-1604 Q5_K). lo, hi: the row's 32 codes;
-// da: its block scale; b0, b1: the sums of its first and second 16 codes.
+// da: its block scale; b0, b1: the sums of its first and second 16 codes; as: its block's s (Q4_1, Q5_1).
 template <int DT>
-__device__ __forceinline__ float piece_dot(const Piece &p, const uint4 &lo, const uint4 &hi, float da, int b0, int b1, float acc) {
+__device__ __forceinline__ float piece_dot(const Piece &p, const uint4 &lo, const uint4 &hi, float da, float as, int b0, int b1, float acc) {
   int t0 = __dp4a((int)p.c[0], (int)lo.x, 0);
   t0 = __dp4a((int)p.c[1], (int)lo.y, t0);
   t0 = __dp4a((int)p.c[2], (int)lo.z, t0);
@@ -307,10 +309,7 @@ __device__ __forceinline__ float piece_dot(const Piece &p, const uint4 &lo, cons
   t1 = __dp4a((int)p.c[5], (int)hi.y, t1);
   t1 = __dp4a((int)p.c[6], (int)hi.z, t1);
   t1 = __dp4a((int)p.c[7], (int)hi.w, t1);
-  if (DT == XNQ_Q4_1 || DT == XNQ_Q5_1) { // the block's min times s = f16(f16(sum) * d), as BlockQ8_1 stores it (k_quants.rs:847-873)
-    const float s = __half2float(__float2half_rn(__fmul_rn(__half2float(__float2half_rn((float)(b0 + b1))), da)));
-    return acc + __fadd_rn(__fmul_rn(__fmul_rn((float)t1, p.d), da), __fmul_rn(p.m, s));
-  }
+  if (DT == XNQ_Q4_1 || DT == XNQ_Q5_1) return acc + __fadd_rn(__fmul_rn(__fmul_rn((float)t1, p.d), da), __fmul_rn(p.m, as));
   if (DT == XNQ_Q5_0) return acc + __fmul_rn(__fmul_rn((float)t1, p.d), da);
   if (DT == XNQ_Q2K) return acc + __fsub_rn(__fmul_rn(__fmul_rn(da, p.d), (float)(p.s0 * t0 + p.s1 * t1)), __fmul_rn(__fmul_rn(da, p.m), (float)(p.m0 * b0 + p.m1 * b1)));
   if (DT == XNQ_Q3K) return acc + __fmul_rn(__fmul_rn(p.d, da), (float)(p.s0 * t0 + p.s1 * t1));
@@ -351,8 +350,9 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
   pdl_wait();
   const int nblk_a = K256 ? pieces >> 3 : pieces;
   const int8_t *aq = act.q + m0 * act.k;
-  const float *ad = act.d + m0 * nblk_a;
-  const int16_t *ab = act.bsum + m0 * (act.k / 16);
+  const float *ad = act.d + m0 * nblk_a;              // K256
+  const int16_t *ab = act.bsum + m0 * (act.k / 16);   // K256
+  const __half *hd = reinterpret_cast<const __half *>(act.d) + m0 * nblk_a, *hs = reinterpret_cast<const __half *>(act.bsum) + m0 * nblk_a; // the others
   float acc[NV];
 #pragma unroll
   for (int i = 0; i < NV; i++) acc[i] = 0.f;
@@ -370,14 +370,16 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
       if (i < rows) {
         const uint4 *a = reinterpret_cast<const uint4 *>(aq + (int64_t)i * act.k + (int64_t)j * 32);
         const uint4 lo = a[0], hi = a[1];
-        const float da = ad[(int64_t)i * nblk_a + (K256 ? j >> 3 : j)];
+        const int64_t blk = (int64_t)i * nblk_a + (K256 ? j >> 3 : j);
+        const float da = K256 ? ad[blk] : __half2float(hd[blk]);
+        const float as = DT == XNQ_Q4_1 || DT == XNQ_Q5_1 ? __half2float(hs[blk]) : 0.f;
         int b0 = 0, b1 = 0;
-        if (DT != XNQ_Q5_0 && DT != XNQ_Q3K) {
+        if (DT == XNQ_Q2K || DT == XNQ_Q5K) {
           const uint32_t b = *reinterpret_cast<const uint32_t *>(ab + (int64_t)i * (act.k / 16) + 2 * (int64_t)j);
           b0 = (int)(int16_t)(b & 0xffffu), b1 = (int)(int16_t)(b >> 16);
         }
 #pragma unroll
-        for (int r = 0; r < GR; r++) acc[i * GR + r] = piece_dot<DT>(p[r], lo, hi, da, b0, b1, acc[i * GR + r]);
+        for (int r = 0; r < GR; r++) acc[i * GR + r] = piece_dot<DT>(p[r], lo, hi, da, as, b0, b1, acc[i * GR + r]);
       }
     }
     if (MT >= 16 && jn < pieces) {
@@ -429,14 +431,15 @@ template <int DT>
 int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes, void *y, int y_dtype, int64_t ldy, cudaStream_t s) {
   const int rows_per_cta = TPB / 32 / k_splits((int)(w.k / 32)) * GR;
   const int mt = act.m >= 9 ? 16 : (act.m >= 5 ? 8 : (act.m >= 3 ? 4 : (int)act.m));
-  // grid.y is limited to 65535 tiles of activation rows
-  const int64_t pass = (int64_t)mt * 65535, nblk_a = w.k / (act.act_dtype == XNQ_Q8_0 ? QK : QK_K);
-  const size_t yes = type_size(y_dtype);
+  const bool k256 = act.act_dtype == XNQ_Q8K;
+  const int64_t pass = (int64_t)mt * 65535; // grid.y is limited to 65535 tiles of activation rows
   for (int64_t r0 = 0; r0 < act.m; r0 += pass) {
     ActView a = act;
-    a.m = act.m - r0 < pass ? act.m - r0 : pass;
-    a.q += r0 * w.k, a.d += r0 * nblk_a, a.bsum += r0 * (w.k / 16);
-    void *yp = static_cast<char *>(y) + (size_t)r0 * ldy * yes;
+    a.m = std::min(act.m - r0, pass);
+    a.q += r0 * w.k;
+    a.d = reinterpret_cast<float *>(reinterpret_cast<char *>(act.d) + r0 * (k256 ? w.k / QK_K * 4 : w.k / QK * 2));
+    if (act.bsum) a.bsum += r0 * (k256 ? w.k / 16 : w.k / QK);
+    void *yp = static_cast<char *>(y) + (size_t)r0 * ldy * type_size(y_dtype);
     const dim3 grid((unsigned)((w.n + rows_per_cta - 1) / rows_per_cta), (unsigned)((a.m + mt - 1) / mt));
     cudaError_t e;
     switch (mt) {
@@ -499,18 +502,31 @@ int launch_quantize_q8_1(const void *x, int x_dtype, int64_t m, int64_t k, int64
   return XNQ_OK;
 }
 
-// The activations' planar image: codes, block scales, 16-sums. Q8_1 blocks have the codes and the (f16-rounded) scale of Q8_0
-// blocks; the sum they also store follows from the 16-sums.
-static int generic_act_dtype(const WeightView &w) { return act_dtype_for(w.dtype) == XNQ_Q8K ? XNQ_Q8K : XNQ_Q8_0; }
-size_t generic_workspace_bytes(const WeightView &w, int64_t m) { return act_workspace_bytes(m, w.k, generic_act_dtype(w)); }
+// The activations' planar image, no larger than the canonical blocks: Q8_K codes, f32 scales and 16-sums; Q8_0 / Q8_1 codes and f16 scales,
+// and for Q8_1 the f16 s of every block.
+static ActView generic_acts(const WeightView &w, void *ws, int64_t m) {
+  const int adt = act_dtype_for(w.dtype);
+  ActView a;
+  a.act_dtype = adt, a.m = m, a.k = w.k;
+  char *p = static_cast<char *>(ws);
+  a.q = reinterpret_cast<int8_t *>(p);
+  a.d = reinterpret_cast<float *>(p += m * w.k);
+  p += m * (adt == XNQ_Q8K ? w.k / QK_K * 4 : w.k / QK * 2);
+  a.bsum = adt == XNQ_Q8_0 ? nullptr : reinterpret_cast<int16_t *>(p);
+  return a;
+}
+size_t generic_workspace_bytes(const WeightView &w, int64_t m) {
+  const int adt = act_dtype_for(w.dtype);
+  return ((size_t)m * (size_t)(w.k / block_size(adt)) * (size_t)type_size(adt) + 255) & ~(size_t)255;
+}
 
 // y[m, n] = x[m, k] . W^T for a weight held as canonical blocks; workspace: generic_workspace_bytes(w, m)
 int launch_generic_matmul(const WeightView &w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
                           cudaStream_t s) {
   // the reference's dots of the 32-element formats refuse an odd number of blocks (k_quants.rs:322-325, 413-415, 523-526)
   if (block_size(w.dtype) == 32 && (w.k / 32) % 2) return fail(XNQ_ERR_SHAPE, "matmul_t: k = %lld is not divisible by 64 (an even number of 32-value blocks)", (long long)w.k);
-  const ActView act = act_view(workspace, m, w.k, generic_act_dtype(w));
-  int rc = launch_quantize_act_planar(act, x, x_dtype, ldx, s);
+  const ActView act = generic_acts(w, workspace, m);
+  int rc = act.act_dtype == XNQ_Q8K ? launch_quantize_act_planar(act, x, x_dtype, ldx, s) : launch_quantize_act_f16_scales(act, x, x_dtype, ldx, s);
   if (rc != XNQ_OK) return rc;
   const int64_t row_bytes = w.k / block_size(w.dtype) * type_size(w.dtype);
   profile_mark(s, true);

@@ -37,7 +37,8 @@ namespace {
 
 constexpr int TPB = 256;
 
-// LAYOUT 0: canonical GGUF activation blocks; LAYOUT 1: planar scratch
+// LAYOUT 0: canonical GGUF activation blocks; 1: planar scratch; 2: planar scratch of Q8_0 / Q8_1 blocks with f16 scales, d and bsum being
+// __half: one value per block each, bsum the s of Q8_1 = f16(f16(sum of codes) * d) (k_quants.rs:847-873) or NULL
 template <int ACT, typename XT, int LAYOUT>
 __global__ void __launch_bounds__(TPB) quantize_act_kernel(const XT *__restrict__ x, int64_t m, int64_t k, int64_t ldx,
                                                            uint8_t *__restrict__ blocks, ActView pl) {
@@ -57,9 +58,17 @@ __global__ void __launch_bounds__(TPB) quantize_act_kernel(const XT *__restrict_
   }
   const int lane = threadIdx.x & 31;
   Quant8 q = ACT == XNQ_Q8_0 ? quantize8_q8_0(v, lane) : quantize8_q8k(v, lane);
+  const int sum32 = LAYOUT == 2 ? q.sum16 + __shfl_xor_sync(0xffffffffu, q.sum16, 2) : 0;
   if (!valid) return;
 
-  if (LAYOUT == 1) {
+  if (LAYOUT == 2) {
+    *reinterpret_cast<uint2 *>(pl.q + row * k + c8 * 8) = make_uint2(q.lo, q.hi);
+    if ((lane & 3) == 0) {
+      const int64_t b = row * (k / QK) + c8 / 4;
+      reinterpret_cast<__half *>(pl.d)[b] = __float2half_rn(q.d_unrounded);
+      if (pl.bsum) reinterpret_cast<__half *>(pl.bsum)[b] = __float2half_rn(__fmul_rn(__half2float(__float2half_rn((float)sum32)), q.d));
+    }
+  } else if (LAYOUT == 1) {
     *reinterpret_cast<uint2 *>(pl.q + row * k + c8 * 8) = make_uint2(q.lo, q.hi);
     if (ACT == XNQ_Q8_0) {
       if ((lane & 3) == 0) pl.d[row * (k / QK) + c8 / 4] = q.d;
@@ -114,8 +123,15 @@ int launch_quantize_act_planar(const ActView &a, const void *x, int x_dtype, int
   return launch_typed<XNQ_Q8K, 1>(x, x_dtype, a.m, a.k, ldx, nullptr, a, s);
 }
 
+int launch_quantize_act_f16_scales(const ActView &a, const void *x, int x_dtype, int64_t ldx, cudaStream_t s) {
+  return launch_typed<XNQ_Q8_0, 2>(x, x_dtype, a.m, a.k, ldx, nullptr, a, s);
+}
+
 int quantize_init(int) {
   cudaFuncAttributes fa;
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_act_kernel<XNQ_Q8_0, float, 2>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_act_kernel<XNQ_Q8_0, __half, 2>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_act_kernel<XNQ_Q8_0, __nv_bfloat16, 2>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_act_kernel<XNQ_Q8_0, float, 0>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_act_kernel<XNQ_Q8_0, float, 1>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, quantize_act_kernel<XNQ_Q8K, float, 0>));
