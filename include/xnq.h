@@ -294,7 +294,8 @@ int xnq_rope_kv_store(const float *qkv, const float *cos_table, const float *sin
                       float *q_out, void *k_cache, void *v_cache, int64_t batch, int heads, int kv_heads,
                       int head_dim, int64_t max_seq, void *stream);
 /* The same for a whole prompt at positions 0 .. seq - 1 of every sequence: qkv[batch, seq, (heads + 2 kv_heads) * head_dim] f32,
- * q_out[batch, heads, seq, head_dim] bf16. seq <= max_seq, head_dim a multiple of 8. */
+ * q_out[batch, heads, seq, head_dim] bf16. seq <= max_seq, head_dim a multiple of 8. Before xnq_rope_attn_decode reads the
+ * caches, a normally launched kernel or copy must lie in between (the one that writes *pos_dev, for instance); see there. */
 int xnq_rope_kv_store_prompt(const float *qkv, const float *cos_table, const float *sin_table, void *q_out, void *k_cache, void *v_cache,
                              int64_t batch, int64_t seq, int heads, int kv_heads, int head_dim, int64_t max_seq, void *stream);
 /* Single-query attention over cache positions 0..*pos_dev: out[batch, heads, head_dim] =

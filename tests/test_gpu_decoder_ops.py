@@ -270,3 +270,32 @@ def test_add_rmsnorm_rows_is_the_torch_operations_bits(shape, with_delta):
     want = want_x * torch.rsqrt(want_x.pow(2).mean(-1, keepdim=True) + 1e-5) * w
     got = ops.add_rmsnorm_rows(x, delta if with_delta else None, w, 1e-5)
     assert torch.equal(x, want_x) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("S", [1, 63, 64, 200])
+def test_decode_attention_right_behind_the_prompt_sees_its_rows(S):
+    """The attention kernel of a decode step reads cache rows before it waits for its predecessor. With the position written by a
+    normal copy in between, as the header asks, the rows that the prompt's store kernel has just written are the ones it reads."""
+    from xn_b200 import decoder_ops as ops
+    B, H, KV, hd, max_seq = 3, 8, 2, 128, 256
+    g = torch.Generator(device="cpu"); g.manual_seed(S)
+    prompts = [torch.randn(B, S, (H + 2 * KV) * hd, generator=g).to(DEV) for _ in range(8)]
+    step = torch.randn(B, (H + 2 * KV) * hd, generator=g).to(DEV)
+    ang = torch.arange(max_seq, dtype=torch.float32)[:, None] / 10000.0 ** (torch.arange(0, hd, 2, dtype=torch.float32) / hd)[None]
+    cos, sin = ang.cos().to(DEV), ang.sin().to(DEV)
+    kc = torch.zeros(B, KV, max_seq, hd, dtype=torch.bfloat16, device=DEV); vc = torch.zeros_like(kc)
+    pos = torch.zeros(1, dtype=torch.int64, device=DEV)
+
+    def run(prompt, wait):
+        out = torch.empty(B, H, hd, device=DEV)
+        ops.rope_kv_store_prompt(prompt, cos, sin, kc, vc, H, KV)
+        wait()
+        pos.fill_(S)
+        wait()
+        ops.rope_attn_decode(step, cos, sin, pos, kc, vc, out, H, KV)
+        return out
+    apart = [run(p, torch.cuda.synchronize) for p in prompts]
+    in_turn = [run(p, lambda: None) for p in prompts]      # every prompt overwrites the rows of the one before
+    for a, b in zip(apart, in_turn):
+        assert torch.equal(a, b)
+    assert not torch.equal(apart[0], apart[1])

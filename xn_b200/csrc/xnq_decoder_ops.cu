@@ -369,10 +369,10 @@ __global__ void rope_store_kernel(const float *qkv, const float *cos_t, const fl
 // A whole prompt: qkv [B, seq, (H + 2 KV) * hd] f32 -> q_out [B, H, seq, hd] bf16 (rotated at position s), rotated k and plain v into
 // the caches at positions 0 .. seq - 1. One CTA per token; a thread takes four rotation pairs (i, i + hd / 2) of a head. Bound by its
 // 6 bytes per value: the rotation, its concatenation, the casts and the cache stores were eleven passes as separate operations
-// (220 us per 512-token prompt of two layers with 6144 values a token; 11 us like this).
+// (220 us per 512-token prompt of two layers with 6144 values a token; 11 us like this). It lets no kernel start while it runs:
+// rope_attn_decode reads cache rows before its wait.
 __global__ void __launch_bounds__(256) rope_store_prompt_kernel(const float *qkv, const float *cos_t, const float *sin_t, __nv_bfloat16 *q_out,
                                                                 __nv_bfloat16 *k_cache, __nv_bfloat16 *v_cache, int seq, int H, int KV, int hd, int max_seq) {
-  pdl_launch_dependents();
   pdl_wait();
   const int pos = blockIdx.x, b = blockIdx.y, half = hd / 2, per_head = hd / 8;
   const float *src = qkv + ((int64_t)b * seq + pos) * (H + 2 * KV) * hd;
