@@ -182,3 +182,12 @@ def test_gguf_file_round_trip_through_device_handles(tmp_path):
         full = c.upload(name, dev).matmul_t(x)
         parts = [c.upload(name, dev, r, 2).matmul_t(x) for r in range(2)]
         assert torch.equal(torch.cat(parts, dim=-1), full)
+
+
+def test_prefill_of_a_model_without_layers_is_the_head_of_the_embedding():
+    from xn_b200.llama import LlamaConfig, QLlama, dense_reference_logits
+    import dataclasses
+    dev = torch.device("cuda", 0)
+    m = QLlama(dataclasses.replace(LlamaConfig.tiny(), n_layers=0), dev, batch=2, max_seq=64, max_prefill_rows=64)
+    prompt = torch.tensor([[3, 5, 7], [11, 13, 17]], device=dev)
+    assert _rel(m.prefill(prompt), dense_reference_logits(m, prompt)) < 2e-2

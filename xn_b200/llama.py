@@ -275,7 +275,8 @@ class QLlama:
         delta = None
         for L in self.layers:
             delta = self._block(L, x, delta, pos_idx, mask, prompt)
-        x = self._rms(x[:, -1:, :] + delta[:, -1:, :], self.norm)
+        x = x[:, -1:, :] if delta is None else x[:, -1:, :] + delta[:, -1:, :]
+        x = self._rms(x, self.norm)
         logits = self._linear_gathered(self.lm_head, x).view(tokens.shape[0], -1)
         return logits if self.pg is None else logits.clone()   # out of the exchange slot before it is reused
 
