@@ -98,3 +98,21 @@ def test_host_mirror_shape_errors_match_reference_messages():
         QTensor(np.zeros(70, np.uint8), (4, 32), D.Q4_0)
     qt = QTensor(np.zeros(72, np.uint8), (4, 32), D.Q4_0)
     assert qt.rank() == 2 and qt.shape() == (4, 32) and qt.dtype() == D.Q4_0 and qt.storage_size_in_bytes() == 72
+
+
+def test_the_current_stream_is_found_without_torchs_private_name(monkeypatch):
+    """The usual call takes the raw stream from a private function of torch; a torch without it gets the public route."""
+    import importlib.util
+    import torch
+    from xn_b200 import quantized
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    spec = importlib.util.spec_from_file_location("xn_b200.quantized_without_raw_stream", quantized.__file__)
+    fresh = importlib.util.module_from_spec(spec)
+    monkeypatch.setitem(__import__("sys").modules, spec.name, fresh)
+    spec.loader.exec_module(fresh)
+    asked = []
+
+    class Stream:
+        cuda_stream = 1234
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda index: asked.append(index) or Stream())
+    assert fresh._raw_stream(3) == 1234 and asked == [3]

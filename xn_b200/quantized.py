@@ -28,6 +28,12 @@ _TORCH_TO_XNQ = {torch.float32: GgmlDType.F32, torch.float16: GgmlDType.F16, tor
 
 _XNQ_IDS = {t: int(d) for t, d in _TORCH_TO_XNQ.items()}
 
+try:   # a private name of torch: a tenth of the time of a Stream object
+    from torch._C import _cuda_getCurrentRawStream as _raw_stream
+except ImportError:
+    def _raw_stream(index: int) -> int:
+        return torch.cuda.current_stream(index).cuda_stream
+
 
 def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
@@ -275,7 +281,7 @@ class QCudaTensor:
         index = device.index
         if index is not None and index == torch.cuda.current_device():
             check(_lib.lib().xnq_matmul_t(self._h, x.data_ptr(), x_dtype, m, ldx, y.data_ptr(), y_dtype, ldy, ws.data_ptr(), ws.numel(),
-                                          torch._C._cuda_getCurrentRawStream(index)))
+                                          _raw_stream(index)))
         else:
             with torch.cuda.device(device):
                 check(_lib.lib().xnq_matmul_t(self._h, x.data_ptr(), x_dtype, m, ldx, y.data_ptr(), y_dtype, ldy, ws.data_ptr(), ws.numel(),
