@@ -191,3 +191,40 @@ def test_prefill_of_a_model_without_layers_is_the_head_of_the_embedding():
     m = QLlama(dataclasses.replace(LlamaConfig.tiny(), n_layers=0), dev, batch=2, max_seq=64, max_prefill_rows=64)
     prompt = torch.tensor([[3, 5, 7], [11, 13, 17]], device=dev)
     assert _rel(m.prefill(prompt), dense_reference_logits(m, prompt)) < 2e-2
+
+
+@pytest.mark.parametrize("S", [1, 63, 64, 65, 130])
+def test_prompts_shorter_than_the_cache(S):
+    """A prompt attends to its own positions, rounded up to 64, of a cache that holds whatever an earlier prompt left behind it."""
+    from xn_b200.llama import LlamaConfig, QLlama, dense_reference_logits
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device="cpu"); g.manual_seed(S)
+    m = QLlama(LlamaConfig.tiny(), dev, batch=3, max_seq=256, max_prefill_rows=3 * 130)
+    prompt = torch.randint(0, m.cfg.vocab, (3, S), generator=g).to(dev)
+    clean = m.prefill(prompt)
+    rows = [(L.k_cache[:, :, :S].clone(), L.v_cache[:, :, :S].clone()) for L in m.layers]
+    for L in m.layers:
+        L.k_cache.fill_(3e4); L.v_cache.fill_(-3e4)
+    logits = m.prefill(prompt)
+    assert torch.equal(logits, clean)
+    for L, (k, v) in zip(m.layers, rows):
+        assert torch.equal(L.k_cache[:, :, :S], k) and torch.equal(L.v_cache[:, :, :S], v)
+        assert bool((L.k_cache[:, :, S:] == L.k_cache[0, 0, 255, 0]).all()) and bool((L.v_cache[:, :, S:] == L.v_cache[0, 0, 255, 0]).all())
+    assert _rel(logits, dense_reference_logits(m, prompt)) < 3e-2
+    whole = m._forward(prompt, torch.arange(S, device=dev))       # over the whole cache, rotated and stored by torch
+    assert _rel(logits, whole) < 2e-2
+    # one decode step from here sees these rows and no others
+    m.prefill(prompt)
+    nxt = m.tokens.clone()
+    m._decode_step()
+    assert _rel(m.last_logits, dense_reference_logits(m, torch.cat([prompt, nxt[:, None]], 1))) < 3e-2
+
+
+def test_a_prompt_longer_than_the_cache_is_refused():
+    from xn_b200.llama import LlamaConfig, QLlama
+    m = QLlama(LlamaConfig.tiny(), torch.device("cuda", 0), batch=1, max_seq=64, max_prefill_rows=64)
+    whole = m.prefill(torch.ones(1, 64, dtype=torch.int64, device="cuda"))
+    assert int(m.pos) == 64 and bool(torch.isfinite(whole).all())
+    with pytest.raises(ValueError, match="65 tokens"):
+        m.prefill(torch.ones(1, 65, dtype=torch.int64, device="cuda"))
+    assert int(m.pos) == 64

@@ -141,8 +141,8 @@ def _f32_bound(O, dt, w, x, n, k):
     return 4 * (k / 16 + 8) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ dense.T + np.abs(x).max() * dense.max() * 32)
 
 
-# the integer kernel around its operand row counts (16, 32, 48, 64) and the row counts where other kernels take over, over one step,
-# a partial step, more steps than its rings have stages, and rows of a last tile
+# the integer kernel around its operand row counts (16, 32, 48, 64) and the row counts where other kernels take over, over one step, a
+# partial step, tiles that several CTAs share, and rows of a last tile (a CTA has two steps here; the test behind it has the long runs)
 @pytest.mark.parametrize("dt", WEIGHT_TYPES)
 @pytest.mark.parametrize("m", [4, 5, 6, 16, 17, 32, 33, 48, 49, 64])
 def test_integer_kernel_row_and_step_edges(Q, O, dt, m):
@@ -154,6 +154,22 @@ def test_integer_kernel_row_and_step_edges(Q, O, dt, m):
         t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
         got = t.matmul_t(torch.from_numpy(x).to(DEV)).cpu().numpy().astype(np.float64)
         assert (np.abs(got - O.matmul(int(dt), x, w, n)) <= _f32_bound(O, dt, w, x, n, k)).all(), (dt.name, m, n, k)
+
+
+# Every CTA of the integer kernel takes an equal run of the (tile, step) space: here more steps than twice the stages of any of its rings
+# but the two of eight (operand 2 or 3, activations 2 to 8, side 8), so every barrier is met in both parities, and the long rings wrap.
+@pytest.mark.parametrize("dt", WEIGHT_TYPES)
+def test_integer_kernel_long_runs_of_steps(Q, O, dt):
+    n, k = 148 * 128 + 1, 256 * 13 - (0 if dt.block_size == 256 else 64)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert -(-n // 128) * 13 >= sms * 13
+    w = synth.make_weight(dt, n, k, seed=31)
+    x = synth.make_activation(64, k, seed=32)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    want, bound = O.matmul(int(dt), x, w, n, threads=O.hw_threads()), _f32_bound(O, dt, w, x, n, k)
+    for m in (6, 16) if dt is D.Q6K else (5, 16, 17, 32, 33, 48, 64):
+        got = t.matmul_t(torch.from_numpy(x[:m]).to(DEV)).cpu().numpy().astype(np.float64)
+        assert (np.abs(got - want[:m]) <= bound[:m]).all(), (dt.name, m)
 
 
 # the fp16 kernel: one and two accumulators, tiles that end with 1 and 16 rows, k-steps that do not fill a super-step or a stage ring,
