@@ -784,6 +784,7 @@ int xnqo_matmul_f64(int dtype, int64_t m, int64_t k, int64_t n, const float *lhs
                     int threads) {
   const int bs = xnqo_block_size(dtype);
   if (bs <= 1 || xnqo_vec_dot_type(dtype) < 0 || dtype == XNQO_Q8K || dtype == XNQO_Q8_1) return -1;
+  if (dtype != XNQO_Q4_0 && dtype != XNQO_Q8_0 && dtype != XNQO_Q4K && dtype != XNQO_Q6K) return -1; /* the formats mm_f64_worker reads */
   if (m < 0 || n < 0 || k < 0 || k % bs != 0) return -1;
   if (m == 0 || n == 0) return 0;
   void *lhs_b = xnqo_quantize_lhs(dtype, m, k, lhs);

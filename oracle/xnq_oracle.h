@@ -75,7 +75,7 @@ int xnqo_vec_dot_avx2(int dtype, int64_t k, const void *w_row, const void *act_r
 int xnqo_matmul(int dtype, int64_t m, int64_t k, int64_t n, const float *lhs, const void *rhs,
                 float *dst, int threads);
 /* f64 dot of the *quantized* operands (the reference's own test oracle, k_quants.rs:2162-2184,
- * extended to the other formats by dequantizing both sides exactly in f64). */
+ * extended to Q4_0, Q4_K and Q6_K by dequantizing both sides exactly in f64; -1 for the other formats). */
 int xnqo_matmul_f64(int dtype, int64_t m, int64_t k, int64_t n, const float *lhs,
                     const void *rhs, double *dst, int threads);
 /* The reference's x86 execution: AVX2-order dots driven as matmul_by_row (rows serial, 128-column

@@ -179,3 +179,9 @@ def test_odd_block_counts_are_refused_like_the_reference():
         w = synth.make_weight(dt, 2, 96, seed=8)
         with pytest.raises(ValueError):
             O.matmul(int(dt), synth.make_activation(1, 96), w, 2)
+
+
+@pytest.mark.parametrize("dt", FORMATS)
+def test_the_f64_matmul_refuses_the_formats_it_does_not_read(dt):
+    with pytest.raises(Exception, match="matmul_f64"):
+        O.matmul(int(dt), synth.make_activation(2, 512, seed=1), synth.make_weight(dt, 3, 512, seed=2), 3, order="f64")
