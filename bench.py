@@ -43,7 +43,7 @@ WORKLOADS = {
     "C3_q4k_14336x4096_m4": (D.Q4K, 14336, 4096, 4),
     "C3_q4k_14336x4096_m16": (D.Q4K, 14336, 4096, 16),
     "C4_q6k_128256x4096_m1": (D.Q6K, 128256, 4096, 1),
-    "C4_q6k_128256x4096_m16": (D.Q6K, 128256, 4096, 16),   # the dp4a small-batch kernel (Q6_K has no integer tensor-core path)
+    "C4_q6k_128256x4096_m16": (D.Q6K, 128256, 4096, 16),
     "C1_q4_0_4096x4096_m16": (D.Q4_0, 4096, 4096, 16),
     "C1_q4_0_4096x4096_m128": (D.Q4_0, 4096, 4096, 128),
     "C4_q6k_128256x4096_m32": (D.Q6K, 128256, 4096, 32),
@@ -54,6 +54,15 @@ WORKLOADS = {
     "C3_q4k_14336x4096_m64": (D.Q4K, 14336, 4096, 64),
     "C3_q4k_14336x4096_m512": (D.Q4K, 14336, 4096, 512),
 }
+
+
+def kernel_of(dt, m: int) -> str:
+    """The kernel that serves m rows of a weight of this format at k = 4096."""
+    if m == 1:
+        return "matvec_ring_kernel"
+    if m <= {D.Q4_0: 4, D.Q8_0: 4, D.Q4K: 1, D.Q6K: 5}[dt]:
+        return f"matvec_{dt.name.lower()} (dp4a)"
+    return "imma_kernel (tcgen05 kind::i8)" if m <= (16 if dt is D.Q6K else 64) else "prefill_persistent_kernel (tcgen05 kind::f16)"
 
 
 def captured_traffic(name: str):
@@ -505,8 +514,7 @@ def measure_matmul(ctx, args, name, dt, n, k, m, with_cpu=True):
                 "unit": "TFLOP/s" if tensor_bound else "GB/s",
                 "frac": ((tflops / peak_tf) if tensor_bound else (achieved / peak)) if achieved else None,
                 "traffic": captured_traffic(name) if world == 1 else None,
-                "kernel": ("matvec_ring_kernel" if m == 1 else "imma_kernel (tcgen05 kind::i8)" if (m <= 64 and dt.name != "Q6K")
-                           else "prefill_persistent_kernel (tcgen05 kind::f16)" if m > 16 else "matvec_q6k (dp4a)"),
+                "kernel": kernel_of(dt, m),
                 "launch_us": kern_ms * 1e3, "launches_timed": cnt.value, "peak_kind": f"of {peak_kind}",
                 "bytes_per_launch": kern_bytes, "flops_per_launch": flops, "hbm_gbs": achieved, "tflops": tflops,
                 "isolated_launch_us": isolated_us,

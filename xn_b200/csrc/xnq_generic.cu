@@ -2,12 +2,11 @@
 // formats and Q8_1 as an activation format (xn-core/src/quantized/k_quants.rs:100-186 block layouts, 307-610 the
 // 32-element formats, 834-878 Q8_1, 880-1316 Q2_K / Q3_K, 1507-1722 Q5_K).
 //
-// Real GGUF files mix types, so a handle must be able to hold any of them; none of these formats is on the measured path.
-// They are therefore kept on the device exactly as in the file (canonical blocks, no re-layout) and served by one plain
-// kernel per operation:
+// Real GGUF files mix types, so a handle must be able to hold any of them. These formats are kept on the device exactly as in the
+// file (canonical blocks, no re-layout) and served by one kernel per operation:
 //   to_float   one thread per element, the reference's arithmetic operation for operation (bit-identical results);
 //   matmul     activations are quantized to the block format of the weight's VecDotType (Q8_0, Q8_1 or Q8_K) as planar codes,
-//              scales and 16-sums, then one kernel unpacks the file's blocks to int8 codes in registers and multiplies them with
+//              scales and sums, then one kernel unpacks the file's blocks to int8 codes in registers and multiplies them with
 //              dp4a: each block's integer sums are exact, scales are applied in f32 as in the reference, and only the order in
 //              which block contributions are added differs from its serial sum (within 2e-3 under its own metric).
 #include <algorithm>

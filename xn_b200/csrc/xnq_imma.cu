@@ -949,7 +949,7 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     // The CTAs are started while the previous kernel drains, and the first SM that is free would take eight of them (3.9 us instead of
     // 1.3): unused shared memory keeps them apart.
     const dim3 prep_grid((unsigned)(paired ? pl.NP / 2 : pl.NP), (unsigned)std::min<int64_t>(16, (k + 2047) / 2048));
-    const size_t spread = MAX_SPREAD / ((prep_grid.x * prep_grid.y + 147) / 148) / 1024 * 1024;
+    const size_t spread = MAX_SPREAD / ((prep_grid.x * prep_grid.y + g_sms - 1) / g_sms) / 1024 * 1024;
 #define XNQ_IMMA_PREP(ACT, XT)                                                                                                          \
   XNQ_CUDA(launch_pdl(imma_prepare<ACT, XT>, prep_grid, dim3(256), spread, s,     \
                       iq ? nullptr : static_cast<const XT *>(x) + r0 * ldx, iq, id, ib, rows, k, ldx, pl.NP, pl.nsteps, bimg, meta, cnt, pl.tiles, paired ? 1 : 0))
@@ -1012,9 +1012,11 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     a.raw_stage_bytes = (uint32_t)(CONV_WARPS / 2) * (32u * (uint32_t)step_code + 512u); // a step in flight: four warp slots of the rows' code bytes and 16 scale bytes per row
     a.b_stage_bytes = (uint32_t)pl.NP * 256;
     a.side_stage_bytes = HDR_BYTES + (uint32_t)pl.NP * 32 + (paired ? TILE_N * 4 : 0);
-    // shared-memory plan: A stages (half steps) | B stages (half as many whole steps) | side stages | raw stages. The MMA
-    // issuer bounds a step, so the converters and the drain need little slack (six half steps of operand image); what remains
-    // goes to raw stages, which hide the memory latency.
+    // Shared-memory plan: A stages (half steps of operand image) | B stages (activations, whole steps) | side stages | raw stages (weights,
+    // whole steps). The first plan of six half steps with the most raw stages that leaves five B stages (NP > 32: two), else of four with two.
+    // The activations' copies queue behind the weights': with three B stages a step takes a third of their latency of 4500 cycles, which is
+    // why NP = 16 has eight. As it comes out, (A, raw, B): Q4_0 / Q4_K (6, 4, 8), (4, 6, 3), (6, 4, 2), (4, 4, 3) for NP = 16, 32, 48, 64;
+    // Q8_0 (4, 2, 8), (4, 2, 8), (4, 2, 5), (4, 2, 3); Q6_K (4, 4, 2). Fewer raw and more B stages were not measured where B is 2 or 3.
     const size_t budget = IMMA_SMEM - 1024; // 1024: alignment slack of the base
     a.a_stages = 0;
     static constexpr int as_order[3] = {6, 4, 8};
@@ -1023,8 +1025,6 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
       for (int rs = MAX_RAW_STAGES; rs >= 2 && !a.a_stages; rs -= 2) { // even: the two converter groups own half of the slots each
         const size_t fixed = (size_t)as * A_STAGE_BYTES + (size_t)SIDE_STAGES * a.side_stage_bytes + (size_t)rs * a.raw_stage_bytes + 256;
         if (rs < 4 && as != 4) continue;
-        // The activations' copies queue behind the weights': with three stages of a step each a step took the 4500 cycles of their
-        // latency divided by three
         const int bs = fixed >= budget ? 0 : (int)std::min<size_t>(MAX_B_STAGES, (budget - fixed) / a.b_stage_bytes);
         if (bs >= (pl.NP <= 32 && ai == 0 ? 5 : 2)) a.a_stages = as, a.raw_stages = rs, a.b_stages = bs;
       }

@@ -1,4 +1,4 @@
-// Prefill (m > 16): quantized weights x activations as a dense contraction on the 5th-generation
+// Prefill (m > 64; Q6_K: m > 16): quantized weights x activations as a dense contraction on the 5th-generation
 // tensor cores (tcgen05.mma, accumulators in TMEM).
 //
 //   D[128 weight rows, mt activation rows] += A[128, 64] . B[mt, 64]^T      per k-step of 64
@@ -12,7 +12,7 @@
 //      as the reference's quantize_lhs does (k_quants.rs:2015-2026), dequantized, scaled by a power of
 //      two per row and stored as fp16 in the same swizzled image, so that one 1-D bulk-async copy
 //      (cp.async.bulk, non-multicast) brings a whole stage.
-//   D  f32 in tensor memory; four epilogue warps read it back with tcgen05.ld, undo the power-of-two
+//   D  f32 in tensor memory; eight epilogue warps read it back with tcgen05.ld, undo the power-of-two
 //      scales and store y.
 //
 // Operand type. The contraction runs in fp16 (kind::f16 with f16 inputs), not bf16: both have the
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       cur.advance(len, KT, TM);
     }
   } else {
-    // ---- drain: four warps, warp q reads accumulator lanes 32q.. (weight rows), all columns -----------------
+    // ---- drain: eight warps, two to a quarter q of the accumulator lanes (weight rows 32 q ..), which take turns in its chunks of 32 columns ----
     const int q = warp & 3; // tensor-memory lanes a warp may read are fixed by its index modulo 4
     const int half = (warp - EPI_WARP0) >> 2; // which half of the 32-column chunks this warp takes
     const int et = threadIdx.x - EPI_WARP0 * 32; // 0..255
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       const int64_t m0 = (int64_t)tile_m * MAX_MT;
       const int mt = (int)min((int64_t)MAX_MT, p.m_pad - m0);
       // one thread waits for the accumulator and, for a tile shared with other CTAs, settles who stores and
-      // who adds; the four warps then act on the same answers
+      // who adds; the eight warps then act on the same answers
       if (et == 0) {
         unsigned int t = mbar_wait(acc_full + 8 * buf, use & 1, 8u) ? 0u : 0x80000000u;
         if (!whole && t == 0) {
@@ -645,7 +645,7 @@ int launch_persistent_fmt(const PrefillArgs &a, unsigned ctas, size_t smem, cuda
   return XNQ_OK;
 }
 
-constexpr size_t SM_SMEM = 228 * 1024, MAX_SPREAD = 200 * 1024;
+constexpr size_t SM_SMEM = 228 * 1024, MAX_SPREAD = SM_SMEM / 2;
 static_assert(RowQ4_0::ROWB == RowQ4K::ROWB && RowQ8_0::ROWB == RowQ4K::ROWB, "the raw ring's plan assumes one slot size for these");
 constexpr size_t PREFILL_SMEM = 226 * 1024; // everything an SM offers minus the static barriers and a reserve
 
@@ -673,10 +673,10 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   uint8_t *xh = reinterpret_cast<uint8_t *>(tile_cnt) + cnt_bytes;
   const int act = act_dtype_for(w.dtype);
   // The rows' CTAs are started while the previous kernel drains, and the first SM that is free would take eight of them (10 us for
-  // 32 rows instead of 3); unused shared memory keeps them apart: at most ceil(rows / SMs) to an SM.
+  // 32 rows instead of 3); unused shared memory, half of the share that ceil(rows / SMs) of them would have, keeps them apart: one to an
+  // SM up to as many rows as SMs, above that less than twice the even share.
   const int64_t sms = g_num_sms > 0 ? g_num_sms : 148;
-  const size_t spread = std::min<size_t>(MAX_SPREAD, (SM_SMEM / (size_t)((m_pad + sms - 1) / sms)) / 2048 * 1024);
-  // (each CTA also takes 1 KB of its own)
+  const size_t spread = SM_SMEM / (size_t)((m_pad + sms - 1) / sms) / 2048 * 1024; // (each CTA also takes 1 KB of its own)
 #define XNQ_PREP(ACT, XT)                                                                                                   \
   XNQ_CUDA(launch_pdl(prefill_prepare_acts<ACT, XT>, dim3((unsigned)m_pad), dim3(256), spread, s, static_cast<const XT *>(x), m, k, ldx, m_pad, ksteps, \
                       w.dtype, wscale, xh, row_unscale, tile_cnt, (int)(cnt_bytes / 4)))

@@ -16,9 +16,9 @@ Tensor parallelism over ``world`` ranks (one process per GPU):
     its summand into every rank's buffer; the next residual-add + RMSNorm adds the summands;
   * the LM head is N-sharded and its output columns are gathered the same way.
 
-Prefill runs attention and the mean of its RMSNorms as torch ops, the rest as the library's operators. A decode step uses the library's fused operators
-between the linears (residual-add + RMSNorm, RoPE + KV-cache store, single-query attention, SwiGLU), so
-one layer is ten launches and the whole step is one CUDA graph.
+Prefill runs attention and the mean of its RMSNorms as torch ops, the rest as the library's operators. A decode step uses the
+library's fused operators between the linears (residual-add + RMSNorm, RoPE + KV-cache store + single-query attention, SwiGLU), so
+one layer is six launches for one sequence and nine for a batch on Q4_K weights, and the whole step is one CUDA graph.
 """
 from __future__ import annotations
 
@@ -166,7 +166,7 @@ class QLlama:
             return ops.ActImage.for_weight(c.linear_dtype, batch, k, device) if wants_image(k) else None
         self._xn_img = image(c.d_model)
         self._h_img = image(c.ffn // G)
-        if isinstance(self._xn_img, ops.OperandImage):   # the LM head is not an integer tensor-core weight: it keeps a planar image, or float rows
+        if isinstance(self._xn_img, ops.OperandImage):   # operand images are the Q4_K kernels' alone: the LM head keeps a planar image, or float rows
             self._head_img = ops.ActImage.for_weight(c.head_dtype, batch, c.d_model, device) if wants_image(c.d_model) else None
         else:
             self._head_img = self._xn_img if c.head_dtype.vec_dot_type == c.linear_dtype.vec_dot_type else None
