@@ -228,3 +228,39 @@ def test_a_prompt_longer_than_the_cache_is_refused():
     with pytest.raises(ValueError, match="65 tokens"):
         m.prefill(torch.ones(1, 65, dtype=torch.int64, device="cuda"))
     assert int(m.pos) == 64
+
+
+def test_a_replayed_batch_step_repeats_itself_and_equals_one_with_every_launch_waited_for(monkeypatch):
+    """Sixteen sequences: the launches of a step overlap (each starts while its predecessor drains), so a read that does not wait for
+    its writer would show as a difference between replays, or between a replay and the step with a synchronize around every operator."""
+    from xn_b200 import decoder_ops as ops, quantized as Q
+    from xn_b200.llama import LlamaConfig, QLlama
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device="cpu"); g.manual_seed(16)
+    m = QLlama(LlamaConfig.tiny(), dev, batch=16, max_seq=64, max_prefill_rows=16 * 20)
+    m.prefill(torch.randint(0, m.cfg.vocab, (16, 20), generator=g).to(dev))
+    m.capture_decode()
+    pos, tokens = m.pos.clone(), torch.randint(0, m.cfg.vocab, (16,), generator=g).to(dev)
+
+    def step():
+        m.pos.copy_(pos); m.tokens.copy_(tokens)
+        m.decode(1)
+        return m.last_logits.clone(), m.tokens.clone()
+    first = step()
+    for _ in range(20):
+        again = step()
+        assert torch.equal(again[0], first[0]) and torch.equal(again[1], first[1])
+
+    def waited(f):
+        def call(*args, **kwargs):
+            torch.cuda.synchronize()
+            out = f(*args, **kwargs)
+            torch.cuda.synchronize()
+            return out
+        return call
+    m._graph = None
+    for name in ("embed_rows", "add_rmsnorm", "rope_attn_decode", "swiglu", "argmax_advance"):
+        monkeypatch.setattr(ops, name, waited(getattr(ops, name)))
+    monkeypatch.setattr(Q.QCudaTensor, "matmul_t", waited(Q.QCudaTensor.matmul_t))
+    apart = step()
+    assert torch.equal(apart[0], first[0]) and torch.equal(apart[1], first[1])

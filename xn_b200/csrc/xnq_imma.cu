@@ -38,7 +38,7 @@
 // Work is the flattened (tile of 128 weight rows, 256-k step) space, cut into equal contiguous ranges, one
 // per CTA, so all SMs finish together however few tiles there are. A tile whose steps are split between
 // CTAs is summed deterministically: every part is written to a scratch slot, an arrival ticket elects the
-// last part, and that CTA adds the parts in k order and stores y.
+// last part, and that CTA adds the parts, in runs in k order, and stores y.
 //
 // Every wait is bounded; on expiry a status bit is set and the roles fall through to the common exit, where
 // tensor memory is released.
@@ -357,6 +357,9 @@ struct ConvQ6K { // 128 ql bytes and 64 qh bytes per row and step. 64 k number 2
 //   Q4_K         hdr = f16 d, f16 dmin, four 24-bit fields sc[2g] | sc[2g+1] << 6 | mn[2g] << 12 | mn[2g+1] << 18;
 //                record = {lo(h=0), hi(h=0), lo(h=1), hi(h=1), f32 d, 0, 0, 0}: the 32-sums of the activation codes of
 //                each half's four sub-blocks, s = 128 * hi + lo with lo in 0..127 (one byte each)
+// The eight block terms of a step are added first, the step's sum then to the running sum: one rounding at the running sum's magnitude
+// per step. One by one they made the results 7 to 20 % less exact than the two chains of half steps that were added before (relative
+// error against the exact dot of the quantized operands, 1000 x 1024: 7.9e-8, with two chains 6.6e-8).
 template <int CH>
 struct DrainBlockScaled {
   __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int c0, const uint32_t (&v)[8][CH], float *acc) {
@@ -365,11 +368,14 @@ struct DrainBlockScaled {
     for (int c = 0; c < CH; c++) {
       const uint4 a = lds128(meta + (uint32_t)(c0 + c) * 32), b = lds128(meta + (uint32_t)(c0 + c) * 32 + 16);
       const uint32_t da[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      float step = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         const __half2 h = *reinterpret_cast<const __half2 *>(&w[j >> 1]);
-        acc[c] += (float)(int)v[j][c] * (((j & 1) ? __high2float(h) : __low2float(h)) * __uint_as_float(da[j]));
+        const float term = ((j & 1) ? __high2float(h) : __low2float(h)) * __uint_as_float(da[j]);
+        step = j == 0 ? (float)(int)v[j][c] * term : fmaf((float)(int)v[j][c], term, step);
       }
+      acc[c] += step;
     }
   }
 };
@@ -404,6 +410,11 @@ __device__ __forceinline__ void q6k_sums(const uint4 &hdr, int h, const uint32_t
 #pragma unroll
     for (int j = 0; j < 8; j++) isum[c] += (int)(int8_t)((w[j >> 2] >> (8 * (j & 3))) & 0xffu) * (int)v[j][c];
 }
+
+// Long f32 chains are cut: after SUM_RUN terms the chain's sum goes to a second one. Q6_K's steps (a CTA may add all of a long row's:
+// 14336 / 256 = 56), and the parts of a tile. (Q6_K, 600 x 14336: 1.06e-7 from the exact dot in one chain; the dp4a kernel, whose 32 lanes
+// take a part each, 8.3e-8.)
+constexpr int SUM_RUN = 8;
 
 // Drain warps: a warp's waits and its decoding of the row's scales cost as much as four columns' arithmetic; with 16 rows eight warps of
 // eight columns each do better than sixteen of four (Q6_K 32000 x 4096, 16 rows: 48.5 -> 46.4 us; Q8_0 11008 x 4096, 8 rows: 21.7 -> 20.9).
@@ -637,6 +648,9 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
     float acc[NPT];
 #pragma unroll
     for (int c = 0; c < NPT; c++) acc[c] = 0.f;
+    float run[Conv::PAIRED ? NPT : 1]; // Q6_K: the finished runs of steps
+#pragma unroll
+    for (int c = 0; c < (Conv::PAIRED ? NPT : 1); c++) run[c] = 0.f;
     int seg_kt0 = kt0; // first step of the current segment inside its tile
     int ap = 0, nb = 0;  // i % AP, i % (NB / 2)
     uint32_t a_ph = 0;   // (i / AP) & 1
@@ -684,6 +698,16 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
       if (alive && lane == 0) mbar_arrive(side_empty + 8 * ss);
       // ---- end of a segment (the tile's last step, or this CTA's last unit): store or hand over the sums ----
       const bool tile_end = kt == KT - 1, range_end = i == nunits - 1;
+      if constexpr (Conv::PAIRED) {
+        if ((kt & (SUM_RUN - 1)) == SUM_RUN - 1 || tile_end || range_end) {
+          const bool last = tile_end || range_end;
+#pragma unroll
+          for (int c = 0; c < NPT; c++) {
+            const float all = run[c] + acc[c];
+            run[c] = last ? 0.f : all, acc[c] = last ? all : 0.f;
+          }
+        }
+      }
       if (tile_end || range_end) {
         const int64_t row = (int64_t)tile * TILE_N + 32 * q + lane;
         const bool whole = seg_kt0 == 0 && tile_end;
@@ -715,16 +739,21 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
           const int t_u0 = tile * KT, t_u1 = t_u0 + KT;
           const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u1 - 1, p.units_q, p.units_r);
           if (et == 0 && (int)ticket == c_last - c_first) p.tile_cnt[tile] = 0u; // every part has its ticket: the word is zero again for the next call
-          if ((int)ticket == c_last - c_first) { // the last part to arrive adds all parts in k order
+          if ((int)ticket == c_last - c_first) { // the last part to arrive adds all parts, in runs in k order
             __threadfence();
             float (&sum)[NPT] = acc; // the segment's own sums are in its scratch slot by now
+            float some[NPT];
 #pragma unroll
-            for (int c = 0; c < NPT; c++) sum[c] = 0.f;
+            for (int c = 0; c < NPT; c++) sum[c] = 0.f, some[c] = 0.f;
             for (int cc = c_first; cc <= c_last; cc++) {
               const int cu0 = cta_first_unit(cc, p.units_q, p.units_r);
               const float *part = p.partials + ((size_t)2 * cc + (cu0 >= t_u0 ? 0 : 1)) * ROWS * TILE_N;
 #pragma unroll
-              for (int c = 0; c < NPT; c++) sum[c] += __ldcg(part + (size_t)(c0 + c) * TILE_N + 32 * q + lane);
+              for (int c = 0; c < NPT; c++) some[c] += __ldcg(part + (size_t)(c0 + c) * TILE_N + 32 * q + lane);
+              if (((cc - c_first) & (SUM_RUN - 1)) == SUM_RUN - 1 || cc == c_last) {
+#pragma unroll
+                for (int c = 0; c < NPT; c++) sum[c] += some[c], some[c] = 0.f;
+              }
             }
             if (row < p.w.n) {
 #pragma unroll

@@ -197,7 +197,7 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q8_0(WeightView w, ActView a, void *y, 
         const int4 av = *reinterpret_cast<const int4 *>(sa.q + (int64_t)i * k + c * 16);
         const float da = sa.d[(int64_t)i * nblk + (c >> 1)];
 #pragma unroll
-        for (int r = 0; r < R; r++) acc[r][i] += (float)dot16(q[r], av, 0) * dw[r] * da;
+        for (int r = 0; r < R; r++) acc[r][i] += (float)dot16(q[r], av, 0) * (dw[r] * da); // two f16 values: their product is exact
       }
     }
   }
