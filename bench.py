@@ -57,7 +57,7 @@ WORKLOADS = {
 
 
 def kernel_of(dt, m: int) -> str:
-    """The kernel that serves m rows of a weight of this format at k = 4096."""
+    """The kernel that serves m rows of an [n >= 3072, 4096] weight of this format."""
     if m == 1:
         return "matvec_ring_kernel"
     if m <= {D.Q4_0: 4, D.Q8_0: 4, D.Q4K: 1, D.Q6K: 5}[dt]:

@@ -336,8 +336,8 @@ int xnq_device_check_record(unsigned long long out[8]);
 /* Tuning switches, for A/B measurements: "matvec_tma" (default 1) selects the persistent bulk-copy ring
  * decode kernel for m == 1; 0 forces the plain streaming-load kernel. "matvec_mma" (default 1)
  * selects the integer-MMA kernel for batches of 5..16 rows on Q4_K weights, 0 the dp4a kernel. "imma" (default 1):
- * batches of 5..64 rows on Q4_0 / Q8_0, 2..64 on Q4_K and 6..16 on Q6_K weights take the tcgen05 integer kernel; 0 sends
- * them to the older kernels. "imma_fold": accepted without effect (it chose a second Q4_K kernel that no batch was faster on).
+ * batches of 5..64 rows on Q4_0 / Q8_0 (2..4 where the dp4a kernel is slower), 2..64 on Q4_K and 6..16 on Q6_K weights take the
+ * tcgen05 integer kernel; 0 sends them to the older kernels. "imma_fold": accepted without effect (it chose a second Q4_K kernel that no batch was faster on).
  * "gather_cta_fence" (default 1): scope of the per-CTA fence before the arrival count of a kernel-side gather, 1 = gpu,
  * 0 = system. No counterpart in the reference. */
 int xnq_set_option(const char *name, int value);

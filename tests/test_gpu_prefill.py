@@ -156,6 +156,34 @@ def test_integer_kernel_row_and_step_edges(Q, O, dt, m):
         assert (np.abs(got - O.matmul(int(dt), x, w, n)) <= _f32_bound(O, dt, w, x, n, k)).all(), (dt.name, m, n, k)
 
 
+# two to four rows of Q4_0 / Q8_0, on both sides of every line between the dp4a and the tensor-core kernel (k 256, 512, 3072, 4096, 5632, 8192;
+# n 512, 3072, 6144, 8192), in every type of rows and with rows apart, against the kernel that the option imma = 0 leaves and the oracle
+@pytest.mark.parametrize("dt", [D.Q4_0, D.Q8_0])
+@pytest.mark.parametrize("n,k", [(511, 5632), (511, 5664), (512, 4096), (512, 3072), (512, 3104), (513, 8192), (513, 8224), (3071, 3104), (3072, 8224), (5, 512), (6144, 512),
+                                 (6143, 512), (6144, 544), (6144, 256), (8191, 5664), (8192, 5664), (8192, 5632)])
+def test_two_to_four_rows_on_either_kernel(Q, O, dt, n, k):
+    from xn_b200 import _lib
+    L = _lib.lib()
+    w = synth.make_weight(dt, n, k, seed=n)
+    x = synth.make_activation(4, 2 * k, seed=k)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    for act in (torch.float32, torch.float16, torch.bfloat16):
+        xd = torch.from_numpy(x).to(act).to(DEV)[:, :k]
+        rows = xd.float().cpu().numpy()
+        want = O.matmul(int(dt), rows, w, n, threads=O.hw_threads())
+        bound = _f32_bound(O, dt, w, rows, n, k) if act is torch.float32 else \
+            2e-5 * np.abs(want).max() + np.abs(want) * 2.0 ** (-11 if act is torch.float16 else -8)   # and rounded to the result's type
+        for m in (2, 3, 4):
+            for imma in (1, 0):
+                try:
+                    _lib.check(L.xnq_set_option(b"imma", imma))
+                    got = t.matmul_t(xd[:m])
+                finally:
+                    _lib.check(L.xnq_set_option(b"imma", 1))
+                assert got.dtype is act
+                assert (np.abs(got.float().cpu().numpy().astype(np.float64) - want[:m]) <= bound[:m]).all(), (dt.name, m, n, k, imma, act)
+
+
 # Every CTA of the integer kernel takes an equal run of the (tile, step) space: here more steps than twice the stages of any of its rings
 # but the two of eight (operand 2 or 3, activations 2 to 8, side 8), so every barrier is met in both parities, and the long rings wrap.
 @pytest.mark.parametrize("dt", WEIGHT_TYPES)

@@ -29,13 +29,28 @@ static std::atomic<int> g_opt_gather_cta_fence{1};
 static std::atomic<int> g_opt_host_direct_y{1};
 static std::atomic<int> g_opt_matvec_mma{1};
 static std::atomic<int> g_opt_imma{1};
-// The integer tensor-core kernel, except up to four rows of Q4_0 / Q8_0 that the dp4a kernel can stage at once: it streams the weight
-// without the operand image and its hand-overs (Q4_0 4096 x 4096, 2 rows: 8.1 us against 12.5; Q8_0 11008 x 4096, 2 rows: 17.0 against
-// 21.1; 4096 x 4096, 3 rows: 11.0 against 13.2). Q4_K stays on one kernel from two rows on, so that operand images and float rows give
-// the same bits.
+// Two to four rows of Q4_0 / Q8_0 that the dp4a kernel can stage at once: where it is faster than the integer tensor-core kernel. It
+// streams the weight without the operand image and its hand-overs, but a row's whole k is one warp's and every activation row costs its
+// own dp4a. Both timed on the device with cold weights at 13 row counts n from 128 to 28672, 12 k from 256 to 14336 and 2, 3 and 4 rows;
+// the rule's choice is on average 1 % above the faster one (dp4a throughout: 7 %), and 1.25 times at most.
+static bool few_rows_on_dp4a(const WeightView &w, int64_t m) {
+  if (m > 4 || (w.dtype != XNQ_Q4_0 && w.dtype != XNQ_Q8_0) || matvec_rows_per_pass(w.dtype, w.k) < m) return false;
+  const bool q8 = w.dtype == XNQ_Q8_0;
+  // one or two steps of k: many tiles are no longer than few on the tensor cores (Q4_0, 4 rows, 28672 x 256: dp4a 12.8 us, tensor cores 5.3;
+  // 14336 x 512: 8.7, 5.2; 256 x 512: 4.6, 4.8)
+  if (w.k <= (q8 && m == 2 ? 256 : 512)) return w.n < 6144;
+  // few weight rows: not enough warps to hide the walk along a long k (Q8_0, 4 rows, 512 x 14336: 26.9, 14.3; 512 x 2048: 6.4, 7.8; Q4_0, 3 rows,
+  // 1024 x 4096: 8.5, 8.4; Q8_0, 2 rows, 128 x 4096: 6.3, 8.2)
+  if (w.n < 512) return w.k <= 5632;
+  if (w.n < 3072) return w.k <= (q8 ? 3072 : (m == 2 ? 8192 : 4096));
+  // many: the dp4a rate bounds three and four rows of Q8_0 (4 rows, 8192 x 11008: 41.0, 30.7; 14336 x 8192: 43.4, 37.2; 3 rows, 11008 x 4096: 18.9, 22.1;
+  // 6144 x 8192: 19.0, 22.9; 2 rows, 8192 x 4096: 11.8, 17.6)
+  return !q8 || m == 2 || w.n < 8192 || w.k <= 5632;
+}
+// Which batches the integer tensor-core kernel takes. Q4_K stays on it from two rows on, so that operand images and float rows give the
+// same bits.
 static bool use_imma(const xnq_weight *w, int64_t m) {
-  if (m < 2 || m > IMMA_MAX_M || !g_opt_imma.load(std::memory_order_relaxed) || !imma_supported(w->v, m)) return false;
-  return m > 4 || w->v.dtype == XNQ_Q4K || matvec_rows_per_pass(w->v.dtype, w->v.k) < m;
+  return m >= 2 && m <= IMMA_MAX_M && g_opt_imma.load(std::memory_order_relaxed) && imma_supported(w->v, m) && !few_rows_on_dp4a(w->v, m);
 }
 // Small batches: the integer-MMA kernel where it serves the weight and wins (Q4_K, five rows and up), else the
 // dp4a kernel. Returns the rows per launch.
