@@ -38,7 +38,7 @@
 // Work is the flattened (tile of 128 weight rows, 256-k step) space, cut into equal contiguous ranges, one
 // per CTA, so all SMs finish together however few tiles there are. A tile whose steps are split between
 // CTAs is summed deterministically: every part is written to a scratch slot, an arrival ticket elects the
-// last part, and that CTA adds the parts, in runs in k order, and stores y.
+// last part, and that CTA adds the parts in k order and stores y.
 //
 // Every wait is bounded; on expiry a status bit is set and the roles fall through to the common exit, where
 // tensor memory is released.
@@ -412,8 +412,9 @@ __device__ __forceinline__ void q6k_sums(const uint4 &hdr, int h, const uint32_t
 }
 
 // Long f32 chains are cut: after SUM_RUN terms the chain's sum goes to a second one. Q6_K's steps (a CTA may add all of a long row's:
-// 14336 / 256 = 56), and the parts of a tile. (Q6_K, 600 x 14336: 1.06e-7 from the exact dot in one chain; the dp4a kernel, whose 32 lanes
-// take a part each, 8.3e-8.)
+// 14336 / 256 = 56) and, with 16 rows, the parts of a tile. (Q6_K, 600 x 14336: 1.06e-7 from the exact dot in one chain; the dp4a kernel, whose
+// 32 lanes take a part each, 8.3e-8. Wider operands add their parts in one chain, as they did before their drain took whole steps: with
+// runs, in 72 registers, the loop over the parts of 600 x 14336 took 44 us instead of 29 at 64 rows.)
 constexpr int SUM_RUN = 8;
 
 // Drain warps: a warp's waits and its decoding of the row's scales cost as much as four columns' arithmetic; with 16 rows eight warps of
@@ -739,21 +740,28 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
           const int t_u0 = tile * KT, t_u1 = t_u0 + KT;
           const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u1 - 1, p.units_q, p.units_r);
           if (et == 0 && (int)ticket == c_last - c_first) p.tile_cnt[tile] = 0u; // every part has its ticket: the word is zero again for the next call
-          if ((int)ticket == c_last - c_first) { // the last part to arrive adds all parts, in runs in k order
+          if ((int)ticket == c_last - c_first) { // the last part to arrive adds all parts in k order (16 rows: in runs)
             __threadfence();
             float (&sum)[NPT] = acc; // the segment's own sums are in its scratch slot by now
-            float some[NPT];
 #pragma unroll
-            for (int c = 0; c < NPT; c++) sum[c] = 0.f, some[c] = 0.f;
-            for (int cc = c_first; cc <= c_last; cc++) {
+            for (int c = 0; c < NPT; c++) sum[c] = 0.f;
+            auto add_part = [&](int cc, float (&to)[NPT]) {
               const int cu0 = cta_first_unit(cc, p.units_q, p.units_r);
               const float *part = p.partials + ((size_t)2 * cc + (cu0 >= t_u0 ? 0 : 1)) * ROWS * TILE_N;
 #pragma unroll
-              for (int c = 0; c < NPT; c++) some[c] += __ldcg(part + (size_t)(c0 + c) * TILE_N + 32 * q + lane);
-              if (((cc - c_first) & (SUM_RUN - 1)) == SUM_RUN - 1 || cc == c_last) {
+              for (int c = 0; c < NPT; c++) to[c] += __ldcg(part + (size_t)(c0 + c) * TILE_N + 32 * q + lane);
+            };
+            if constexpr (DW == 8) {
+              for (int cc = c_first; cc <= c_last;) {
+                float some[NPT];
 #pragma unroll
-                for (int c = 0; c < NPT; c++) sum[c] += some[c], some[c] = 0.f;
+                for (int c = 0; c < NPT; c++) some[c] = 0.f;
+                for (const int end = min(cc + SUM_RUN, c_last + 1); cc < end; cc++) add_part(cc, some);
+#pragma unroll
+                for (int c = 0; c < NPT; c++) sum[c] += some[c];
               }
+            } else {
+              for (int cc = c_first; cc <= c_last; cc++) add_part(cc, sum);
             }
             if (row < p.w.n) {
 #pragma unroll
