@@ -215,3 +215,40 @@ def test_fp16_kernel_tile_and_step_edges(Q, O, dt, m):
         _check(got.cpu().numpy(), want, f"{dt.name} m={m} n={n} k={k}")
         half = t.matmul_t(xd, out=torch.empty(m, n, dtype=torch.float16, device=DEV))
         assert torch.allclose(half.float(), got, rtol=2.0 ** -10, atol=1e-4 * float(got.abs().max()))   # rounded once; parts of a split tile may meet in another order
+
+
+# 16-bit results of the fp16 kernel on pairs of CTAs: an odd number of row tiles and one row in the last, m-tiles of unequal halves, k-steps that
+# do not fill a super-step; against the oracle, and against the f32 results of single CTAs
+@pytest.mark.parametrize("dt", WEIGHT_TYPES)
+@pytest.mark.parametrize("n,k,m", [(3841, 2048, 881), (3841, 2048, 1024), (14209, 4096, 209)])
+def test_fp16_kernel_on_pairs(Q, O, dt, n, k, m):
+    k -= 0 if dt.block_size == 256 else 32
+    w = synth.make_weight(dt, n, k, seed=m)
+    x = synth.make_activation(m, k, seed=m + k)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    xd = torch.from_numpy(x).to(DEV)
+    got = t.matmul_t(xd)
+    _check(got.cpu().numpy(), O.matmul(int(dt), x, w, n, threads=O.hw_threads()), f"{dt.name} m={m} n={n} k={k}")
+    for out in (torch.float16, torch.bfloat16):
+        buf = torch.full((m * n + 128,), 777.0, device=DEV, dtype=out)
+        half = t.matmul_t(xd, out=buf[:m * n].view(m, n))
+        assert torch.all(buf[m * n:] == 777.0), "wrote past the output"
+        assert torch.allclose(half.float(), got, rtol=2.0 ** (-10 if out is torch.float16 else -7), atol=1e-4 * float(got.abs().max()))
+
+
+# several tiles of unequal widths (256 and 192, 256 and 16 rows) on one CTA's single accumulator, whose halves are given back one by one; rows of y that
+# start on 16 bytes (n a multiple of 8) and rows that do not
+@pytest.mark.parametrize("dt", WEIGHT_TYPES)
+@pytest.mark.parametrize("n,m", [(515, 700), (512, 700), (516, 528), (1029, 260)])
+def test_fp16_kernel_unequal_tiles(Q, O, dt, n, m):
+    k = 512 if dt.block_size == 256 else 352
+    w = synth.make_weight(dt, n, k, seed=m + n)
+    x = synth.make_activation(m, k, seed=m)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    xd = torch.from_numpy(x).to(DEV)
+    got = t.matmul_t(xd)
+    _check(got.cpu().numpy(), O.matmul(int(dt), x, w, n, threads=O.hw_threads()), f"{dt.name} m={m} n={n}")
+    wide = torch.full((m, n + 7), 777.0, dtype=torch.bfloat16, device=DEV)   # rows apart
+    t.matmul_t(xd, out=wide[:, :n]) if n % 8 else t.matmul_t(xd, out=wide.view(-1)[: m * n].view(m, n))
+    half = wide[:, :n] if n % 8 else wide.view(-1)[: m * n].view(m, n)
+    assert torch.allclose(half.float(), got, rtol=2.0 ** -7, atol=1e-4 * float(got.abs().max()))

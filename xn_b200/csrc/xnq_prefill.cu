@@ -12,7 +12,8 @@
 //      as the reference's quantize_lhs does (k_quants.rs:2015-2026), dequantized, scaled by a power of
 //      two per row and stored as fp16 in the same swizzled image, so that one 1-D bulk-async copy
 //      (cp.async.bulk, non-multicast) brings a whole stage.
-//   D  f32 in tensor memory; eight epilogue warps read it back with tcgen05.ld, undo the power-of-two
+//   D  f32 in tensor memory; eight drain warps read it back with tcgen05.ld, turn it over in shared memory
+//      (in tensor memory a lane is a weight row, y is contiguous along weight rows), undo the power-of-two
 //      scales and store y.
 //
 // Operand type. The contraction runs in fp16 (kind::f16 with f16 inputs), not bf16: both have the
@@ -30,6 +31,7 @@
 // bulk copy adds its transaction bytes) and empty (tcgen05.commit by the MMA warp). Every wait is bounded; on
 // expiry a status bit is set and every role falls through to the common exit, where tensor memory is released.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 
 #include "xnq_common.cuh"
@@ -47,8 +49,15 @@ constexpr int BK = 64;             // k-step (elements) = one 128-byte swizzle r
 constexpr int TILE_N = 128;        // weight rows per CTA = UMMA M
 constexpr int MAX_MT = 256;        // activation rows per CTA = UMMA N
 constexpr int PRODUCER_WARPS = 16; // four row groups of 32 rows x four warps
-constexpr int LOADER_WARP = PRODUCER_WARPS, MMA_WARP = LOADER_WARP + 1;
-constexpr int NTHREADS = PRODUCER_WARPS * 32 + 64; // warps 0-15 producers, then the loader warp and the MMA warp
+constexpr int EPI_WARPS = 8;       // two per accumulator lane quarter, which take turns in its chunks of 16 columns
+constexpr int LOADER_WARP = PRODUCER_WARPS, MMA_WARP = LOADER_WARP + 1, EPI_WARP0 = MMA_WARP + 1, COPY_WARP0 = EPI_WARP0 + EPI_WARPS;
+// Copy warps: two, and four for Q8_0, whose k-steps are twice the bytes (11008 x 4096, 160 rows: 31.9 us with four, 32.9 with two; Q4_K 14336 x
+// 4096, 100 rows: 30.7 and 30.0: the other formats' conversion wants the registers).
+template <typename RowT>
+__host__ __device__ constexpr int copy_warps() { return RowT::KPS == 2 ? 4 : 2; }
+template <typename RowT>
+__host__ __device__ constexpr int nthreads() { return (COPY_WARP0 + copy_warps<RowT>()) * 32; }
+constexpr uint32_t EPI_SLOT = 16 * 32 * 4; // a drain warp's chunk: 16 columns of 32 weight rows, f32
 constexpr uint32_t WAIT_LIMIT = 1u << 26; // polls of a flag in global memory
 constexpr int A_COLS = BK / 2;     // tensor-memory columns of a stage's weights
 constexpr int A_COL0 = 256;        // they start behind the accumulators: one of 256 columns or two of 128
@@ -104,6 +113,25 @@ __device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity,
   const bool ok = mbar_wait(bar, parity, bit);
   return __all_sync(0xffffffffu, ok);
 }
+// ---- CTA pairs (a cluster of two) ----
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() { // by every thread of both CTAs
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// the same barrier in the leader's (rank 0's) shared memory
+__device__ __forceinline__ uint32_t leader_addr(uint32_t bar) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(bar));
+  return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
 // true in one lane of a converged warp
 __device__ __forceinline__ bool elect_one() {
   uint32_t e;
@@ -121,39 +149,49 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
 }
 
 // ---- tcgen05 wrappers --------------------------------------------------------------------------------
+// CG: CTAs that work together on a tile. All of a kernel's tcgen05 instructions name the same number.
+template <int CG>
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+  if (CG == 2) asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+  else asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
 }
-__device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory"); }
+template <int CG>
+__device__ __forceinline__ void tmem_relinquish() {
+  if (CG == 2) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  else asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+template <int CG>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// A from tensor memory, B from shared memory
+// A from tensor memory, B from shared memory. CG 2: every CTA of the pair has its 128 weight rows in its own tensor memory and half of the
+// activation rows in its own shared memory, both at the addresses that are named here, and gets its 128 rows of the result.
+template <int CG>
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  if (CG == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
-// arrives on the mbarrier once every MMA issued so far by this thread has finished reading smem / writing tmem
+// arrives on the mbarrier (CG 2: on that of each CTA of the pair) once every MMA issued so far by this thread has finished reading and writing
+template <int CG>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
+  if (CG == 2)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+  else asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -173,7 +211,7 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
 }
 // kind::f16 instruction descriptor: D f32 (bit 4), A/B format (0 = f16) at [7,10) / [10,13), both K-major,
 // N >> 3 at [17,23), M >> 4 at [24,29).
-__device__ __forceinline__ uint32_t idesc_f16(int umma_n) { return (1u << 4) | ((uint32_t)(umma_n >> 3) << 17) | ((uint32_t)(TILE_N >> 4) << 24); }
+__device__ __forceinline__ uint32_t idesc_f16(int umma_m, int umma_n) { return (1u << 4) | ((uint32_t)(umma_n >> 3) << 17) | ((uint32_t)(umma_m >> 4) << 24); }
 
 struct PrefillArgs {
   WeightView w;
@@ -183,77 +221,126 @@ struct PrefillArgs {
   int y_dtype;
   int64_t ldy;
   int64_t m, m_pad;
+  int mt;                 // activation rows of a tile (the last one may have fewer)
   int ksteps;
   int nstages;            // stages: weights in tensor memory, activations in shared memory
   int acc_bufs;           // accumulators: 1 of 256 columns, 2 of 128 (tiles of up to 128 activation rows)
   int raw_slots;          // raw super-steps in shared memory, the one being converted included
+  int vec_out;            // rows of y start on 16 bytes and hold whole 16-byte pieces
   uint32_t b_stride;      // bytes between B stages (largest mt of the grid x 128, multiple of 1024)
-  uint32_t raw_off;       // offset of the raw ring behind the B ring
+  uint32_t raw_off, epi_off; // offsets of the raw ring and of the drain warps' chunks behind the B ring
   float wscale;           // power of two applied to every dequantized weight
-  // persistent kernel: tile t = tile_n * tiles_m + tile_m; work unit u = t * ksteps + kt; CTA c takes units
-  // [units * c / G, units * (c + 1) / G), or whole tiles when the output cannot be accumulated atomically
-  int tiles_n, tiles_m;
-  long long units;
+  // persistent kernel: tile t = tile_n * tiles_m + tile_m; work unit u = t * ksteps + kt; CTA (or pair) c takes units
+  // [units * c / G, units * (c + 1) / G), or whole tiles when the output cannot be accumulated atomically. share_q, share_r: what is divided
+  // (units or tiles) by G and its remainder, set at launch: the 64-bit divisions held every thread of every CTA back before its first copy
+  int tiles_n, tiles_m;   // tiles_n: of 128 weight rows, or of a pair's 256
+  long long units, share_q;
+  int share_r;
   int whole_tiles;
-  unsigned int *tile_cnt; // [tiles] arrival tickets then [tiles] "first partial stored" flags; zeroed by the prepare kernel
+  int row_tiles;          // tiles of 128 weight rows: the last pair's second CTA may have none
+  unsigned int *tile_cnt; // per (row tile, m-tile) arrival tickets, then "first partial stored" flags; zeroed by the prepare kernel
 };
 
 using namespace prefill_rows;
 
-// waits until at most `pending` of this thread's committed copy groups are still in flight
-__device__ __forceinline__ void cp_async_wait(int pending) {
-  switch (pending) {
-    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+
+// How a chunk (16 columns = activation rows, 32 weight rows) reaches y. In the accumulator a lane is a weight row, and y is contiguous along
+// weight rows.
+enum Store { STORE_F32, ADD_F32, STORE_F16, STORE_BF16 };
+template <int ST>
+__device__ __forceinline__ uint32_t pack16(float a, float b) {
+  if (ST == STORE_F16) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
+  }
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+// Rows of y that start on 16 bytes: the chunk is turned over in shared memory (column j of weight row l at j * 128 + 4 l, 16-byte pieces
+// swapped in odd columns so that the 16-bit types' reads of two neighbouring pieces touch all banks) and leaves in 16-byte stores, 8 or 4
+// lanes to a row: a quarter of the store instructions. yp: this warp's first weight row in the chunk's first activation row; cols: how many
+// columns exist; rows: how many of the 32 weight rows; ru: shared address of the chunk's row factors.
+template <int ST>
+__device__ __forceinline__ void store_turned(uint32_t slot, uint32_t ru, char *yp, int64_t row_bytes, int cols, int rows, int lane) {
+  if (ST <= ADD_F32) {
+    const int j0 = lane >> 3, piece = lane & 7;
+    const uint32_t at = slot + (uint32_t)(j0 * 128 + ((piece ^ (j0 & 1)) << 4));
+    char *p = yp + j0 * row_bytes + piece * 16;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint4 v = lds128(at + i * 512);
+      const float f = __uint_as_float(lds32(ru + (uint32_t)((4 * i + j0) * 4)));
+      const float4 o = make_float4(__uint_as_float(v.x) * f, __uint_as_float(v.y) * f, __uint_as_float(v.z) * f, __uint_as_float(v.w) * f);
+      if (4 * i + j0 < cols && piece * 4 < rows) {
+        if (ST == STORE_F32) *reinterpret_cast<float4 *>(p) = o;
+        else atomicAdd(reinterpret_cast<float4 *>(p), o);
+      }
+      p += 4 * row_bytes;
+    }
+  } else {
+    const int j0 = lane >> 2, piece = (lane & 3) * 2;
+    const uint32_t at = slot + (uint32_t)(j0 * 128);
+    const uint32_t p0 = (uint32_t)((piece ^ (j0 & 1)) << 4), p1 = p0 ^ 16u;
+    char *p = yp + j0 * row_bytes + piece * 8;
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const uint4 a = lds128(at + i * 1024 + p0), b = lds128(at + i * 1024 + p1);
+      const float f = __uint_as_float(lds32(ru + (uint32_t)((8 * i + j0) * 4)));
+      const uint4 o = make_uint4(pack16<ST>(__uint_as_float(a.x) * f, __uint_as_float(a.y) * f), pack16<ST>(__uint_as_float(a.z) * f, __uint_as_float(a.w) * f),
+                                 pack16<ST>(__uint_as_float(b.x) * f, __uint_as_float(b.y) * f), pack16<ST>(__uint_as_float(b.z) * f, __uint_as_float(b.w) * f));
+      if (8 * i + j0 < cols && piece * 4 < rows) *reinterpret_cast<uint4 *>(p) = o;
+      p += 8 * row_bytes;
+    }
   }
 }
-
-// Writes one 32-column chunk of an accumulator row block: column j of the chunk is activation row
-// m_first + j, this lane's accumulator lane is weight row `row`. MODE: 0 f32 store, 1 f32 atomic add,
-// 2 f16 store, 3 bf16 store.
-template <int MODE>
-__device__ __forceinline__ void drain_chunk(const uint32_t (&v)[32], float ru_lane, void *y, int64_t ldy, int64_t row, int64_t m_first, int64_t m_end,
-                                            bool row_ok) {
-  // a running pointer and one small count: the few warps that drain have nobody to hide instruction latency
-  // behind, so every instruction per column counts
-  const int es = MODE <= 1 ? 4 : 2;
-  char *yp = static_cast<char *>(y) + (m_first * ldy + row) * es;
-  const int64_t step = ldy * es;
-  const int nvalid = row_ok ? (int)min((int64_t)32, m_end - m_first) : 0;
+// Other rows: a lane stores its weight row's values one by one, neighbouring lanes to neighbouring addresses.
+template <int ST>
+__device__ __forceinline__ void store_direct(const uint32_t (&v)[16], uint32_t ru, char *yp, int64_t row_bytes, int cols, bool row_ok, int lane) {
+  char *p = yp + lane * (ST <= ADD_F32 ? 4 : 2);
 #pragma unroll
-  for (int j = 0; j < 32; j++) {
-    const float val = __uint_as_float(v[j]) * __shfl_sync(0xffffffffu, ru_lane, j);
-    if (j < nvalid) {
-      if (MODE == 0) *reinterpret_cast<float *>(yp) = val;
-      else if (MODE == 1) atomicAdd(reinterpret_cast<float *>(yp), val);
-      else if (MODE == 2) *reinterpret_cast<__half *>(yp) = __float2half_rn(val);
-      else *reinterpret_cast<__nv_bfloat16 *>(yp) = __float2bfloat16_rn(val);
+  for (int j = 0; j < 16; j++) {
+    const float val = __uint_as_float(v[j]) * __uint_as_float(lds32(ru + (uint32_t)(j * 4)));
+    if (j < cols && row_ok) {
+      if (ST == STORE_F32) *reinterpret_cast<float *>(p) = val;
+      else if (ST == ADD_F32) atomicAdd(reinterpret_cast<float *>(p), val);
+      else if (ST == STORE_F16) *reinterpret_cast<__half *>(p) = __float2half_rn(val);
+      else *reinterpret_cast<__nv_bfloat16 *>(p) = __float2bfloat16_rn(val);
     }
-    yp += step;
+    p += row_bytes;
   }
 }
 
 // ---- the kernel ------------------------------------------------------------------------------------------------
-// One CTA per SM walks a contiguous range of the flattened (tile, k-step) space, so all SMs finish
+// CG 2: the CTAs of a cluster of two take 128 weight rows each of a tile and one MMA (cta_group::2) works for both, so that each CTA brings
+// only half of the tile's activation rows: per k-step of 256 rows 16 KB instead of 32 through L2 and shared memory, which at 512 cycles of
+// MMA were what bounded such tiles (28672 x 4096, 2000 rows: 415 -> 390 us at full clock). The leader issues the MMAs; the other CTA's warp
+// of that role tells it when its half of a stage is there, and the commits arrive on both CTAs' barriers. (The relay's arrival and the
+// leader's wait have the default semantics: with .release.cluster and .acquire.cluster each costs a fence of some 1000 cycles and the kernel
+// took 654 us. What they order, tensor-memory stores and bulk copies, has completed before the local barrier lets the relay pass.)
+// One CTA per SM (or pair per two) walks a contiguous range of the flattened (tile, k-step) space, so all SMs finish
 // together whatever the tile count, and a tile whose k-steps are split between CTAs is summed in
 // global memory: the first CTA to finish its part stores it and raises the tile's flag, the others add
 // theirs atomically after seeing the flag (two to three parts per split tile; f32 output only - other
 // output types get whole tiles). Tiles of up to 128 activation rows have two accumulators, so the drain of one
-// segment overlaps the MMAs of the next; wider ones have one, and the producers fill the stages meanwhile.
+// segment overlaps the MMAs of the next. Wider ones have one, whose halves of columns the drain gives back one by one: the first
+// MMAs of the next segment go to the half that is free.
 // Roles: 16 producer warps, one activation-loader warp (one bulk copy per stage), one MMA-issuing warp, eight drain
-// warps. Stage counters run on across segments.
-// Producers: the four warps of a row group (32 weight rows) fetch the group's bytes of a super-step together, several
-// super-steps ahead, and each then converts its own k-step of it (or its half of one), so the k-steps of a super-step are
-// converted side by side and a warp's chain of waits, loads, arithmetic and stores has a super-step's MMAs to run in. One
-// barrier of the row group's four warps per super-step makes the copies visible to all of them and tells that the slot of
-// the previous super-step has been read.
-constexpr int EPI_WARPS = 8; // two per accumulator lane quarter, splitting the columns
-constexpr int EPI_WARP0 = MMA_WARP + 1;
-constexpr int NTHREADS_SK = NTHREADS + EPI_WARPS * 32;
-
+// warps, two or four warps that copy raw weights. Stage counters run on across segments.
+// Producers: the four warps of a row group (32 weight rows) convert a k-step each of a super-step (or a half of one), so the k-steps of a
+// super-step are converted side by side and a warp's chain of waits, loads, arithmetic and stores has a super-step's MMAs to run in.
+// Measured together, the turned drain, the halves and the copy warps (long stream of calls, f32 results): Q4_0 4096 x 4096, 200 rows 32.5 ->
+// 25.6 us; Q4_K 4096 x 4096, 300 rows 31.9 -> 29.3; Q6_K 8192 x 4096, 700 rows 69.5 -> 65.6; Q8_0 11008 x 4096, 512 rows 66.5 -> 64.0; Q4_K 14336 x
+// 4096, 512 rows 73.1 -> 72.2 (power limit).
 struct Cursor { // position in the flattened (tile, k-step) space; tile = tile_n * tiles_m + tile_m
   int tile_n, tile_m, kt;
   __device__ __forceinline__ void advance(int steps, int KT, int tiles_m) {
@@ -266,132 +353,109 @@ struct Cursor { // position in the flattened (tile, k-step) space; tile = tile_n
       }
     }
   }
-  __device__ __forceinline__ int tile(int tiles_m) const { return tile_n * tiles_m + tile_m; }
 };
 
-template <typename RowT>
-__global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(PrefillArgs p) {
+// columns of an accumulator's first half, which is given back to the MMAs on its own; n: the widest tile's (narrower ones are divided there too,
+// as a segment's first MMAs go by what the segment before has given back)
+template <int CG>
+__device__ __forceinline__ int first_half(int n) { return (n / 2 + 16 * CG - 1) / (16 * CG) * (16 * CG); }
+// The activation row of a tile whose products are in accumulator column c. Pairs: each half of the n columns holds first rows of the leader's
+// half of the tile, then rows of the other CTA's.
+template <int CG>
+__device__ __forceinline__ int row_of_column(int c, int n) {
+  if (CG == 1) return c;
+  const int h0 = first_half<2>(n), upper = c >= h0, q = (upper ? n - h0 : h0) / 2, cc = upper ? c - h0 : c;
+  const int cta = cc >= q;
+  return cta * (n / 2) + (upper ? h0 / 2 : 0) + cc - cta * q;
+}
+
+template <typename RowT, int CG>
+__global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel(PrefillArgs p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 4]; // full, empty (8 each), acc_full[2], acc_empty[2]
+  __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 4 + 2 * MAX_RAW_SLOTS]; // full, empty (8 each), acc_full[2], acc_empty[2], raw_full, raw_empty
+  __shared__ float s_ru[MAX_MT]; // the tile's row factors
   __shared__ uint32_t tmem_slot;
   __shared__ unsigned int s_ticket;
   const int S = p.nstages;
-  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, acc_full = empty + 8 * MAX_STAGES, acc_empty = acc_full + 16;
+  const uint32_t full = smem_u32(bars), empty = full + 8 * MAX_STAGES, acc_full = empty + 8 * MAX_STAGES, acc_empty = acc_full + 16, raw_full = acc_empty + 16,
+                 raw_empty = raw_full + 8 * MAX_RAW_SLOTS;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // so that the compiler knows `warp` to be uniform
   const uint32_t b_ring = smem_base;
   const int NACC = p.acc_bufs;
   const int KT = p.ksteps;
+  const uint32_t rank = CG == 2 ? cluster_rank() : 0u; // 0: the pair's leader, which issues its MMAs
 
-  // this CTA's range of work units
-  long long u0, u1;
-  if (p.whole_tiles) {
-    const long long T = (long long)p.tiles_n * p.tiles_m;
-    u0 = (T * blockIdx.x / gridDim.x) * KT;
-    u1 = (T * (blockIdx.x + 1) / gridDim.x) * KT;
-  } else {
-    u0 = p.units * blockIdx.x / gridDim.x;
-    u1 = p.units * (blockIdx.x + 1) / gridDim.x;
-  }
+  // this CTA's (or pair's) range of work units
+  const int cta = (int)blockIdx.x / CG, ctas = (int)gridDim.x / CG;
+  long long u0 = p.share_q * cta + cta * p.share_r / ctas, u1 = p.share_q * (cta + 1) + (cta + 1) * p.share_r / ctas;
+  if (p.whole_tiles) u0 *= KT, u1 *= KT;
   const int nsteps = (int)(u1 - u0);
   const int TM = p.tiles_m;
-  const Cursor start{(int)((u0 / KT) / TM), (int)((u0 / KT) % TM), (int)(u0 % KT)};
+  const int tile0 = p.units <= INT_MAX ? (int)u0 / KT : (int)(u0 / KT);
+  const Cursor start{tile0 / TM, tile0 % TM, (int)(u0 - (long long)tile0 * KT)};
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; s++) {
-      mbar_init(full + 8 * s, PRODUCER_WARPS / RowT::KPS + 1);
+      mbar_init(full + 8 * s, PRODUCER_WARPS / RowT::KPS + 1 + (CG == 2 && rank == 0 ? 1 : 0)); // the leader's: and one by the other CTA's relay
       mbar_init(empty + 8 * s, 1);
+    }
+    for (int r = 0; r < p.raw_slots; r++) {
+      mbar_init(raw_full + 8 * r, copy_warps<RowT>() * 32);
+      mbar_init(raw_empty + 8 * r, PRODUCER_WARPS);
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(acc_full + 8 * b, 1);
-      mbar_init(acc_empty + 8 * b, EPI_WARPS);
+      mbar_init(acc_empty + 8 * b, EPI_WARPS * CG); // (used in the leader only)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == LOADER_WARP) {
-    tmem_alloc(smem_u32(&tmem_slot), 512);
-    tmem_relinquish();
+    tmem_alloc<CG>(smem_u32(&tmem_slot), 512);
+    tmem_relinquish<CG>();
   }
   tc_fence_before();
+  if (CG == 2) cluster_sync(); // the other CTA's barriers are set up
   __syncthreads();
   tc_fence_after();
   pdl_launch_dependents();
   const uint32_t tmem_d = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
+  constexpr int KPS = RowT::KPS;
+  constexpr uint32_t SLOT = TILE_N * RowT::ROWB;
+  const int SPT = (KT + KPS - 1) / KPS; // super-steps per tile
+  const int R = p.raw_slots;
+  const int last_kt = nsteps - 1 + start.kt; // counted from the start of the first tile
+  const int nsuper = nsteps > 0 ? (last_kt / KT) * SPT + (last_kt % KT) / KPS - start.kt / KPS + 1 : 0; // super-steps of this CTA
   if (warp < PRODUCER_WARPS) {
-    // ---- producers (nothing here waits for the kernel that prepares the activations: weights are immutable) ----
-    constexpr int KPS = RowT::KPS, NCOPY = (32 * RowT::ITEMS + 127) / 128;
+    // ---- producers: the four warps of a row group convert a k-step of a super-step each (KPS 2: half of one) ----
     const int rg = warp & 3, kg = warp >> 2;
     const int kk = kg % KPS, hf = kg / KPS; // this warp's k-step of a super-step; which half of it (KPS = 2)
-    const int t = kg * 32 + lane; // 0..127 in the row group
-    const uint32_t raw = smem_base + p.raw_off + (uint32_t)(rg * 32 * RowT::ROWB);
-    constexpr uint32_t SLOT = TILE_N * RowT::ROWB;
-    const int SPT = (KT + KPS - 1) / KPS; // super-steps per tile
-    const int R = p.raw_slots;
-    // position of the copies in the super-step space
-    int l_n = start.tile_n, l_m = start.tile_m, l_s = start.kt / KPS, l_slot = 0;
-    const int last_kt = nsteps - 1 + start.kt; // counted from the start of the first tile
-    int l_left = nsteps > 0 ? (last_kt / KT) * SPT + (last_kt % KT) / KPS - l_s + 1 : 0; // super-steps still to be copied
-    int left = l_left;
-    Item it[NCOPY]; // this thread's copies; their addresses change with the tile only
-    auto bind = [&]() {
-#pragma unroll
-      for (int i = 0; i < NCOPY; i++) {
-        const int item = min(i * 128 + t, 32 * RowT::ITEMS - 1);
-        it[i] = RowT::item(p.w, min((int64_t)l_n * TILE_N + 32 * rg + item / RowT::ITEMS, p.w.n - 1), item % RowT::ITEMS);
-      }
-    };
-    bind();
-    uint32_t to[NCOPY]; // where they go in a slot
-#pragma unroll
-    for (int i = 0; i < NCOPY; i++) to[i] = raw + (uint32_t)(((i * 128 + t) / RowT::ITEMS) * RowT::ROWB + ((i * 128 + t) % RowT::ITEMS) * 16);
-    auto issue = [&]() {
-      if (l_left > 0) {
-        l_left--;
-        const uint32_t slot = (uint32_t)l_slot * SLOT;
-#pragma unroll
-        for (int i = 0; i < NCOPY; i++) {
-          if ((32 * RowT::ITEMS) % 128 == 0 || i * 128 + t < 32 * RowT::ITEMS) {
-            const uint32_t off = ((uint32_t)l_s * it[i].mul) & ~15u;
-            if (RowT::LIMITED) cp_async16(to[i] + slot, it[i].p + (off < it[i].lim ? off : 0u), off < it[i].lim ? 16u : 0u);
-            else cp_async16(to[i] + slot, it[i].p + off, 16u);
-          }
-        }
-        if (++l_slot == R) l_slot = 0;
-        if (++l_s == SPT) {
-          l_s = 0;
-          if (++l_m == TM) {
-            l_m = 0, l_n++;
-            bind();
-          }
-        }
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    for (int j = 0; j < R - 1; j++) issue();
-    int c_s = start.kt / KPS, c_slot = 0;
+    const uint32_t raw = smem_base + p.raw_off + (uint32_t)((rg * 32 + lane) * RowT::ROWB);
+    int c_s = start.kt / KPS, slot = 0;
+    uint32_t raw_lap = 0;
     int base_i = -start.kt; // the CTA's step number of the current tile's first k-step
     int at = 0, s = 0;      // s = at % S, lap: parity of at / S, of the last step this warp looked at
     uint32_t lap = 0;
     bool alive = true;
-    for (; left > 0; left--) {
-      cp_async_wait(R - 2); // the super-step's copies of this thread have landed
-      asm volatile("bar.sync %0, 128;" ::"r"(2 + rg) : "memory"); // ... and those of the row group's other threads; all have read the previous slot
-      issue();              // into the previous slot
-      const int kt = c_s * KPS + kk, i = base_i + kt;
-      if (alive && kt < KT && i >= 0 && i < nsteps) {
+    for (int left = nsuper; left > 0; left--) {
+      if (alive) alive = mbar_wait_uniform(raw_full + 8 * slot, raw_lap, 1u);
+      // A warp whose k-step a tile's last super-step does not have waits for the last one that it has, so that two of its waits are never
+      // more than KPS steps apart (see MIN_STAGES).
+      const int kt = c_s * KPS + kk, i = base_i + min(kt, KT - 1);
+      if (alive && i >= 0 && i < nsteps) {
         for (s += i - at, at = i; s >= S; lap ^= 1u) s -= S;
-        if (i >= S) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 1u); // a warp that gave up still takes part in the barriers
-        if (alive) {
+        if (i >= S) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 1u);
+        if (alive && kt < KT) {
           tc_fence_after();
-          const uint32_t slot = raw + (uint32_t)c_slot * SLOT + (uint32_t)(lane * RowT::ROWB);
+          const uint32_t row = raw + (uint32_t)slot * SLOT;
           const uint32_t dst = tmem_d + ((uint32_t)(32 * rg) << 16) + (uint32_t)(A_COL0 + s * A_COLS);
-          const typename RowT::Head head = RowT::head(slot, c_s, kk, p.wscale);
+          const typename RowT::Head head = RowT::head(row, c_s, kk, p.wscale);
 #pragma unroll
           for (int h = 0; h < KPS / 2; h++) {
             const int half = KPS == 2 ? hf : h;
             uint32_t o[16];
-            RowT::half(head, slot, kk, half, o); // a lane past the weight's last row repeats that row and is not stored
+            RowT::half(head, row, kk, half, o); // a lane past the weight's last row repeats that row and is not stored
             tmem_st16(dst + 16 * half, o);
           }
           tmem_st_wait();
@@ -400,13 +464,57 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
           if (lane == 0) mbar_arrive(full + 8 * s);
         }
       }
-      if (++c_slot == R) c_slot = 0;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(raw_empty + 8 * slot); // (also by a warp that gave up)
+      if (++slot == R) slot = 0, raw_lap ^= 1u;
       if (++c_s == SPT) {
         c_s = 0;
         base_i += KT;
       }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  } else if (warp >= COPY_WARP0) {
+    // ---- copies of the raw weights: two or four warps fetch the 128 rows of a super-step, up to R super-steps ahead. (While the producers fetched
+    // their rows themselves, issuing those copies took 1100 to 1700 of a super-step's 3000 cycles: they queue behind the loader's bulk
+    // copies.) A thread has one of the ITEMS pieces of every RPP-th row, so consecutive threads take consecutive 16 bytes of a row. Nothing
+    // here waits for the kernel that prepares the activations: weights are immutable. ----
+    constexpr int RPP = copy_warps<RowT>() * 32 / RowT::ITEMS; // rows per pass
+    const int t = (int)threadIdx.x - COPY_WARP0 * 32;
+    const int piece = t % RowT::ITEMS, first = t < RPP * RowT::ITEMS ? t / RowT::ITEMS : TILE_N;
+    const uint32_t pitch = (uint32_t)(RowT::item(p.w, 1, piece).p - RowT::item(p.w, 0, piece).p);
+    const uint32_t to = smem_base + p.raw_off + (uint32_t)(first * RowT::ROWB + piece * 16);
+    Cursor cur = start;
+    int l_s = start.kt / KPS, slot = 0;
+    uint32_t lap = 0;
+    Item it;
+    int last_row = 0; // rows past the weight's last one repeat it
+    auto bind = [&]() {
+      const int64_t row0 = min(((int64_t)cur.tile_n * CG + rank) * TILE_N, p.w.n - 1);
+      it = RowT::item(p.w, row0, piece);
+      last_row = (int)min((int64_t)(TILE_N - 1), p.w.n - 1 - row0);
+    };
+    bind();
+    for (int j = 0; j < nsuper; j++) {
+      if (j >= R && !mbar_wait_uniform(raw_empty + 8 * slot, lap ^ 1u, 1u)) break;
+      const uint32_t off = ((uint32_t)l_s * it.mul) & ~15u;
+      const bool there = !RowT::LIMITED || off < it.lim;
+      const uint8_t *src = it.p + (there ? off : 0u);
+      const uint32_t dst = to + (uint32_t)slot * SLOT;
+#pragma unroll 8
+      for (int i = 0; i < (TILE_N + RPP - 1) / RPP; i++) {
+        const int r = first + i * RPP;
+        if (r < TILE_N) cp_async16(dst + (uint32_t)(i * RPP * RowT::ROWB), src + (uint64_t)(uint32_t)min(r, last_row) * pitch, there ? 16u : 0u);
+      }
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(raw_full + 8 * slot) : "memory"); // when this thread's copies have landed
+      if (++slot == R) slot = 0, lap ^= 1u;
+      if (++l_s == SPT) {
+        l_s = 0;
+        const int n = cur.tile_n;
+        cur.kt = 0;
+        cur.advance(KT, KT, TM);
+        if (cur.tile_n != n) bind();
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory"); // nothing in flight into this CTA's shared memory when it exits
   } else if (warp == LOADER_WARP) {
     // ---- activation loader: the whole warp runs the loop, one elected lane issues (see the MMA issuer) ----
     pdl_wait(); // the activation image is the previous kernel's output
@@ -415,11 +523,17 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     uint32_t lap = 0;
     for (int i = 0; i < nsteps; i++) {
       if (i >= S && !mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 2u)) break;
-      const int64_t m0 = (int64_t)cur.tile_m * MAX_MT;
-      const uint32_t bytes = (uint32_t)min((int64_t)MAX_MT, p.m_pad - m0) * 128;
+      // a pair's CTAs bring half of the tile's rows each (the last tile's second half may have fewer, or none: what is then left in the
+      // stage reaches only columns that are not stored)
+      const int64_t tm0 = (int64_t)cur.tile_m * p.mt, m0 = tm0 + (CG == 2 ? (int)rank * (p.mt / 2) : 0);
+      const int rows = (int)min((int64_t)(p.mt / CG), min(tm0 + p.mt, p.m_pad) - m0);
       if (elect_one()) {
-        mbar_expect_tx(full + 8 * s, bytes);
-        bulk_g2s(b_ring + s * p.b_stride, p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128, bytes, full + 8 * s);
+        if (rows > 0) {
+          mbar_expect_tx(full + 8 * s, (uint32_t)rows * 128);
+          bulk_g2s(b_ring + s * p.b_stride, p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128, (uint32_t)rows * 128, full + 8 * s);
+        } else {
+          mbar_arrive(full + 8 * s);
+        }
       }
       __syncwarp();
       issued = i + 1;
@@ -427,6 +541,21 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       if (++s == S) s = 0, lap ^= 1u;
     }
     for (int i = max(0, issued - S); i < issued; i++) mbar_wait_uniform(full + 8 * (i % S), (i / S) & 1, 2u); // nothing in flight at exit
+  } else if (CG == 2 && warp == MMA_WARP && rank != 0) {
+    // ---- relay: tells the leader that this CTA's half of a stage is there ----
+    const uint32_t to = leader_addr(full);
+    bool alive = true;
+    for (int i = 0, s = 0, round = 0; i < nsteps && alive; i++) {
+      alive = mbar_wait_uniform(full + 8 * s, round & 1, 4u);
+      tc_fence_after();
+      tc_fence_before();
+      if (alive && elect_one()) mbar_arrive_cluster(to + 8 * s);
+      __syncwarp();
+      if (++s == S) {
+        s = 0;
+        round++;
+      }
+    }
   } else if (warp == MMA_WARP) {
     // ---- MMA issuer: the whole warp runs the loop and one elected lane issues. Everything that decides a loop's course or a
     // descriptor is a function of launch parameters and counters (a wait that gave up only makes the rest of the loop idle), so
@@ -439,11 +568,55 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
     uint32_t round = 0;
     for (int seg = 0; i < nsteps; seg++) {
       const int len = min(KT - cur.kt, nsteps - i);
-      const int buf = NACC == 2 ? seg & 1 : 0, use = NACC == 2 ? seg >> 1 : seg;
-      if (use > 0 && alive) alive = mbar_wait(acc_empty + 8 * buf, (use - 1) & 1, 4u); // the drain of this buffer's previous segment
-      const uint32_t idesc = idesc_f16(min(MAX_MT, (int)p.m_pad - cur.tile_m * MAX_MT));
+      const int N = CG == 2 ? p.mt : min(p.mt, (int)p.m_pad - cur.tile_m * p.mt);
+      // A pair's MMAs always take the two halves of the columns one after the other: which CTA's activation rows are in which columns depends
+      // on an instruction's width.
+      const int h0 = min(first_half<CG>(p.mt), N);
+      const uint32_t idesc = idesc_f16(TILE_N * CG, N), id0 = idesc_f16(TILE_N * CG, h0), id1 = idesc_f16(TILE_N * CG, N - h0);
+      int j = 0;
+      if (NACC == 1 && seg > 0) {
+        // One accumulator: its first half of columns is free while the second is still drained. The first steps of the segment go there
+        // alone and catch up in the second half when that is free too.
+        const int early = min(len, S / 2), s0 = s;
+        if (alive) alive = mbar_wait(acc_empty, (seg - 1) & 1, 4u);
+        for (; j < early; j++) {
+          if (alive) alive = mbar_wait(full + 8 * s, round & 1, 4u);
+          tc_fence_after();
+          __syncwarp();
+          const uint32_t a = tmem_d + (uint32_t)(A_COL0 + s * A_COLS);
+          const uint64_t bdesc = smem_desc_sw128(b_ring + s * p.b_stride);
+          if (elect_one() && alive) {
+#pragma unroll
+            for (int ks = 0; ks < BK / 16; ks++) umma_f16<CG>(tmem_d, a + (uint32_t)(ks * 8), bdesc + (uint64_t)(ks * 2), id0, (j | ks) ? 1u : 0u);
+          }
+          __syncwarp();
+          if (++s == S) {
+            s = 0;
+            round++;
+          }
+        }
+        if (alive) alive = mbar_wait(acc_empty + 8, (seg - 1) & 1, 4u);
+        tc_fence_after();
+        __syncwarp();
+        for (int t = 0, ts = s0; t < early; t++) {
+          const uint32_t a = tmem_d + (uint32_t)(A_COL0 + ts * A_COLS);
+          const uint64_t bdesc = smem_desc_sw128(b_ring + ts * p.b_stride + (uint32_t)(h0 / CG) * 128);
+          if (elect_one() && alive) {
+            if (N > h0) { // (an instruction of no columns is an illegal one)
+#pragma unroll
+              for (int ks = 0; ks < BK / 16; ks++) umma_f16<CG>(tmem_d + (uint32_t)h0, a + (uint32_t)(ks * 8), bdesc + (uint64_t)(ks * 2), id1, (t | ks) ? 1u : 0u);
+            }
+            umma_commit<CG>(empty + 8 * ts);
+            if (t == len - 1) umma_commit<CG>(acc_full);
+          }
+          __syncwarp();
+          if (++ts == S) ts = 0;
+        }
+      }
+      const int buf = NACC == 2 ? seg & 1 : 0;
+      if (NACC == 2 && seg >= 2 && alive) alive = mbar_wait(acc_empty + 8 * buf, ((seg >> 1) - 1) & 1, 4u); // the drain of this buffer's previous segment
       const uint32_t d = tmem_d + (uint32_t)(buf * 128);
-      for (int j = 0; j < len; j++) {
+      for (; j < len; j++) {
         if (alive) alive = mbar_wait(full + 8 * s, round & 1, 4u);
         tc_fence_after();
         __syncwarp();
@@ -451,9 +624,14 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
         const uint64_t bdesc = smem_desc_sw128(b_ring + s * p.b_stride);
         if (elect_one() && alive) {
 #pragma unroll
-          for (int ks = 0; ks < BK / 16; ks++) umma_f16(d, a + (uint32_t)(ks * 8), bdesc + (uint64_t)(ks * 2), idesc, (j | ks) ? 1u : 0u);
-          umma_commit(empty + 8 * s);
-          if (j == len - 1) umma_commit(acc_full + 8 * buf);
+          for (int ks = 0; ks < BK / 16; ks++) umma_f16<CG>(d, a + (uint32_t)(ks * 8), bdesc + (uint64_t)(ks * 2), CG == 2 ? id0 : idesc, (j | ks) ? 1u : 0u);
+          if (CG == 2 && N > h0) {
+#pragma unroll
+            for (int ks = 0; ks < BK / 16; ks++)
+              umma_f16<CG>(d + (uint32_t)h0, a + (uint32_t)(ks * 8), bdesc + (uint64_t)(h0 / CG * 8) + (uint64_t)(ks * 2), id1, (j | ks) ? 1u : 0u);
+          }
+          umma_commit<CG>(empty + 8 * s);
+          if (j == len - 1) umma_commit<CG>(acc_full + 8 * buf);
         }
         __syncwarp();
         if (++s == S) {
@@ -465,22 +643,31 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
       cur.advance(len, KT, TM);
     }
   } else {
-    // ---- drain: eight warps, two to a quarter q of the accumulator lanes (weight rows 32 q ..), which take turns in its chunks of 32 columns ----
+    // ---- drain: eight warps, two to a quarter q of the accumulator lanes (weight rows 32 q ..), which take turns in its chunks of 16 columns ----
     const int q = warp & 3; // tensor-memory lanes a warp may read are fixed by its index modulo 4
-    const int half = (warp - EPI_WARP0) >> 2; // which half of the 32-column chunks this warp takes
+    const int half = (warp - EPI_WARP0) >> 2; // which of the quarter's two warps
     const int et = threadIdx.x - EPI_WARP0 * 32; // 0..255
+    const uint32_t slot = smem_base + p.epi_off + (uint32_t)(warp - EPI_WARP0) * EPI_SLOT;
+    auto give_back = [&](uint32_t bar) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 2) mbar_arrive_cluster(leader_addr(bar));
+        else mbar_arrive(bar);
+      }
+    };
     pdl_wait(); // the previous kernel writes the row factors and zeroes the tiles' tickets
     Cursor cur = start;
     bool alive = true;
     int i = 0;
     for (int seg = 0; i < nsteps && alive; seg++) {
       const int len = min(KT - cur.kt, nsteps - i);
-      const bool whole = cur.kt == 0 && len == KT;
+      const int row_tile = cur.tile_n * CG + (int)rank, tile = row_tile * TM + cur.tile_m; // each CTA of a pair settles its own 128 rows of a split tile
+      const bool whole = (cur.kt == 0 && len == KT) || row_tile >= p.row_tiles;
       const int buf = NACC == 2 ? seg & 1 : 0, use = NACC == 2 ? seg >> 1 : seg;
-      const int tile_n = cur.tile_n, tile_m = cur.tile_m, tile = cur.tile(TM);
-      const int64_t row = (int64_t)tile_n * TILE_N + 32 * q + lane;
-      const int64_t m0 = (int64_t)tile_m * MAX_MT;
-      const int mt = (int)min((int64_t)MAX_MT, p.m_pad - m0);
+      const int64_t m0 = (int64_t)cur.tile_m * p.mt;
+      const int mt = CG == 2 ? p.mt : (int)min((int64_t)p.mt, p.m_pad - m0); // columns
+      const int64_t m_end = min(p.m, m0 + mt);
       // one thread waits for the accumulator and, for a tile shared with other CTAs, settles who stores and
       // who adds; the eight warps then act on the same answers
       if (et == 0) {
@@ -488,7 +675,7 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
         if (!whole && t == 0) {
           t = atomicAdd(p.tile_cnt + tile, 1u);
           if (t > 0) { // wait (bounded) until the first finisher's stores are visible
-            const unsigned int *flag = p.tile_cnt + (size_t)p.tiles_n * p.tiles_m + tile;
+            const unsigned int *flag = p.tile_cnt + (size_t)p.row_tiles * TM + tile;
             uint32_t spins = 0;
             unsigned int v = 0;
             do {
@@ -503,36 +690,75 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
         s_ticket = t;
       }
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+      if (et < mt) {
+        const int64_t r = m0 + row_of_column<CG>(et, mt);
+        s_ru[et] = r < p.m_pad ? p.row_unscale[r] : 0.f;
+      }
       const unsigned int ticket = s_ticket & 0x7fffffffu;
       alive = (s_ticket & 0x80000000u) == 0;
-      asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); // s_ticket may be rewritten from here on
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); // s_ticket may be rewritten from here on, s_ru is filled
       if (alive) {
         tc_fence_after();
         const uint32_t lane_addr = tmem_d + (uint32_t)(buf * 128) + ((uint32_t)(32 * q) << 16);
-        for (int c0 = 32 * half; c0 < mt; c0 += 32 * (EPI_WARPS / 4)) {
-          uint32_t v[32];
-          tmem_ld32(lane_addr + c0, v);
-          const float ru_lane = (m0 + c0 + lane < p.m_pad) ? p.row_unscale[m0 + c0 + lane] : 0.f; // the chunk's 32 row factors
+        const int es = p.y_dtype == XNQ_F32 ? 4 : 2;
+        const int64_t row_bytes = p.ldy * es, row0 = (int64_t)row_tile * TILE_N + 32 * q;
+        const int rows = (int)max((int64_t)0, min((int64_t)32, p.w.n - row0)); // of this warp's 32
+        char *const y0 = static_cast<char *>(p.y) + m0 * row_bytes + row0 * es;
+        const uint32_t ru0 = smem_u32(s_ru);
+        const int h0 = NACC == 2 ? mt : min(first_half<CG>(p.mt), mt);
+        int c = 16 * half;
+        bool first_given = NACC == 2; // the barrier of the accumulator's first half of columns
+        uint32_t v[16];
+        if (c < mt) tmem_ld16(lane_addr + c, v);
+        while (c < mt) {
+          const int next = c + 16 * (EPI_WARPS / 4), r0 = row_of_column<CG>(c, mt), cols = (int)(m_end - m0) - r0; // (cols: none of a pair's may be left)
+          const uint32_t ru = ru0 + (uint32_t)c * 4;
+          char *const yp = y0 + r0 * row_bytes;
           tmem_ld_wait();
-          const bool row_ok = row < p.w.n;
-          if (p.y_dtype == XNQ_F32) {
-            if (ticket == 0) drain_chunk<0>(v, ru_lane, p.y, p.ldy, row, m0 + c0, p.m, row_ok);
-            else drain_chunk<1>(v, ru_lane, p.y, p.ldy, row, m0 + c0, p.m, row_ok);
-          } else if (p.y_dtype == XNQ_F16) {
-            drain_chunk<2>(v, ru_lane, p.y, p.ldy, row, m0 + c0, p.m, row_ok);
-          } else {
-            drain_chunk<3>(v, ru_lane, p.y, p.ldy, row, m0 + c0, p.m, row_ok);
+          if (!first_given && next >= h0) { // this warp has read all it needs of the first half: its columns may be overwritten
+            first_given = true;
+            give_back(acc_empty);
           }
+          if (next >= mt) give_back(acc_empty + 8 * (NACC == 2 ? buf : 1));
+          if (p.vec_out) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) sts32(slot + (uint32_t)(j * 128) + ((uint32_t)(lane * 4) ^ ((j & 1) << 4)), v[j]);
+            if (next < mt) tmem_ld16(lane_addr + next, v); // arrives while the chunk is stored
+            __syncwarp();
+            if (p.y_dtype == XNQ_F32) {
+              if (ticket == 0) store_turned<STORE_F32>(slot, ru, yp, row_bytes, cols, rows, lane);
+              else store_turned<ADD_F32>(slot, ru, yp, row_bytes, cols, rows, lane);
+            } else if (p.y_dtype == XNQ_F16) {
+              store_turned<STORE_F16>(slot, ru, yp, row_bytes, cols, rows, lane);
+            } else {
+              store_turned<STORE_BF16>(slot, ru, yp, row_bytes, cols, rows, lane);
+            }
+            __syncwarp();
+          } else {
+            const bool row_ok = lane < rows;
+            if (p.y_dtype == XNQ_F32) {
+              if (ticket == 0) store_direct<STORE_F32>(v, ru, yp, row_bytes, cols, row_ok, lane);
+              else store_direct<ADD_F32>(v, ru, yp, row_bytes, cols, row_ok, lane);
+            } else if (p.y_dtype == XNQ_F16) {
+              store_direct<STORE_F16>(v, ru, yp, row_bytes, cols, row_ok, lane);
+            } else {
+              store_direct<STORE_BF16>(v, ru, yp, row_bytes, cols, row_ok, lane);
+            }
+            if (next < mt) tmem_ld16(lane_addr + next, v);
+          }
+          c = next;
         }
-        tc_fence_before();
+        // a warp that had no chunk (16 columns, the second warp of a quarter)
+        if (16 * half >= mt) {
+          if (NACC == 1) give_back(acc_empty);
+          give_back(acc_empty + 8 * (NACC == 2 ? buf : 1));
+        }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty + 8 * buf); // this warp has read its lanes: the buffer may be overwritten
       if (!whole && alive) {
         if (ticket == 0) __threadfence();
         asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
         if (ticket == 0 && et == 0) {
-          unsigned int *flag = p.tile_cnt + (size_t)p.tiles_n * p.tiles_m + tile;
+          unsigned int *flag = p.tile_cnt + (size_t)p.row_tiles * TM + tile;
           asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory");
         }
       }
@@ -543,7 +769,8 @@ __global__ void __launch_bounds__(NTHREADS_SK, 1) prefill_persistent_kernel(Pref
 
   tc_fence_before();
   __syncthreads();
-  if (warp == LOADER_WARP) tmem_dealloc(tmem_d, 512);
+  if (CG == 2) cluster_sync(); // nothing of the pair reaches for this CTA's barriers or tensor memory any more
+  if (warp == LOADER_WARP) tmem_dealloc<CG>(tmem_d, 512);
 }
 
 // ---- activation image -----------------------------------------------------------------------------------
@@ -636,18 +863,52 @@ __global__ void __launch_bounds__(256) prefill_prepare_acts(const XT *__restrict
   }
 }
 
-int g_num_sms = 0;
+int g_num_sms = 0, g_num_pairs = 0;
 
+void pair_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute (&attr)[2], unsigned ctas, int threads, size_t smem, cudaStream_t s) {
+  cfg->gridDim = dim3(ctas);
+  cfg->blockDim = dim3(threads);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = s;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 2;
+}
+// ctas: CTAs, or pairs of them
 template <typename RowT>
-int launch_persistent_fmt(const PrefillArgs &a, unsigned ctas, size_t smem, cudaStream_t s) {
-  XNQ_CUDA(launch_pdl(prefill_persistent_kernel<RowT>, dim3(ctas), dim3(NTHREADS_SK), smem, s, a));
+int launch_persistent_fmt(const PrefillArgs &a, bool pairs, unsigned ctas, size_t smem, cudaStream_t s) {
+  if (pairs) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    pair_config(&cfg, attr, 2 * ctas, nthreads<RowT>(), smem, s);
+    XNQ_CUDA(cudaLaunchKernelEx(&cfg, prefill_persistent_kernel<RowT, 2>, a));
+  } else {
+    XNQ_CUDA(launch_pdl(prefill_persistent_kernel<RowT, 1>, dim3(ctas), dim3(nthreads<RowT>()), smem, s, a));
+  }
   count_launch();
   return XNQ_OK;
 }
 
 constexpr size_t SM_SMEM = 228 * 1024, MAX_SPREAD = SM_SMEM / 2;
 static_assert(RowQ4_0::ROWB == RowQ4K::ROWB && RowQ8_0::ROWB == RowQ4K::ROWB, "the raw ring's plan assumes one slot size for these");
-constexpr size_t PREFILL_SMEM = 226 * 1024; // everything an SM offers minus the static barriers and a reserve
+constexpr size_t PREFILL_SMEM = 225 * 1024; // everything an SM offers minus the static barriers and a reserve
+
+template <typename RowT>
+int init_fmt(int *pairs) { // pairs: lowered to what the device holds at a time of this kernel (0: not set yet)
+  XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
+  XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  pair_config(&cfg, attr, 2, nthreads<RowT>(), PREFILL_SMEM, nullptr);
+  int clusters = 0;
+  XNQ_CUDA(cudaOccupancyMaxActiveClusters(&clusters, prefill_persistent_kernel<RowT, 2>, &cfg));
+  clusters = std::min(clusters, g_num_sms / 2);
+  *pairs = *pairs ? std::min(*pairs, clusters) : clusters;
+  return XNQ_OK;
+}
 
 } // namespace
 
@@ -702,35 +963,52 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   a.m = m;
   a.m_pad = m_pad;
   a.ksteps = ksteps;
+  const int row_tiles = (int)((w.n + TILE_N - 1) / TILE_N);
+  a.tiles_m = (int)((m_pad + MAX_MT - 1) / MAX_MT);
+  a.whole_tiles = y_dtype == XNQ_F32 ? 0 : 1;
+  // 16-bit results, whose tiles are whole: equal tiles of activation rows, in the MMA's steps of 16 columns (pairs: 32, 16 of each CTA).
+  // Pairs halve the activation operand's traffic, which is what bounds wide tiles: from 224 rows a tile on they are the faster or the equal
+  // ones (in a long stream of calls, Q4_K 14336 x 4096: 224 rows 41.8 against 42.6 us, 512 rows 74.5 / 77.5, 1024 rows 128 / 139; but 176 rows
+  // 39.0 / 37.0). With few tiles a pair's coarser share of the work costs more than that (Q4_K 1536 x 2048, 2000 rows, 21 k-steps a pair: 35.2 / 33.5).
+  // f32 results: tiles of 256 rows on single CTAs. Where the CTAs' shares cut a tile decides the last bits of its sums, and a last bit that
+  // differs in a decoder's first linear moves its logits by 3 % of their norm (8-bit activation codes flip).
+  const int even_mt = (int)((m_pad + a.tiles_m - 1) / a.tiles_m), pair_mt = (even_mt + 31) / 32 * 32;
+  const bool pairs = a.whole_tiles && g_num_pairs > 0 && pair_mt >= 224 && (long long)((row_tiles + 1) / 2) * a.tiles_m * ksteps >= 24ll * g_num_pairs;
+  const int cg = pairs ? 2 : 1;
+  a.mt = pairs ? pair_mt : (a.whole_tiles ? (even_mt + 15) / 16 * 16 : (int)std::min<int64_t>(MAX_MT, m_pad));
   // Shared-memory plan: B ring | raw ring. With up to eight stages a producer warp can be a whole super-step ahead of the MMAs; what is
   // left goes to the raw ring (it covers the memory latency of the weights). At 256 activation rows that is five stages and three
-  // raw slots (two for Q6_K).
+  // raw slots (two for Q6_K), for a pair eight and five (three).
   const uint32_t slot = TILE_N * (w.dtype == XNQ_Q6K ? RowQ6K::ROWB : RowQ4K::ROWB);
-  const uint32_t mt_max = (uint32_t)std::min<int64_t>(MAX_MT, m_pad);
-  a.b_stride = (mt_max * 128 + 1023) & ~1023u;
-  const size_t budget = PREFILL_SMEM - 1024; // alignment slack
-  a.nstages = (int)std::min<size_t>(MAX_STAGES, (budget - 2 * slot) / a.b_stride);
+  a.b_stride = ((uint32_t)(a.mt / cg) * 128 + 1023) & ~1023u;
+  const size_t budget = PREFILL_SMEM - 1024 - EPI_WARPS * EPI_SLOT; // 1024: alignment slack
+  for (int raw = 3; raw >= 2; raw--) { // at least so many raw slots
+    a.nstages = (int)std::min<size_t>(MAX_STAGES, (budget - raw * slot) / a.b_stride);
+    if (a.nstages >= MIN_STAGES) break;
+  }
   if (a.nstages < MIN_STAGES) return fail(XNQ_ERR_SIZE, "prefill: shared-memory plan does not fit");
   a.raw_slots = (int)std::min<size_t>(MAX_RAW_SLOTS, (budget - (size_t)a.nstages * a.b_stride) / slot);
   a.raw_off = a.nstages * a.b_stride;
-  a.acc_bufs = m_pad <= 128 ? 2 : 1;
+  a.epi_off = a.raw_off + a.raw_slots * slot;
+  const size_t yes = type_size(y_dtype), piece = 16 / yes;
+  a.vec_out = (reinterpret_cast<uintptr_t>(y) & 15) == 0 && ldy % piece == 0 && w.n % piece == 0;
+  a.acc_bufs = a.mt <= 128 ? 2 : 1;
   a.wscale = wscale;
-  const dim3 grid((unsigned)((w.n + TILE_N - 1) / TILE_N), (unsigned)((m_pad + MAX_MT - 1) / MAX_MT));
-  a.tiles_n = (int)grid.x;
-  a.tiles_m = (int)grid.y;
-  a.units = (long long)grid.x * grid.y * ksteps;
-  a.whole_tiles = y_dtype == XNQ_F32 ? 0 : 1;
+  a.row_tiles = row_tiles;
+  a.tiles_n = (row_tiles + cg - 1) / cg;
+  const long long tiles = (long long)a.tiles_n * a.tiles_m;
+  a.units = tiles * ksteps;
   a.tile_cnt = tile_cnt;
   profile_mark(s, true);
   int rc;
-  const long long tiles = (long long)grid.x * grid.y;
   const long long want = a.whole_tiles ? tiles : std::max<long long>(1, a.units / 8); // at least 8 k-steps per CTA
-  const unsigned ctas = (unsigned)std::min<long long>(g_num_sms, want);
+  const unsigned ctas = (unsigned)std::min<long long>(pairs ? g_num_pairs : g_num_sms, want);
+  a.share_q = (a.whole_tiles ? tiles : a.units) / ctas, a.share_r = (int)((a.whole_tiles ? tiles : a.units) % ctas);
   switch (w.dtype) {
-    case XNQ_Q4_0: rc = launch_persistent_fmt<RowQ4_0>(a, ctas, PREFILL_SMEM, s); break;
-    case XNQ_Q8_0: rc = launch_persistent_fmt<RowQ8_0>(a, ctas, PREFILL_SMEM, s); break;
-    case XNQ_Q4K: rc = launch_persistent_fmt<RowQ4K>(a, ctas, PREFILL_SMEM, s); break;
-    case XNQ_Q6K: rc = launch_persistent_fmt<RowQ6K>(a, ctas, PREFILL_SMEM, s); break;
+    case XNQ_Q4_0: rc = launch_persistent_fmt<RowQ4_0>(a, pairs, ctas, PREFILL_SMEM, s); break;
+    case XNQ_Q8_0: rc = launch_persistent_fmt<RowQ8_0>(a, pairs, ctas, PREFILL_SMEM, s); break;
+    case XNQ_Q4K: rc = launch_persistent_fmt<RowQ4K>(a, pairs, ctas, PREFILL_SMEM, s); break;
+    case XNQ_Q6K: rc = launch_persistent_fmt<RowQ6K>(a, pairs, ctas, PREFILL_SMEM, s); break;
     default: rc = fail(XNQ_ERR_DTYPE, "prefill: dtype %d", w.dtype);
   }
   profile_mark(s, false);
@@ -741,10 +1019,12 @@ int prefill_init(int device) {
   cudaDeviceProp prop;
   XNQ_CUDA(cudaGetDeviceProperties(&prop, device));
   g_num_sms = prop.multiProcessorCount;
-  XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowQ4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowQ8_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowQ4K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowQ6K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
+  // pairs that are resident together: the CTAs of a split tile wait for one another
+  int pairs = 0, rc = XNQ_OK;
+  if ((rc = init_fmt<RowQ4_0>(&pairs)) != XNQ_OK || (rc = init_fmt<RowQ8_0>(&pairs)) != XNQ_OK || (rc = init_fmt<RowQ4K>(&pairs)) != XNQ_OK ||
+      (rc = init_fmt<RowQ6K>(&pairs)) != XNQ_OK)
+    return rc;
+  g_num_pairs = pairs;
 #define XNQ_PREP_INIT(ACT, XT) XNQ_CUDA(cudaFuncSetAttribute(prefill_prepare_acts<ACT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SPREAD))
   XNQ_PREP_INIT(XNQ_Q8_0, float);
   XNQ_PREP_INIT(XNQ_Q8_0, __half);
