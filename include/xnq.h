@@ -162,6 +162,10 @@ size_t xnq_matmul_workspace_bytes(const xnq_weight *w, int64_t max_m);
  * Enqueues on `stream` only; allocates nothing. */
 int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y,
                  int y_dtype, int64_t ldy, void *workspace, size_t ws_bytes, void *stream);
+/* The same on float activations with a bias: n_local values of y's type in device memory, added to the f32 sums before they are
+ * rounded to y's type (Q8Linear::forward's broadcast_add, q8.rs:172-175); NULL: none. */
+int xnq_matmul_t_bias(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, const void *bias, void *y,
+                      int y_dtype, int64_t ldy, void *workspace, size_t ws_bytes, void *stream);
 
 /* A prefetch hint (no counterpart in the reference): names the weight that the calling thread will multiply
  * AFTER its next one-row (m == 1) xnq_matmul_t / xnq_matmul_t_gather call. That next call's kernel then asks for

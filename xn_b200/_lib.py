@@ -56,6 +56,7 @@ def lib() -> ctypes.CDLL:
     L.xnq_matmul_workspace_bytes.argtypes = [vp, i64]
     L.xnq_matmul_workspace_bytes.restype = sz
     L.xnq_matmul_t.argtypes = [vp, vp, ci, i64, i64, vp, ci, i64, vp, sz, vp]
+    L.xnq_matmul_t_bias.argtypes = [vp, vp, ci, i64, i64, vp, vp, ci, i64, vp, sz, vp]
     L.xnq_linear_forward_host.argtypes = [vp, vp, i64, vp, vp, vp]
     L.xnq_weight_reserve_host_staging.argtypes = [vp, i64]
     L.xnq_hint_next_weight.argtypes = [vp]

@@ -587,10 +587,16 @@ size_t xnq_matmul_workspace_bytes(const xnq_weight *w, int64_t max_m) {
 
 int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
                  size_t ws_bytes, void *stream) {
+  return xnq_matmul_t_bias(w, x, x_dtype, m, ldx, nullptr, y, y_dtype, ldy, workspace, ws_bytes, stream);
+}
+
+int xnq_matmul_t_bias(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, const void *bias, void *y, int y_dtype, int64_t ldy,
+                      void *workspace, size_t ws_bytes, void *stream) {
   clear_error();
   if (!w) return fail(XNQ_ERR_NULL, "matmul_t: weight is NULL");
   const int64_t k = w->v.k, n = w->v.n;
   if (x_dtype == XNQ_ACT_IMAGE && is_generic_dtype(w->v.dtype)) return fail(XNQ_ERR_UNSUPPORTED, "matmul_t: dtype %d takes float activations only (no activation image)", w->v.dtype);
+  if (bias && (x_dtype == XNQ_ACT_OPERAND || x_dtype == XNQ_ACT_IMAGE)) return fail(XNQ_ERR_UNSUPPORTED, "matmul_t: a bias goes with float activations");
   if (x_dtype == XNQ_ACT_OPERAND) return matmul_from_operand(w, x, m, y, y_dtype, ldy, workspace, ws_bytes, static_cast<cudaStream_t>(stream));
   if (x_dtype == XNQ_ACT_IMAGE) return matmul_from_image(w, x, m, y, y_dtype, ldy, workspace, ws_bytes, static_cast<cudaStream_t>(stream));
   int rc = check_activations("matmul_t", x, x_dtype, m, k, ldx);
@@ -600,12 +606,13 @@ int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int
   if (m == 0 || n == 0) return XNQ_OK;
   if (!y) return fail(XNQ_ERR_NULL, "matmul_t: y is NULL");
   if (!aligned(y, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "matmul_t: y is not aligned to its element size");
+  if (!aligned(bias, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "matmul_t: the bias is not aligned to its element size");
   const size_t need = least_workspace_bytes(w, m);
   if (!workspace) return fail(XNQ_ERR_NULL, "matmul_t: workspace is NULL (need %zu bytes)", need);
   if (!aligned(workspace, 256)) return fail(XNQ_ERR_ALIGN, "matmul_t: workspace must be 256-byte aligned");
   if (ws_bytes < need) return fail(XNQ_ERR_SIZE, "matmul_t: workspace has %zu bytes, m = %lld needs %zu", ws_bytes, (long long)m, need);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (is_generic_dtype(w->v.dtype)) return launch_generic_matmul(w->v, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s);
+  if (is_generic_dtype(w->v.dtype)) return launch_generic_matmul(w->v, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s, bias);
   if (g_opt_matvec_tma.load(std::memory_order_relaxed) && matvec_tma_supported(w->v, m)) {
     // decode fast path: one kernel; activations quantized in its prologue (k <= 4096, no scratch) or, for longer
     // rows, by the stand-alone quantizer into the workspace as an activation image
@@ -618,13 +625,13 @@ int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int
       xin_dtype = XNQ_ACT_IMAGE;
     }
     profile_mark(s, true);
-    rc = launch_matvec_tma(w->v, xin, xin_dtype, y, y_dtype, s);
+    rc = launch_matvec_tma(w->v, xin, xin_dtype, y, y_dtype, s, nullptr, nullptr, bias);
     profile_mark(s, false);
     return rc;
   }
   if (use_imma(w, m) && ws_bytes >= imma_workspace_bytes(w->v, m)) // exact integer dots on the tensor cores
-    return launch_imma(w->v, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s);
-  if (m > MATVEC_MAX_M) return launch_prefill(w->v, w->wscale, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s);
+    return launch_imma(w->v, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s, bias);
+  if (m > MATVEC_MAX_M) return launch_prefill(w->v, w->wscale, x, x_dtype, m, ldx, y, y_dtype, ldy, workspace, s, bias);
   bool use_mma = false;
   const int64_t pass = small_batch_pass(w, m, y_dtype, &use_mma);
   if (pass == 0) return fail(XNQ_ERR_SIZE, "matmul_t: k = %lld is too large for the shared-memory staging of one activation row", (long long)k);
@@ -637,9 +644,10 @@ int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int
     char *yp = static_cast<char *>(y) + (size_t)r0 * ldy * yes;
     if ((rc = launch_quantize_act_planar(a, xp, x_dtype, ldx, s)) != XNQ_OK) return rc;
     profile_mark(s, true);
-    rc = use_mma ? launch_matvec_mma(w->v, a, yp, y_dtype, ldy, s) : launch_matvec(w->v, a, yp, y_dtype, ldy, s);
+    rc = use_mma ? launch_matvec_mma(w->v, a, yp, y_dtype, ldy, s) : launch_matvec(w->v, a, yp, y_dtype, ldy, s, bias);
     profile_mark(s, false);
     if (rc != XNQ_OK) return rc;
+    if (use_mma && bias && (rc = launch_add_bias(yp, y_dtype, bias, rows, n, ldy, s)) != XNQ_OK) return rc;
   }
   return XNQ_OK;
 }
@@ -709,9 +717,8 @@ int xnq_linear_forward_host(xnq_weight *w, const float *x_host, int64_t m, const
     else
       (void)cudaGetLastError(); // an unregistered pointer is not an error here
   }
-  int rc = xnq_matmul_t(w, xd, XNQ_F32, m, k, y_direct ? y_direct : yd, XNQ_F32, n, ws, wsb, s);
+  const int rc = xnq_matmul_t_bias(w, xd, XNQ_F32, m, k, bias_host ? bd : nullptr, y_direct ? y_direct : yd, XNQ_F32, n, ws, wsb, s);
   if (rc != XNQ_OK) return rc;
-  if (bias_host && (rc = launch_add_bias(yd, bd, m, n, n, s)) != XNQ_OK) return rc;
   if (!y_direct) XNQ_CUDA(cudaMemcpyAsync(y_host, yd, (size_t)m * n * 4, cudaMemcpyDeviceToHost, s));
   XNQ_CUDA(cudaStreamSynchronize(s));
   return XNQ_OK;

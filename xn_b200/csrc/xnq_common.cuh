@@ -260,7 +260,7 @@ int launch_generic_dequantize(const WeightView &w, int out_dtype, void *dst, cud
 int launch_quantize_q8_1(const void *x, int x_dtype, int64_t m, int64_t k, int64_t ldx, void *dst, cudaStream_t s);
 size_t generic_workspace_bytes(const WeightView &w, int64_t m);
 int launch_generic_matmul(const WeightView &w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
-                          cudaStream_t s);
+                          cudaStream_t s, const void *bias = nullptr);
 int layout_init(int device);
 
 // xnq_quantize_act.cu
@@ -275,7 +275,7 @@ int launch_quantize_weight(int dtype, const float *x, int64_t n, int64_t k, void
 
 // xnq_matvec.cu  (m <= 16)
 constexpr int MATVEC_MAX_M = 16;
-int launch_matvec(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s);
+int launch_matvec(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias = nullptr);
 int matvec_init(int device);
 // activation rows one matvec launch can stage in shared memory for this k (0: k is too large)
 int64_t matvec_rows_per_pass(int wdtype, int64_t k);
@@ -310,7 +310,7 @@ struct NormArgs {
 };
 int comm_fill_wait(const xnq_comm *c, NormArgs *na); // xnq_comm.cu
 int launch_matvec_tma(const WeightView &w, const void *x, int x_dtype, void *y, int y_dtype, cudaStream_t s, const GatherArgs *g = nullptr,
-                      const NormArgs *norm = nullptr);
+                      const NormArgs *norm = nullptr, const void *bias = nullptr);
 bool matvec_tma_enabled(); // the "matvec_tma" library option
 int gather_cta_fence_scope(); // the "gather_cta_fence" library option
 // shared argument checks of the matmul entries (dtype, leading dimension, 16-byte row alignment)
@@ -323,7 +323,7 @@ int matvec_check_record(unsigned long long out[8]);
 bool imma_supported(const WeightView &w, int64_t m);
 size_t imma_workspace_bytes(const WeightView &w, int64_t m);
 int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
-                cudaStream_t s);
+                cudaStream_t s, const void *bias = nullptr);
 int imma_init(int device);
 int imma_status(unsigned int *bits);
 int decoder_ops_init();
@@ -346,14 +346,30 @@ constexpr int64_t IMMA_MAX_M = 64; // batches up to here take the integer tensor
 // xnq_prefill.cu  (m > 64, and Q6_K above 16 rows: tcgen05 / TMEM contraction on fp16 operands)
 size_t prefill_workspace_bytes(int64_t m, int64_t k, int64_t n);
 int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy,
-                   void *workspace, cudaStream_t s);
+                   void *workspace, cudaStream_t s, const void *bias = nullptr);
 int prefill_init(int device);
 int prefill_status(unsigned int *bits);
 
 // largest |dequantized weight| of the tensor, written to *dev_out (a float in device memory)
 int launch_max_abs(const WeightView &w, float *dev_out, cudaStream_t s);
 
-// xnq_bias.cu-ish helper in xnq_layout.cu: y[m, n] += bias[n]
-int launch_add_bias(float *y, const float *bias, int64_t m, int64_t n, int64_t ldy, cudaStream_t s);
+// A bias (n values of y's type, or null) is added to the results as an addition in y's type would (rounded to that type, added in f32, rounded
+// again), by the matmul kernels as they store (as a torch operator of its own it cost 5 to 8 us of a call). launch_add_bias does it where no
+// thread holds the finished sum (the parts of split f32 tiles meet in memory) and after the legacy-MMA kernel.
+#ifdef __CUDACC__
+__device__ __forceinline__ float bias_at(const void *bias, int y_dtype, int64_t row) {
+  if (y_dtype == XNQ_F32) return static_cast<const float *>(bias)[row];
+  if (y_dtype == XNQ_F16) return __half2float(static_cast<const __half *>(bias)[row]);
+  return __bfloat162float(static_cast<const __nv_bfloat16 *>(bias)[row]);
+}
+#endif
+#ifdef __CUDACC__
+__device__ __forceinline__ float with_bias(float v, float bias, int y_dtype) {
+  if (y_dtype == XNQ_F16) v = __half2float(__float2half_rn(v));
+  else if (y_dtype == XNQ_BF16) v = __bfloat162float(__float2bfloat16_rn(v));
+  return __fadd_rn(v, bias);
+}
+#endif
+int launch_add_bias(void *y, int y_dtype, const void *bias, int64_t m, int64_t n, int64_t ldy, cudaStream_t s); // xnq_layout.cu: y[m, n] += bias[n]
 
 } // namespace xnq

@@ -332,7 +332,7 @@ __host__ __device__ constexpr int k_splits(int pieces) { return pieces < 64 ? 1 
 
 template <int DT, int MT>
 __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *__restrict__ w, ActView act, int64_t n, int64_t row_bytes, void *y, int y_dtype,
-                                                             int64_t ldy) {
+                                                             int64_t ldy, const void *__restrict__ bias) {
   constexpr int NV = GR * MT;
   constexpr bool K256 = DT == XNQ_Q2K || DT == XNQ_Q3K || DT == XNQ_Q5K;
   using Sum = typename LaneSum<DT>::T;
@@ -430,7 +430,8 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
   const int64_t row = row0 + v % GR;
   if (lane % PER == 0 && i < rows && row < n) {
     const int64_t idx = (m0 + i) * ldy + row;
-    const float sum = (float)tot[0];
+    float sum = (float)tot[0];
+    if (bias) sum = with_bias(sum, bias_at(bias, y_dtype, row), y_dtype);
     if (y_dtype == XNQ_F32) static_cast<float *>(y)[idx] = sum;
     else if (y_dtype == XNQ_F16) static_cast<__half *>(y)[idx] = __float2half_rn(sum);
     else static_cast<__nv_bfloat16 *>(y)[idx] = __float2bfloat16_rn(sum);
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
 }
 
 template <int DT>
-int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes, void *y, int y_dtype, int64_t ldy, cudaStream_t s) {
+int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias) {
   const int rows_per_cta = TPB / 32 / k_splits((int)(w.k / 32)) * GR;
   const int mt = act.m >= 9 ? 16 : (act.m >= 5 ? 8 : (act.m >= 3 ? 4 : (int)act.m));
   const bool k256 = act.act_dtype == XNQ_Q8K;
@@ -453,11 +454,11 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
     const dim3 grid((unsigned)((w.n + rows_per_cta - 1) / rows_per_cta), (unsigned)((a.m + mt - 1) / mt));
     cudaError_t e;
     switch (mt) {
-      case 1: e = launch_pdl(generic_matmul_kernel<DT, 1>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
-      case 2: e = launch_pdl(generic_matmul_kernel<DT, 2>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
-      case 4: e = launch_pdl(generic_matmul_kernel<DT, 4>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
-      case 8: e = launch_pdl(generic_matmul_kernel<DT, 8>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
-      default: e = launch_pdl(generic_matmul_kernel<DT, 16>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy); break;
+      case 1: e = launch_pdl(generic_matmul_kernel<DT, 1>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
+      case 2: e = launch_pdl(generic_matmul_kernel<DT, 2>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
+      case 4: e = launch_pdl(generic_matmul_kernel<DT, 4>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
+      case 8: e = launch_pdl(generic_matmul_kernel<DT, 8>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
+      default: e = launch_pdl(generic_matmul_kernel<DT, 16>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
     }
     XNQ_CUDA(e);
     count_launch();
@@ -532,7 +533,7 @@ size_t generic_workspace_bytes(const WeightView &w, int64_t m) {
 
 // y[m, n] = x[m, k] . W^T for a weight held as canonical blocks; workspace: generic_workspace_bytes(w, m)
 int launch_generic_matmul(const WeightView &w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
-                          cudaStream_t s) {
+                          cudaStream_t s, const void *bias) {
   // the reference's dots of the 32-element formats refuse an odd number of blocks (k_quants.rs:322-325, 413-415, 523-526)
   if (block_size(w.dtype) == 32 && (w.k / 32) % 2) return fail(XNQ_ERR_SHAPE, "matmul_t: k = %lld is not divisible by 64 (an even number of 32-value blocks)", (long long)w.k);
   const ActView act = generic_acts(w, workspace, m);
@@ -541,12 +542,12 @@ int launch_generic_matmul(const WeightView &w, const void *x, int x_dtype, int64
   const int64_t row_bytes = w.k / block_size(w.dtype) * type_size(w.dtype);
   profile_mark(s, true);
   switch (w.dtype) {
-    case XNQ_Q4_1: rc = launch_matmul_dt<XNQ_Q4_1>(w, act, row_bytes, y, y_dtype, ldy, s); break;
-    case XNQ_Q5_0: rc = launch_matmul_dt<XNQ_Q5_0>(w, act, row_bytes, y, y_dtype, ldy, s); break;
-    case XNQ_Q5_1: rc = launch_matmul_dt<XNQ_Q5_1>(w, act, row_bytes, y, y_dtype, ldy, s); break;
-    case XNQ_Q2K: rc = launch_matmul_dt<XNQ_Q2K>(w, act, row_bytes, y, y_dtype, ldy, s); break;
-    case XNQ_Q3K: rc = launch_matmul_dt<XNQ_Q3K>(w, act, row_bytes, y, y_dtype, ldy, s); break;
-    case XNQ_Q5K: rc = launch_matmul_dt<XNQ_Q5K>(w, act, row_bytes, y, y_dtype, ldy, s); break;
+    case XNQ_Q4_1: rc = launch_matmul_dt<XNQ_Q4_1>(w, act, row_bytes, y, y_dtype, ldy, s, bias); break;
+    case XNQ_Q5_0: rc = launch_matmul_dt<XNQ_Q5_0>(w, act, row_bytes, y, y_dtype, ldy, s, bias); break;
+    case XNQ_Q5_1: rc = launch_matmul_dt<XNQ_Q5_1>(w, act, row_bytes, y, y_dtype, ldy, s, bias); break;
+    case XNQ_Q2K: rc = launch_matmul_dt<XNQ_Q2K>(w, act, row_bytes, y, y_dtype, ldy, s, bias); break;
+    case XNQ_Q3K: rc = launch_matmul_dt<XNQ_Q3K>(w, act, row_bytes, y, y_dtype, ldy, s, bias); break;
+    case XNQ_Q5K: rc = launch_matmul_dt<XNQ_Q5K>(w, act, row_bytes, y, y_dtype, ldy, s, bias); break;
     default: rc = fail(XNQ_ERR_DTYPE, "matmul_t: dtype %d", w.dtype);
   }
   profile_mark(s, false);

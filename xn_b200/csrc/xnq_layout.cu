@@ -173,11 +173,27 @@ __global__ void max_abs_kernel(WeightView w, unsigned int *out) {
   if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m)); // non-negative floats order like their bit patterns
 }
 
-__global__ void add_bias_kernel(float *__restrict__ y, const float *__restrict__ bias, int64_t m, int64_t n, int64_t ldy) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= m * n) return;
-  const int64_t r = i / n, c = i % n;
-  y[r * ldy + c] = __fadd_rn(y[r * ldy + c], bias[c]);
+// One row of y per grid row, VEC values a thread (what its 16 bytes hold, where y's rows allow that). Bound by y's traffic; it starts while the
+// matmul before it drains.
+template <typename T, int VEC>
+__global__ void __launch_bounds__(TPB) add_bias_kernel(T *__restrict__ y, const T *__restrict__ bias, int64_t m, int64_t n, int64_t ldy, int y_dtype) {
+  const int64_t c = ((int64_t)blockIdx.x * TPB + threadIdx.x) * VEC;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (c >= n) return;
+  float b[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; i++) b[i] = bias_at(bias, y_dtype, c + i);
+  for (int64_t r = blockIdx.y; r < m; r += gridDim.y) {
+    T *p = y + r * ldy + c;
+    __align__(16) T v[VEC];
+    if (VEC > 1) *reinterpret_cast<uint4 *>(v) = *reinterpret_cast<const uint4 *>(p);
+    else v[0] = p[0];
+#pragma unroll
+    for (int i = 0; i < VEC; i++) v[i] = cast_out<T>(__fadd_rn(bias_at(v, y_dtype, i), b[i]));
+    if (VEC > 1) *reinterpret_cast<uint4 *>(p) = *reinterpret_cast<const uint4 *>(v);
+    else p[0] = v[0];
+  }
 }
 
 inline unsigned grid_for(int64_t work) { return (unsigned)((work + TPB - 1) / TPB); }
@@ -246,12 +262,21 @@ int launch_max_abs(const WeightView &w, float *dev_out, cudaStream_t s) {
   return XNQ_OK;
 }
 
-int launch_add_bias(float *y, const float *bias, int64_t m, int64_t n, int64_t ldy, cudaStream_t s) {
-  if (m == 0 || n == 0) return XNQ_OK;
-  add_bias_kernel<<<grid_for(m * n), TPB, 0, s>>>(y, bias, m, n, ldy);
-  XNQ_CUDA(cudaGetLastError());
+template <typename T>
+static int add_bias_as(void *y, int y_dtype, const void *bias, int64_t m, int64_t n, int64_t ldy, cudaStream_t s) {
+  constexpr int VEC = 16 / sizeof(T);
+  const bool vec = (reinterpret_cast<uintptr_t>(y) & 15) == 0 && n % VEC == 0 && ldy % VEC == 0;
+  const dim3 grid(grid_for(vec ? n / VEC : n), (unsigned)std::min<int64_t>(m, 65535));
+  if (vec) XNQ_CUDA(launch_pdl(add_bias_kernel<T, VEC>, grid, dim3(TPB), 0, s, static_cast<T *>(y), static_cast<const T *>(bias), m, n, ldy, y_dtype));
+  else XNQ_CUDA(launch_pdl(add_bias_kernel<T, 1>, grid, dim3(TPB), 0, s, static_cast<T *>(y), static_cast<const T *>(bias), m, n, ldy, y_dtype));
   count_launch();
   return XNQ_OK;
+}
+int launch_add_bias(void *y, int y_dtype, const void *bias, int64_t m, int64_t n, int64_t ldy, cudaStream_t s) {
+  if (m == 0 || n == 0) return XNQ_OK;
+  if (y_dtype == XNQ_F32) return add_bias_as<float>(y, y_dtype, bias, m, n, ldy, s);
+  if (y_dtype == XNQ_F16) return add_bias_as<__half>(y, y_dtype, bias, m, n, ldy, s);
+  return add_bias_as<__nv_bfloat16>(y, y_dtype, bias, m, n, ldy, s);
 }
 
 int layout_init(int) {
@@ -267,7 +292,12 @@ int layout_init(int) {
   XNQ_CUDA(cudaFuncGetAttributes(&fa, dequantize_kernel<float>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, dequantize_kernel<__half>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, dequantize_kernel<__nv_bfloat16>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, add_bias_kernel));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, add_bias_kernel<float, 1>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, add_bias_kernel<float, 4>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, add_bias_kernel<__half, 1>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, add_bias_kernel<__half, 8>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, add_bias_kernel<__nv_bfloat16, 1>));
+  XNQ_CUDA(cudaFuncGetAttributes(&fa, add_bias_kernel<__nv_bfloat16, 8>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, max_abs_kernel));
   return XNQ_OK;
 }

@@ -106,13 +106,13 @@ __device__ __forceinline__ SmemAct stage_activations(unsigned char *smem, const 
 
 template <int MT, int R>
 __device__ __forceinline__ void reduce_store(float (&acc)[R][MT], int lane, int64_t row0, int64_t n, int m, void *y, int y_dtype,
-                                             int64_t ldy) {
+                                             int64_t ldy, const void *bias) {
 #pragma unroll
   for (int r = 0; r < R; r++) {
 #pragma unroll
     for (int i = 0; i < MT; i++) {
       const float v = warp_sum(acc[r][i]);
-      if (lane == 0 && i < m && row0 + r < n) store_y(y, y_dtype, (int64_t)i * ldy + row0 + r, v);
+      if (lane == 0 && i < m && row0 + r < n) store_y(y, y_dtype, (int64_t)i * ldy + row0 + r, bias ? with_bias(v, bias_at(bias, y_dtype, row0 + r), y_dtype) : v);
     }
   }
 }
@@ -121,7 +121,7 @@ __device__ __forceinline__ void reduce_store(float (&acc)[R][MT], int lane, int6
 
 // ---- Q4_0: one 16-byte chunk = one block (32 codes) ----------------------------------------------
 template <int MT, int R>
-__global__ void XNQ_MATVEC_BOUNDS matvec_q4_0(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy) {
+__global__ void XNQ_MATVEC_BOUNDS matvec_q4_0(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK, true);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -162,13 +162,13 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q4_0(WeightView w, ActView a, void *y, 
       }
     }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy);
+  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
 // ---- Q8_0: one 16-byte chunk = half a block -------------------------------------------------------
 template <int MT, int R>
-__global__ void XNQ_MATVEC_BOUNDS matvec_q8_0(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy) {
+__global__ void XNQ_MATVEC_BOUNDS matvec_q8_0(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK, false);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -201,13 +201,13 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q8_0(WeightView w, ActView a, void *y, 
       }
     }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy);
+  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
 // ---- Q4_K: 8 lanes per 144-byte super-block (header + 8 chunks of 16 nibble bytes) -----------------
 template <int MT, int R>
-__global__ void XNQ_MATVEC_BOUNDS matvec_q4k(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy) {
+__global__ void XNQ_MATVEC_BOUNDS matvec_q4k(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK_K, true);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -292,13 +292,13 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q4k(WeightView w, ActView a, void *y, i
       }
     }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy);
+  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
 // ---- Q6_K: 4 lanes per super-block; a lane takes 2 ql chunks + 1 qh chunk = 64 codes ---------------
 template <int MT, int R>
-__global__ void XNQ_MATVEC_BOUNDS matvec_q6k(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy) {
+__global__ void XNQ_MATVEC_BOUNDS matvec_q6k(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK_K, true, true);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -405,12 +405,12 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q6k(WeightView w, ActView a, void *y, i
     }
   }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy);
+  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
 template <int MT, int R>
-int launch_mt(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s) {
+int launch_mt(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias) {
   const int64_t groups = (w.n + (int64_t)WARPS * R - 1) / ((int64_t)WARPS * R);
   const int blk = (w.dtype == XNQ_Q4_0 || w.dtype == XNQ_Q8_0) ? QK : QK_K;
   const size_t image = smem_act_bytes(a.m, a.k, blk, w.dtype != XNQ_Q8_0);
@@ -420,22 +420,22 @@ int launch_mt(const WeightView &w, const ActView &a, void *y, int y_dtype, int64
   switch (w.dtype) {
     case XNQ_Q4_0: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK, true);
-      matvec_q4_0<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy);
+      matvec_q4_0<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     case XNQ_Q8_0: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK, false);
-      matvec_q8_0<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy);
+      matvec_q8_0<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     case XNQ_Q4K: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK_K, true);
-      matvec_q4k<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy);
+      matvec_q4k<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     case XNQ_Q6K: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK_K, true);
-      matvec_q6k<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy);
+      matvec_q6k<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     default: return fail(XNQ_ERR_DTYPE, "matvec: dtype %d", w.dtype);
@@ -468,14 +468,14 @@ int64_t matvec_rows_per_pass(int wdtype, int64_t k) {
   return rows;
 }
 
-int launch_matvec(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s) {
+int launch_matvec(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias) {
   if (w.n == 0 || a.m == 0) return XNQ_OK;
   if (a.m > MATVEC_MAX_M) return fail(XNQ_ERR_SHAPE, "matvec: m=%lld exceeds %d", (long long)a.m, MATVEC_MAX_M);
-  if (a.m == 1) return w.dtype == XNQ_Q4K ? launch_mt<1, 4>(w, a, y, y_dtype, ldy, s) : launch_mt<1, 2>(w, a, y, y_dtype, ldy, s);
-  if (a.m == 2) return launch_mt<2, 2>(w, a, y, y_dtype, ldy, s);
-  if (a.m <= 4) return launch_mt<4, 2>(w, a, y, y_dtype, ldy, s);
-  if (a.m <= 8) return launch_mt<8, 2>(w, a, y, y_dtype, ldy, s);
-  return launch_mt<16, 2>(w, a, y, y_dtype, ldy, s);
+  if (a.m == 1) return w.dtype == XNQ_Q4K ? launch_mt<1, 4>(w, a, y, y_dtype, ldy, s, bias) : launch_mt<1, 2>(w, a, y, y_dtype, ldy, s, bias);
+  if (a.m == 2) return launch_mt<2, 2>(w, a, y, y_dtype, ldy, s, bias);
+  if (a.m <= 4) return launch_mt<4, 2>(w, a, y, y_dtype, ldy, s, bias);
+  if (a.m <= 8) return launch_mt<8, 2>(w, a, y, y_dtype, ldy, s, bias);
+  return launch_mt<16, 2>(w, a, y, y_dtype, ldy, s, bias);
 }
 
 int matvec_init(int device) {

@@ -535,9 +535,10 @@ __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 15, %0;
 // GATHER: this rank holds rows [col0, col0 + n) of an N-sharded weight; every result goes straight
 // into the gathered output of every rank (plain stores through peer mappings), and the last CTA to
 // finish publishes this rank's next epoch to every peer.
-template <typename LaneT, int ACT, int R, bool GATHER>
+// BIAS: a variant of its own, because the step of a decoder is sensitive to the size of the function that its linears share.
+template <typename LaneT, int ACT, int R, bool GATHER, bool BIAS = false>
 __global__ void __launch_bounds__(NTHREADS, 1)
-matvec_ring_kernel(WeightView w, const void *x, int x_dtype, void *y, int y_dtype, Ring ring, GatherArgs g, NormArgs na) {
+matvec_ring_kernel(WeightView w, const void *x, int x_dtype, void *y, int y_dtype, Ring ring, GatherArgs g, NormArgs na, const void *bias) {
   extern __shared__ __align__(128) unsigned char smem[];
   const uint32_t full0 = smem_u32(smem), empty0 = full0 + 8 * MAX_STAGES; // full[MAX_STAGES], empty[MAX_STAGES]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -738,6 +739,8 @@ matvec_ring_kernel(WeightView w, const void *x, int x_dtype, void *y, int y_dtyp
     float acc[R];
 #pragma unroll
     for (int r = 0; r < R; r++) acc[r] = 0.f;
+    float add = 0.f; // the bias of the row that this lane stores, requested before the wait
+    if (BIAS && seg == 0 && lane < R && rl * R + lane < nrows - it * RPS) add = bias_at(bias, y_dtype, row_begin + (int64_t)it * RPS + rl * R + lane);
     if (alive) alive = mbar_wait_warp(full0 + 8 * s, ph);
 #ifdef XNQ_DEV_TRACE
     if (it == 0) XNQ_TRACE_POINT(4);
@@ -776,7 +779,7 @@ matvec_ring_kernel(WeightView w, const void *x, int x_dtype, void *y, int y_dtyp
     if (seg == 0 && lane < R && slot0 + lane < rows && alive) {
       const int64_t idx = row_begin + (int64_t)it * RPS + slot0 + lane;
       if (idx < 0 || idx >= w.n) record_violation(0x200, it, (unsigned long long)idx, slot0, w.n);
-      else if (!GATHER) store_out(y, y_dtype, idx, v);
+      else if (!GATHER) store_out(y, y_dtype, idx, BIAS ? with_bias(v, add, y_dtype) : v);
       else store_out(g.dst[g.rank], y_dtype, g.col0 + idx, v); // the peers get the CTA's whole run of rows in one sweep below
     }
   }
@@ -886,7 +889,8 @@ int plan_ring(const WeightView &w, Ring &r) {
 }
 
 template <typename LaneT, int ACT>
-int launch_fmt(const WeightView &w, const void *x, int x_dtype, void *y, int y_dtype, const Ring &r, cudaStream_t s, const GatherArgs *g, const NormArgs *norm) {
+int launch_fmt(const WeightView &w, const void *x, int x_dtype, void *y, int y_dtype, const Ring &r, cudaStream_t s, const GatherArgs *g, const NormArgs *norm,
+               const void *bias) {
   const NormArgs na = norm ? *norm : NormArgs{};
   const int64_t max_ctas = (w.n + r.stage_rows - 1) / r.stage_rows; // at least one stage of rows per CTA
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)g_num_sms, max_ctas));
@@ -907,11 +911,13 @@ int launch_fmt(const WeightView &w, const void *x, int x_dtype, void *y, int y_d
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (r.rows_per_warp == 2) {
-    if (g) XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 2, true>, w, x, x_dtype, y, y_dtype, rr, *g, na));
-    else XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 2, false>, w, x, x_dtype, y, y_dtype, rr, GatherArgs{}, na));
+    if (g) XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 2, true>, w, x, x_dtype, y, y_dtype, rr, *g, na, nullptr));
+    else if (bias) XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 2, false, true>, w, x, x_dtype, y, y_dtype, rr, GatherArgs{}, na, bias));
+    else XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 2, false>, w, x, x_dtype, y, y_dtype, rr, GatherArgs{}, na, nullptr));
   } else {
-    if (g) XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 1, true>, w, x, x_dtype, y, y_dtype, rr, *g, na));
-    else XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 1, false>, w, x, x_dtype, y, y_dtype, rr, GatherArgs{}, na));
+    if (g) XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 1, true>, w, x, x_dtype, y, y_dtype, rr, *g, na, nullptr));
+    else if (bias) XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 1, false, true>, w, x, x_dtype, y, y_dtype, rr, GatherArgs{}, na, bias));
+    else XNQ_CUDA(cudaLaunchKernelEx(&cfg, matvec_ring_kernel<LaneT, ACT, 1, false>, w, x, x_dtype, y, y_dtype, rr, GatherArgs{}, na, nullptr));
   }
   count_launch();
   return XNQ_OK;
@@ -923,6 +929,8 @@ int init_fmt() {
   XNQ_CUDA(cudaFuncSetAttribute(matvec_ring_kernel<LaneT, ACT, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET));
   XNQ_CUDA(cudaFuncSetAttribute(matvec_ring_kernel<LaneT, ACT, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET));
   XNQ_CUDA(cudaFuncSetAttribute(matvec_ring_kernel<LaneT, ACT, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET));
+  XNQ_CUDA(cudaFuncSetAttribute(matvec_ring_kernel<LaneT, ACT, 1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET));
+  XNQ_CUDA(cudaFuncSetAttribute(matvec_ring_kernel<LaneT, ACT, 2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BUDGET));
   return XNQ_OK;
 }
 
@@ -943,7 +951,8 @@ bool matvec_tma_wants_image(const WeightView &w) {
 
 void matvec_hint_next(const xnq_weight *w) { t_hint_next = w; }
 
-int launch_matvec_tma(const WeightView &w, const void *x, int x_dtype, void *y, int y_dtype, cudaStream_t s, const GatherArgs *g, const NormArgs *norm) {
+int launch_matvec_tma(const WeightView &w, const void *x, int x_dtype, void *y, int y_dtype, cudaStream_t s, const GatherArgs *g, const NormArgs *norm,
+                      const void *bias) {
   Ring r;
   const int ks = plan_ring(w, r);
   if (!ks) return fail(XNQ_ERR_SIZE, "matvec_ring: no ring fits k = %lld", (long long)w.k);
@@ -955,10 +964,10 @@ int launch_matvec_tma(const WeightView &w, const void *x, int x_dtype, void *y, 
     t_hint_next = nullptr;
   }
   switch (w.dtype) {
-    case XNQ_Q4_0: return launch_fmt<Q4_0Lane, XNQ_Q8_0>(w, x, x_dtype, y, y_dtype, r, s, g, norm);
-    case XNQ_Q8_0: return launch_fmt<Q8_0Lane, XNQ_Q8_0>(w, x, x_dtype, y, y_dtype, r, s, g, norm);
-    case XNQ_Q4K: return launch_fmt<Q4KLane, XNQ_Q8K>(w, x, x_dtype, y, y_dtype, r, s, g, norm);
-    case XNQ_Q6K: return launch_fmt<Q6KLane, XNQ_Q8K>(w, x, x_dtype, y, y_dtype, r, s, g, norm);
+    case XNQ_Q4_0: return launch_fmt<Q4_0Lane, XNQ_Q8_0>(w, x, x_dtype, y, y_dtype, r, s, g, norm, bias);
+    case XNQ_Q8_0: return launch_fmt<Q8_0Lane, XNQ_Q8_0>(w, x, x_dtype, y, y_dtype, r, s, g, norm, bias);
+    case XNQ_Q4K: return launch_fmt<Q4KLane, XNQ_Q8K>(w, x, x_dtype, y, y_dtype, r, s, g, norm, bias);
+    case XNQ_Q6K: return launch_fmt<Q6KLane, XNQ_Q8K>(w, x, x_dtype, y, y_dtype, r, s, g, norm, bias);
   }
   return fail(XNQ_ERR_DTYPE, "matvec_ring: dtype %d", w.dtype);
 }

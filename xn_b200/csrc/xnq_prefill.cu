@@ -218,6 +218,7 @@ struct PrefillArgs {
   const uint8_t *xh;      // activation image: [k-steps][m_pad][64] fp16, swizzled rows, k-step-permuted
   const float *row_unscale; // [m_pad]: 1 / (activation row scale * weight scale)
   void *y;
+  const void *bias;       // n values of y's type, or null
   int y_dtype;
   int64_t ldy;
   int64_t m, m_pad;
@@ -269,9 +270,16 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
 // Rows of y that start on 16 bytes: the chunk is turned over in shared memory (column j of weight row l at j * 128 + 4 l, 16-byte pieces
 // swapped in odd columns so that the 16-bit types' reads of two neighbouring pieces touch all banks) and leaves in 16-byte stores, 8 or 4
 // lanes to a row: a quarter of the store instructions. yp: this warp's first weight row in the chunk's first activation row; cols: how many
-// columns exist; rows: how many of the 32 weight rows; ru: shared address of the chunk's row factors.
+// columns exist; rows: how many of the 32 weight rows; ru: shared address of the chunk's row factors; bias: of the weight rows' bias in f32, or 0.
 template <int ST>
-__device__ __forceinline__ void store_turned(uint32_t slot, uint32_t ru, char *yp, int64_t row_bytes, int cols, int rows, int lane) {
+__device__ __forceinline__ float plus(float v, float bias) { return with_bias(v, bias, ST == STORE_F16 ? XNQ_F16 : (ST == STORE_BF16 ? XNQ_BF16 : XNQ_F32)); }
+template <int ST>
+__device__ __forceinline__ float4 add4(float4 o, uint32_t bias) {
+  const uint4 b = lds128(bias);
+  return make_float4(plus<ST>(o.x, __uint_as_float(b.x)), plus<ST>(o.y, __uint_as_float(b.y)), plus<ST>(o.z, __uint_as_float(b.z)), plus<ST>(o.w, __uint_as_float(b.w)));
+}
+template <int ST>
+__device__ __forceinline__ void store_turned(uint32_t slot, uint32_t ru, uint32_t bias, char *yp, int64_t row_bytes, int cols, int rows, int lane) {
   if (ST <= ADD_F32) {
     const int j0 = lane >> 3, piece = lane & 7;
     const uint32_t at = slot + (uint32_t)(j0 * 128 + ((piece ^ (j0 & 1)) << 4));
@@ -280,7 +288,8 @@ __device__ __forceinline__ void store_turned(uint32_t slot, uint32_t ru, char *y
     for (int i = 0; i < 4; i++) {
       const uint4 v = lds128(at + i * 512);
       const float f = __uint_as_float(lds32(ru + (uint32_t)((4 * i + j0) * 4)));
-      const float4 o = make_float4(__uint_as_float(v.x) * f, __uint_as_float(v.y) * f, __uint_as_float(v.z) * f, __uint_as_float(v.w) * f);
+      float4 o = make_float4(__uint_as_float(v.x) * f, __uint_as_float(v.y) * f, __uint_as_float(v.z) * f, __uint_as_float(v.w) * f);
+      if (ST != ADD_F32 && bias) o = add4<ST>(o, bias + piece * 16);
       if (4 * i + j0 < cols && piece * 4 < rows) {
         if (ST == STORE_F32) *reinterpret_cast<float4 *>(p) = o;
         else atomicAdd(reinterpret_cast<float4 *>(p), o);
@@ -296,8 +305,10 @@ __device__ __forceinline__ void store_turned(uint32_t slot, uint32_t ru, char *y
     for (int i = 0; i < 2; i++) {
       const uint4 a = lds128(at + i * 1024 + p0), b = lds128(at + i * 1024 + p1);
       const float f = __uint_as_float(lds32(ru + (uint32_t)((8 * i + j0) * 4)));
-      const uint4 o = make_uint4(pack16<ST>(__uint_as_float(a.x) * f, __uint_as_float(a.y) * f), pack16<ST>(__uint_as_float(a.z) * f, __uint_as_float(a.w) * f),
-                                 pack16<ST>(__uint_as_float(b.x) * f, __uint_as_float(b.y) * f), pack16<ST>(__uint_as_float(b.z) * f, __uint_as_float(b.w) * f));
+      float4 l = make_float4(__uint_as_float(a.x) * f, __uint_as_float(a.y) * f, __uint_as_float(a.z) * f, __uint_as_float(a.w) * f);
+      float4 h = make_float4(__uint_as_float(b.x) * f, __uint_as_float(b.y) * f, __uint_as_float(b.z) * f, __uint_as_float(b.w) * f);
+      if (bias) l = add4<ST>(l, bias + piece * 16), h = add4<ST>(h, bias + piece * 16 + 16);
+      const uint4 o = make_uint4(pack16<ST>(l.x, l.y), pack16<ST>(l.z, l.w), pack16<ST>(h.x, h.y), pack16<ST>(h.z, h.w));
       if (8 * i + j0 < cols && piece * 4 < rows) *reinterpret_cast<uint4 *>(p) = o;
       p += 8 * row_bytes;
     }
@@ -305,11 +316,13 @@ __device__ __forceinline__ void store_turned(uint32_t slot, uint32_t ru, char *y
 }
 // Other rows: a lane stores its weight row's values one by one, neighbouring lanes to neighbouring addresses.
 template <int ST>
-__device__ __forceinline__ void store_direct(const uint32_t (&v)[16], uint32_t ru, char *yp, int64_t row_bytes, int cols, bool row_ok, int lane) {
+__device__ __forceinline__ void store_direct(const uint32_t (&v)[16], uint32_t ru, uint32_t bias, char *yp, int64_t row_bytes, int cols, bool row_ok, int lane) {
+  const float add = ST != ADD_F32 && bias ? __uint_as_float(lds32(bias + lane * 4)) : 0.f;
   char *p = yp + lane * (ST <= ADD_F32 ? 4 : 2);
 #pragma unroll
   for (int j = 0; j < 16; j++) {
-    const float val = __uint_as_float(v[j]) * __uint_as_float(lds32(ru + (uint32_t)(j * 4)));
+    float val = __uint_as_float(v[j]) * __uint_as_float(lds32(ru + (uint32_t)(j * 4)));
+    if (ST != ADD_F32 && bias) val = plus<ST>(val, add);
     if (j < cols && row_ok) {
       if (ST == STORE_F32) *reinterpret_cast<float *>(p) = val;
       else if (ST == ADD_F32) atomicAdd(reinterpret_cast<float *>(p), val);
@@ -374,7 +387,8 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 4 + 2 * MAX_RAW_SLOTS]; // full, empty (8 each), acc_full[2], acc_empty[2], raw_full, raw_empty
-  __shared__ float s_ru[MAX_MT]; // the tile's row factors
+  __shared__ float s_ru[MAX_MT];   // the tile's row factors
+  __shared__ __align__(16) float s_bias[TILE_N]; // and the bias of its weight rows
   __shared__ uint32_t tmem_slot;
   __shared__ unsigned int s_ticket;
   const int S = p.nstages;
@@ -694,6 +708,10 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
         const int64_t r = m0 + row_of_column<CG>(et, mt);
         s_ru[et] = r < p.m_pad ? p.row_unscale[r] : 0.f;
       }
+      if (p.bias && et < TILE_N) {
+        const int64_t r = (int64_t)row_tile * TILE_N + et;
+        s_bias[et] = r < p.w.n ? bias_at(p.bias, p.y_dtype, r) : 0.f;
+      }
       const unsigned int ticket = s_ticket & 0x7fffffffu;
       alive = (s_ticket & 0x80000000u) == 0;
       asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); // s_ticket may be rewritten from here on, s_ru is filled
@@ -704,7 +722,7 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
         const int64_t row_bytes = p.ldy * es, row0 = (int64_t)row_tile * TILE_N + 32 * q;
         const int rows = (int)max((int64_t)0, min((int64_t)32, p.w.n - row0)); // of this warp's 32
         char *const y0 = static_cast<char *>(p.y) + m0 * row_bytes + row0 * es;
-        const uint32_t ru0 = smem_u32(s_ru);
+        const uint32_t ru0 = smem_u32(s_ru), bias = p.bias ? smem_u32(s_bias) + 128 * q : 0u;
         const int h0 = NACC == 2 ? mt : min(first_half<CG>(p.mt), mt);
         int c = 16 * half;
         bool first_given = NACC == 2; // the barrier of the accumulator's first half of columns
@@ -726,23 +744,23 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
             if (next < mt) tmem_ld16(lane_addr + next, v); // arrives while the chunk is stored
             __syncwarp();
             if (p.y_dtype == XNQ_F32) {
-              if (ticket == 0) store_turned<STORE_F32>(slot, ru, yp, row_bytes, cols, rows, lane);
-              else store_turned<ADD_F32>(slot, ru, yp, row_bytes, cols, rows, lane);
+              if (ticket == 0) store_turned<STORE_F32>(slot, ru, bias, yp, row_bytes, cols, rows, lane);
+              else store_turned<ADD_F32>(slot, ru, bias, yp, row_bytes, cols, rows, lane);
             } else if (p.y_dtype == XNQ_F16) {
-              store_turned<STORE_F16>(slot, ru, yp, row_bytes, cols, rows, lane);
+              store_turned<STORE_F16>(slot, ru, bias, yp, row_bytes, cols, rows, lane);
             } else {
-              store_turned<STORE_BF16>(slot, ru, yp, row_bytes, cols, rows, lane);
+              store_turned<STORE_BF16>(slot, ru, bias, yp, row_bytes, cols, rows, lane);
             }
             __syncwarp();
           } else {
             const bool row_ok = lane < rows;
             if (p.y_dtype == XNQ_F32) {
-              if (ticket == 0) store_direct<STORE_F32>(v, ru, yp, row_bytes, cols, row_ok, lane);
-              else store_direct<ADD_F32>(v, ru, yp, row_bytes, cols, row_ok, lane);
+              if (ticket == 0) store_direct<STORE_F32>(v, ru, bias, yp, row_bytes, cols, row_ok, lane);
+              else store_direct<ADD_F32>(v, ru, bias, yp, row_bytes, cols, row_ok, lane);
             } else if (p.y_dtype == XNQ_F16) {
-              store_direct<STORE_F16>(v, ru, yp, row_bytes, cols, row_ok, lane);
+              store_direct<STORE_F16>(v, ru, bias, yp, row_bytes, cols, row_ok, lane);
             } else {
-              store_direct<STORE_BF16>(v, ru, yp, row_bytes, cols, row_ok, lane);
+              store_direct<STORE_BF16>(v, ru, bias, yp, row_bytes, cols, row_ok, lane);
             }
             if (next < mt) tmem_ld16(lane_addr + next, v);
           }
@@ -924,7 +942,7 @@ size_t prefill_workspace_bytes(int64_t m, int64_t k, int64_t n) {
 }
 
 int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy,
-                   void *workspace, cudaStream_t s) {
+                   void *workspace, cudaStream_t s, const void *bias) {
   const int64_t k = w.k;
   const int64_t m_pad = (m + 15) / 16 * 16;
   const int ksteps = (int)((k + BK - 1) / BK);
@@ -958,6 +976,7 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   a.xh = xh;
   a.row_unscale = row_unscale;
   a.y = y;
+  a.bias = bias;
   a.y_dtype = y_dtype;
   a.ldy = ldy;
   a.m = m;
@@ -1003,6 +1022,9 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   int rc;
   const long long want = a.whole_tiles ? tiles : std::max<long long>(1, a.units / 8); // at least 8 k-steps per CTA
   const unsigned ctas = (unsigned)std::min<long long>(pairs ? g_num_pairs : g_num_sms, want);
+  // The bias of split tiles is added when their parts have met, so that its addition is the last one.
+  const bool bias_after = bias && !a.whole_tiles && tiles % ctas != 0;
+  if (bias_after) a.bias = nullptr;
   a.share_q = (a.whole_tiles ? tiles : a.units) / ctas, a.share_r = (int)((a.whole_tiles ? tiles : a.units) % ctas);
   switch (w.dtype) {
     case XNQ_Q4_0: rc = launch_persistent_fmt<RowQ4_0>(a, pairs, ctas, PREFILL_SMEM, s); break;
@@ -1012,7 +1034,7 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
     default: rc = fail(XNQ_ERR_DTYPE, "prefill: dtype %d", w.dtype);
   }
   profile_mark(s, false);
-  return rc;
+  return rc == XNQ_OK && bias_after ? launch_add_bias(y, y_dtype, bias, m, w.n, ldy, s) : rc;
 }
 
 int prefill_init(int device) {

@@ -19,6 +19,7 @@ from typing import Optional, Sequence
 
 import numpy as np
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from ._lib import XnqError, check
@@ -253,6 +254,10 @@ class QCudaTensor:
                                               ctypes.c_void_p(ws.data_ptr()) if ws is not None else None, ws.numel() if ws is not None else 0,
                                               _stream_ptr(self.device)))
             return out
+        return self._matmul_float(lhs, out, None)
+
+    def _matmul_float(self, lhs: torch.Tensor, out: Optional[torch.Tensor], bias: Optional[torch.Tensor]) -> torch.Tensor:
+        """``matmul_t`` of float rows; ``bias``: n contiguous values of the result's type, added by the matmul's kernel."""
         k, n, device = self.k, self.n, self.device
         shape = lhs.shape
         if shape[-1] != k:
@@ -280,12 +285,12 @@ class QCudaTensor:
         # take several times as long as the call).
         index = device.index
         if index is not None and index == torch.cuda.current_device():
-            check(_lib.lib().xnq_matmul_t(self._h, x.data_ptr(), x_dtype, m, ldx, y.data_ptr(), y_dtype, ldy, ws.data_ptr(), ws.numel(),
-                                          _raw_stream(index)))
+            check(_lib.lib().xnq_matmul_t_bias(self._h, x.data_ptr(), x_dtype, m, ldx, None if bias is None else bias.data_ptr(), y.data_ptr(), y_dtype, ldy,
+                                               ws.data_ptr(), ws.numel(), _raw_stream(index)))
         else:
             with torch.cuda.device(device):
-                check(_lib.lib().xnq_matmul_t(self._h, x.data_ptr(), x_dtype, m, ldx, y.data_ptr(), y_dtype, ldy, ws.data_ptr(), ws.numel(),
-                                              _stream_ptr(device)))
+                check(_lib.lib().xnq_matmul_t_bias(self._h, x.data_ptr(), x_dtype, m, ldx, None if bias is None else bias.data_ptr(), y.data_ptr(), y_dtype, ldy,
+                                                   ws.data_ptr(), ws.numel(), _stream_ptr(device)))
         return out
 
     def forward_host(self, x: np.ndarray, bias: Optional[np.ndarray] = None, out: Optional[np.ndarray] = None) -> np.ndarray:
@@ -311,6 +316,9 @@ class QCudaTensor:
         return y
 
 
+_PLAIN_TENSORS = (torch.Tensor, torch.nn.Parameter)
+
+
 class QCudaLinear:
     """A linear layer with GGUF-quantized weights on the device (``Q8Linear``, q8.rs:160-185)."""
 
@@ -331,8 +339,16 @@ class QCudaLinear:
     def forward(self, xs: torch.Tensor) -> torch.Tensor:
         if xs.dim() < 2:
             raise ValueError(f"input tensor has only one dimension {tuple(xs.shape)}")  # mod.rs:363-365
+        bias = self.bias
+        if bias is None:
+            return self.weight.matmul_t(xs)
+        # broadcast_add, q8.rs:172-175: by the matmul's kernel, but for a bias that torch has to see the addition of (gradients, transforms)
+        # or that the kernel cannot read (another device, strides)
+        if type(bias) in _PLAIN_TENSORS and not hasattr(xs, "act_dtype") and bias.device == self.weight.device and bias.shape == (self.weight.n,) and not (
+                bias.requires_grad and torch.is_grad_enabled()) and not torch._C._functorch.is_functorch_wrapped_tensor(bias) and forward_ad._current_level < 0:
+            return self.weight._matmul_float(xs, None, bias.to(xs.dtype).contiguous())
         out = self.weight.matmul_t(xs)
-        return out if self.bias is None else out.add_(self.bias.to(out.dtype))  # broadcast_add, q8.rs:172-175
+        return out.add_(bias.to(out.dtype))
 
     __call__ = forward
 
