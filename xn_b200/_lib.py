@@ -23,6 +23,7 @@ class XnqError(RuntimeError):
 
 
 _lib = None
+_native = None
 
 
 def lib() -> ctypes.CDLL:
@@ -100,3 +101,18 @@ def lib() -> ctypes.CDLL:
 def check(rc: int) -> None:
     if rc != XNQ_OK:
         raise XnqError(rc, lib().xnq_last_error().decode("utf-8", "replace"))
+
+
+def native():
+    """The torch side of a linear's call (``csrc/torch_linear.cpp``), bound to the library that :func:`lib` loaded."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        try:
+            from . import _xnq_torch as m
+        except ImportError as e:
+            raise RuntimeError(f"xn_b200/_xnq_torch.so cannot be loaded ({e}). Build it with `python -m xn_b200.build`.") from e
+        L = lib()
+        m.bind(ctypes.cast(L.xnq_matmul_t_bias, ctypes.c_void_p).value, ctypes.cast(L.xnq_matmul_workspace_bytes, ctypes.c_void_p).value, check)
+        _native = m
+    return _native

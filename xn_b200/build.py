@@ -1,4 +1,5 @@
-"""Builds ``libxnq.so`` (the C-ABI CUDA library) in-tree with nvcc, for sm_100a only.
+"""Builds ``libxnq.so`` (the C-ABI CUDA library) in-tree with nvcc, for sm_100a only, and ``_xnq_torch.so`` (the torch side of a linear's call)
+with the host compiler.
 
 Usage: ``python -m xn_b200.build [--force]``.  No other architecture, no PTX fallback.
 """
@@ -14,6 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libxnq.so")
+TORCH_MODULE = os.path.join(HERE, "_xnq_torch.so")
 
 EXTRA = os.environ.get("XNQ_EXTRA_NVCC_FLAGS", "").split()
 if os.environ.get("XNQ_LIB_NAME"):
@@ -50,7 +52,27 @@ def is_stale() -> bool:
     return any(os.path.getmtime(p) > t for p in sources() + _deps())
 
 
+def build_torch_module(force: bool = False) -> str:
+    src = os.path.join(CSRC, "torch_linear.cpp")
+    if not force and os.path.exists(TORCH_MODULE) and os.path.getmtime(TORCH_MODULE) >= os.path.getmtime(src):
+        return TORCH_MODULE
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = [*include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{p}" for p in inc), src, "-o", TORCH_MODULE, *(f"-L{p}" for p in library_paths()),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ltorch"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"the host compiler failed on {src}:\n{r.stdout}\n{r.stderr}")
+    return TORCH_MODULE
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
+    build_torch_module(force)
     if not force and not is_stale():
         return LIB
     os.makedirs(OBJ, exist_ok=True)

@@ -1,0 +1,155 @@
+// The torch side of a linear's call, in C++: what QCudaTensor.matmul_t and QCudaLinear.forward do for the ordinary case (float rows on the
+// weight's device, which is the current one, no `out`).
+//
+// A one-row call is bound by the host, not by its kernel (Q4_0 4096 x 4096: the kernel takes 3.3 us). In Python, with the library called through
+// ctypes, it took 10.5 us: some 25 attribute reads and comparisons, a tensor made through the dispatcher, twelve arguments converted one by one, and
+// the launch. Everything that is not ordinary returns None, and the Python code takes the call; nothing is kept from one call for the next but
+// the shared scratch, as there.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <map>
+#include <vector>
+
+namespace {
+
+using MatmulFn = int (*)(const void *, const void *, int, int64_t, int64_t, const void *, void *, int, int64_t, void *, size_t, void *);
+using WorkspaceFn = size_t (*)(const void *, int64_t);
+MatmulFn g_matmul = nullptr;         // xnq_matmul_t_bias
+WorkspaceFn g_workspace_bytes = nullptr; // xnq_matmul_workspace_bytes
+PyObject *g_check = nullptr;         // raises the error of a status
+
+struct Weight { // what a call needs of a weight; owned by the capsule that the Python weight keeps
+  const void *handle;
+  int64_t n, k;
+  c10::DeviceIndex device;
+  int64_t ws_rows; // rows asked for last and the scratch they need: a program calls a linear with the same few row counts
+  size_t ws_bytes;
+};
+constexpr const char *NAME = "xnq.weight";
+void free_weight(PyObject *capsule) { delete static_cast<Weight *>(PyCapsule_GetPointer(capsule, NAME)); }
+
+// Scratch: all weights of a device share one buffer, which only grows; outgrown ones stay alive because a captured graph may still point at
+// them. (Touched under the interpreter's lock only.)
+std::map<int, std::vector<at::Tensor>> *g_pools = nullptr;
+at::Tensor &scratch(int device, size_t bytes) {
+  std::vector<at::Tensor> &pool = (*g_pools)[device];
+  if (pool.empty() || (size_t)pool.back().numel() < bytes)
+    pool.push_back(at::empty({(int64_t)std::max<size_t>(bytes, 256)}, at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, (c10::DeviceIndex)device))));
+  return pool.back();
+}
+
+int xnq_dtype(at::ScalarType t) { // F32 0, F16 1, BF16 30: the ggml ids
+  return t == at::kFloat ? 0 : (t == at::kHalf ? 1 : (t == at::kBFloat16 ? 30 : -1));
+}
+// an ordinary dense CUDA tensor: no subclass, no wrapper of a transform
+bool plain(PyObject *o) {
+  if (!THPVariable_CheckExact(o)) return false;
+  constexpr c10::DispatchKeySet allowed({c10::DispatchKey::CUDA, c10::DispatchKey::ADInplaceOrView, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::AutocastCUDA});
+  const c10::DispatchKeySet ks = THPVariable_Unpack(o).key_set();
+  return (ks.raw_repr() & ~allowed.raw_repr()) == 0 && ks.has(c10::DispatchKey::CUDA);
+}
+bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled(); }
+
+// linear(weight capsule, x, bias or None) -> y, or None where the general code has to take the call
+PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 3) {
+    PyErr_SetString(PyExc_TypeError, "linear(weight, x, bias)");
+    return nullptr;
+  }
+  Weight *w = static_cast<Weight *>(PyCapsule_GetPointer(args[0], NAME));
+  if (!w) return nullptr;
+  if (!plain(args[1]) || modes_active()) Py_RETURN_NONE;
+  const at::Tensor &x = THPVariable_Unpack(args[1]);
+  const int xt = xnq_dtype(x.scalar_type());
+  const int64_t dims = x.dim();
+  if (xt < 0 || dims < 2 || x.size(dims - 1) != w->k || x.device().index() != w->device || c10::cuda::current_device() != w->device) Py_RETURN_NONE;
+  const int64_t m = x.numel() / w->k;
+  int64_t ldx = w->k;
+  if (!x.is_contiguous()) {
+    if (dims != 2 || x.stride(1) != 1 || (m > 1 && x.stride(0) < w->k)) Py_RETURN_NONE;
+    if (m > 1) ldx = x.stride(0);
+  }
+  const void *bias = nullptr;
+  if (args[2] != Py_None) {
+    if (!plain(args[2])) Py_RETURN_NONE;
+    const at::Tensor &b = THPVariable_Unpack(args[2]);
+    if (b.dim() != 1 || b.size(0) != w->n || b.scalar_type() != x.scalar_type() || b.device() != x.device() || !b.is_contiguous() ||
+        (b.requires_grad() && c10::GradMode::is_enabled()) || b._fw_grad(0).defined())
+      Py_RETURN_NONE;
+    bias = b.const_data_ptr();
+  }
+  c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
+  shape[dims - 1] = w->n;
+  at::Tensor y = at::Tensor(at::detail::empty_cuda(shape, x.scalar_type(), x.device(), std::nullopt));
+  if (w->ws_rows != m) w->ws_rows = m, w->ws_bytes = g_workspace_bytes(w->handle, m);
+  at::Tensor &ws = scratch(w->device, w->ws_bytes);
+  void *const wsp = ws.mutable_data_ptr(), *const yp = y.mutable_data_ptr();
+  const size_t wsb = (size_t)ws.numel();
+  const void *const xp = x.const_data_ptr();
+  void *const stream = c10::cuda::getCurrentCUDAStream(w->device).stream();
+  int rc;
+  Py_BEGIN_ALLOW_THREADS // a launch may block while the device's queue is full
+  rc = g_matmul(w->handle, xp, xt, m, ldx, bias, yp, xt, w->n, wsp, wsb, stream);
+  Py_END_ALLOW_THREADS
+  if (rc != 0) return PyObject_CallFunction(g_check, "i", rc);
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// workspace(weight capsule, rows) -> the shared scratch, large enough for that many rows
+PyObject *workspace(PyObject *, PyObject *args) {
+  HANDLE_TH_ERRORS
+  PyObject *capsule;
+  long long m;
+  if (!PyArg_ParseTuple(args, "OL", &capsule, &m)) return nullptr;
+  Weight *w = static_cast<Weight *>(PyCapsule_GetPointer(capsule, NAME));
+  if (!w) return nullptr;
+  if (w->ws_rows != m) w->ws_rows = m, w->ws_bytes = g_workspace_bytes(w->handle, m);
+  return THPVariable_Wrap(scratch(w->device, w->ws_bytes));
+  END_HANDLE_TH_ERRORS
+}
+
+// weight(handle, n, k, device index) -> capsule
+PyObject *weight(PyObject *, PyObject *args) {
+  unsigned long long handle;
+  long long n, k;
+  int device;
+  if (!PyArg_ParseTuple(args, "KLLi", &handle, &n, &k, &device)) return nullptr;
+  return PyCapsule_New(new Weight{reinterpret_cast<const void *>(handle), n, k, (c10::DeviceIndex)device, -1, 0}, NAME, free_weight);
+}
+
+// bind(xnq_matmul_t_bias, xnq_matmul_workspace_bytes, check): the library that ctypes has loaded
+PyObject *bind(PyObject *, PyObject *args) {
+  unsigned long long matmul, ws;
+  PyObject *check;
+  if (!PyArg_ParseTuple(args, "KKO", &matmul, &ws, &check)) return nullptr;
+  g_matmul = reinterpret_cast<MatmulFn>(matmul), g_workspace_bytes = reinterpret_cast<WorkspaceFn>(ws);
+  Py_INCREF(check);
+  Py_XSETREF(g_check, check);
+  if (!g_pools) g_pools = new std::map<int, std::vector<at::Tensor>>(); // never destroyed: the allocator may be gone by then
+  Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(linear)), METH_FASTCALL, "linear(weight, x, bias) -> y or None"},
+    {"workspace", workspace, METH_VARARGS, "workspace(weight, rows) -> scratch"},
+    {"weight", weight, METH_VARARGS, "weight(handle, n, k, device index) -> capsule"},
+    {"bind", bind, METH_VARARGS, "bind(matmul, workspace_bytes, check)"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_xnq_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+} // namespace
+
+PyMODINIT_FUNC PyInit__xnq_torch() { return PyModule_Create(&module_def); }

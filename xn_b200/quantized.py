@@ -36,12 +36,14 @@ except ImportError:
         return torch.cuda.current_stream(index).cuda_stream
 
 
+_linear = None   # the ordinary call of a linear, in C++ (set by the first weight)
+
+
 def _stream_ptr(device: torch.device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
 _inited: set[int] = set()
-_workspaces: dict[int, list[torch.Tensor]] = {}
 
 
 def init(device: torch.device | int | str = "cuda:0") -> None:
@@ -105,7 +107,9 @@ class QCudaTensor:
         check(_lib.lib().xnq_weight_info(self._h, dt, nt, nl, r0, k, nb))
         self._dtype = GgmlDType(dt.value)
         self.n_total, self.n, self.row0, self.k, self.device_bytes = nt.value, nl.value, r0.value, k.value, nb.value
-        self._ws_need: tuple[int, int] = (-1, 0)
+        global _linear
+        _linear = _lib.native().linear
+        self._native = _lib.native().weight(handle, self.n, self.k, device.index if device.index is not None else torch.cuda.current_device())
 
     # -- construction ---------------------------------------------------------------------------
     @classmethod
@@ -201,14 +205,7 @@ class QCudaTensor:
         """Scratch for ``m`` activation rows. All weights of a device share one buffer (the reference's device
         has a single stream, cuda_backend/mod.rs:141-167, so calls never overlap); it only ever grows, and
         outgrown buffers stay alive because a captured graph may still point at them."""
-        last = self._ws_need   # (rows, bytes) of the size asked for last: a program calls a linear with the same few row counts
-        if last[0] != m:
-            last = self._ws_need = (m, _lib.lib().xnq_matmul_workspace_bytes(self._h, m))
-        need = last[1]
-        pool = _workspaces.setdefault(self.device.index or 0, [])
-        if not pool or pool[-1].numel() < need:
-            pool.append(torch.empty(max(need, 256), dtype=torch.uint8, device=self.device))
-        return pool[-1]
+        return _lib.native().workspace(self._native, m)
 
     def hint_next(self) -> None:
         """Names this weight as the one the calling thread multiplies after its next one-row matmul: that matmul's kernel
@@ -240,6 +237,10 @@ class QCudaTensor:
 
     def matmul_t(self, lhs: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``lhs @ self^T`` with ``lhs`` of shape ``(.., k)``; the result is ``(.., n)`` (q8.rs:116-157)."""
+        if out is None:
+            y = _linear(self._native, lhs, None)   # the ordinary case; None: what follows takes the call
+            if y is not None:
+                return y
         if hasattr(lhs, "act_dtype"):   # an ActImage: activations quantized ahead of the call
             if lhs.k != self.k or lhs.act_dtype != self._dtype.vec_dot_type:
                 raise ValueError(f"cuda quantized matmul: image [{lhs.m}, {lhs.k}] {lhs.act_dtype.name} does not fit weight (k={self.k}, {self._dtype.name})")
@@ -337,6 +338,9 @@ class QCudaLinear:
         return cls(QCudaTensor.from_dense(weight, dtype), bias)
 
     def forward(self, xs: torch.Tensor) -> torch.Tensor:
+        y = _linear(self.weight._native, xs, self.bias)
+        if y is not None:
+            return y
         if xs.dim() < 2:
             raise ValueError(f"input tensor has only one dimension {tuple(xs.shape)}")  # mod.rs:363-365
         bias = self.bias
