@@ -106,3 +106,20 @@ def test_matmul_row_and_tile_edges(dt, kb):
         assert (np.abs(got.cpu().numpy().astype(np.float64) - want) <= bound).all(), (dt.name, n, k, m)
         for r in (0, m - 1):   # the sum's order depends on k alone
             assert torch.equal(w.matmul_t(xd[r:r + 1]), got[r:r + 1])
+
+
+# How many activation rows a warp takes, and whether a CTA walks over several groups of weight rows, depends on the shape (one, two and four warps
+# to a row of k; many and few groups; tiles of eight, four, two rows and one): a row's bits do not.
+@pytest.mark.parametrize("dt", FORMATS)
+@pytest.mark.parametrize("n,k,ms", [(9001, 512, (5, 8, 9, 24)), (4097, 2048, (2, 7, 17)), (3001, 4096, (3, 8, 13)), (130, 1024, (2, 3, 4, 5, 10, 40)), (1, 512, (9,))])
+def test_a_rows_bits_do_not_depend_on_the_batch(dt, n, k, ms):
+    from xn_b200 import quantized as Q
+    Q.init(DEV)
+    w = synth.make_weight(dt, n, k, seed=n)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    x = torch.from_numpy(synth.make_activation(max(ms), k, seed=k)).to(DEV)
+    alone = torch.cat([t.matmul_t(x[i:i + 1]) for i in range(max(ms))])
+    for m in ms:
+        buf = torch.full((m * n + 64,), 777.0, device=DEV)
+        t.matmul_t(x[:m], out=buf[: m * n].view(m, n))
+        assert torch.equal(buf[: m * n].view(m, n), alone[:m]) and torch.all(buf[m * n:] == 777.0), (dt.name, n, k, m)

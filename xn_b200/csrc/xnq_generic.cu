@@ -330,28 +330,37 @@ template <>
 struct LaneSum<XNQ_Q2K> { using T = double; };
 __host__ __device__ constexpr int k_splits(int pieces) { return pieces < 64 ? 1 : (pieces < 128 ? 2 : 4); }
 
+// Eight rows: the device's CTAs walk all groups of weight rows, and the first pieces of a CTA's next group are requested while it multiplies
+// the last ones of this (Q5_K 4096 x 4096, 7 rows 16.5 -> 13.9 us; Q4_1 3840 x 576, 62 rows 23.2 -> 17.7). With fewer rows more CTAs in flight do
+// better (Q5_1 26309 x 2752, one row: 21.5 us, walking 31.8), and with Q3_K's 22 words a piece (20256 x 2304, 6 rows: 41.8, walking 43.5): a
+// CTA has one group.
+__host__ __device__ constexpr bool walks(int dt, int mt) { return mt >= 8 && dt != XNQ_Q3K; }
+
 template <int DT, int MT>
 __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *__restrict__ w, ActView act, int64_t n, int64_t row_bytes, void *y, int y_dtype,
-                                                             int64_t ldy, const void *__restrict__ bias) {
+                                                             int64_t ldy, const void *__restrict__ bias, int64_t groups) {
   constexpr int NV = GR * MT;
   constexpr bool K256 = DT == XNQ_Q2K || DT == XNQ_Q3K || DT == XNQ_Q5K;
   using Sum = typename LaneSum<DT>::T;
-  __shared__ Sum red[TPB / 32][NV];
+  __shared__ Sum red[2][TPB / 32][NV];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int pieces = (int)(act.k / 32), ks_n = k_splits(pieces);
   const int ks = warp & (ks_n - 1), grp = warp / ks_n;
-  const int64_t row0 = ((int64_t)blockIdx.x * (TPB / 32 / ks_n) + grp) * GR;
   const int64_t m0 = (int64_t)blockIdx.y * MT;
   const int rows = (int)min((int64_t)MT, act.m - m0);
   const int s = lane & 7;
-  const uint8_t *wr[GR];
+  const uint8_t *wr[GR]; // the warp's rows of a group; past the last row: a duplicate, never stored
+  auto bind = [&](int64_t group) {
+    const int64_t row0 = (group * (TPB / 32 / ks_n) + grp) * GR;
 #pragma unroll
-  for (int r = 0; r < GR; r++) wr[r] = w + min(row0 + r, n - 1) * row_bytes; // past the last row: a duplicate, never stored
+    for (int r = 0; r < GR; r++) wr[r] = w + min(row0 + r, n - 1) * row_bytes;
+  };
+  bind(blockIdx.x);
   Raw<DT> raw[GR];
-  int j = ks * 32 + lane;
-  if (j < pieces) {
+  const int j0 = ks * 32 + lane;
+  if (j0 < pieces) {
 #pragma unroll
-    for (int r = 0; r < GR; r++) raw[r].load(wr[r], j);
+    for (int r = 0; r < GR; r++) raw[r].load(wr[r], j0);
   }
   pdl_wait();
   const int nblk_a = K256 ? pieces >> 3 : pieces;
@@ -359,17 +368,27 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
   const float *ad = act.d + m0 * nblk_a;              // K256
   const int16_t *ab = act.bsum + m0 * (act.k / 16);   // K256
   const __half *hd = reinterpret_cast<const __half *>(act.d) + m0 * nblk_a, *hs = reinterpret_cast<const __half *>(act.bsum) + m0 * nblk_a; // the others
+  constexpr bool WALK = walks(DT, MT);
+  int turn = 0;
+  int64_t group = blockIdx.x;
+  do {
+  const int64_t row0 = (group * (TPB / 32 / ks_n) + grp) * GR;
   float acc[NV];
 #pragma unroll
   for (int i = 0; i < NV; i++) acc[i] = 0.f;
-  while (j < pieces) {
+  for (int j = j0; j < pieces;) {
     Piece p[GR];
 #pragma unroll
     for (int r = 0; r < GR; r++) raw[r].unpack(s, p[r]);
+    // the next pieces, of these rows or of the CTA's next ones, are on their way while these are multiplied
     const int jn = j + 32 * ks_n;
-    if (MT < 16 && jn < pieces) { // the next pieces are on their way while these are multiplied (16 rows: no registers left for them)
+    if (jn < pieces) {
 #pragma unroll
       for (int r = 0; r < GR; r++) raw[r].load(wr[r], jn);
+    } else if (WALK && group + gridDim.x < groups) {
+      bind(group + gridDim.x);
+#pragma unroll
+      for (int r = 0; r < GR; r++) raw[r].load(wr[r], j0);
     }
 #pragma unroll
     for (int i = 0; i < MT; i++) {
@@ -387,10 +406,6 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
 #pragma unroll
         for (int r = 0; r < GR; r++) acc[i * GR + r] = piece_dot<DT>(p[r], lo, hi, da, as, b0, b1, acc[i * GR + r]);
       }
-    }
-    if (MT >= 16 && jn < pieces) {
-#pragma unroll
-      for (int r = 0; r < GR; r++) raw[r].load(wr[r], jn);
     }
     j = jn;
   }
@@ -420,11 +435,11 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
   }
   constexpr int PER = 32 / NV; // lanes that hold the same value
   const int v = lane / PER;
-  if (ks_n > 1) {
-    if (lane % PER == 0) red[warp][v] = tot[0];
+  if (ks_n > 1) { // (two buffers: a warp may be a group ahead of the one that adds)
+    if (lane % PER == 0) red[turn][warp][v] = tot[0];
     __syncthreads();
-    if (ks > 0) return;
-    for (int i = 1; i < ks_n; i++) tot[0] += red[warp + i][v];
+    if (ks > 0) continue;
+    for (int i = 1; i < ks_n; i++) tot[0] += red[turn][warp + i][v];
   }
   const int i = v / GR;
   const int64_t row = row0 + v % GR;
@@ -436,12 +451,20 @@ __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *_
     else if (y_dtype == XNQ_F16) static_cast<__half *>(y)[idx] = __float2half_rn(sum);
     else static_cast<__nv_bfloat16 *>(y)[idx] = __float2bfloat16_rn(sum);
   }
+  } while (WALK && (turn ^= 1, (group += gridDim.x) < groups));
 }
+
+int g_sms = 148;
 
 template <int DT>
 int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias) {
   const int rows_per_cta = TPB / 32 / k_splits((int)(w.k / 32)) * GR;
-  const int mt = act.m >= 9 ? 16 : (act.m >= 5 ? 8 : (act.m >= 3 ? 4 : (int)act.m));
+  const int64_t groups = (w.n + rows_per_cta - 1) / rows_per_cta;
+  // Activation rows a warp takes at a time: eight, as far as that leaves the device enough CTAs (Q5_K 384 x 1536, 38 rows: 10.1 us with eight,
+  // 6.4 with four; Q5_1 384 x 512, 10 rows: 5.9, 4.1, 3.3 and 2.9 with eight to one); Q2_K, whose lanes' sums are f64, four (1280 x 6656, 39 rows:
+  // 62 and 49). Sixteen, with spilled registers, were slower everywhere (Q5_K 384 x 1536: 25; Q4_1 3840 x 576, 62 rows: 32.3, eight 23.2).
+  int mt = act.m >= 5 && DT != XNQ_Q2K ? 8 : (act.m >= 3 ? 4 : (int)act.m);
+  while (mt > 1 && groups * ((act.m + mt - 1) / mt) < 200) mt /= 2;
   const bool k256 = act.act_dtype == XNQ_Q8K;
   const int64_t pass = (int64_t)mt * 65535; // grid.y is limited to 65535 tiles of activation rows
   for (int64_t r0 = 0; r0 < act.m; r0 += pass) {
@@ -451,14 +474,14 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
     a.d = reinterpret_cast<float *>(reinterpret_cast<char *>(act.d) + r0 * (k256 ? w.k / QK_K * 4 : w.k / QK * 2));
     if (act.bsum) a.bsum += r0 * (k256 ? w.k / 16 : w.k / QK);
     void *yp = static_cast<char *>(y) + (size_t)r0 * ldy * type_size(y_dtype);
-    const dim3 grid((unsigned)((w.n + rows_per_cta - 1) / rows_per_cta), (unsigned)((a.m + mt - 1) / mt));
+    const int64_t tiles = (a.m + mt - 1) / mt;
+    const dim3 grid((unsigned)(walks(DT, mt) ? std::min(groups, std::max<int64_t>(1, 2 * g_sms / tiles)) : groups), (unsigned)tiles);
     cudaError_t e;
     switch (mt) {
-      case 1: e = launch_pdl(generic_matmul_kernel<DT, 1>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
-      case 2: e = launch_pdl(generic_matmul_kernel<DT, 2>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
-      case 4: e = launch_pdl(generic_matmul_kernel<DT, 4>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
-      case 8: e = launch_pdl(generic_matmul_kernel<DT, 8>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
-      default: e = launch_pdl(generic_matmul_kernel<DT, 16>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias); break;
+      case 1: e = launch_pdl(generic_matmul_kernel<DT, 1>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias, groups); break;
+      case 2: e = launch_pdl(generic_matmul_kernel<DT, 2>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias, groups); break;
+      case 4: e = launch_pdl(generic_matmul_kernel<DT, 4>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias, groups); break;
+      default: e = launch_pdl(generic_matmul_kernel<DT, 8>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias, groups); break;
     }
     XNQ_CUDA(e);
     count_launch();
@@ -472,7 +495,6 @@ int init_matmul_dt() { // kernels are loaded before any stream capture
   XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 2>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 4>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 8>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, 16>));
   return XNQ_OK;
 }
 
@@ -554,7 +576,8 @@ int launch_generic_matmul(const WeightView &w, const void *x, int x_dtype, int64
   return rc;
 }
 
-int generic_init(int) { // kernels are loaded before any stream capture
+int generic_init(int device) { // kernels are loaded before any stream capture
+  XNQ_CUDA(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, device));
   cudaFuncAttributes fa;
   XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_dequantize_kernel<float>));
   XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_dequantize_kernel<__half>));
