@@ -375,9 +375,11 @@ int xnq_weight_upload_rows(int dtype, const void *blocks, size_t nbytes, int64_t
   w->v.sc = dtype == XNQ_Q6K ? reinterpret_cast<const int8_t *>(b + p.sc) : nullptr;
   w->v.d = dtype == XNQ_Q4K ? nullptr : reinterpret_cast<const __half *>(b + p.d);
 
-  int rc = XNQ_OK;
+  w->v.maps = &w->maps;
+  int rc = make_weight_maps(w->v, &w->maps);
   void *staging = nullptr;
   do {
+    if (rc != XNQ_OK) break;
     if ((e = cudaMemsetAsync(w->base, 0, p.total, s)) != cudaSuccess) break;
     if (nbytes == 0) break;
     if ((e = cudaMalloc(&staging, nbytes)) != cudaSuccess) break;

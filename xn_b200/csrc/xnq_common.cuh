@@ -2,6 +2,7 @@
 // error plumbing, launch entry points of each translation unit. sm_100a only.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -100,6 +101,14 @@ inline int act_dtype_for(int wdt) {
 // dstride (elements) is the scale count per row rounded up to 8, so every row of d starts 16-byte
 // aligned. Total bytes equal the GGUF bytes (plus that padding).
 // ------------------------------------------------------------------------------------------------
+// Tensor maps of a weight's code streams, boxes of 128 rows (a tile): Q4_K 144 bytes, a whole super-block, as it lies; Q4_0 and Q6_K's ql 128 bytes
+// (256 k) and Q8_0 128 bytes (128 k) with the 128-byte swizzle (16-byte chunk c of row r at c ^ (r & 7)); Q6_K's qh 64 bytes with the 64-byte
+// swizzle (c ^ ((r >> 1) & 3)). Rows and columns past the weight's ends arrive as zeros. Measured on boxes from DRAM, 148 CTAs with four in
+// flight: 19.8 bytes a cycle and SM for Q4_K's (5.6 TB/s), 4.7 cycles a row where they are in L2, whatever the row's length up to 256 bytes;
+// 16-byte cp.async copies of the same rows by 16 warps: 21 at best, and their issue took a third of the instructions of the kernels.
+struct WeightMaps {
+  CUtensorMap codes, high;
+};
 struct WeightView {
   int dtype;
   int64_t n; // rows held
@@ -109,6 +118,7 @@ struct WeightView {
   const uint8_t *qh;
   const int8_t *sc;
   const __half *d;
+  const WeightMaps *maps; // in host memory
 };
 
 // Planar device layout of quantized activations (the matmul scratch):
@@ -215,6 +225,7 @@ struct xnq_weight {
   size_t stage_dev_bytes;
   void *stage_host;
   size_t stage_host_bytes;
+  xnq::WeightMaps maps;
 };
 
 namespace xnq {
@@ -252,6 +263,7 @@ void profile_mark(cudaStream_t s, bool start);
 
 // xnq_layout.cu
 int launch_relayout(const WeightView &dst, const uint8_t *canonical_dev, cudaStream_t s);   // GGUF -> device layout
+int make_weight_maps(const WeightView &w, WeightMaps *maps);                                 // tensor maps of the device layout
 int launch_to_canonical(const WeightView &src, uint8_t *canonical_dev, cudaStream_t s);     // device layout -> GGUF
 int launch_dequantize(const WeightView &w, int out_dtype, void *dst, cudaStream_t s);
 // formats held as canonical blocks (xnq_generic.cu)

@@ -16,21 +16,20 @@
 // upper and once with the lower 16 of each 32 codes zeroed, so that one MMA yields both 16-sums; the drain multiplies the sixteen sums
 // of a super-block with the int8 scales, adds them as integers and scales once, as the CPU code does (k_quants.rs:1743-1799).
 //
-// Roles of the 19 or 27 warps of a CTA (one CTA per SM, persistent):
-//   producer (1)    one thread requests, per 256-k step, the 1-D bulk copies of the quantized activations (already in
+// Roles of the 20 or 28 warps of a CTA (one CTA per SM, persistent):
+//   activations (1) one elected thread requests, per 256-k step, the 1-D bulk copies of the quantized activations (already in
 //                   the MMA's shared-memory layout) and of their per-block metadata into rings of stages guarded by
-//                   mbarriers; when the kernel starts it also asks for the CTA's share of the weight's bytes to be
-//                   brought into L2 in long contiguous runs.
+//                   mbarriers.
+//   weights (1)     one elected thread requests a step's boxes of the weight's tensor maps (xnq_common.cuh), up to six steps ahead. Q8_0's
+//                   codes arrive as the operand image the MMA reads.
 //   converters (8)  two groups of four warps, one thread per weight row; the groups take alternate 256-k steps, so a step's
-//                   chain of waits, loads, stores and fences has two steps' time to run in. Every warp fetches the code bytes of its own 32 rows itself, several steps ahead, with
-//                   16-byte cp.async copies into a ring of warp-private slots (consecutive lanes take consecutive
-//                   16 bytes of a row, so the requests are whole sectors; nothing but the warp's own
-//                   cp.async.wait_group and __syncwarp orders them), unpacks 4-bit codes to int8 (or copies int8
-//                   codes) into the 128-byte-swizzled K-major operand image the MMA reads, and hands the rows' scale
-//                   bytes on to the drain. (Tiled TMA boxes of 128 rows x 144..256 bytes were tried first:
-//                   a box took 5000 to 7000 cycles to arrive, with or without the bytes in L2, about 17 cycles per box
-//                   row, which held the whole kernel at a third of the memory's rate. One bulk copy per row before
-//                   that: the copy engine takes some 60 ns per copy whatever its size.)
+//                   chain of waits, loads, stores and fences has two steps' time to run in. They unpack the 4- and 6-bit codes of a raw stage
+//                   to int8 into the 128-byte-swizzled K-major operand image, and hand the rows' scale bytes on to the drain.
+//                   (Until the boxes, every warp copied its 32 rows with 16-byte cp.async and the CTA asked its share of the weight into
+//                   L2 first: a third of all instructions, and 17 to 24 cycles a copy instruction whatever was done, 16 to 30 bytes a cycle.
+//                   With the boxes, in a stream of calls: Q8_0 11008 x 4096, 45 rows 30.9 -> 26.4 us, 16 rows 21.4 -> 18.8; Q4_K 28672 x 4096, 16 rows
+//                   34.0 -> 30.5; 14336 x 4096, 64 rows 36.6 -> 34.7; Q6_K 32000 x 4096, 16 rows 46.5 -> 39.3. An earlier trial of boxes had the
+//                   L2 requests queue in front of them in the same unit: 5000 cycles a box.)
 //   MMA issuers (2) one warp per half step issues its four K = 32 MMAs into accumulator buffer h and commits them;
 //   drain (16, or 8 with 16 activation rows) read the slices of a step back with tcgen05.ld, scale, and keep f32 sums in registers
 //                   across the k steps of a tile; the warps of an accumulator lane quarter split the columns.
@@ -55,15 +54,14 @@ namespace {
 constexpr int TILE_N = 128;         // weight rows per tile = UMMA M
 constexpr int MAX_NP = 64;          // activation rows per pass = UMMA N (multiple of 16)
 constexpr int CONV_WARPS = 8, DRAIN_WARPS = 16;
-constexpr int ACT_PRODUCER_WARP = 0, MMA_WARP = 1, CONV_WARP0 = 3, DRAIN_WARP0 = CONV_WARP0 + CONV_WARPS; // MMA issuers: warps 1 and 2
+constexpr int ACT_PRODUCER_WARP = 0, MMA_WARP = 1, WEIGHT_PRODUCER_WARP = 3, CONV_WARP0 = 4, DRAIN_WARP0 = CONV_WARP0 + CONV_WARPS; // MMA issuers: warps 1 and 2
 constexpr int A_STAGE_BYTES = TILE_N * 128; // one 128-k half step of int8 codes
-constexpr int SIDE_STAGES = 8, MAX_RAW_STAGES = 8, MAX_B_STAGES = 8; // side stages are small (scale bytes and records of one step): enough of them that
+constexpr int SIDE_STAGES = 8, MAX_B_STAGES = 8; // side stages are small (scale bytes and records of one step): enough of them that
                                                                    // the converters, which fill them, never wait for the drain, which frees them
 constexpr int HDR_BYTES = TILE_N * 16;      // per 256-k step: 16 bytes of scale data per weight row
 constexpr int TMEM_COLS = 512;              // all of the SM's tensor memory: 512 / (4 slices x NP) accumulator buffers, at most 8
 constexpr size_t IMMA_SMEM = 226 * 1024, MAX_SPREAD = 120 * 1024;
-constexpr uint32_t PF_CHUNK = 16384;              // bytes per L2 prefetch request
-constexpr size_t PF_MAX_BYTES = 80ull << 20;      // larger weights are not prefetched whole: they would push each other out of L2
+constexpr int SCALE_SLOTS = 2;              // a converter warp's slots of scale bytes (Q4_0, Q8_0, Q6_K): copied that many of its steps ahead
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -145,28 +143,17 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
                "r"(bytes), "r"(bar)
                : "memory");
 }
-// asks for a run of global memory to be brought into L2 (a hint; nothing waits for it)
-__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+// a box of a tensor map: x in bytes (a multiple of 16), y the first row
+__device__ __forceinline__ void tma_box(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+               : "memory");
 }
 // 16-byte asynchronous copy global -> shared, bypassing L1; src_bytes 0 writes zeros instead (the address is not read)
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// waits until at most `pending` of this thread's committed groups are still in flight
-__device__ __forceinline__ void cp_async_wait(int pending) {
-  switch (pending) {
-    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-    case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-    case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
-    case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
-  }
-}
+__device__ __forceinline__ void cp_async_wait_oldest() { asm volatile("cp.async.wait_group %0;" ::"n"(SCALE_SLOTS - 1) : "memory"); }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
@@ -258,18 +245,13 @@ struct ImmaArgs {
                         // no thread divides 64-bit numbers before its first copy
   unsigned int *tile_cnt; // [tiles] arrival tickets of split tiles, zeroed by the prepare kernel
   float *partials;        // [2 * grid][activation rows of the operand][128] partial sums of split tiles
-  // raw weight bytes: stream 0 holds the codes (Q4_K: the whole 144-byte super-blocks), stream 1 the f16 block scales of Q4_0 / Q8_0
-  const uint8_t *src[2];
-  int nstreams;
-  uint32_t row_bytes[2];  // bytes of one weight row in the stream
-  uint32_t step_bytes[2]; // bytes of one 256-k step of a row
-  uint32_t code_off;      // where the codes start inside a step of stream 0 (Q4_K: after the 16 header bytes)
-  // each CTA asks for its share of every stream (whole, contiguous rows) to be brought into L2 when it starts
-  const uint8_t *pf_base[2];
-  unsigned long long pf_bytes[2], pf_share[2]; // share: a multiple of PF_CHUNK; bytes 0: no prefetch
+  uint32_t step_x;        // bytes of one 256-k step of a row in the code stream
+  // a row's 16 scale bytes of a step (Q4_0, Q8_0: eight f16 block scales, Q6_K: sixteen int8 ones; Q4_K has them in the code stream)
+  const uint8_t *scales;
+  uint32_t scale_row_bytes;
   int raw_stages, b_stages, a_stages;
-  uint32_t raw_stage_bytes, b_stage_bytes, side_stage_bytes;
-  uint32_t a_off, b_off, raw_off0, side_off; // offsets from the 1024-aligned base of dynamic shared memory; a raw stage holds eight warp slots
+  uint32_t b_stage_bytes, side_stage_bytes;
+  uint32_t a_off, b_off, raw_off, side_off, scale_off; // offsets from the 1024-aligned base of dynamic shared memory
 };
 
 // the flattened (tile, step) space is cut into contiguous ranges: the first units_r CTAs take units_q + 1 units, the others units_q
@@ -280,51 +262,48 @@ __device__ __forceinline__ int cta_of(int u, int q, int r) {
 }
 
 // ---- converters: raw bytes of (row, 64 of the step's 256 k) -> 64 bytes of int8 codes ------------------------
-// A warp slot holds the step's code bytes of the warp's 32 rows, STEP bytes per row; the 16-byte chunk c of row r sits
-// at r * STEP + ((c ^ (r & (STEP / 16 - 1))) << 4), so that 32 lanes reading chunk c of their own rows touch all the
-// banks. row: shared address of the lane's row in the slot; key: the lane's row number in the slot; h: half step;
-// p: which 64 k of the half step.
-template <int STEP>
-__device__ __forceinline__ uint4 raw_chunk(uint32_t row, int key, int c) {
-  return lds128(row + (uint32_t)((c ^ (key & (STEP / 16 - 1))) << 4));
-}
+// A raw stage holds a step's boxes of the tile as the tensor maps lay them out (WeightMaps). raw: shared address of the stage; r: row in the
+// tile; h: half step; p: which 64 k of the half step. Lanes read chunk c of their own rows: the swizzles and Q4_K's 144-byte rows spread
+// a quarter warp's reads over all banks.
+__device__ __forceinline__ uint4 chunk128(uint32_t raw, int r, int c) { return lds128(raw + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4))); }
+__device__ __forceinline__ uint4 chunk64(uint32_t raw, int r, int c) { return lds128(raw + (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4))); }
 template <int CH>
 struct DrainBlockScaled;
 template <int CH>
 struct DrainQ4K;
-struct ConvQ8_0 { // 256 code bytes per row and step
-  static constexpr int STEP = 256, HI = 0; // HI: bytes per row and step of a second code stream
+struct ConvQ8_0 { // the boxes are the MMA's operand as they are: they go straight to the operand stages
+  static constexpr uint32_t RAW = 0;       // bytes of a raw stage
+  static constexpr int SCALES = 512;       // bytes of scale data that a converter warp copies for a step
   static constexpr bool PAIRED = false;    // two operand columns per activation row
   template <int CH>
   using Drain = DrainBlockScaled<CH>;
-  __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) out[i] = raw_chunk<STEP>(row, key, 8 * h + 4 * p + i);
-  }
 };
 __device__ __forceinline__ uint32_t nib_lo_s8(uint32_t w) { return (((w & 0x0f0f0f0fu) | 0x80808080u) - 0x08080808u) ^ 0x80808080u; } // code - 8 per byte
 __device__ __forceinline__ uint32_t nib_hi_s8(uint32_t w) { return ((((w >> 4) & 0x0f0f0f0fu) | 0x80808080u) - 0x08080808u) ^ 0x80808080u; }
 struct ConvQ4_0 { // eight blocks of 16 nibble bytes per row and step; element j < 16 low nibble of byte j, j >= 16 high nibble of byte j - 16
-  static constexpr int STEP = 128, HI = 0;
+  static constexpr uint32_t RAW = TILE_N * 128;
+  static constexpr int SCALES = 512;
   static constexpr bool PAIRED = false;
   template <int CH>
   using Drain = DrainBlockScaled<CH>;
-  __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
+  __device__ static __forceinline__ void run(uint32_t raw, int r, int h, int p, uint4 (&out)[4]) {
 #pragma unroll
     for (int bb = 0; bb < 2; bb++) {
-      const uint4 q = raw_chunk<STEP>(row, key, 4 * h + 2 * p + bb);
+      const uint4 q = chunk128(raw, r, 4 * h + 2 * p + bb);
       out[2 * bb] = make_uint4(nib_lo_s8(q.x), nib_lo_s8(q.y), nib_lo_s8(q.z), nib_lo_s8(q.w));
       out[2 * bb + 1] = make_uint4(nib_hi_s8(q.x), nib_hi_s8(q.y), nib_hi_s8(q.z), nib_hi_s8(q.w));
     }
   }
 };
-struct ConvQ4K { // 128 code bytes per row and step: four 32-byte chunks; chunk c = sub-block 2c in the low nibbles, 2c+1 in the high ones
-  static constexpr int STEP = 128, HI = 0;
+struct ConvQ4K { // super-blocks: 16 header bytes, then four 32-byte chunks; chunk c = sub-block 2c in the low nibbles, 2c+1 in the high ones
+  static constexpr uint32_t RAW = TILE_N * 144;
+  static constexpr int SCALES = 0;
   static constexpr bool PAIRED = false;
   template <int CH>
   using Drain = DrainQ4K<CH>;
-  __device__ static __forceinline__ void run(uint32_t row, int key, int h, int p, uint4 (&out)[4]) {
-    const uint4 a = raw_chunk<STEP>(row, key, 2 * (2 * h + p)), b = raw_chunk<STEP>(row, key, 2 * (2 * h + p) + 1);
+  __device__ static __forceinline__ void run(uint32_t raw, int r, int h, int p, uint4 (&out)[4]) {
+    const uint32_t at = raw + (uint32_t)(r * 144 + 16 + 32 * (2 * h + p));
+    const uint4 a = lds128(at), b = lds128(at + 16);
     out[0] = make_uint4(a.x & 0x0f0f0f0fu, a.y & 0x0f0f0f0fu, a.z & 0x0f0f0f0fu, a.w & 0x0f0f0f0fu);
     out[1] = make_uint4(b.x & 0x0f0f0f0fu, b.y & 0x0f0f0f0fu, b.z & 0x0f0f0f0fu, b.w & 0x0f0f0f0fu);
     out[2] = make_uint4((a.x >> 4) & 0x0f0f0f0fu, (a.y >> 4) & 0x0f0f0f0fu, (a.z >> 4) & 0x0f0f0f0fu, (a.w >> 4) & 0x0f0f0f0fu);
@@ -336,14 +315,15 @@ __device__ __forceinline__ uint32_t q6_code(uint32_t ql, int sh, uint32_t qh, in
   const uint32_t c = ((ql >> sh) & 0x0f0f0f0fu) | (((qh >> hsh) & 0x03030303u) << 4);
   return ((c | 0x80808080u) - 0x20202020u) ^ 0x80808080u;
 }
-struct ConvQ6K { // 128 ql bytes and 64 qh bytes per row and step. 64 k number 2 h + p: the two 32-element groups 2 p, 2 p + 1 of half h
-  static constexpr int STEP = 128, HI = 64;
+struct ConvQ6K { // 128 ql bytes, behind the rows' 64 qh bytes. 64 k number 2 h + p: the two 32-element groups 2 p, 2 p + 1 of half h
+  static constexpr uint32_t RAW = TILE_N * 192;
+  static constexpr int SCALES = 1024;      // and the 16 bytes that hold the super-block's f16 d
   static constexpr bool PAIRED = true;
-  // row / hi: the row's 128 and 64 bytes in the slot
-  __device__ static __forceinline__ void run(uint32_t row, uint32_t hi, int key, int h, int p, uint4 (&out)[4]) {
+  __device__ static __forceinline__ void run(uint32_t raw, int r, int h, int p, uint4 (&out)[4]) {
+    const uint32_t hi = raw + TILE_N * 128;
 #pragma unroll
     for (int half = 0; half < 2; half++) { // elements 0..15 and 16..31 of the groups
-      const uint4 a = raw_chunk<STEP>(row, key, 4 * h + half), b = raw_chunk<STEP>(row, key, 4 * h + 2 + half), q = raw_chunk<HI>(hi, key, 2 * h + half);
+      const uint4 a = chunk128(raw, r, 4 * h + half), b = chunk128(raw, r, 4 * h + 2 + half), q = chunk64(hi, r, 2 * h + half);
       const int sh = 4 * p, h0 = 4 * p, h1 = 4 * p + 2; // groups 0, 1: low nibbles of ql[l], ql[l + 32]; groups 2, 3: the high nibbles
       out[half] = make_uint4(q6_code(a.x, sh, q.x, h0), q6_code(a.y, sh, q.y, h0), q6_code(a.z, sh, q.z, h0), q6_code(a.w, sh, q.w, h0));
       out[2 + half] = make_uint4(q6_code(b.x, sh, q.x, h1), q6_code(b.y, sh, q.y, h1), q6_code(b.z, sh, q.z, h1), q6_code(b.w, sh, q.w, h1));
@@ -425,7 +405,7 @@ __host__ __device__ constexpr int imma_threads(int rows) { return (DRAIN_WARP0 +
 
 // BIAS: a variant of its own (one kernel with a test of p.bias took 22.1 instead of 21.4 us for Q4_K 4096 x 14336, 16 rows without a bias).
 template <typename Conv, int NP, bool BIAS>
-__global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) imma_kernel(const __grid_constant__ ImmaArgs p) {
+__global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) imma_kernel(const __grid_constant__ ImmaArgs p, const __grid_constant__ CUtensorMap codes, const __grid_constant__ CUtensorMap high) {
   constexpr int ROWS = Conv::PAIRED ? NP / 2 : NP; // activation rows of the operand; NP: its columns
   constexpr int DW = drain_warps(ROWS);
   constexpr int NPT = ROWS / (DW / 4); // rows per drain thread: the warps of an accumulator lane quarter split them
@@ -434,12 +414,12 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u; // operand stages need 1024-byte alignment
   constexpr int NBUF = TMEM_COLS / (8 * NP) > 4 ? 8 : TMEM_COLS / (8 * NP) * 2; // accumulator buffers (even: buffer parity = half step parity)
   constexpr int BUF_COLS = 4 * NP;
-  // barriers: b_full/b_empty [8], side_full/side_empty [8], a_full/mma_done [8], acc_empty [8]
-  __shared__ __align__(8) uint64_t bars[56];
+  // barriers: b_full/b_empty [8], side_full/side_empty [8], a_full/mma_done [8], acc_empty [8], raw_full/raw_empty [8]
+  __shared__ __align__(8) uint64_t bars[72];
   __shared__ uint32_t tmem_slot;
   __shared__ unsigned int s_ticket;
   const uint32_t b_full = smem_u32(bars), b_empty = b_full + 64, side_full = b_full + 128, side_empty = b_full + 192, a_full = b_full + 256,
-                 mma_done = b_full + 320, acc_empty = b_full + 384;
+                 mma_done = b_full + 320, acc_empty = b_full + 384, raw_full = b_full + 448, raw_empty = b_full + 512;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // so that the compiler knows `warp` to be uniform
   const int RS = p.raw_stages, BS = p.b_stages, AS = p.a_stages, AP = AS / 2; // AP: operand stages in whole steps
   const int NB = min(NBUF, AS); // accumulator buffers in use: a drain group waiting on mma_done must not be lapped by the MMA thread,
@@ -451,13 +431,15 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 8; s++) {
-      mbar_init(a_full + 8 * s, CONV_WARPS / 2); // the four converter warps of the step's group (one barrier per step: entries 0 .. AP - 1)
+      mbar_init(a_full + 8 * s, Conv::RAW ? CONV_WARPS / 2 : 1); // the four converter warps of the step's group (one barrier per step: entries 0 .. AP - 1); Q8_0: the boxes
       mbar_init(mma_done + 8 * s, 1);            // the half step's MMAs have read their operands and written their slices
       mbar_init(acc_empty + 8 * s, DW);
       mbar_init(side_full + 8 * s, 1 + CONV_WARPS / 2); // the producer's transaction + the four converter warps that copy the scale bytes
       mbar_init(side_empty + 8 * s, DW);
       mbar_init(b_full + 8 * s, 1);
       mbar_init(b_empty + 8 * s, 2); // both half steps' MMAs
+      mbar_init(raw_full + 8 * s, 1);
+      mbar_init(raw_empty + 8 * s, CONV_WARPS / 2);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -474,16 +456,6 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
   if (warp == ACT_PRODUCER_WARP) {
     // ---- activation producer: per 256-k step the activations' operand image and their records. The whole warp runs the loop and
     // one elected lane issues (see the MMA issuers). ----
-    // A 256-k step of a tile is 128 separate runs of 144 to 256 bytes, 2 to 4 KB apart. So that DRAM is read in long
-    // contiguous runs all the same, the weight is asked into L2 whole when the kernel starts, every CTA asking for its
-    // share of the bytes (not of the work: any CTA's copies then hit in L2, or go to DRAM when they are early).
-    if (elect_one()) {
-      for (int st = 0; st < p.nstreams; st++) {
-        const unsigned long long o0 = p.pf_share[st] * blockIdx.x, o1 = min(o0 + p.pf_share[st], p.pf_bytes[st]);
-        for (unsigned long long o = o0; o < o1; o += PF_CHUNK) bulk_prefetch_l2(p.pf_base[st] + o, (uint32_t)min((unsigned long long)PF_CHUNK, o1 - o));
-      }
-    }
-    __syncwarp();
     pdl_wait();
     bool alive = true;
     int kt = kt0, bs = 0;
@@ -535,108 +507,122 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
       if (++bs == BS) bs = 0, b_ph ^= 1u;
       if (2 * ++nb == NB) nb = 0, acc_ph ^= 1u;
     }
+  } else if (warp == WEIGHT_PRODUCER_WARP) {
+    // ---- weight producer: the boxes of a step, as many steps ahead as there are stages (weights are immutable after upload: nothing here waits
+    // for the kernel that prepares the activations). Q8_0's are the operand stages themselves, free again when both halves' MMAs are done. ----
+    const int S = Conv::RAW ? RS : AP;
+    int kt = kt0, tile = tile0, s = 0, issued = 0;
+    uint32_t lap = 0; // (i / S) & 1
+    bool alive = true;
+    for (int i = 0; i < nunits && alive; i++) {
+      if (i >= S) {
+        if (Conv::RAW) alive = mbar_wait_warp(raw_empty + 8 * s, lap ^ 1u, 1u);
+        else alive = mbar_wait_warp(mma_done + 8 * (2 * s), lap ^ 1u, 1u) && mbar_wait_warp(mma_done + 8 * (2 * s + 1), lap ^ 1u, 1u);
+      }
+      if (alive && elect_one()) {
+        const int x = kt * (int)p.step_x, y = tile * TILE_N;
+        if (Conv::RAW) {
+          const uint32_t dst = base + p.raw_off + (uint32_t)s * Conv::RAW, bar = raw_full + 8 * s;
+          mbar_expect_tx(bar, Conv::RAW);
+          tma_box(dst, &codes, x, y, bar);
+          if (Conv::PAIRED) tma_box(dst + TILE_N * 128, &high, x / 2, y, bar);
+        } else {
+          const uint32_t dst = base + p.a_off + (uint32_t)(2 * s) * A_STAGE_BYTES, bar = a_full + 8 * s;
+          mbar_expect_tx(bar, 2 * A_STAGE_BYTES);
+          tma_box(dst, &codes, x, y, bar);
+          tma_box(dst + A_STAGE_BYTES, &codes, x + 128, y, bar);
+        }
+      }
+      __syncwarp();
+      if (alive) issued = i + 1;
+      if (++kt == KT) kt = 0, tile++;
+      if (++s == S) s = 0, lap ^= 1u;
+    }
+    for (int i = max(0, issued - S); i < issued; i++) mbar_wait_warp((Conv::RAW ? raw_full : a_full) + 8 * (i % S), (i / S) & 1, 1u); // nothing in flight at exit
   } else if (warp < DRAIN_WARP0) {
     // ---- converters: group g (four warps, one thread per weight row) produces the steps i = g, g + 2, ... of this CTA: a
     // step's chain of waits, loads, stores and fences has the time of two steps' MMAs to run in ----
-    constexpr int STEP = Conv::STEP, CPR = STEP / 16, RPI = 32 / CPR; // code bytes per row and step; 16-byte chunks per row; rows per copy instruction
-    constexpr uint32_t SIDE = 32 * (STEP + Conv::HI), SLOT = SIDE + 512 + (Conv::PAIRED ? 512 : 0); // a warp's slot: its rows' code bytes, then 16 scale bytes per row (Q6_K: and 16 that hold d)
     const int cw = warp - CONV_WARP0;
-    const int r0 = (cw & 3) * 32, r = r0 + lane, g = cw >> 2;
+    const int r = (cw & 3) * 32 + lane, g = cw >> 2;
     const int sw = r & 7;
-    const int D = RS >> 1; // slots per warp: RS steps are in flight per CTA, half of them this group's
-    const uint32_t slot0 = base + p.raw_off0 + (uint32_t)(cw * D) * SLOT;
-    const int64_t n = p.w.n;
-    // the warp's own loads, D of its steps ahead: lane l copies chunk l % CPR of row q * RPI + l / CPR in instruction q
+    // the rows' scale bytes, SCALE_SLOTS of the warp's steps ahead, into slots of its own: lane l copies those of its row
+    const uint32_t slot0 = base + p.scale_off + (uint32_t)(cw * SCALE_SLOTS * Conv::SCALES);
     int l_i = g, l_tile = tile0, l_kt = kt0 + g, l_s = 0;
     while (l_kt >= KT) l_kt -= KT, l_tile++;
     auto issue = [&]() {
-      const uint32_t dst = slot0 + (uint32_t)l_s * SLOT;
-      const int c = lane % CPR;
-      const uint32_t in_row = (uint32_t)l_kt * p.step_bytes[0] + p.code_off + (uint32_t)(c * 16); // a row's bytes end at a multiple of 16
-      const uint32_t bytes = in_row + 16 <= p.row_bytes[0] ? 16u : 0u;
-#pragma unroll
-      for (int q = 0; q < CPR; q++) {
-        const int rw = q * RPI + lane / CPR;
-        const int64_t grow = (int64_t)l_tile * TILE_N + r0 + rw;
-        const bool ok = grow < n;
-        cp_async16(dst + (uint32_t)(rw * STEP + ((c ^ (rw & (CPR - 1))) << 4)), p.src[0] + (size_t)(ok ? grow : n - 1) * p.row_bytes[0] + in_row, ok ? bytes : 0u);
-      }
-      if constexpr (Conv::HI > 0) { // Q6_K: the qh bytes, then the 16 bytes that hold the super-block's f16 d
-        constexpr int HPR = Conv::HI / 16;
-#pragma unroll
-        for (int q = 0; q < HPR; q++) {
-          const int rw = q * (32 / HPR) + lane / HPR, hc = lane % HPR;
-          const int64_t grow = min((int64_t)l_tile * TILE_N + r0 + rw, n - 1);
-          cp_async16(dst + 32 * STEP + (uint32_t)(rw * Conv::HI + ((hc ^ (rw & (HPR - 1))) << 4)), p.w.qh + (size_t)grow * (p.row_bytes[0] / 2) + (uint32_t)l_kt * Conv::HI + hc * 16, 16u);
-        }
-        const int64_t grow = min((int64_t)l_tile * TILE_N + r, n - 1);
-        cp_async16(dst + SIDE + 512 + lane * 16, p.w.d + grow * p.w.dstride + (l_kt & ~7), 16u);
-      }
-      { // the rows' 16 scale bytes of the step: the head of the Q4_K super-block, eight f16 block scales, or the sixteen int8 scales of Q6_K
-        const int st = p.nstreams - 1;
-        const int64_t grow = (int64_t)l_tile * TILE_N + r;
-        const bool ok = grow < n && (uint32_t)l_kt * p.step_bytes[st] + 16 <= p.row_bytes[st];
-        cp_async16(dst + SIDE + lane * 16, p.src[st] + (size_t)(grow < n ? grow : n - 1) * p.row_bytes[st] + (ok ? (size_t)l_kt * p.step_bytes[st] : 0), ok ? 16u : 0u);
-      }
+      const int64_t grow = (int64_t)l_tile * TILE_N + r, at = min(grow, p.w.n - 1);
+      const uint32_t dst = slot0 + (uint32_t)(l_s * Conv::SCALES) + lane * 16;
+      const bool ok = grow < p.w.n && (uint32_t)l_kt * 16 + 16 <= p.scale_row_bytes;
+      cp_async16(dst, p.scales + (size_t)at * p.scale_row_bytes + (ok ? (size_t)l_kt * 16 : 0), ok ? 16u : 0u);
+      if constexpr (Conv::PAIRED) cp_async16(dst + 512, p.w.d + at * p.w.dstride + (l_kt & ~7), 16u);
       l_i += 2, l_kt += 2;
       while (l_kt >= KT) l_kt -= KT, l_tile++;
-      if (++l_s == D) l_s = 0;
+      if (++l_s == SCALE_SLOTS) l_s = 0;
     };
-    for (int u = 0; u < D; u++) { // weights are immutable after upload: nothing here waits for the kernel that prepares the activations
-      if (l_i < nunits) issue();
-      cp_async_commit();
+    if constexpr (Conv::SCALES > 0) {
+      for (int u = 0; u < SCALE_SLOTS; u++) { // weights are immutable after upload: nothing here waits for the kernel that prepares the activations
+        if (l_i < nunits) issue();
+        cp_async_commit();
+      }
     }
     bool alive = true;
-    int rs = 0, bs = g % AP;
-    uint32_t a_ph = (uint32_t)(g / AP) & 1u; // (i / AP) & 1
+    int ls = 0, rs = g % RS, bs = g % AP;
+    uint32_t a_ph = (uint32_t)(g / AP) & 1u, raw_ph = (uint32_t)(g / RS) & 1u; // (i / AP) & 1, (i / RS) & 1
     for (int i = g; i < nunits && alive; i += 2) {
       const int ss = i % SIDE_STAGES;
-      cp_async_wait(D - 1); // one group per step and lane, committed in step order: step i's has landed
-      __syncwarp();         // ... for every lane of the warp
-      const uint32_t slot = slot0 + (uint32_t)rs * SLOT;
+      const uint32_t raw = base + p.raw_off + (uint32_t)rs * Conv::RAW;
+      if constexpr (Conv::RAW > 0) alive = mbar_wait_warp(raw_full + 8 * rs, raw_ph, 2u);
+      if (alive && i >= SIDE_STAGES) alive = mbar_wait_warp(side_empty + 8 * ss, ((i / SIDE_STAGES) - 1) & 1, 2u);
+      if (!alive) break;
       { // hand the row's 16 scale bytes to the drain
-        if (i >= SIDE_STAGES) alive = mbar_wait_warp(side_empty + 8 * ss, ((i / SIDE_STAGES) - 1) & 1, 2u);
-        if (!alive) break;
-        const uint4 hv = lds128(slot + SIDE + lane * 16);
-        if constexpr (Conv::PAIRED) { // the super-block's d, widened, behind the records
-          const int sb = (kt0 + i) % KT;
-          const uint32_t dd = lds32(slot + SIDE + 512 + lane * 16 + 4 * ((sb >> 1) & 3));
-          const float d = __half2float(__ushort_as_half((unsigned short)((sb & 1) ? (dd >> 16) : (dd & 0xffffu))));
-          asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + p.side_off + ss * p.side_stage_bytes + HDR_BYTES + (uint32_t)(NP * 32) + (uint32_t)r * 4), "f"(d) : "memory");
+        uint4 hv;
+        if constexpr (Conv::SCALES > 0) {
+          cp_async_wait_oldest(); // one group per step and lane, committed in step order: step i's has landed (a lane reads what it copied itself)
+          const uint32_t slot = slot0 + (uint32_t)(ls * Conv::SCALES) + lane * 16;
+          hv = lds128(slot);
+          if constexpr (Conv::PAIRED) { // the super-block's d, widened, behind the records
+            const int sb = (kt0 + i) % KT;
+            const uint32_t dd = lds32(slot + 512 + 4 * ((sb >> 1) & 3));
+            const float d = __half2float(__ushort_as_half((unsigned short)((sb & 1) ? (dd >> 16) : (dd & 0xffffu))));
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + p.side_off + ss * p.side_stage_bytes + HDR_BYTES + (uint32_t)(NP * 32) + (uint32_t)r * 4), "f"(d) : "memory");
+          }
+        } else {
+          hv = lds128(raw + (uint32_t)(r * 144)); // the head of the Q4_K super-block
         }
         sts128(base + p.side_off + ss * p.side_stage_bytes + (uint32_t)r * 16, hv);
         __syncwarp();
         if (lane == 0) mbar_arrive(side_full + 8 * ss);
       }
-      if (i >= AP) alive = mbar_wait_warp(mma_done + 8 * (2 * bs), a_ph ^ 1u, 2u) && mbar_wait_warp(mma_done + 8 * (2 * bs + 1), a_ph ^ 1u, 2u); // both halves of the stage have been multiplied
-      if (!alive) break;
+      if constexpr (Conv::RAW > 0) {
+        if (i >= AP) alive = mbar_wait_warp(mma_done + 8 * (2 * bs), a_ph ^ 1u, 2u) && mbar_wait_warp(mma_done + 8 * (2 * bs + 1), a_ph ^ 1u, 2u); // both halves of the stage have been multiplied
+        if (!alive) break;
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        uint4 lo[4], hi[4];
-        if constexpr (Conv::HI > 0) {
-          Conv::run(slot + (uint32_t)lane * STEP, slot + 32 * STEP + (uint32_t)(lane * Conv::HI), lane, h, 0, lo);
-          Conv::run(slot + (uint32_t)lane * STEP, slot + 32 * STEP + (uint32_t)(lane * Conv::HI), lane, h, 1, hi);
-        } else {
-          Conv::run(slot + (uint32_t)lane * STEP, lane, h, 0, lo);
-          Conv::run(slot + (uint32_t)lane * STEP, lane, h, 1, hi);
+        for (int h = 0; h < 2; h++) {
+          uint4 lo[4], hi[4];
+          Conv::run(raw, r, h, 0, lo);
+          Conv::run(raw, r, h, 1, hi);
+          const uint32_t dst_row = base + p.a_off + (2 * bs + h) * A_STAGE_BYTES + (uint32_t)r * 128;
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            sts128(dst_row + (uint32_t)((c ^ sw) << 4), lo[c]);
+            sts128(dst_row + (uint32_t)(((4 + c) ^ sw) << 4), hi[c]);
+          }
         }
-        const uint32_t dst_row = base + p.a_off + (2 * bs + h) * A_STAGE_BYTES + (uint32_t)r * 128;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          sts128(dst_row + (uint32_t)((c ^ sw) << 4), lo[c]);
-          sts128(dst_row + (uint32_t)(((4 + c) ^ sw) << 4), hi[c]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the tensor core
+        __syncwarp(); // every lane has stored its row and has read all it needs of the stage
+        if (lane == 0) mbar_arrive(a_full + 8 * bs), mbar_arrive(raw_empty + 8 * rs);
+        for (int t = 0; t < 2; t++) {
+          if (++bs == AP) bs = 0, a_ph ^= 1u;
+          if (++rs == RS) rs = 0, raw_ph ^= 1u;
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> visible to the tensor core
-      __syncwarp(); // every lane has stored its row and has read all it needs of the slot
-      if (lane == 0) mbar_arrive(a_full + 8 * bs);
-      if (l_i < nunits) issue(); // into the slot just read
-      cp_async_commit();
-      if (++rs == D) rs = 0;
-      for (int t = 0; t < 2; t++)
-        if (++bs == AP) bs = 0, a_ph ^= 1u;
+      if constexpr (Conv::SCALES > 0) {
+        if (l_i < nunits) issue(); // into the slot just read
+        cp_async_commit();
+        if (++ls == SCALE_SLOTS) ls = 0;
+      }
     }
-    cp_async_wait(0); // nothing may be in flight into this CTA's shared memory when it exits
+    asm volatile("cp.async.wait_all;" ::: "memory"); // nothing may be in flight into this CTA's shared memory when it exits
   } else {
     // ---- drain: warp quarter q reads accumulator lanes 32q.. (weight rows), the warps of a quarter split the columns; every warp
     // takes both half steps of every step and keeps f32 sums in registers. (Two groups of eight warps that took one half step each had
@@ -907,11 +893,11 @@ int launch_np(const ImmaArgs &a, int NP, unsigned grid, cudaStream_t s) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if constexpr (Conv::PAIRED) { // 16 rows, 32 columns
-    XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 32, BIAS>, a));
-  } else if (NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 16, BIAS>, a));
-  else if (NP == 32) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 32, BIAS>, a));
-  else if (NP == 48) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 48, BIAS>, a));
-  else XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 64, BIAS>, a));
+    XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 32, BIAS>, a, a.w.maps->codes, a.w.maps->high));
+  } else if (NP == 16) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 16, BIAS>, a, a.w.maps->codes, a.w.maps->high));
+  else if (NP == 32) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 32, BIAS>, a, a.w.maps->codes, a.w.maps->high));
+  else if (NP == 48) XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 48, BIAS>, a, a.w.maps->codes, a.w.maps->high));
+  else XNQ_CUDA(cudaLaunchKernelEx(&cfg, imma_kernel<Conv, 64, BIAS>, a, a.w.maps->codes, a.w.maps->high));
   count_launch();
   return XNQ_OK;
 }
@@ -1024,59 +1010,43 @@ int launch_imma(const WeightView &w, const void *x, int x_dtype, int64_t m, int6
     a.units_q = a.units / pl.grid, a.units_r = a.units % pl.grid;
     a.tile_cnt = cnt;
     a.partials = partials;
-    int rc, step_code; // step_code: code bytes per row and step
+    int rc;
+    uint32_t raw = 0, scales = 0; // bytes of a raw stage and of a converter warp's scale slot
     switch (w.dtype) {
-      case XNQ_Q4K:
-        a.nstreams = 1, a.src[0] = w.qs, a.row_bytes[0] = (uint32_t)(k / QK_K * 144), a.step_bytes[0] = 144, a.code_off = 16, step_code = ConvQ4K::STEP;
-        break;
+      case XNQ_Q4K: a.step_x = 144, raw = ConvQ4K::RAW; break;
       case XNQ_Q8_0:
-        a.nstreams = 2, a.src[0] = w.qs, a.row_bytes[0] = (uint32_t)k, a.step_bytes[0] = 256, a.code_off = 0, step_code = ConvQ8_0::STEP;
-        a.src[1] = reinterpret_cast<const uint8_t *>(w.d), a.row_bytes[1] = (uint32_t)(w.dstride * 2), a.step_bytes[1] = 16;
+        a.step_x = 256, scales = ConvQ8_0::SCALES, a.scales = reinterpret_cast<const uint8_t *>(w.d), a.scale_row_bytes = (uint32_t)(w.dstride * 2);
         break;
       case XNQ_Q4_0:
-        a.nstreams = 2, a.src[0] = w.qs, a.row_bytes[0] = (uint32_t)(k / 2), a.step_bytes[0] = 128, a.code_off = 0, step_code = ConvQ4_0::STEP;
-        a.src[1] = reinterpret_cast<const uint8_t *>(w.d), a.row_bytes[1] = (uint32_t)(w.dstride * 2), a.step_bytes[1] = 16;
+        a.step_x = 128, raw = ConvQ4_0::RAW, scales = ConvQ4_0::SCALES, a.scales = reinterpret_cast<const uint8_t *>(w.d), a.scale_row_bytes = (uint32_t)(w.dstride * 2);
         break;
-      case XNQ_Q6K: // a row's qh bytes are half its ql bytes; they and d are addressed from the weight itself
-        a.nstreams = 2, a.src[0] = w.qs, a.row_bytes[0] = (uint32_t)(k / 2), a.step_bytes[0] = 128, a.code_off = 0, step_code = ConvQ6K::STEP + ConvQ6K::HI + 16;
-        a.src[1] = reinterpret_cast<const uint8_t *>(w.sc), a.row_bytes[1] = (uint32_t)(k / 16), a.step_bytes[1] = 16;
+      case XNQ_Q6K:
+        a.step_x = 128, raw = ConvQ6K::RAW, scales = ConvQ6K::SCALES, a.scales = reinterpret_cast<const uint8_t *>(w.sc), a.scale_row_bytes = (uint32_t)(k / 16);
         break;
       default: return fail(XNQ_ERR_DTYPE, "imma: dtype %d", w.dtype);
     }
-    {
-      size_t total = 0;
-      for (int st = 0; st < a.nstreams; st++) total += (size_t)a.row_bytes[st] * (size_t)w.n;
-      for (int st = 0; st < 2; st++) {
-        a.pf_base[st] = st < a.nstreams ? a.src[st] : nullptr;
-        a.pf_bytes[st] = st < a.nstreams && total <= PF_MAX_BYTES ? (unsigned long long)(((size_t)a.row_bytes[st] * (size_t)w.n) & ~(size_t)15) : 0ull;
-        a.pf_share[st] = ((a.pf_bytes[st] / (unsigned)pl.grid) + PF_CHUNK - 1) & ~(unsigned long long)(PF_CHUNK - 1);
-      }
-    }
-    a.raw_stage_bytes = (uint32_t)(CONV_WARPS / 2) * (32u * (uint32_t)step_code + 512u); // a step in flight: four warp slots of the rows' code bytes and 16 scale bytes per row
     a.b_stage_bytes = (uint32_t)pl.NP * 256;
     a.side_stage_bytes = HDR_BYTES + (uint32_t)pl.NP * 32 + (paired ? TILE_N * 4 : 0);
-    // Shared-memory plan: A stages (half steps of operand image) | B stages (activations, whole steps) | side stages | raw stages (weights,
-    // whole steps). The first plan of six half steps with the most raw stages that leaves five B stages (NP > 32: two), else of four with two.
-    // The activations' copies queue behind the weights': with three B stages a step takes a third of their latency of 4500 cycles, which is
-    // why NP = 16 has eight. As it comes out, (A, raw, B): Q4_0 / Q4_K (6, 4, 8), (4, 6, 3), (6, 4, 2), (4, 4, 3) for NP = 16, 32, 48, 64;
-    // Q8_0 (4, 2, 8), (4, 2, 8), (4, 2, 5), (4, 2, 3); Q6_K (4, 4, 2). Fewer raw and more B stages were not measured where B is 2 or 3.
+    // Shared-memory plan: A stages (half steps of operand image) | raw stages (weights, whole steps) | B stages (activations, whole steps) | side
+    // stages | scale slots. The first plan that leaves as many B stages as it names. Four raw stages in flight (Q8_0: operand stages) are what
+    // DRAM's latency takes at its rate; an even number of them, so that a stage is always read by the same group of converter warps (a group
+    // that took turns with the other could test a barrier two phases behind, which reads as complete).
+    struct { int as, rs, bs; } static constexpr direct[] = {{8, 2, 3}, {6, 2, 2}, {4, 2, 2}}, converted[] = {{6, 4, 5}, {4, 6, 4}, {4, 4, 2}, {4, 2, 2}};
     const size_t budget = IMMA_SMEM - 1024; // 1024: alignment slack of the base
     a.a_stages = 0;
-    static constexpr int as_order[3] = {6, 4, 8};
-    for (int ai = 0; ai < 3 && !a.a_stages; ai++) {
-      const int as = as_order[ai];
-      for (int rs = MAX_RAW_STAGES; rs >= 2 && !a.a_stages; rs -= 2) { // even: the two converter groups own half of the slots each
-        const size_t fixed = (size_t)as * A_STAGE_BYTES + (size_t)SIDE_STAGES * a.side_stage_bytes + (size_t)rs * a.raw_stage_bytes + 256;
-        if (rs < 4 && as != 4) continue;
-        const int bs = fixed >= budget ? 0 : (int)std::min<size_t>(MAX_B_STAGES, (budget - fixed) / a.b_stage_bytes);
-        if (bs >= (pl.NP <= 32 && ai == 0 ? 5 : 2)) a.a_stages = as, a.raw_stages = rs, a.b_stages = bs;
-      }
-    }
+    auto try_plan = [&](int as, int rs, int least) {
+      const size_t fixed = (size_t)as * A_STAGE_BYTES + (size_t)rs * raw + (size_t)SIDE_STAGES * a.side_stage_bytes + (size_t)CONV_WARPS * SCALE_SLOTS * scales;
+      const int bs = fixed >= budget ? 0 : (int)std::min<size_t>(MAX_B_STAGES, (budget - fixed) / a.b_stage_bytes);
+      if (!a.a_stages && bs >= least) a.a_stages = as, a.raw_stages = rs, a.b_stages = bs;
+    };
+    if (raw) for (const auto &c : converted) try_plan(c.as, c.rs, c.bs);
+    else for (const auto &c : direct) try_plan(c.as, c.rs, c.bs);
     if (!a.a_stages) return fail(XNQ_ERR_SIZE, "imma: shared-memory plan does not fit");
     a.a_off = 0;
-    a.b_off = (uint32_t)a.a_stages * A_STAGE_BYTES;
+    a.raw_off = (uint32_t)a.a_stages * A_STAGE_BYTES;
+    a.b_off = a.raw_off + (uint32_t)a.raw_stages * raw;
     a.side_off = a.b_off + a.b_stages * a.b_stage_bytes;
-    a.raw_off0 = (a.side_off + SIDE_STAGES * a.side_stage_bytes + 127) & ~127u;
+    a.scale_off = a.side_off + SIDE_STAGES * a.side_stage_bytes;
     profile_mark(s, true);
     if (w.dtype == XNQ_Q4K) rc = launch_fmt<ConvQ4K>(a, pl.NP, (unsigned)pl.grid, s);
     else if (w.dtype == XNQ_Q8_0) rc = launch_fmt<ConvQ8_0>(a, pl.NP, (unsigned)pl.grid, s);

@@ -200,6 +200,34 @@ inline unsigned grid_for(int64_t work) { return (unsigned)((work + TPB - 1) / TP
 
 } // namespace
 
+int make_weight_maps(const WeightView &v, WeightMaps *maps) {
+  if (v.n == 0) return XNQ_OK;
+  using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  XNQ_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found));
+  if (found != cudaDriverEntryPointSuccess || !fn) return fail(XNQ_ERR_UNSUPPORTED, "weight_upload: the driver has no cuTensorMapEncodeTiled");
+  auto encode = [&](CUtensorMap *m, const void *base, int64_t row_bytes, uint32_t box_bytes, CUtensorMapSwizzle swizzle) {
+    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)v.n}, strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {box_bytes, 128}, steps[2] = {1, 1};
+    const CUresult r = reinterpret_cast<Encode>(fn)(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? XNQ_OK : fail(XNQ_ERR_CUDA, "weight_upload: cuTensorMapEncodeTiled of [%lld, %lld bytes] failed: %d", (long long)v.n, (long long)row_bytes, (int)r);
+  };
+  int rc = XNQ_OK;
+  switch (v.dtype) {
+    case XNQ_Q4K: rc = encode(&maps->codes, v.qs, v.k / QK_K * 144, 144, CU_TENSOR_MAP_SWIZZLE_NONE); break;
+    case XNQ_Q4_0: rc = encode(&maps->codes, v.qs, v.k / 2, 128, CU_TENSOR_MAP_SWIZZLE_128B); break;
+    case XNQ_Q8_0: rc = encode(&maps->codes, v.qs, v.k, 128, CU_TENSOR_MAP_SWIZZLE_128B); break;
+    case XNQ_Q6K:
+      rc = encode(&maps->codes, v.qs, v.k / 2, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+      if (rc == XNQ_OK) rc = encode(&maps->high, v.qh, v.k / 4, 64, CU_TENSOR_MAP_SWIZZLE_64B);
+      break;
+  }
+  return rc;
+}
+
 int launch_relayout(const WeightView &v, const uint8_t *src, cudaStream_t s) {
   if (v.n == 0) return XNQ_OK;
   const int64_t nblk = v.k / block_size(v.dtype);
