@@ -252,3 +252,20 @@ def test_fp16_kernel_unequal_tiles(Q, O, dt, n, m):
     t.matmul_t(xd, out=wide[:, :n]) if n % 8 else t.matmul_t(xd, out=wide.view(-1)[: m * n].view(m, n))
     half = wide[:, :n] if n % 8 else wide.view(-1)[: m * n].view(m, n)
     assert torch.allclose(half.float(), got, rtol=2.0 ** -7, atol=1e-4 * float(got.abs().max()))
+
+
+# a tile's last super-step lacks some of its k-steps (k-steps not a multiple of two or four) while the CTA goes on to further tiles: the warps of a missing
+# step must neither miss nor outrun a phase of a stage's barrier. f32 (ranges of k-steps) and 16-bit (whole tiles)
+@pytest.mark.parametrize("dt", [d for d in WEIGHT_TYPES if d.block_size == 32])
+@pytest.mark.parametrize("n,k,m", [(640, 8384, 814), (640, 8288, 814), (1029, 8512, 700), (300, 1312, 814), (4096, 352, 257), (2048, 96, 1100), (520, 4128, 100)])
+def test_fp16_kernel_missing_steps(Q, O, dt, n, k, m):
+    w = synth.make_weight(dt, n, k, seed=m + n)
+    x = synth.make_activation(m, k, seed=m)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    xd = torch.from_numpy(x).to(DEV)
+    want = O.matmul(int(dt), x, w, n, threads=O.hw_threads())
+    for _ in range(20):
+        got = t.matmul_t(xd)
+    _check(got.cpu().numpy(), want, f"{dt.name} m={m} n={n} k={k}")
+    half = t.matmul_t(xd, out=torch.empty(m, n, dtype=torch.bfloat16, device=DEV))
+    assert torch.allclose(half.float(), got, rtol=2.0 ** -7, atol=1e-4 * float(got.abs().max()))

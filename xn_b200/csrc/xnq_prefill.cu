@@ -451,16 +451,20 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
     int base_i = -start.kt; // the CTA's step number of the current tile's first k-step
     int at = 0, s = 0;      // s = at % S, lap: parity of at / S, of the last step this warp looked at
     uint32_t lap = 0;
+    const bool lockstep = KT % KPS != 0 && KPS + KT % KPS > S;
     bool alive = true;
     for (int left = nsuper; left > 0; left--) {
       if (alive) alive = mbar_wait_uniform(raw_full + 8 * slot, raw_lap, 1u);
-      // A warp whose k-step a tile's last super-step does not have waits for the last one that it has, so that two of its waits are never
-      // more than KPS steps apart (see MIN_STAGES).
-      const int kt = c_s * KPS + kk, i = base_i + min(kt, KT - 1);
-      if (alive && i >= 0 && i < nsteps) {
+      // A warp waits for a stage only on behalf of a step that it fills: that step's MMAs, and so the stage's next phase, wait for this warp in
+      // turn, while a barrier that runs on without it may be two phases ahead by the time it looks, which a parity cannot tell from none. Where
+      // a warp's k-step is missing from a tile's last super-step, two of its waits may then be more than S steps apart, and the second could
+      // take an older phase for its own: there (Q4_0 with k not a multiple of 256) the four warps of a row group keep step with one another.
+      if (lockstep) asm volatile("bar.sync %0, 128;" ::"r"(2 + rg) : "memory");
+      const int kt = c_s * KPS + kk, i = base_i + kt;
+      if (alive && kt < KT && i >= 0 && i < nsteps) {
         for (s += i - at, at = i; s >= S; lap ^= 1u) s -= S;
         if (i >= S) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 1u);
-        if (alive && kt < KT) {
+        if (alive) {
           tc_fence_after();
           const uint32_t row = raw + (uint32_t)slot * SLOT;
           const uint32_t dst = tmem_d + ((uint32_t)(32 * rg) << 16) + (uint32_t)(A_COL0 + s * A_COLS);
