@@ -50,13 +50,8 @@ constexpr int TILE_N = 128;        // weight rows per CTA = UMMA M
 constexpr int MAX_MT = 256;        // activation rows per CTA = UMMA N
 constexpr int PRODUCER_WARPS = 16; // four row groups of 32 rows x four warps
 constexpr int EPI_WARPS = 8;       // two per accumulator lane quarter, which take turns in its chunks of 16 columns
-constexpr int LOADER_WARP = PRODUCER_WARPS, MMA_WARP = LOADER_WARP + 1, EPI_WARP0 = MMA_WARP + 1, COPY_WARP0 = EPI_WARP0 + EPI_WARPS;
-// Copy warps: two, and four for Q8_0, whose k-steps are twice the bytes (11008 x 4096, 160 rows: 31.9 us with four, 32.9 with two; Q4_K 14336 x
-// 4096, 100 rows: 30.7 and 30.0: the other formats' conversion wants the registers).
-template <typename RowT>
-__host__ __device__ constexpr int copy_warps() { return RowT::KPS == 2 ? 4 : 2; }
-template <typename RowT>
-__host__ __device__ constexpr int nthreads() { return (COPY_WARP0 + copy_warps<RowT>()) * 32; }
+constexpr int LOADER_WARP = PRODUCER_WARPS, MMA_WARP = LOADER_WARP + 1, EPI_WARP0 = MMA_WARP + 1, COPY_WARP = EPI_WARP0 + EPI_WARPS;
+constexpr int NTHREADS = (COPY_WARP + 1) * 32;
 constexpr uint32_t EPI_SLOT = 16 * 32 * 4; // a drain warp's chunk: 16 columns of 32 weight rows, f32
 constexpr uint32_t WAIT_LIMIT = 1u << 26; // polls of a flag in global memory
 constexpr int A_COLS = BK / 2;     // tensor-memory columns of a stage's weights
@@ -348,12 +343,14 @@ __device__ __forceinline__ void store_direct(const uint32_t (&v)[16], uint32_t r
 // segment overlaps the MMAs of the next. Wider ones have one, whose halves of columns the drain gives back one by one: the first
 // MMAs of the next segment go to the half that is free.
 // Roles: 16 producer warps, one activation-loader warp (one bulk copy per stage), one MMA-issuing warp, eight drain
-// warps, two or four warps that copy raw weights. Stage counters run on across segments.
+// warps, one warp that requests raw weights. Stage counters run on across segments.
 // Producers: the four warps of a row group (32 weight rows) convert a k-step each of a super-step (or a half of one), so the k-steps of a
 // super-step are converted side by side and a warp's chain of waits, loads, arithmetic and stores has a super-step's MMAs to run in.
-// Measured together, the turned drain, the halves and the copy warps (long stream of calls, f32 results): Q4_0 4096 x 4096, 200 rows 32.5 ->
-// 25.6 us; Q4_K 4096 x 4096, 300 rows 31.9 -> 29.3; Q6_K 8192 x 4096, 700 rows 69.5 -> 65.6; Q8_0 11008 x 4096, 512 rows 66.5 -> 64.0; Q4_K 14336 x
-// 4096, 512 rows 73.1 -> 72.2 (power limit).
+// Measured, start of each -> with it (long stream of calls): the turned drain, the halves and copies by warps of their own, Q4_0 4096 x 4096, 200 rows
+// 32.5 -> 25.6 us, Q4_K 4096 x 4096, 300 rows 31.9 -> 29.3; weights in boxes of tensor maps and a short turn of the activation loader, Q4_K 28672 x
+// 4096, 2000 rows (bf16 results) 443 -> 417, Q8_0 11008 x 4096, 512 rows 64.0 -> 61.4, Q6_K 128256 x 4096, 32 rows 155 -> 138, Q4_K 14336 x 4096, 512
+// rows 72.2 -> 70.3. What bounds it now: wide tiles the power limit and the tensor core's 512 cycles a k-step, Q6_K and narrow tiles the
+// instructions of the conversion (Q6_K 540 cycles a k-step, of which its four warps' instructions are 85 %).
 struct Cursor { // position in the flattened (tile, k-step) space; tile = tile_n * tiles_m + tile_m
   int tile_n, tile_m, kt;
   __device__ __forceinline__ void advance(int steps, int KT, int tiles_m) {
@@ -383,7 +380,7 @@ __device__ __forceinline__ int row_of_column(int c, int n) {
 }
 
 template <typename RowT, int CG>
-__global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel(PrefillArgs p) {
+__global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const __grid_constant__ PrefillArgs p, const __grid_constant__ CUtensorMap codes, const __grid_constant__ CUtensorMap high) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   __shared__ __align__(8) uint64_t bars[2 * MAX_STAGES + 4 + 2 * MAX_RAW_SLOTS]; // full, empty (8 each), acc_full[2], acc_empty[2], raw_full, raw_empty
@@ -415,7 +412,7 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
       mbar_init(empty + 8 * s, 1);
     }
     for (int r = 0; r < p.raw_slots; r++) {
-      mbar_init(raw_full + 8 * r, copy_warps<RowT>() * 32);
+      mbar_init(raw_full + 8 * r, 1 + (RowT::SCALES ? 32 : 0)); // the boxes, and the lanes that copy scale data
       mbar_init(raw_empty + 8 * r, PRODUCER_WARPS);
     }
     for (int b = 0; b < 2; b++) {
@@ -436,7 +433,8 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
   const uint32_t tmem_d = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
   constexpr int KPS = RowT::KPS;
-  constexpr uint32_t SLOT = TILE_N * RowT::ROWB;
+  constexpr uint32_t SLOT = RowT::SLOT;
+  static_assert(ROWS == TILE_N && SLOT % 1024 == 0, "swizzled boxes start on 1024 bytes");
   const int SPT = (KT + KPS - 1) / KPS; // super-steps per tile
   const int R = p.raw_slots;
   const int last_kt = nsteps - 1 + start.kt; // counted from the start of the first tile
@@ -445,7 +443,8 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
     // ---- producers: the four warps of a row group convert a k-step of a super-step each (KPS 2: half of one) ----
     const int rg = warp & 3, kg = warp >> 2;
     const int kk = kg % KPS, hf = kg / KPS; // this warp's k-step of a super-step; which half of it (KPS = 2)
-    const uint32_t raw = smem_base + p.raw_off + (uint32_t)((rg * 32 + lane) * RowT::ROWB);
+    const uint32_t raw = smem_base + p.raw_off;
+    const int r = rg * 32 + lane; // row in the tile
     int c_s = start.kt / KPS, slot = 0;
     uint32_t raw_lap = 0;
     int base_i = -start.kt; // the CTA's step number of the current tile's first k-step
@@ -466,14 +465,14 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
         if (i >= S) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 1u);
         if (alive) {
           tc_fence_after();
-          const uint32_t row = raw + (uint32_t)slot * SLOT;
+          const uint32_t at_slot = raw + (uint32_t)slot * SLOT;
           const uint32_t dst = tmem_d + ((uint32_t)(32 * rg) << 16) + (uint32_t)(A_COL0 + s * A_COLS);
-          const typename RowT::Head head = RowT::head(row, c_s, kk, p.wscale);
+          const typename RowT::Head head = RowT::head(at_slot, r, c_s, kk, p.wscale);
 #pragma unroll
           for (int h = 0; h < KPS / 2; h++) {
             const int half = KPS == 2 ? hf : h;
             uint32_t o[16];
-            RowT::half(head, row, kk, half, o); // a lane past the weight's last row repeats that row and is not stored
+            RowT::half(head, at_slot, r, kk, half, o); // (what a lane past the weight's last row makes is not stored)
             tmem_st16(dst + 16 * half, o);
           }
           tmem_st_wait();
@@ -490,75 +489,75 @@ __global__ void __launch_bounds__(nthreads<RowT>(), 1) prefill_persistent_kernel
         base_i += KT;
       }
     }
-  } else if (warp >= COPY_WARP0) {
-    // ---- copies of the raw weights: two or four warps fetch the 128 rows of a super-step, up to R super-steps ahead. (While the producers fetched
-    // their rows themselves, issuing those copies took 1100 to 1700 of a super-step's 3000 cycles: they queue behind the loader's bulk
-    // copies.) A thread has one of the ITEMS pieces of every RPP-th row, so consecutive threads take consecutive 16 bytes of a row. Nothing
+  } else if (warp == COPY_WARP) {
+    // ---- raw weights: one warp requests a super-step's boxes, and copies the rows' scale data where it lies apart, up to R super-steps ahead.
+    // (While the rows were copied by cp.async, by the producers or by warps of their own, that took 1100 to 1700 cycles a super-step.) Nothing
     // here waits for the kernel that prepares the activations: weights are immutable. ----
-    constexpr int RPP = copy_warps<RowT>() * 32 / RowT::ITEMS; // rows per pass
-    const int t = (int)threadIdx.x - COPY_WARP0 * 32;
-    const int piece = t % RowT::ITEMS, first = t < RPP * RowT::ITEMS ? t / RowT::ITEMS : TILE_N;
-    const uint32_t pitch = (uint32_t)(RowT::item(p.w, 1, piece).p - RowT::item(p.w, 0, piece).p);
-    const uint32_t to = smem_base + p.raw_off + (uint32_t)(first * RowT::ROWB + piece * 16);
     Cursor cur = start;
-    int l_s = start.kt / KPS, slot = 0;
+    int l_s = start.kt / KPS, slot = 0, issued = 0;
     uint32_t lap = 0;
-    Item it;
-    int last_row = 0; // rows past the weight's last one repeat it
-    auto bind = [&]() {
-      const int64_t row0 = min(((int64_t)cur.tile_n * CG + rank) * TILE_N, p.w.n - 1);
-      it = RowT::item(p.w, row0, piece);
-      last_row = (int)min((int64_t)(TILE_N - 1), p.w.n - 1 - row0);
-    };
-    bind();
     for (int j = 0; j < nsuper; j++) {
       if (j >= R && !mbar_wait_uniform(raw_empty + 8 * slot, lap ^ 1u, 1u)) break;
-      const uint32_t off = ((uint32_t)l_s * it.mul) & ~15u;
-      const bool there = !RowT::LIMITED || off < it.lim;
-      const uint8_t *src = it.p + (there ? off : 0u);
-      const uint32_t dst = to + (uint32_t)slot * SLOT;
-#pragma unroll 8
-      for (int i = 0; i < (TILE_N + RPP - 1) / RPP; i++) {
-        const int r = first + i * RPP;
-        if (r < TILE_N) cp_async16(dst + (uint32_t)(i * RPP * RowT::ROWB), src + (uint64_t)(uint32_t)min(r, last_row) * pitch, there ? 16u : 0u);
+      const int64_t row0 = ((int64_t)cur.tile_n * CG + rank) * TILE_N;
+      const uint32_t dst = smem_base + p.raw_off + (uint32_t)slot * SLOT, bar = raw_full + 8 * slot;
+      if (elect_one()) {
+        mbar_expect_tx(bar, RowT::BOX);
+        RowT::boxes(dst, &codes, &high, l_s, (int)row0, bar);
       }
-      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(raw_full + 8 * slot) : "memory"); // when this thread's copies have landed
+      __syncwarp();
+      if constexpr (RowT::SCALES > 0) {
+#pragma unroll
+        for (int i = 0; i < 4 * RowT::SCALES; i++) {
+          const int r = (i & 3) * 32 + lane;
+          cp_async16(dst + RowT::BOX + (uint32_t)((i >> 2) * TILE_N * 16 + r * 16), RowT::scales(p.w, min(row0 + r, p.w.n - 1), l_s, i >> 2));
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory"); // when this lane's copies have landed
+      }
+      issued = j + 1;
       if (++slot == R) slot = 0, lap ^= 1u;
       if (++l_s == SPT) {
         l_s = 0;
-        const int n = cur.tile_n;
         cur.kt = 0;
         cur.advance(KT, KT, TM);
-        if (cur.tile_n != n) bind();
       }
     }
+    for (int j = max(0, issued - R); j < issued; j++) mbar_wait_uniform(raw_full + 8 * (j % R), (j / R) & 1, 1u);
     asm volatile("cp.async.wait_all;" ::: "memory"); // nothing in flight into this CTA's shared memory when it exits
   } else if (warp == LOADER_WARP) {
-    // ---- activation loader: the whole warp runs the loop, one elected lane issues (see the MMA issuer) ----
+    // ---- activation loader: the whole warp runs the loop and one elected lane issues (see the MMA issuer). A turn is kept short (a wait, an
+    // arrival, a copy, with what a tile needs worked out beforehand): it shares its scheduler with busy warps. (When every step was worked out in
+    // 64 bits a turn took 650 cycles, more than the MMAs of 256 rows, and the activations were what every step waited for; as long with one
+    // thread in a branch, whose copy's operands move to uniform registers one by one.) ----
     pdl_wait(); // the activation image is the previous kernel's output
     Cursor cur = start;
-    int s = 0, issued = 0;
+    int s = 0, i = 0;
     uint32_t lap = 0;
-    for (int i = 0; i < nsteps; i++) {
-      if (i >= S && !mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 2u)) break;
+    bool alive = true;
+    while (i < nsteps) {
       // a pair's CTAs bring half of the tile's rows each (the last tile's second half may have fewer, or none: what is then left in the
       // stage reaches only columns that are not stored)
       const int64_t tm0 = (int64_t)cur.tile_m * p.mt, m0 = tm0 + (CG == 2 ? (int)rank * (p.mt / 2) : 0);
       const int rows = (int)min((int64_t)(p.mt / CG), min(tm0 + p.mt, p.m_pad) - m0);
-      if (elect_one()) {
-        if (rows > 0) {
-          mbar_expect_tx(full + 8 * s, (uint32_t)rows * 128);
-          bulk_g2s(b_ring + s * p.b_stride, p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128, (uint32_t)rows * 128, full + 8 * s);
-        } else {
-          mbar_arrive(full + 8 * s);
+      const uint32_t bytes = (uint32_t)max(rows, 0) * 128;
+      const uint8_t *src = p.xh + ((size_t)cur.kt * p.m_pad + m0) * 128;
+      const size_t step = (size_t)p.m_pad * 128;
+      const int len = min(KT - cur.kt, nsteps - i), end = i + len;
+      for (; i < end; i++, src += step) {
+        if (i >= S && alive) alive = mbar_wait(empty + 8 * s, lap ^ 1u, 2u);
+        if (elect_one() && alive) {
+          if (bytes) {
+            mbar_expect_tx(full + 8 * s, bytes);
+            bulk_g2s(b_ring + s * p.b_stride, src, bytes, full + 8 * s);
+          } else {
+            mbar_arrive(full + 8 * s);
+          }
         }
+        __syncwarp();
+        if (++s == S) s = 0, lap ^= 1u;
       }
-      __syncwarp();
-      issued = i + 1;
-      cur.advance(1, KT, TM);
-      if (++s == S) s = 0, lap ^= 1u;
+      cur.advance(len, KT, TM);
     }
-    for (int i = max(0, issued - S); i < issued; i++) mbar_wait_uniform(full + 8 * (i % S), (i / S) & 1, 2u); // nothing in flight at exit
+    for (int j = max(0, nsteps - S); j < nsteps && alive; j++) alive = mbar_wait(full + 8 * (j % S), (j / S) & 1, 2u); // nothing in flight at exit
   } else if (CG == 2 && warp == MMA_WARP && rank != 0) {
     // ---- relay: tells the leader that this CTA's half of a stage is there ----
     const uint32_t to = leader_addr(full);
@@ -905,17 +904,17 @@ int launch_persistent_fmt(const PrefillArgs &a, bool pairs, unsigned ctas, size_
   if (pairs) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
-    pair_config(&cfg, attr, 2 * ctas, nthreads<RowT>(), smem, s);
-    XNQ_CUDA(cudaLaunchKernelEx(&cfg, prefill_persistent_kernel<RowT, 2>, a));
+    pair_config(&cfg, attr, 2 * ctas, NTHREADS, smem, s);
+    XNQ_CUDA(cudaLaunchKernelEx(&cfg, prefill_persistent_kernel<RowT, 2>, a, a.w.maps->codes, a.w.maps->high));
   } else {
-    XNQ_CUDA(launch_pdl(prefill_persistent_kernel<RowT, 1>, dim3(ctas), dim3(nthreads<RowT>()), smem, s, a));
+    XNQ_CUDA(launch_pdl(prefill_persistent_kernel<RowT, 1>, dim3(ctas), dim3(NTHREADS), smem, s, a, a.w.maps->codes, a.w.maps->high));
   }
   count_launch();
   return XNQ_OK;
 }
 
 constexpr size_t SM_SMEM = 228 * 1024, MAX_SPREAD = SM_SMEM / 2;
-static_assert(RowQ4_0::ROWB == RowQ4K::ROWB && RowQ8_0::ROWB == RowQ4K::ROWB, "the raw ring's plan assumes one slot size for these");
+static_assert(RowQ4_0::SLOT == RowQ4K::SLOT && RowQ8_0::SLOT == RowQ4K::SLOT, "the raw ring's plan assumes one slot size for these");
 constexpr size_t PREFILL_SMEM = 225 * 1024; // everything an SM offers minus the static barriers and a reserve
 
 template <typename RowT>
@@ -924,7 +923,7 @@ int init_fmt(int *pairs) { // pairs: lowered to what the device holds at a time 
   XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowT, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
-  pair_config(&cfg, attr, 2, nthreads<RowT>(), PREFILL_SMEM, nullptr);
+  pair_config(&cfg, attr, 2, NTHREADS, PREFILL_SMEM, nullptr);
   int clusters = 0;
   XNQ_CUDA(cudaOccupancyMaxActiveClusters(&clusters, prefill_persistent_kernel<RowT, 2>, &cfg));
   clusters = std::min(clusters, g_num_sms / 2);
@@ -1002,7 +1001,7 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   // Shared-memory plan: B ring | raw ring. With up to eight stages a producer warp can be a whole super-step ahead of the MMAs; what is
   // left goes to the raw ring (it covers the memory latency of the weights). At 256 activation rows that is five stages and three
   // raw slots (two for Q6_K), for a pair eight and five (three).
-  const uint32_t slot = TILE_N * (w.dtype == XNQ_Q6K ? RowQ6K::ROWB : RowQ4K::ROWB);
+  const uint32_t slot = w.dtype == XNQ_Q6K ? RowQ6K::SLOT : RowQ4K::SLOT;
   a.b_stride = ((uint32_t)(a.mt / cg) * 128 + 1023) & ~1023u;
   const size_t budget = PREFILL_SMEM - 1024 - EPI_WARPS * EPI_SLOT; // 1024: alignment slack
   for (int raw = 3; raw >= 2; raw--) { // at least so many raw slots

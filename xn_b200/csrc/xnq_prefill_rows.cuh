@@ -1,14 +1,14 @@
 // Per-format weight producers of the prefill kernel.
 //
-// The weight rows of a tile are fetched and dequantized in row groups of 32 rows. A row group's bytes of one super-step (256 k,
-// Q8_0: 128 k) are one slot of a shared-memory ring: ROWB bytes per row, an odd multiple of 16, so that a quarter warp's 128-bit
-// reads of eight neighbouring rows fall into eight different bank groups.
-//   item()   one of the ITEMS 16-byte copies that make up a row's super-step: where it comes from and how that moves with the
-//            super-step. Consecutive threads take consecutive copies, so that a copy instruction of a warp touches four to six runs
-//            of memory (one thread per row would touch 32).
+// The weight rows of a tile are fetched one super-step (256 k, Q8_0: 128 k) at a time into a slot of a shared-memory ring: the boxes of the weight's
+// tensor maps (xnq_common.cuh), as they lay the rows out, and behind them 16 bytes of scale data per row where the format keeps its scales
+// apart.
+//   boxes()  requests the boxes of super-step ss of the tile that starts at a row
+//   scales() where the 16 bytes of scale data of a row and super-step lie (piece 0 .. SCALES - 1)
 //   head()   what the two halves of a row's 64-wide k-step share (scales, high bits)
-//   half()   reads the row's bytes of half a k-step from the slot and dequantizes them to fp16: the 16 packed pairs that go to the
-//            row's lane of tensor memory, where the MMA reads its weight operand.
+//   half()   reads the bytes of half a k-step of row r from the slot and dequantizes them to fp16: the 16 packed pairs that go to the
+//            row's lane of tensor memory, where the MMA reads its weight operand. Lanes are rows: the swizzles and the 144-byte rows spread a
+//            quarter warp's 128-bit reads over all bank groups.
 //
 // Stored k order inside a k-step (the activation image uses the same one, see kpair_shift in xnq_prefill.cu):
 //   Q8_0, Q6_K  natural
@@ -22,9 +22,8 @@
 namespace xnq {
 namespace prefill_rows {
 
-// bytes 0: zeros are written and nothing is read
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
@@ -44,29 +43,31 @@ __device__ __forceinline__ __half2 scaled_half2(uint32_t f16_bits, float wscale)
   return __float2half2_rn(__half2float(__ushort_as_half((unsigned short)f16_bits)) * wscale);
 }
 
-// A copy's bytes of super-step ss are at p + ((ss * mul) & ~15); from lim on there is nothing (zeros are stored).
-struct Item {
-  const uint8_t *p;
-  uint32_t mul, lim;
-};
-constexpr uint32_t NO_LIMIT = 0xffffffffu;
+// a box of a tensor map: x in bytes (a multiple of 16), y the first row
+__device__ __forceinline__ void tma_box(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+               : "memory");
+}
+constexpr uint32_t ROWS = 128; // of a tile
+__device__ __forceinline__ uint4 chunk128(uint32_t at, int r, int c) { return lds128(at + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4))); }
+__device__ __forceinline__ uint4 chunk64(uint32_t at, int r, int c) { return lds128(at + (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4))); }
 
 // KPS k-steps per super-step ss. KPS = 4: one thread converts both halves of a row's k-step kk; KPS = 2: two threads, a half each.
 
-struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
-  static constexpr bool LIMITED = true; // rows may end inside a super-step
-  static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
-  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { // scales beyond the last block are zero
-    if (c < 8) return Item{w.qs + row * (w.k / 2) + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k / 2 - 16 * c)};
-    return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 16u, NO_LIMIT};
+struct RowQ4_0 { // 128 nibble bytes per row, then eight f16 scales
+  static constexpr int KPS = 4, SCALES = 1;
+  static constexpr uint32_t BOX = ROWS * 128, SLOT = BOX + ROWS * 16;
+  __device__ static __forceinline__ void boxes(uint32_t slot, const CUtensorMap *codes, const CUtensorMap *, int ss, int row, uint32_t bar) { tma_box(slot, codes, ss * 128, row, bar); }
+  __device__ static __forceinline__ const void *scales(const WeightView &w, int64_t row, int ss, int) { // (beyond the last block they are zero)
+    return reinterpret_cast<const uint8_t *>(w.d + row * w.dstride) + ss * 16;
   }
   struct Head {
     uint32_t dd;
     float wscale;
   };
-  __device__ static __forceinline__ Head head(uint32_t slot, int, int kk, float wscale) { return Head{lds32(slot + 128 + 4 * kk), wscale}; }
-  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int kk, int hf, uint32_t (&o)[16]) { // half = one block
-    const uint4 q = lds128(slot + 32 * kk + 16 * hf);
+  __device__ static __forceinline__ Head head(uint32_t slot, int r, int, int kk, float wscale) { return Head{lds32(slot + BOX + r * 16 + 4 * kk), wscale}; }
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int r, int kk, int hf, uint32_t (&o)[16]) { // half = one block
+    const uint4 q = chunk128(slot, r, 2 * kk + hf);
     const __half2 off = h2_from_bits(0x64086408u); // 1032 = 1024 + 8
     const __half2 d2 = scaled_half2(hf ? (hd.dd >> 16) : (hd.dd & 0xffffu), hd.wscale);
     const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
@@ -78,17 +79,19 @@ struct RowQ4_0 { // 128 nibble bytes | eight f16 scales
   }
 };
 
-struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighbour
-  static constexpr bool LIMITED = true;
-  static constexpr int KPS = 2, ROWB = 144, ITEMS = 9;
-  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) {
-    if (c < 8) return Item{w.qs + row * w.k + 16 * c, 128u, (uint32_t)max((int64_t)0, w.k - 16 * c)};
-    return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 8u, NO_LIMIT};
+struct RowQ8_0 { // 128 codes per row, then the f16 scales of this super-step and its neighbour
+  static constexpr int KPS = 2, SCALES = 1;
+  static constexpr uint32_t BOX = ROWS * 128, SLOT = BOX + ROWS * 16;
+  __device__ static __forceinline__ void boxes(uint32_t slot, const CUtensorMap *codes, const CUtensorMap *, int ss, int row, uint32_t bar) { tma_box(slot, codes, ss * 128, row, bar); }
+  __device__ static __forceinline__ const void *scales(const WeightView &w, int64_t row, int ss, int) {
+    return reinterpret_cast<const uint8_t *>(w.d + row * w.dstride) + ((ss * 8) & ~15);
   }
   using Head = RowQ4_0::Head;
-  __device__ static __forceinline__ Head head(uint32_t slot, int ss, int kk, float wscale) { return Head{lds32(slot + 128 + 8 * (ss & 1) + 4 * kk), wscale}; }
-  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int kk, int hf, uint32_t (&o)[16]) { // half = one block
-    const uint4 q[2] = {lds128(slot + 64 * kk + 32 * hf), lds128(slot + 64 * kk + 32 * hf + 16)};
+  __device__ static __forceinline__ Head head(uint32_t slot, int r, int ss, int kk, float wscale) {
+    return Head{lds32(slot + BOX + r * 16 + 8 * (ss & 1) + 4 * kk), wscale};
+  }
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int r, int kk, int hf, uint32_t (&o)[16]) { // half = one block
+    const uint4 q[2] = {chunk128(slot, r, 4 * kk + 2 * hf), chunk128(slot, r, 4 * kk + 2 * hf + 1)};
     const __half2 d2 = scaled_half2(hf ? (hd.dd >> 16) : (hd.dd & 0xffffu), hd.wscale);
     const __half2 off = h2_from_bits(0x64806480u); // 1152 = 1024 + 128
 #pragma unroll
@@ -106,23 +109,24 @@ struct RowQ8_0 { // 128 codes | the f16 scales of this super-step and its neighb
 };
 
 struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
-  static constexpr bool LIMITED = false;
-  static constexpr int KPS = 4, ROWB = 144, ITEMS = 9;
-  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) { return Item{w.qs + row * (w.k / QK_K) * 144 + 16 * c, 144u, NO_LIMIT}; }
+  static constexpr int KPS = 4, SCALES = 0;
+  static constexpr uint32_t BOX = ROWS * 144, SLOT = BOX;
+  __device__ static __forceinline__ void boxes(uint32_t slot, const CUtensorMap *codes, const CUtensorMap *, int ss, int row, uint32_t bar) { tma_box(slot, codes, ss * 144, row, bar); }
+  __device__ static __forceinline__ const void *scales(const WeightView &, int64_t, int, int) { return nullptr; }
   struct Head {
     __half2 a_lo, a_hi, b_lo, b_hi;
   };
   // value = (d*sc) * code - (dmin*m): low nibbles are sub-block 2g, high nibbles sub-block 2g+1
-  __device__ static __forceinline__ Head head(uint32_t slot, int, int g, float wscale) {
-    const uint4 hdr = lds128(slot);
+  __device__ static __forceinline__ Head head(uint32_t slot, int r, int, int g, float wscale) {
+    const uint4 hdr = lds128(slot + r * 144);
     const __half2 dm = *reinterpret_cast<const __half2 *>(&hdr.x);
     const uint32_t f = k4_field(hdr.y, hdr.z, hdr.w, g);
     const float d = __low2float(dm) * wscale, mn = __high2float(dm) * wscale;
     return Head{__float2half2_rn(d * (float)(f & 63)), __float2half2_rn(d * (float)((f >> 6) & 63)), __float2half2_rn(-mn * (float)((f >> 12) & 63)),
                 __float2half2_rn(-mn * (float)(f >> 18))};
   }
-  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int g, int hf, uint32_t (&o)[16]) { // half = words 4 hf .. of the group
-    const uint4 q = lds128(slot + 16 + 32 * g + 16 * hf);
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int r, int g, int hf, uint32_t (&o)[16]) { // half = words 4 hf .. of the group
+    const uint4 q = lds128(slot + r * 144 + 16 + 32 * g + 16 * hf);
     const __half2 k1024 = h2_from_bits(0x64006400u);
     const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
@@ -135,15 +139,16 @@ struct RowQ4K { // the 144-byte super-block: header | 128 nibble bytes
   }
 };
 
-struct RowQ6K { // 128 ql bytes | 64 qh bytes | 16 scales | the f16 d of eight super-blocks
-  static constexpr bool LIMITED = false;
-  static constexpr int KPS = 4, ROWB = 240, ITEMS = 14;
-  __device__ static __forceinline__ Item item(const WeightView &w, int64_t row, int c) {
-    const int64_t blk = row * (w.k / QK_K);
-    if (c < 8) return Item{w.qs + blk * 128 + 16 * c, 128u, NO_LIMIT};
-    if (c < 12) return Item{w.qh + blk * 64 + 16 * (c - 8), 64u, NO_LIMIT};
-    if (c == 12) return Item{reinterpret_cast<const uint8_t *>(w.sc + blk * 16), 16u, NO_LIMIT};
-    return Item{reinterpret_cast<const uint8_t *>(w.d + row * w.dstride), 2u, NO_LIMIT};
+struct RowQ6K { // 128 ql bytes per row, then 64 qh bytes, 16 scales, the f16 d of eight super-blocks
+  static constexpr int KPS = 4, SCALES = 2;
+  static constexpr uint32_t BOX = ROWS * 192, SLOT = BOX + ROWS * 32, HI = ROWS * 128;
+  __device__ static __forceinline__ void boxes(uint32_t slot, const CUtensorMap *codes, const CUtensorMap *high, int ss, int row, uint32_t bar) {
+    tma_box(slot, codes, ss * 128, row, bar);
+    tma_box(slot + HI, high, ss * 64, row, bar);
+  }
+  __device__ static __forceinline__ const void *scales(const WeightView &w, int64_t row, int ss, int piece) {
+    if (piece == 0) return w.sc + (row * (w.k / QK_K) + ss) * 16;
+    return reinterpret_cast<const uint8_t *>(w.d + row * w.dstride) + ((ss * 2) & ~15);
   }
   // k-step kk = 2 h + hi_pair of the super-block: group 0 takes ql[l] of half h, group 1 ql[l + 32], both the low (hi_pair 0) or high nibbles
   struct Head {
@@ -151,19 +156,19 @@ struct RowQ6K { // 128 ql bytes | 64 qh bytes | 16 scales | the f16 d of eight s
     uint32_t sc4;
     float d;
   };
-  __device__ static __forceinline__ Head head(uint32_t slot, int ss, int kk, float wscale) {
+  __device__ static __forceinline__ Head head(uint32_t slot, int r, int ss, int kk, float wscale) {
     const int h = kk >> 1;
     Head hd;
-    hd.qh[0] = lds128(slot + 128 + 32 * h), hd.qh[1] = lds128(slot + 144 + 32 * h);
-    hd.sc4 = lds32(slot + 192 + 8 * h + 4 * (kk & 1));
-    const uint32_t dd = lds32(slot + 208 + 4 * ((ss >> 1) & 3));
+    hd.qh[0] = chunk64(slot + HI, r, 2 * h), hd.qh[1] = chunk64(slot + HI, r, 2 * h + 1);
+    hd.sc4 = lds32(slot + BOX + r * 16 + 8 * h + 4 * (kk & 1));
+    const uint32_t dd = lds32(slot + BOX + ROWS * 16 + r * 16 + 4 * ((ss >> 1) & 3));
     hd.d = __half2float(__ushort_as_half((unsigned short)((ss & 1) ? (dd >> 16) : (dd & 0xffffu)))) * wscale;
     return hd;
   }
-  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int kk, int hf, uint32_t (&o)[16]) {
+  __device__ static __forceinline__ void half(const Head &hd, uint32_t slot, int r, int kk, int hf, uint32_t (&o)[16]) {
     const int h = kk >> 1, sh = 4 * (kk & 1);
     const uint4 (&qh)[2] = hd.qh;
-    const uint4 ql[2] = {lds128(slot + 64 * h + 32 * hf), lds128(slot + 64 * h + 32 * hf + 16)};
+    const uint4 ql[2] = {chunk128(slot, r, 4 * h + 2 * hf), chunk128(slot, r, 4 * h + 2 * hf + 1)};
     const __half2 off = h2_from_bits(0x64206420u); // 1056 = 1024 + 32
     const int hsh = sh + 2 * hf; // bit position of this group's two high bits inside a qh byte
 #pragma unroll
