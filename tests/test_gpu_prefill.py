@@ -269,3 +269,20 @@ def test_fp16_kernel_missing_steps(Q, O, dt, n, k, m):
     _check(got.cpu().numpy(), want, f"{dt.name} m={m} n={n} k={k}")
     half = t.matmul_t(xd, out=torch.empty(m, n, dtype=torch.bfloat16, device=DEV))
     assert torch.allclose(half.float(), got, rtol=2.0 ** -7, atol=1e-4 * float(got.abs().max()))
+
+
+# tiles in more parts than are requested at once (28 of two steps; 16 and more rows), CTAs whose range starts in one tile and ends in another, and with both ends
+# inside one; the parts are added in k order, so that every call has the same bits
+@pytest.mark.parametrize("dt", WEIGHT_TYPES)
+@pytest.mark.parametrize("n,k", [(129, 14336), (3 * 128, 256 * 5), (1000, 2048), (128 * 90, 1024)])
+def test_integer_kernel_parts_of_tiles(Q, O, dt, n, k):
+    w = synth.make_weight(dt, n, k, seed=n)
+    x = synth.make_activation(64, k, seed=k)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    want, bound = O.matmul(int(dt), x, w, n, threads=O.hw_threads()), _f32_bound(O, dt, w, x, n, k)
+    for m in (6, 16) if dt is D.Q6K else (5, 16, 20, 33, 48, 64):
+        xd = torch.from_numpy(x[:m]).to(DEV)
+        got = t.matmul_t(xd)
+        assert (np.abs(got.cpu().numpy().astype(np.float64) - want[:m]) <= bound[:m]).all(), (dt.name, m)
+        for _ in range(10):
+            assert torch.equal(t.matmul_t(xd), got), (dt.name, m)

@@ -128,6 +128,24 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, un
   const bool ok = mbar_wait(bar, parity, bit);
   return __all_sync(0xffffffffu, ok);
 }
+// whether the phase has completed, without waiting for it
+__device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// a ticket of a tile: releases what the CTA stored before the barrier that precedes it, acquires what the others released
+__device__ __forceinline__ unsigned int take_ticket(unsigned int *word) {
+  unsigned int t;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(t) : "l"(word) : "memory");
+  return t;
+}
 // true in one lane of a converged warp
 __device__ __forceinline__ bool elect_one() {
   uint32_t e;
@@ -417,7 +435,7 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
   // barriers: b_full/b_empty [8], side_full/side_empty [8], a_full/mma_done [8], acc_empty [8], raw_full/raw_empty [8]
   __shared__ __align__(8) uint64_t bars[72];
   __shared__ uint32_t tmem_slot;
-  __shared__ unsigned int s_ticket;
+  __shared__ unsigned int s_ticket[2];
   const uint32_t b_full = smem_u32(bars), b_empty = b_full + 64, side_full = b_full + 128, side_empty = b_full + 192, a_full = b_full + 256,
                  mma_done = b_full + 320, acc_empty = b_full + 384, raw_full = b_full + 448, raw_empty = b_full + 512;
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // so that the compiler knows `warp` to be uniform
@@ -428,6 +446,7 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
   const int u0 = cta_first_unit((int)blockIdx.x, p.units_q, p.units_r);
   const int nunits = p.units_q + ((int)blockIdx.x < p.units_r ? 1 : 0);
   const int tile0 = u0 / KT, kt0 = u0 - tile0 * KT;
+  const bool first_part = kt0 != 0 && nunits > KT - kt0; // the CTA's range starts inside a tile and goes on after it
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 8; s++) {
@@ -537,6 +556,12 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
       if (alive) issued = i + 1;
       if (++kt == KT) kt = 0, tile++;
       if (++s == S) s = 0, lap ^= 1u;
+    }
+    if (first_part) { // a release takes about a microsecond, which stops a drain warp in the middle of the range; this warp is done with its own work
+      asm volatile("bar.sync 2, %0;" ::"n"(DW * 32 + 32) : "memory");
+      if (elect_one()) s_ticket[0] = take_ticket(p.tile_cnt + tile0);
+      __syncwarp();
+      asm volatile("bar.arrive 3, %0;" ::"n"(DW * 32 + 32) : "memory");
     }
     for (int i = max(0, issued - S); i < issued; i++) mbar_wait_warp((Conv::RAW ? raw_full : a_full) + 8 * (i % S), (i / S) & 1, 1u); // nothing in flight at exit
   } else if (warp < DRAIN_WARP0) {
@@ -656,19 +681,24 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
         }
       }
     };
-    int seg_kt0 = kt0; // first step of the current segment inside its tile
     int ap = 0, nb = 0;  // i % AP, i % (NB / 2)
     uint32_t a_ph = 0;   // (i / AP) & 1
+    // The next step's records and products were seen to be there while this step's were read back. The three waits one after the other took 500
+    // cycles even when nothing was left to wait for, of 1400 that a step of 16 rows takes a drain warp.
+    bool ready = false;
     for (int i = 0; i < nunits; i++) {
       const int ss = i % SIDE_STAGES;
-      if (alive) alive = mbar_wait_warp(side_full + 8 * ss, (i / SIDE_STAGES) & 1, 8u);
+      if (!__all_sync(0xffffffffu, ready)) { // else the step was there when the one before was read back
+        if (alive) alive = mbar_wait_warp(side_full + 8 * ss, (i / SIDE_STAGES) & 1, 8u);
+        if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap), a_ph, 8u);
+        if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap + 1), a_ph, 8u);
+      }
+      ready = false;
       const uint32_t side = base + p.side_off + ss * p.side_stage_bytes;
       uint4 hdr = make_uint4(0, 0, 0, 0);
       float dw = 0.f;
       if (alive) hdr = lds128(side + (uint32_t)(32 * q + lane) * 16);
       if (Conv::PAIRED && alive) dw = __uint_as_float(lds32(side + HDR_BYTES + (uint32_t)(NP * 32 + (32 * q + lane) * 4)));
-      if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap), a_ph, 8u);
-      if (alive) alive = mbar_wait_warp(mma_done + 8 * (2 * ap + 1), a_ph, 8u);
       if (alive) {
         tc_fence_after();
         const uint32_t taddr = tmem_d + ((uint32_t)(32 * q) << 16) + (uint32_t)(2 * nb * BUF_COLS + c0); // the halves' buffers are neighbours
@@ -695,6 +725,8 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty + 8 * (2 * nb)), mbar_arrive(acc_empty + 8 * (2 * nb + 1));
+            const uint32_t next = mma_done + (ap + 1 == AP ? 0u : 16u * (uint32_t)(ap + 1)), ph = ap + 1 == AP ? a_ph ^ 1u : a_ph;
+            ready = (i + 1 < nunits) & mbar_peek(side_full + 8 * ((i + 1) % SIDE_STAGES), ((i + 1) / SIDE_STAGES) & 1) & mbar_peek(next, ph) & mbar_peek(next + 8, ph);
           }
           if constexpr (!Conv::PAIRED) Conv::template Drain<CH>::run(hdr, side + HDR_BYTES, c0 + ch * CH, v, acc + ch * CH);
         }
@@ -715,53 +747,18 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
       }
       if (tile_end || range_end) {
         const int64_t row = (int64_t)tile * TILE_N + 32 * q + lane;
-        const bool whole = seg_kt0 == 0 && tile_end;
-        if (whole) {
+        if (tile_end && (tile != tile0 || kt0 == 0)) {
           if (alive) store_rows(row, acc);
         } else {
-          // this CTA's first segment (it starts where the CTA's range starts) uses scratch slot 2c, a later one 2c + 1
-          const int seg_u0 = tile * KT + seg_kt0;
-          float *mine = p.partials + ((size_t)2 * blockIdx.x + (seg_u0 == u0 ? 0 : 1)) * ROWS * TILE_N;
+          // this CTA's first segment (it starts where the CTA's range starts) uses scratch slot 2c, its last one, if another, 2c + 1
+          const int slot = tile == tile0 ? 0 : 1;
+          float *mine = p.partials + ((size_t)2 * blockIdx.x + slot) * ROWS * TILE_N;
 #pragma unroll
           for (int c = 0; c < NPT; c++) mine[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
-          __threadfence();
-          asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
-          if (et == 0) s_ticket = atomicAdd(p.tile_cnt + tile, 1u);
-          asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
-          const unsigned int ticket = s_ticket;
-          asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory"); // s_ticket may be rewritten from here on
-          const int t_u0 = tile * KT, t_u1 = t_u0 + KT;
-          const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u1 - 1, p.units_q, p.units_r);
-          if (et == 0 && (int)ticket == c_last - c_first) p.tile_cnt[tile] = 0u; // every part has its ticket: the word is zero again for the next call
-          if ((int)ticket == c_last - c_first) { // the last part to arrive adds all parts in k order (16 rows: in runs)
-            __threadfence();
-            float (&sum)[NPT] = acc; // the segment's own sums are in its scratch slot by now
-#pragma unroll
-            for (int c = 0; c < NPT; c++) sum[c] = 0.f;
-            auto add_part = [&](int cc, float (&to)[NPT]) {
-              const int cu0 = cta_first_unit(cc, p.units_q, p.units_r);
-              const float *part = p.partials + ((size_t)2 * cc + (cu0 >= t_u0 ? 0 : 1)) * ROWS * TILE_N;
-#pragma unroll
-              for (int c = 0; c < NPT; c++) to[c] += __ldcg(part + (size_t)(c0 + c) * TILE_N + 32 * q + lane);
-            };
-            if constexpr (DW == 8) {
-              for (int cc = c_first; cc <= c_last;) {
-                float some[NPT];
-#pragma unroll
-                for (int c = 0; c < NPT; c++) some[c] = 0.f;
-                for (const int end = min(cc + SUM_RUN, c_last + 1); cc < end; cc++) add_part(cc, some);
-#pragma unroll
-                for (int c = 0; c < NPT; c++) sum[c] += some[c];
-              }
-            } else {
-              for (int cc = c_first; cc <= c_last; cc++) add_part(cc, sum);
-            }
-            store_rows(row, sum);
-          }
+          if (!range_end) asm volatile("bar.arrive 2, %0;" ::"n"(DW * 32 + 32) : "memory"); // a first segment (first_part): the weight producer takes its ticket
         }
 #pragma unroll
         for (int c = 0; c < NPT; c++) acc[c] = 0.f;
-        seg_kt0 = 0;
       }
       if (++kt == KT) {
         kt = 0;
@@ -769,6 +766,62 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
       }
       if (++ap == AP) ap = 0, a_ph ^= 1u;
       if (2 * ++nb == NB) nb = 0;
+    }
+    // ---- tiles that other CTAs have parts of: the last part to arrive adds all parts in k order (16 rows: in runs) ----
+    // A release of the CTA's stores and the ticket take a microsecond, a trip to the parts 0.8. So: a first segment's ticket is taken by the weight
+    // producer while this warp goes on with the next tile (in the loop, by a drain warp, it held up everything: Q8_0 11008 x 4096, 45 rows 28.5 us
+    // instead of 25.0; both tickets at the end made one CTA the last of two tiles: Q8_0 4096 x 4096, 8 rows 14.1 instead of 10.8), one thread releases
+    // for all, and several parts are requested at once. With the look ahead at the barriers, before -> now in a stream of calls: Q4_K 4096 x 14336,
+    // 16 rows 21.0 -> 18.5 us; 28672 x 4096 30.0 -> 25.4; 4096 x 4096 11.9 -> 10.9; Q8_0 11008 x 4096, 16 rows 18.5 -> 15.7; Q6_K 32000 x 4096, 16 rows
+    // 38.8 -> 34.8; Q4_K 4096 x 4096, 64 rows 19.6 -> 17.7.
+    const int last = tile0 + (kt0 + nunits - 1) / KT; // the tiles whose parts are in this CTA's scratch slots, or -1
+    const int part0 = kt0 != 0 || nunits < KT ? tile0 : -1, part1 = last != tile0 && (kt0 + nunits) % KT != 0 ? last : -1;
+    if (part0 >= 0 || part1 >= 0) {
+      asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
+      const int ticket_of = et == 0 ? (first_part ? -1 : part0) : et == 1 ? part1 : -1;
+      if (ticket_of >= 0) s_ticket[et] = take_ticket(p.tile_cnt + ticket_of);
+      asm volatile("bar.sync 1, %0;" ::"n"(DW * 32) : "memory");
+      if (first_part) asm volatile("bar.sync 3, %0;" ::"n"(DW * 32 + 32) : "memory");
+#pragma unroll 1
+      for (int slot = 0; slot < 2; slot++) {
+        const int t = slot ? part1 : part0;
+        if (t < 0) continue;
+        const int t_u0 = t * KT;
+        const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u0 + KT - 1, p.units_q, p.units_r);
+        if ((int)s_ticket[slot] != c_last - c_first) continue;
+        if (et == 0) p.tile_cnt[t] = 0u; // every part has its ticket: the word is zero again for the next call
+        constexpr int AHEAD = DW == 8 ? SUM_RUN : 48 / NPT; // parts requested together: what the registers hold
+        float sum[NPT], some[DW == 8 ? NPT : 1];
+#pragma unroll
+        for (int c = 0; c < NPT; c++) sum[c] = 0.f;
+#pragma unroll
+        for (int c = 0; c < (DW == 8 ? NPT : 1); c++) some[c] = 0.f;
+#pragma unroll 1
+        for (int cc = c_first; cc <= c_last; cc += AHEAD) {
+          float v[AHEAD][NPT];
+#pragma unroll
+          for (int a = 0; a < AHEAD; a++) {
+            const int from = min(cc + a, c_last);
+            const float *part = p.partials + ((size_t)2 * from + (cta_first_unit(from, p.units_q, p.units_r) >= t_u0 ? 0 : 1)) * ROWS * TILE_N + (size_t)c0 * TILE_N + 32 * q + lane;
+#pragma unroll
+            for (int c = 0; c < NPT; c++) v[a][c] = __ldcg(part + c * TILE_N);
+          }
+#pragma unroll
+          for (int a = 0; a < AHEAD; a++) {
+            if (cc + a > c_last) break;
+#pragma unroll
+            for (int c = 0; c < NPT; c++) {
+              if constexpr (DW == 8) some[c] += v[a][c];
+              else sum[c] += v[a][c];
+            }
+          }
+          if constexpr (DW == 8) { // a run is complete
+#pragma unroll
+            for (int c = 0; c < NPT; c++) sum[c] += some[c], some[c] = 0.f;
+          }
+        }
+        store_rows((int64_t)t * TILE_N + 32 * q + lane, sum);
+      }
     }
   }
 
