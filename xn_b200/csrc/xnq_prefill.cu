@@ -108,6 +108,21 @@ __device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity,
   const bool ok = mbar_wait(bar, parity, bit);
   return __all_sync(0xffffffffu, ok);
 }
+// Whether the phase has completed, without waiting for it. A wait takes 120 to 250 cycles even when there is nothing to wait for, and with 32 rows every
+// role took a turn of 550 cycles that way. The loops below look at the next turn's barrier while this turn's work is under way and wait only for what was
+// not there yet. With Q6_K's shorter conversion, a stream of calls, best and median clock: Q6_K 128256 x 4096, 32 rows 130 and 139 -> 114 and 129 us; Q4_K
+// 28672 x 4096, 65 rows 38.0 -> 36.2; Q8_0 8192 x 4096, 128 rows 29.4 -> 28.4. (Two k-steps a turn on top: no difference.)
+__device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // ---- CTA pairs (a cluster of two) ----
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -349,8 +364,9 @@ __device__ __forceinline__ void store_direct(const uint32_t (&v)[16], uint32_t r
 // Measured, start of each -> with it (long stream of calls): the turned drain, the halves and copies by warps of their own, Q4_0 4096 x 4096, 200 rows
 // 32.5 -> 25.6 us, Q4_K 4096 x 4096, 300 rows 31.9 -> 29.3; weights in boxes of tensor maps and a short turn of the activation loader, Q4_K 28672 x
 // 4096, 2000 rows (bf16 results) 443 -> 417, Q8_0 11008 x 4096, 512 rows 64.0 -> 61.4, Q6_K 128256 x 4096, 32 rows 155 -> 138, Q4_K 14336 x 4096, 512
-// rows 72.2 -> 70.3. What bounds it now: wide tiles the power limit and the tensor core's 512 cycles a k-step, Q6_K and narrow tiles the
-// instructions of the conversion (Q6_K 540 cycles a k-step, of which its four warps' instructions are 85 %).
+// rows 72.2 -> 70.3. What bounds it now: wide tiles the power limit and the tensor core's 512 cycles a k-step (pairs) or the 32 KB of activations that a
+// k-step brings through L2 (single CTAs: 750 to 800 cycles), narrow ones the instructions of the conversion and the latencies between the roles (500
+// cycles a k-step).
 struct Cursor { // position in the flattened (tile, k-step) space; tile = tile_n * tiles_m + tile_m
   int tile_n, tile_m, kt;
   __device__ __forceinline__ void advance(int steps, int KT, int tiles_m) {
@@ -451,9 +467,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
     int at = 0, s = 0;      // s = at % S, lap: parity of at / S, of the last step this warp looked at
     uint32_t lap = 0;
     const bool lockstep = KT % KPS != 0 && KPS + KT % KPS > S;
-    bool alive = true;
+    bool alive = true, raw_ready = false, empty_ready = false;
     for (int left = nsuper; left > 0; left--) {
-      if (alive) alive = mbar_wait_uniform(raw_full + 8 * slot, raw_lap, 1u);
+      if (alive && !__all_sync(0xffffffffu, raw_ready)) alive = mbar_wait_uniform(raw_full + 8 * slot, raw_lap, 1u);
       // A warp waits for a stage only on behalf of a step that it fills: that step's MMAs, and so the stage's next phase, wait for this warp in
       // turn, while a barrier that runs on without it may be two phases ahead by the time it looks, which a parity cannot tell from none. Where
       // a warp's k-step is missing from a tile's last super-step, two of its waits may then be more than S steps apart, and the second could
@@ -462,7 +478,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       const int kt = c_s * KPS + kk, i = base_i + kt;
       if (alive && kt < KT && i >= 0 && i < nsteps) {
         for (s += i - at, at = i; s >= S; lap ^= 1u) s -= S;
-        if (i >= S) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 1u);
+        if (i >= S && !__all_sync(0xffffffffu, empty_ready)) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 1u);
+        empty_ready = false;
         if (alive) {
           tc_fence_after();
           const uint32_t at_slot = raw + (uint32_t)slot * SLOT;
@@ -475,6 +492,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
             RowT::half(head, at_slot, r, kk, half, o); // (what a lane past the weight's last row makes is not stored)
             tmem_st16(dst + 16 * half, o);
           }
+          const int next = s + KPS - (s + KPS >= S ? S : 0); // of this warp's next step, if this tile has one
+          empty_ready = kt + KPS < KT && mbar_peek(empty + 8 * next, s + KPS >= S ? lap : lap ^ 1u);
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
@@ -484,6 +503,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       __syncwarp();
       if (lane == 0) mbar_arrive(raw_empty + 8 * slot); // (also by a warp that gave up)
       if (++slot == R) slot = 0, raw_lap ^= 1u;
+      raw_ready = mbar_peek(raw_full + 8 * slot, raw_lap);
       if (++c_s == SPT) {
         c_s = 0;
         base_i += KT;
@@ -532,7 +552,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
     Cursor cur = start;
     int s = 0, i = 0;
     uint32_t lap = 0;
-    bool alive = true;
+    bool alive = true, ready = false;
     while (i < nsteps) {
       // a pair's CTAs bring half of the tile's rows each (the last tile's second half may have fewer, or none: what is then left in the
       // stage reaches only columns that are not stored)
@@ -543,7 +563,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       const size_t step = (size_t)p.m_pad * 128;
       const int len = min(KT - cur.kt, nsteps - i), end = i + len;
       for (; i < end; i++, src += step) {
-        if (i >= S && alive) alive = mbar_wait(empty + 8 * s, lap ^ 1u, 2u);
+        if (i >= S && alive && !__all_sync(0xffffffffu, ready)) alive = mbar_wait(empty + 8 * s, lap ^ 1u, 2u);
         if (elect_one() && alive) {
           if (bytes) {
             mbar_expect_tx(full + 8 * s, bytes);
@@ -554,6 +574,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
         }
         __syncwarp();
         if (++s == S) s = 0, lap ^= 1u;
+        ready = mbar_peek(empty + 8 * s, lap ^ 1u);
       }
       cur.advance(len, KT, TM);
     }
@@ -633,8 +654,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       const int buf = NACC == 2 ? seg & 1 : 0;
       if (NACC == 2 && seg >= 2 && alive) alive = mbar_wait(acc_empty + 8 * buf, ((seg >> 1) - 1) & 1, 4u); // the drain of this buffer's previous segment
       const uint32_t d = tmem_d + (uint32_t)(buf * 128);
+      bool ready = false;
       for (; j < len; j++) {
-        if (alive) alive = mbar_wait(full + 8 * s, round & 1, 4u);
+        if (alive && !__all_sync(0xffffffffu, ready)) alive = mbar_wait(full + 8 * s, round & 1, 4u);
         tc_fence_after();
         __syncwarp();
         const uint32_t a = tmem_d + (uint32_t)(A_COL0 + s * A_COLS);
@@ -655,6 +677,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
           s = 0;
           round++;
         }
+        ready = mbar_peek(full + 8 * s, round & 1);
       }
       i += len;
       cur.advance(len, KT, TM);
