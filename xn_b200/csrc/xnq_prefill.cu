@@ -473,8 +473,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       // A warp waits for a stage only on behalf of a step that it fills: that step's MMAs, and so the stage's next phase, wait for this warp in
       // turn, while a barrier that runs on without it may be two phases ahead by the time it looks, which a parity cannot tell from none. Where
       // a warp's k-step is missing from a tile's last super-step, two of its waits may then be more than S steps apart, and the second could
-      // take an older phase for its own: there (Q4_0 with k not a multiple of 256) the four warps of a row group keep step with one another.
-      if (lockstep) asm volatile("bar.sync %0, 128;" ::"r"(2 + rg) : "memory");
+      // take an older phase for its own: there (Q4_0 with k not a multiple of 256) the four warps of a row group start a tile together.
+      if (lockstep && c_s == 0) asm volatile("bar.sync %0, 128;" ::"r"(2 + rg) : "memory");
       const int kt = c_s * KPS + kk, i = base_i + kt;
       if (alive && kt < KT && i >= 0 && i < nsteps) {
         for (s += i - at, at = i; s >= S; lap ^= 1u) s -= S;
@@ -1011,16 +1011,34 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   const int row_tiles = (int)((w.n + TILE_N - 1) / TILE_N);
   a.tiles_m = (int)((m_pad + MAX_MT - 1) / MAX_MT);
   a.whole_tiles = y_dtype == XNQ_F32 ? 0 : 1;
-  // 16-bit results, whose tiles are whole: equal tiles of activation rows, in the MMA's steps of 16 columns (pairs: 32, 16 of each CTA).
+  // 16-bit results, whose tiles are whole: equal tiles of activation rows, in the MMA's steps of 16 columns (pairs: 32, 16 of each CTA), as many as
+  // finish first: rounds of the CTAs times a tile's time. Measured for one round (18944 x 1024 and 4096; Q4_K, Q8_0 and Q6_K alike), a k-step takes
+  // the same up to 128 rows (what bounds it is the conversion of the weights) and then a 256th more for every further row: 66 rows 0.277 us, 128
+  // 0.290, 192 0.374, 256 0.423; a tile's start and end take two k-steps and another for 64 rows.
   // Pairs halve the activation operand's traffic, which is what bounds wide tiles: from 224 rows a tile on they are the faster or the equal
   // ones (in a long stream of calls, Q4_K 14336 x 4096: 224 rows 41.8 against 42.6 us, 512 rows 74.5 / 77.5, 1024 rows 128 / 139; but 176 rows
   // 39.0 / 37.0). With few tiles a pair's coarser share of the work costs more than that (Q4_K 1536 x 2048, 2000 rows, 21 k-steps a pair: 35.2 / 33.5).
   // f32 results: tiles of 256 rows on single CTAs. Where the CTAs' shares cut a tile decides the last bits of its sums, and a last bit that
   // differs in a decoder's first linear moves its logits by 3 % of their norm (8-bit activation codes flip).
-  const int even_mt = (int)((m_pad + a.tiles_m - 1) / a.tiles_m), pair_mt = (even_mt + 31) / 32 * 32;
-  const bool pairs = a.whole_tiles && g_num_pairs > 0 && pair_mt >= 224 && (long long)((row_tiles + 1) / 2) * a.tiles_m * ksteps >= 24ll * g_num_pairs;
+  bool pairs = false;
+  a.mt = (int)std::min<int64_t>(MAX_MT, m_pad);
+  if (a.whole_tiles) {
+    double best = 0;
+    const auto consider = [&](int mt, bool pair) {
+      const long long tiles_m = (m_pad + mt - 1) / mt, ctas = pair ? g_num_pairs : sms, count = (pair ? (row_tiles + 1) / 2 : row_tiles) * tiles_m;
+      const double time = (double)((count + ctas - 1) / ctas) * (ksteps * (256. + std::max(0, mt - 128)) * (pair ? 0.95 : 1.) + 512. + 4. * mt);
+      if (best == 0 || time < 0.98 * best) best = time, a.mt = mt, a.tiles_m = (int)tiles_m, pairs = pair; // fewer and wider ones where it makes no difference
+    };
+    const int64_t fewest = a.tiles_m;
+    for (int64_t t = fewest, last = 0; t <= std::min(4 * fewest, fewest + 12); t++) {
+      const int even_mt = (int)((m_pad + t - 1) / t), pair_mt = (even_mt + 31) / 32 * 32, mt = (even_mt + 15) / 16 * 16;
+      if (mt == last) continue;
+      last = mt;
+      if (g_num_pairs > 0 && pair_mt >= 224 && (long long)((row_tiles + 1) / 2) * t * ksteps >= 24ll * g_num_pairs) consider(pair_mt, true);
+      consider(mt, false);
+    }
+  }
   const int cg = pairs ? 2 : 1;
-  a.mt = pairs ? pair_mt : (a.whole_tiles ? (even_mt + 15) / 16 * 16 : (int)std::min<int64_t>(MAX_MT, m_pad));
   // Shared-memory plan: B ring | raw ring. With up to eight stages a producer warp can be a whole super-step ahead of the MMAs; what is
   // left goes to the raw ring (it covers the memory latency of the weights). At 256 activation rows that is five stages and three
   // raw slots (two for Q6_K), for a pair eight and five (three).
