@@ -665,21 +665,13 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
     float run[Conv::PAIRED ? NPT : 1]; // Q6_K: the finished runs of steps
 #pragma unroll
     for (int c = 0; c < (Conv::PAIRED ? NPT : 1); c++) run[c] = 0.f;
-    auto store_rows = [&](int64_t row, const float (&val)[NPT]) {
-      if (row >= p.w.n) return;
-      float add = 0.f;
-      if constexpr (BIAS) add = bias_at(p.bias, p.y_dtype, row);
-#pragma unroll
-      for (int c = 0; c < NPT; c++) {
-        const int64_t col = c0 + c;
-        if (col < p.m) {
-          const int64_t idx = col * p.ldy + row;
-          const float v = BIAS ? with_bias(val[c], add, p.y_dtype) : val[c];
-          if (p.y_dtype == XNQ_F32) static_cast<float *>(p.y)[idx] = v;
-          else if (p.y_dtype == XNQ_F16) static_cast<__half *>(p.y)[idx] = __float2half_rn(v);
-          else static_cast<__nv_bfloat16 *>(p.y)[idx] = __float2bfloat16_rn(v);
-        }
-      }
+    auto store_one = [&](int64_t row, int64_t col, float val) {
+      if (row >= p.w.n || col >= p.m) return;
+      const int64_t idx = col * p.ldy + row;
+      const float v = BIAS ? with_bias(val, bias_at(p.bias, p.y_dtype, row), p.y_dtype) : val;
+      if (p.y_dtype == XNQ_F32) static_cast<float *>(p.y)[idx] = v;
+      else if (p.y_dtype == XNQ_F16) static_cast<__half *>(p.y)[idx] = __float2half_rn(v);
+      else static_cast<__nv_bfloat16 *>(p.y)[idx] = __float2bfloat16_rn(v);
     };
     int ap = 0, nb = 0;  // i % AP, i % (NB / 2)
     uint32_t a_ph = 0;   // (i / AP) & 1
@@ -748,13 +740,17 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
       if (tile_end || range_end) {
         const int64_t row = (int64_t)tile * TILE_N + 32 * q + lane;
         if (tile_end && (tile != tile0 || kt0 == 0)) {
-          if (alive) store_rows(row, acc);
+          if (alive) {
+#pragma unroll
+            for (int c = 0; c < NPT; c++) store_one(row, c0 + c, acc[c]);
+          }
         } else {
           // this CTA's first segment (it starts where the CTA's range starts) uses scratch slot 2c, its last one, if another, 2c + 1
           const int slot = tile == tile0 ? 0 : 1;
           float *mine = p.partials + ((size_t)2 * blockIdx.x + slot) * ROWS * TILE_N;
 #pragma unroll
-          for (int c = 0; c < NPT; c++) mine[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
+          for (int c = 0; c < NPT; c++)
+            if (c0 + c < p.m) mine[(size_t)(c0 + c) * TILE_N + 32 * q + lane] = acc[c];
           if (!range_end) asm volatile("bar.arrive 2, %0;" ::"n"(DW * 32 + 32) : "memory"); // a first segment (first_part): the weight producer takes its ticket
         }
 #pragma unroll
@@ -771,8 +767,8 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
     // A release of the CTA's stores and the ticket take a microsecond, a trip to the parts 0.8. So: a first segment's ticket is taken by the weight
     // producer while this warp goes on with the next tile (in the loop, by a drain warp, it held up everything: Q8_0 11008 x 4096, 45 rows 28.5 us
     // instead of 25.0; both tickets at the end made one CTA the last of two tiles: Q8_0 4096 x 4096, 8 rows 14.1 instead of 10.8), one thread releases
-    // for all, and several parts are requested at once. With the look ahead at the barriers, before -> now in a stream of calls: Q4_K 4096 x 14336,
-    // 16 rows 21.0 -> 18.5 us; 28672 x 4096 30.0 -> 25.4; 4096 x 4096 11.9 -> 10.9; Q8_0 11008 x 4096, 16 rows 18.5 -> 15.7; Q6_K 32000 x 4096, 16 rows
+    // for all. With the look ahead at the barriers, before -> now in a stream of calls: Q4_K 4096 x 14336, 16 rows 21.0 -> 18.2 us;
+    // 512 x 13568 14.8 -> 12.4; 28672 x 4096 30.0 -> 25.4; 4096 x 4096 11.9 -> 10.9; Q8_0 11008 x 4096, 16 rows 18.5 -> 15.7; Q6_K 32000 x 4096, 16 rows
     // 38.8 -> 34.8; Q4_K 4096 x 4096, 64 rows 19.6 -> 17.7.
     const int last = tile0 + (kt0 + nunits - 1) / KT; // the tiles whose parts are in this CTA's scratch slots, or -1
     const int part0 = kt0 != 0 || nunits < KT ? tile0 : -1, part1 = last != tile0 && (kt0 + nunits) % KT != 0 ? last : -1;
@@ -790,37 +786,43 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
         const int c_first = cta_of(t_u0, p.units_q, p.units_r), c_last = cta_of(t_u0 + KT - 1, p.units_q, p.units_r);
         if ((int)s_ticket[slot] != c_last - c_first) continue;
         if (et == 0) p.tile_cnt[t] = 0u; // every part has its ticket: the word is zero again for the next call
-        constexpr int AHEAD = DW == 8 ? SUM_RUN : 48 / NPT; // parts requested together: what the registers hold
-        float sum[NPT], some[DW == 8 ? NPT : 1];
-#pragma unroll
-        for (int c = 0; c < NPT; c++) sum[c] = 0.f;
-#pragma unroll
-        for (int c = 0; c < (DW == 8 ? NPT : 1); c++) some[c] = 0.f;
+        // A thread adds four rows (4 lane ..) of the columns et / 32 + e DW. This code runs once and its instructions come from memory: 16 rows' parts are
+        // requested four at a time, wider operands' one by one (three or four at a time took 20.4 us instead of 17.6 for Q4_K 4096 x 4096, 64 rows).
+        constexpr int EV = ROWS * TILE_N / 4 / (DW * 32), AHEAD = DW == 8 ? 4 : 1;
+        float sum[EV][4] = {}, some[DW == 8 ? EV : 1][4] = {};
+        const float4 *parts = reinterpret_cast<const float4 *>(p.partials) + et;
 #pragma unroll 1
         for (int cc = c_first; cc <= c_last; cc += AHEAD) {
-          float v[AHEAD][NPT];
+          float4 v[AHEAD][EV];
 #pragma unroll
           for (int a = 0; a < AHEAD; a++) {
             const int from = min(cc + a, c_last);
-            const float *part = p.partials + ((size_t)2 * from + (cta_first_unit(from, p.units_q, p.units_r) >= t_u0 ? 0 : 1)) * ROWS * TILE_N + (size_t)c0 * TILE_N + 32 * q + lane;
+            const float4 *part = parts + (size_t)(2 * from + (cta_first_unit(from, p.units_q, p.units_r) >= t_u0 ? 0 : 1)) * (ROWS * TILE_N / 4);
 #pragma unroll
-            for (int c = 0; c < NPT; c++) v[a][c] = __ldcg(part + c * TILE_N);
+            for (int e = 0; e < EV; e++) v[a][e] = et / 32 + e * DW < p.m ? __ldcg(part + e * DW * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
           }
 #pragma unroll
           for (int a = 0; a < AHEAD; a++) {
             if (cc + a > c_last) break;
 #pragma unroll
-            for (int c = 0; c < NPT; c++) {
-              if constexpr (DW == 8) some[c] += v[a][c];
-              else sum[c] += v[a][c];
+            for (int e = 0; e < EV; e++) {
+              float (&to)[4] = DW == 8 ? some[DW == 8 ? e : 0] : sum[e];
+              to[0] += v[a][e].x, to[1] += v[a][e].y, to[2] += v[a][e].z, to[3] += v[a][e].w;
             }
           }
-          if constexpr (DW == 8) { // a run is complete
+          if constexpr (DW == 8) {
+            if ((cc - c_first) % SUM_RUN == SUM_RUN - AHEAD || cc + AHEAD > c_last) { // a run is complete
 #pragma unroll
-            for (int c = 0; c < NPT; c++) sum[c] += some[c], some[c] = 0.f;
+              for (int e = 0; e < EV; e++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) sum[e][j] += some[e][j], some[e][j] = 0.f;
+            }
           }
         }
-        store_rows((int64_t)t * TILE_N + 32 * q + lane, sum);
+#pragma unroll
+        for (int e = 0; e < EV; e++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) store_one((int64_t)t * TILE_N + lane * 4 + j, et / 32 + e * DW, sum[e][j]);
       }
     }
   }
