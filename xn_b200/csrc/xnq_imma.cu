@@ -359,28 +359,57 @@ struct ConvQ6K { // 128 ql bytes, behind the rows' 64 qh bytes. 64 k number 2 h 
 // The eight block terms of a step are added first, the step's sum then to the running sum: one rounding at the running sum's magnitude
 // per step. One by one they made the results 7 to 20 % less exact than the two chains of half steps that were added before (relative
 // error against the exact dot of the quantized operands, 1000 x 1024: 7.9e-8, with two chains 6.6e-8).
+// Two columns to an instruction (f32x2): with 33 and more rows the drain's issue slots bound the kernel. Same operations in the same order.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 template <int CH>
 struct DrainBlockScaled {
-  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int c0, const uint32_t (&v)[8][CH], float *acc) {
+  // np: rows of the records, which are stored block by block
+  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int np, int c0, const uint32_t (&v)[8][CH], float *acc) {
     const uint32_t w[4] = {hdr.x, hdr.y, hdr.z, hdr.w};
+    uint64_t step[CH / 2];
 #pragma unroll
-    for (int c = 0; c < CH; c++) {
-      const uint4 a = lds128(meta + (uint32_t)(c0 + c) * 32), b = lds128(meta + (uint32_t)(c0 + c) * 32 + 16);
-      const uint32_t da[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-      float step = 0.f;
+    for (int j = 0; j < 8; j++) {
+      const __half2 h = *reinterpret_cast<const __half2 *>(&w[j >> 1]);
+      const float d = (j & 1) ? __high2float(h) : __low2float(h);
+      const uint64_t d2 = pack2(d, d);
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const __half2 h = *reinterpret_cast<const __half2 *>(&w[j >> 1]);
-        const float term = ((j & 1) ? __high2float(h) : __low2float(h)) * __uint_as_float(da[j]);
-        step = j == 0 ? (float)(int)v[j][c] * term : fmaf((float)(int)v[j][c], term, step);
+      for (int c = 0; c < CH; c += 4) {
+        const uint4 a = lds128(meta + (uint32_t)(j * np + c0 + c) * 4);
+        const uint64_t t0 = mul2(d2, pack2(__uint_as_float(a.x), __uint_as_float(a.y))), t1 = mul2(d2, pack2(__uint_as_float(a.z), __uint_as_float(a.w)));
+        const uint64_t v0 = pack2((float)(int)v[j][c], (float)(int)v[j][c + 1]), v1 = pack2((float)(int)v[j][c + 2], (float)(int)v[j][c + 3]);
+        step[c / 2] = j == 0 ? mul2(v0, t0) : fma2(v0, t0, step[c / 2]);
+        step[c / 2 + 1] = j == 0 ? mul2(v1, t1) : fma2(v1, t1, step[c / 2 + 1]);
       }
-      acc[c] += step;
+    }
+#pragma unroll
+    for (int c = 0; c < CH; c += 2) {
+      const uint64_t sum = add2(pack2(acc[c], acc[c + 1]), step[c / 2]);
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[c]), "=f"(acc[c + 1]) : "l"(sum));
     }
   }
 };
 template <int CH>
 struct DrainQ4K { // integer sums over the whole super-block, scaled once, as the CPU code does
-  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int c0, const uint32_t (&v)[8][CH], float *acc) {
+  __device__ static __forceinline__ void run(const uint4 &hdr, uint32_t meta, int, int c0, const uint32_t (&v)[8][CH], float *acc) {
     const __half2 dm = *reinterpret_cast<const __half2 *>(&hdr.x);
     const float d = __low2float(dm), dmin = __high2float(dm);
     const uint32_t F[4] = {hdr.y & 0xffffffu, __funnelshift_r(hdr.y, hdr.z, 24) & 0xffffffu, __funnelshift_r(hdr.z, hdr.w, 16) & 0xffffffu, hdr.w >> 8};
@@ -720,7 +749,7 @@ __global__ void __launch_bounds__(imma_threads(Conv::PAIRED ? NP / 2 : NP), 1) i
             const uint32_t next = mma_done + (ap + 1 == AP ? 0u : 16u * (uint32_t)(ap + 1)), ph = ap + 1 == AP ? a_ph ^ 1u : a_ph;
             ready = (i + 1 < nunits) & mbar_peek(side_full + 8 * ((i + 1) % SIDE_STAGES), ((i + 1) / SIDE_STAGES) & 1) & mbar_peek(next, ph) & mbar_peek(next + 8, ph);
           }
-          if constexpr (!Conv::PAIRED) Conv::template Drain<CH>::run(hdr, side + HDR_BYTES, c0 + ch * CH, v, acc + ch * CH);
+          if constexpr (!Conv::PAIRED) Conv::template Drain<CH>::run(hdr, side + HDR_BYTES, NP, c0 + ch * CH, v, acc + ch * CH);
         }
       }
       __syncwarp();
@@ -885,7 +914,8 @@ __global__ void __launch_bounds__(256) imma_prepare(const XT *__restrict__ x, co
       }
       uint32_t *rec = reinterpret_cast<uint32_t *>(meta + ((size_t)(k8 >> 8) * NP + row) * 32);
       if (ACT == XNQ_Q8_0) {
-        if ((lane & 3) == 0) rec[(k8 & 255) >> 5] = __float_as_uint(d); // eight f32 block scales (0 beyond k)
+        // eight f32 block scales (0 beyond k), those of a block's rows side by side
+        if ((lane & 3) == 0) reinterpret_cast<float *>(meta)[((size_t)(k8 >> 8) * 8 + ((k8 & 255) >> 5)) * NP + row] = d;
       } else {
         // 32-sums of the block's eight sub-blocks: lanes 4s .. 4s+3 hold sub-block s; sum16 is the pair sum on both lanes of a pair
         const int s32 = sum16 + __shfl_xor_sync(0xffffffffu, sum16, 2);
