@@ -104,7 +104,8 @@ __device__ __forceinline__ SmemAct stage_activations(unsigned char *smem, const 
   return SmemAct{sq, sd, sb};
 }
 
-template <int MT, int R>
+// BIAS: variants of their own; a test of the pointer beside every store cost Q6_K 4480 x 7424, 5 rows, without a bias, 20.2 us instead of 18.6.
+template <int MT, int R, bool BIAS>
 __device__ __forceinline__ void reduce_store(float (&acc)[R][MT], int lane, int64_t row0, int64_t n, int m, void *y, int y_dtype,
                                              int64_t ldy, const void *bias) {
 #pragma unroll
@@ -112,7 +113,7 @@ __device__ __forceinline__ void reduce_store(float (&acc)[R][MT], int lane, int6
 #pragma unroll
     for (int i = 0; i < MT; i++) {
       const float v = warp_sum(acc[r][i]);
-      if (lane == 0 && i < m && row0 + r < n) store_y(y, y_dtype, (int64_t)i * ldy + row0 + r, bias ? with_bias(v, bias_at(bias, y_dtype, row0 + r), y_dtype) : v);
+      if (lane == 0 && i < m && row0 + r < n) store_y(y, y_dtype, (int64_t)i * ldy + row0 + r, BIAS ? with_bias(v, bias_at(bias, y_dtype, row0 + r), y_dtype) : v);
     }
   }
 }
@@ -120,7 +121,7 @@ __device__ __forceinline__ void reduce_store(float (&acc)[R][MT], int lane, int6
 #define XNQ_MATVEC_BOUNDS __launch_bounds__(THREADS, (R >= 4 ? 2 : (MT <= 2 ? 4 : (MT <= 4 ? 3 : 2))))
 
 // ---- Q4_0: one 16-byte chunk = one block (32 codes) ----------------------------------------------
-template <int MT, int R>
+template <int MT, int R, bool BIAS>
 __global__ void XNQ_MATVEC_BOUNDS matvec_q4_0(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK, true);
@@ -162,12 +163,12 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q4_0(WeightView w, ActView a, void *y, 
       }
     }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
+  reduce_store<MT, R, BIAS>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
 // ---- Q8_0: one 16-byte chunk = half a block -------------------------------------------------------
-template <int MT, int R>
+template <int MT, int R, bool BIAS>
 __global__ void XNQ_MATVEC_BOUNDS matvec_q8_0(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK, false);
@@ -201,12 +202,12 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q8_0(WeightView w, ActView a, void *y, 
       }
     }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
+  reduce_store<MT, R, BIAS>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
 // ---- Q4_K: 8 lanes per 144-byte super-block (header + 8 chunks of 16 nibble bytes) -----------------
-template <int MT, int R>
+template <int MT, int R, bool BIAS>
 __global__ void XNQ_MATVEC_BOUNDS matvec_q4k(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK_K, true);
@@ -292,12 +293,12 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q4k(WeightView w, ActView a, void *y, i
       }
     }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
+  reduce_store<MT, R, BIAS>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
 // ---- Q6_K: 4 lanes per super-block; a lane takes 2 ql chunks + 1 qh chunk = 64 codes ---------------
-template <int MT, int R>
+template <int MT, int R, bool BIAS>
 __global__ void XNQ_MATVEC_BOUNDS matvec_q6k(WeightView w, ActView a, void *y, int y_dtype, int64_t ldy, const void *bias) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemAct sa = stage_activations(smem, a, QK_K, true, true);
@@ -405,12 +406,12 @@ __global__ void XNQ_MATVEC_BOUNDS matvec_q6k(WeightView w, ActView a, void *y, i
     }
   }
   }
-  reduce_store<MT, R>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
+  reduce_store<MT, R, BIAS>(acc, lane, row0, w.n, m, y, y_dtype, ldy, bias);
   }
 }
 
-template <int MT, int R>
-int launch_mt(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias) {
+template <int MT, int R, bool BIAS>
+int launch_variant(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias) {
   const int64_t groups = (w.n + (int64_t)WARPS * R - 1) / ((int64_t)WARPS * R);
   const int blk = (w.dtype == XNQ_Q4_0 || w.dtype == XNQ_Q8_0) ? QK : QK_K;
   const size_t image = smem_act_bytes(a.m, a.k, blk, w.dtype != XNQ_Q8_0);
@@ -420,22 +421,22 @@ int launch_mt(const WeightView &w, const ActView &a, void *y, int y_dtype, int64
   switch (w.dtype) {
     case XNQ_Q4_0: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK, true);
-      matvec_q4_0<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
+      matvec_q4_0<MT, R, BIAS><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     case XNQ_Q8_0: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK, false);
-      matvec_q8_0<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
+      matvec_q8_0<MT, R, BIAS><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     case XNQ_Q4K: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK_K, true);
-      matvec_q4k<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
+      matvec_q4k<MT, R, BIAS><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     case XNQ_Q6K: {
       const size_t sm = smem_act_bytes(a.m, a.k, QK_K, true);
-      matvec_q6k<MT, R><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
+      matvec_q6k<MT, R, BIAS><<<grid, THREADS, sm, s>>>(w, a, y, y_dtype, ldy, bias);
       break;
     }
     default: return fail(XNQ_ERR_DTYPE, "matvec: dtype %d", w.dtype);
@@ -445,15 +446,25 @@ int launch_mt(const WeightView &w, const ActView &a, void *y, int y_dtype, int64
   return XNQ_OK;
 }
 
+template <int MT, int R>
+int launch_mt(const WeightView &w, const ActView &a, void *y, int y_dtype, int64_t ldy, cudaStream_t s, const void *bias) {
+  return bias ? launch_variant<MT, R, true>(w, a, y, y_dtype, ldy, s, bias) : launch_variant<MT, R, false>(w, a, y, y_dtype, ldy, s, nullptr);
+}
+
 constexpr size_t MAX_DYN_SMEM = 200 * 1024;
 
+template <int MT, int R, bool BIAS>
+int init_variant() {
+  XNQ_CUDA(cudaFuncSetAttribute(matvec_q4_0<MT, R, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
+  XNQ_CUDA(cudaFuncSetAttribute(matvec_q8_0<MT, R, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
+  XNQ_CUDA(cudaFuncSetAttribute(matvec_q4k<MT, R, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
+  XNQ_CUDA(cudaFuncSetAttribute(matvec_q6k<MT, R, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
+  return XNQ_OK;
+}
 template <int MT, int R>
 int init_mt() {
-  XNQ_CUDA(cudaFuncSetAttribute(matvec_q4_0<MT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(matvec_q8_0<MT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(matvec_q4k<MT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
-  XNQ_CUDA(cudaFuncSetAttribute(matvec_q6k<MT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM));
-  return XNQ_OK;
+  const int rc = init_variant<MT, R, false>();
+  return rc != XNQ_OK ? rc : init_variant<MT, R, true>();
 }
 
 } // namespace
