@@ -103,7 +103,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
   atomicOr(&g_prefill_status, bit);
   return false;
 }
-// by a whole warp that stays converged; the result is the same in all lanes
+// by a whole warp that stays converged; the result is the same in all lanes. (Each lane polls and reads the clock for itself, so one may give up while
+// another sees the phase complete. A role that votes on what it looked at ahead has to go on with one answer: lanes that had given up would pass by a
+// vote that the others wait in, without a limit.)
 __device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity, unsigned int bit) {
   const bool ok = mbar_wait(bar, parity, bit);
   return __all_sync(0xffffffffu, ok);
@@ -563,7 +565,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       const size_t step = (size_t)p.m_pad * 128;
       const int len = min(KT - cur.kt, nsteps - i), end = i + len;
       for (; i < end; i++, src += step) {
-        if (i >= S && alive && !__all_sync(0xffffffffu, ready)) alive = mbar_wait(empty + 8 * s, lap ^ 1u, 2u);
+        if (i >= S && alive && !__all_sync(0xffffffffu, ready)) alive = mbar_wait_uniform(empty + 8 * s, lap ^ 1u, 2u);
         if (elect_one() && alive) {
           if (bytes) {
             mbar_expect_tx(full + 8 * s, bytes);
@@ -578,7 +580,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       }
       cur.advance(len, KT, TM);
     }
-    for (int j = max(0, nsteps - S); j < nsteps && alive; j++) alive = mbar_wait(full + 8 * (j % S), (j / S) & 1, 2u); // nothing in flight at exit
+    for (int j = max(0, nsteps - S); j < nsteps && alive; j++) alive = mbar_wait_uniform(full + 8 * (j % S), (j / S) & 1, 2u); // nothing in flight at exit
   } else if (CG == 2 && warp == MMA_WARP && rank != 0) {
     // ---- relay: tells the leader that this CTA's half of a stage is there ----
     const uint32_t to = leader_addr(full);
@@ -616,9 +618,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
         // One accumulator: its first half of columns is free while the second is still drained. The first steps of the segment go there
         // alone and catch up in the second half when that is free too.
         const int early = min(len, S / 2), s0 = s;
-        if (alive) alive = mbar_wait(acc_empty, (seg - 1) & 1, 4u);
+        if (alive) alive = mbar_wait_uniform(acc_empty, (seg - 1) & 1, 4u);
         for (; j < early; j++) {
-          if (alive) alive = mbar_wait(full + 8 * s, round & 1, 4u);
+          if (alive) alive = mbar_wait_uniform(full + 8 * s, round & 1, 4u);
           tc_fence_after();
           __syncwarp();
           const uint32_t a = tmem_d + (uint32_t)(A_COL0 + s * A_COLS);
@@ -633,7 +635,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
             round++;
           }
         }
-        if (alive) alive = mbar_wait(acc_empty + 8, (seg - 1) & 1, 4u);
+        if (alive) alive = mbar_wait_uniform(acc_empty + 8, (seg - 1) & 1, 4u);
         tc_fence_after();
         __syncwarp();
         for (int t = 0, ts = s0; t < early; t++) {
@@ -652,11 +654,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
         }
       }
       const int buf = NACC == 2 ? seg & 1 : 0;
-      if (NACC == 2 && seg >= 2 && alive) alive = mbar_wait(acc_empty + 8 * buf, ((seg >> 1) - 1) & 1, 4u); // the drain of this buffer's previous segment
+      if (NACC == 2 && seg >= 2 && alive) alive = mbar_wait_uniform(acc_empty + 8 * buf, ((seg >> 1) - 1) & 1, 4u); // the drain of this buffer's previous segment
       const uint32_t d = tmem_d + (uint32_t)(buf * 128);
       bool ready = false;
       for (; j < len; j++) {
-        if (alive && !__all_sync(0xffffffffu, ready)) alive = mbar_wait(full + 8 * s, round & 1, 4u);
+        if (alive && !__all_sync(0xffffffffu, ready)) alive = mbar_wait_uniform(full + 8 * s, round & 1, 4u);
         tc_fence_after();
         __syncwarp();
         const uint32_t a = tmem_d + (uint32_t)(A_COL0 + s * A_COLS);
