@@ -338,20 +338,22 @@ class QCudaLinear:
         return cls(QCudaTensor.from_dense(weight, dtype), bias)
 
     def forward(self, xs: torch.Tensor) -> torch.Tensor:
-        y = _linear(self.weight._native, xs, self.bias)
+        # One name each for the whole call: another thread may replace the layer's weight while a launch waits for the device's queue (the
+        # interpreter's lock is free meanwhile), and the weight that is being launched must not be freed under it.
+        weight, bias = self.weight, self.bias
+        y = _linear(weight._native, xs, bias)
         if y is not None:
             return y
         if xs.dim() < 2:
             raise ValueError(f"input tensor has only one dimension {tuple(xs.shape)}")  # mod.rs:363-365
-        bias = self.bias
         if bias is None:
-            return self.weight.matmul_t(xs)
+            return weight.matmul_t(xs)
         # broadcast_add, q8.rs:172-175: by the matmul's kernel, but for a bias that torch has to see the addition of (gradients, transforms)
         # or that the kernel cannot read (another device, strides)
-        if type(bias) in _PLAIN_TENSORS and not hasattr(xs, "act_dtype") and bias.device == self.weight.device and bias.shape == (self.weight.n,) and not (
+        if type(bias) in _PLAIN_TENSORS and not hasattr(xs, "act_dtype") and bias.device == weight.device and bias.shape == (weight.n,) and not (
                 bias.requires_grad and torch.is_grad_enabled()) and not torch._C._functorch.is_functorch_wrapped_tensor(bias) and forward_ad._current_level < 0:
-            return self.weight._matmul_float(xs, None, bias.to(xs.dtype).contiguous())
-        out = self.weight.matmul_t(xs)
+            return weight._matmul_float(xs, None, bias.to(xs.dtype).contiguous())
+        out = weight.matmul_t(xs)
         return out.add_(bias.to(out.dtype))
 
     __call__ = forward
