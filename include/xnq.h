@@ -166,6 +166,9 @@ int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int
  * rounded to y's type (Q8Linear::forward's broadcast_add, q8.rs:172-175); NULL: none. */
 int xnq_matmul_t_bias(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, const void *bias, void *y,
                       int y_dtype, int64_t ldy, void *workspace, size_t ws_bytes, void *stream);
+/* xnq_matmul_t_bias of one row where that needs no scratch: Q4_0, Q8_0, Q4_K and Q6_K weights of up to 4096 columns. Others: XNQ_ERR_UNSUPPORTED
+ * (call xnq_matmul_t_bias instead). */
+int xnq_matvec(const xnq_weight *w, const void *x, int x_dtype, const void *bias, void *y, int y_dtype, void *stream);
 
 /* A prefetch hint (no counterpart in the reference): names the weight that the calling thread will multiply
  * AFTER its next one-row (m == 1) xnq_matmul_t / xnq_matmul_t_gather call. That next call's kernel then asks for

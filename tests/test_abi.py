@@ -79,6 +79,7 @@ def test_null_handles_are_rejected():
     assert L.xnq_weight_dequantize(None, 0, None, None) == -1
     assert L.xnq_weight_canonical_bytes(None, None, 0, None) == -1
     assert L.xnq_matmul_t(None, None, 0, 1, 32, None, 0, 1, None, 0, None) == -1
+    assert L.xnq_matvec(None, None, 0, None, None, 0, None) == -1
     assert L.xnq_matmul_workspace_bytes(None, 4) == 0
     assert L.xnq_linear_forward_host(None, None, 1, None, None, None) == -1
     assert L.xnq_quantize_act(2, None, 0, 1, 32, 32, None, None) == -2    # Q4_0 is not an activation format

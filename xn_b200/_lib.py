@@ -58,6 +58,7 @@ def lib() -> ctypes.CDLL:
     L.xnq_matmul_workspace_bytes.restype = sz
     L.xnq_matmul_t.argtypes = [vp, vp, ci, i64, i64, vp, ci, i64, vp, sz, vp]
     L.xnq_matmul_t_bias.argtypes = [vp, vp, ci, i64, i64, vp, vp, ci, i64, vp, sz, vp]
+    L.xnq_matvec.argtypes = [vp, vp, ci, vp, vp, ci, vp]
     L.xnq_linear_forward_host.argtypes = [vp, vp, i64, vp, vp, vp]
     L.xnq_weight_reserve_host_staging.argtypes = [vp, i64]
     L.xnq_hint_next_weight.argtypes = [vp]
@@ -113,6 +114,7 @@ def native():
         except ImportError as e:
             raise RuntimeError(f"xn_b200/_xnq_torch.so cannot be loaded ({e}). Build it with `python -m xn_b200.build`.") from e
         L = lib()
-        m.bind(ctypes.cast(L.xnq_matmul_t_bias, ctypes.c_void_p).value, ctypes.cast(L.xnq_matmul_workspace_bytes, ctypes.c_void_p).value, check)
+        address = lambda f: ctypes.cast(f, ctypes.c_void_p).value
+        m.bind(address(L.xnq_matmul_t_bias), address(L.xnq_matvec), address(L.xnq_matmul_workspace_bytes), check)
         _native = m
     return _native

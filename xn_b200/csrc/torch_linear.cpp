@@ -3,8 +3,7 @@
 //
 // A one-row call is bound by the host, not by its kernel (Q4_0 4096 x 4096: the kernel takes 3.3 us). In Python, with the library called through
 // ctypes, it took 10.5 us: some 25 attribute reads and comparisons, a tensor made through the dispatcher, twelve arguments converted one by one, and
-// the launch. Everything that is not ordinary returns None, and the Python code takes the call; nothing is kept from one call for the next but
-// the shared scratch, as there.
+// the launch. Everything that is not ordinary returns None, and the Python code takes the call; nothing is kept from one call for the next.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -13,19 +12,21 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/GradMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <map>
-#include <vector>
+#include <algorithm>
 
 namespace {
 
 using MatmulFn = int (*)(const void *, const void *, int, int64_t, int64_t, const void *, void *, int, int64_t, void *, size_t, void *);
+using MatvecFn = int (*)(const void *, const void *, int, const void *, void *, int, void *);
 using WorkspaceFn = size_t (*)(const void *, int64_t);
 MatmulFn g_matmul = nullptr;         // xnq_matmul_t_bias
+MatvecFn g_matvec = nullptr;         // xnq_matvec
 WorkspaceFn g_workspace_bytes = nullptr; // xnq_matmul_workspace_bytes
 PyObject *g_check = nullptr;         // raises the error of a status
 
@@ -35,18 +36,19 @@ struct Weight { // what a call needs of a weight; owned by the capsule that the 
   c10::DeviceIndex device;
   int64_t ws_rows; // rows asked for last and the scratch they need: a program calls a linear with the same few row counts
   size_t ws_bytes;
+  bool row_without_scratch; // until xnq_matvec has said that it does not serve this weight
 };
+constexpr int UNSUPPORTED = -8; // XNQ_ERR_UNSUPPORTED
 constexpr const char *NAME = "xnq.weight";
 void free_weight(PyObject *capsule) { delete static_cast<Weight *>(PyCapsule_GetPointer(capsule, NAME)); }
 
-// Scratch: all weights of a device share one buffer, which only grows; outgrown ones stay alive because a captured graph may still point at
-// them. (Touched under the interpreter's lock only.)
-std::map<int, std::vector<at::Tensor>> *g_pools = nullptr;
-at::Tensor &scratch(int device, size_t bytes) {
-  std::vector<at::Tensor> &pool = (*g_pools)[device];
-  if (pool.empty() || (size_t)pool.back().numel() < bytes)
-    pool.push_back(at::empty({(int64_t)std::max<size_t>(bytes, 256)}, at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, (c10::DeviceIndex)device))));
-  return pool.back();
+// Scratch (the quantized activations, the tickets and partial sums of split tiles) is a call's own, from torch's caching allocator, which gives a
+// block out again in the order of the stream that it was allocated for, or within the graph that is being captured. One buffer for all calls of a
+// device was overwritten by calls on another stream, by another thread's call between a call's kernels, and by graphs replayed side by side. A block
+// costs 0.35 us of a one-row call (Q4_0 4096 x 4096: 4.1 us instead of 3.75), so that rows that need none get none.
+size_t scratch_bytes(Weight *w, int64_t rows) {
+  if (w->ws_rows != rows) w->ws_rows = rows, w->ws_bytes = std::max<size_t>(g_workspace_bytes(w->handle, rows), 256);
+  return w->ws_bytes;
 }
 
 int xnq_dtype(at::ScalarType t) { // F32 0, F16 1, BF16 30: the ggml ids
@@ -93,22 +95,29 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
   shape[dims - 1] = w->n;
   at::Tensor y = at::Tensor(at::detail::empty_cuda(shape, x.scalar_type(), x.device(), std::nullopt));
-  if (w->ws_rows != m) w->ws_rows = m, w->ws_bytes = g_workspace_bytes(w->handle, m);
-  at::Tensor &ws = scratch(w->device, w->ws_bytes);
-  void *const wsp = ws.mutable_data_ptr(), *const yp = y.mutable_data_ptr();
-  const size_t wsb = (size_t)ws.numel();
+  void *const yp = y.mutable_data_ptr();
   const void *const xp = x.const_data_ptr();
   void *const stream = c10::cuda::getCurrentCUDAStream(w->device).stream();
-  int rc;
-  Py_BEGIN_ALLOW_THREADS // a launch may block while the device's queue is full
-  rc = g_matmul(w->handle, xp, xt, m, ldx, bias, yp, xt, w->n, wsp, wsb, stream);
-  Py_END_ALLOW_THREADS
+  int rc = UNSUPPORTED;
+  if (m == 1 && w->row_without_scratch) {
+    Py_BEGIN_ALLOW_THREADS // a launch may block while the device's queue is full
+    rc = g_matvec(w->handle, xp, xt, bias, yp, xt, stream);
+    Py_END_ALLOW_THREADS
+    if (rc == UNSUPPORTED) w->row_without_scratch = false;
+  }
+  if (rc == UNSUPPORTED) {
+    const size_t wsb = scratch_bytes(w, m);
+    const c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(wsb); // for the current device and stream, where the call launches
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_matmul(w->handle, xp, xt, m, ldx, bias, yp, xt, w->n, ws.get(), wsb, stream);
+    Py_END_ALLOW_THREADS
+  }
   if (rc != 0) return PyObject_CallFunction(g_check, "i", rc);
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
 }
 
-// workspace(weight capsule, rows) -> the shared scratch, large enough for that many rows
+// workspace(weight capsule, rows) -> scratch for one call of that many rows
 PyObject *workspace(PyObject *, PyObject *args) {
   HANDLE_TH_ERRORS
   PyObject *capsule;
@@ -116,8 +125,7 @@ PyObject *workspace(PyObject *, PyObject *args) {
   if (!PyArg_ParseTuple(args, "OL", &capsule, &m)) return nullptr;
   Weight *w = static_cast<Weight *>(PyCapsule_GetPointer(capsule, NAME));
   if (!w) return nullptr;
-  if (w->ws_rows != m) w->ws_rows = m, w->ws_bytes = g_workspace_bytes(w->handle, m);
-  return THPVariable_Wrap(scratch(w->device, w->ws_bytes));
+  return THPVariable_Wrap(at::Tensor(at::detail::empty_cuda({(int64_t)scratch_bytes(w, m)}, at::kByte, at::Device(at::kCUDA, w->device), std::nullopt)));
   END_HANDLE_TH_ERRORS
 }
 
@@ -127,18 +135,17 @@ PyObject *weight(PyObject *, PyObject *args) {
   long long n, k;
   int device;
   if (!PyArg_ParseTuple(args, "KLLi", &handle, &n, &k, &device)) return nullptr;
-  return PyCapsule_New(new Weight{reinterpret_cast<const void *>(handle), n, k, (c10::DeviceIndex)device, -1, 0}, NAME, free_weight);
+  return PyCapsule_New(new Weight{reinterpret_cast<const void *>(handle), n, k, (c10::DeviceIndex)device, -1, 0, true}, NAME, free_weight);
 }
 
-// bind(xnq_matmul_t_bias, xnq_matmul_workspace_bytes, check): the library that ctypes has loaded
+// bind(xnq_matmul_t_bias, xnq_matvec, xnq_matmul_workspace_bytes, check): the library that ctypes has loaded
 PyObject *bind(PyObject *, PyObject *args) {
-  unsigned long long matmul, ws;
+  unsigned long long matmul, matvec, ws;
   PyObject *check;
-  if (!PyArg_ParseTuple(args, "KKO", &matmul, &ws, &check)) return nullptr;
-  g_matmul = reinterpret_cast<MatmulFn>(matmul), g_workspace_bytes = reinterpret_cast<WorkspaceFn>(ws);
+  if (!PyArg_ParseTuple(args, "KKKO", &matmul, &matvec, &ws, &check)) return nullptr;
+  g_matmul = reinterpret_cast<MatmulFn>(matmul), g_matvec = reinterpret_cast<MatvecFn>(matvec), g_workspace_bytes = reinterpret_cast<WorkspaceFn>(ws);
   Py_INCREF(check);
   Py_XSETREF(g_check, check);
-  if (!g_pools) g_pools = new std::map<int, std::vector<at::Tensor>>(); // never destroyed: the allocator may be gone by then
   Py_RETURN_NONE;
 }
 
@@ -146,7 +153,7 @@ PyMethodDef methods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(linear)), METH_FASTCALL, "linear(weight, x, bias) -> y or None"},
     {"workspace", workspace, METH_VARARGS, "workspace(weight, rows) -> scratch"},
     {"weight", weight, METH_VARARGS, "weight(handle, n, k, device index) -> capsule"},
-    {"bind", bind, METH_VARARGS, "bind(matmul, workspace_bytes, check)"},
+    {"bind", bind, METH_VARARGS, "bind(matmul, matvec, workspace_bytes, check)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_xnq_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -587,6 +587,33 @@ size_t xnq_matmul_workspace_bytes(const xnq_weight *w, int64_t max_m) {
   return w->v.dtype == XNQ_Q6K && imma_supported(w->v, q6k_rows) ? std::max(need, imma_workspace_bytes(w->v, q6k_rows)) : need;
 }
 
+// the result and the bias of a product of float rows; the two pointers only if there is something to compute
+static int check_result(const char *what, const xnq_weight *w, int64_t m, const void *bias, const void *y, int y_dtype, int64_t ldy) {
+  const int64_t n = w->v.n;
+  if (!is_float_dtype(y_dtype)) return fail(XNQ_ERR_DTYPE, "%s: output dtype %d is not f32/f16/bf16", what, y_dtype);
+  if (ldy < n) return fail(XNQ_ERR_SHAPE, "%s: ldy = %lld is smaller than n = %lld", what, (long long)ldy, (long long)n);
+  if (m == 0 || n == 0) return XNQ_OK;
+  if (!y) return fail(XNQ_ERR_NULL, "%s: y is NULL", what);
+  if (!aligned(y, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "%s: y is not aligned to its element size", what);
+  if (!aligned(bias, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "%s: the bias is not aligned to its element size", what);
+  return XNQ_OK;
+}
+
+int xnq_matvec(const xnq_weight *w, const void *x, int x_dtype, const void *bias, void *y, int y_dtype, void *stream) {
+  clear_error();
+  if (!w) return fail(XNQ_ERR_NULL, "matvec: weight is NULL");
+  if (is_generic_dtype(w->v.dtype) || !g_opt_matvec_tma.load(std::memory_order_relaxed) || !matvec_tma_supported(w->v, 1) || matvec_tma_wants_image(w->v))
+    return fail(XNQ_ERR_UNSUPPORTED, "matvec: this weight needs scratch; use xnq_matmul_t");
+  int rc = check_activations("matvec", x, x_dtype, 1, w->v.k, w->v.k);
+  if (rc == XNQ_OK) rc = check_result("matvec", w, 1, bias, y, y_dtype, w->v.n);
+  if (rc != XNQ_OK) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  profile_mark(s, true);
+  rc = launch_matvec_tma(w->v, x, x_dtype, y, y_dtype, s, nullptr, nullptr, bias);
+  profile_mark(s, false);
+  return rc;
+}
+
 int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y, int y_dtype, int64_t ldy, void *workspace,
                  size_t ws_bytes, void *stream) {
   return xnq_matmul_t_bias(w, x, x_dtype, m, ldx, nullptr, y, y_dtype, ldy, workspace, ws_bytes, stream);
@@ -602,13 +629,8 @@ int xnq_matmul_t_bias(const xnq_weight *w, const void *x, int x_dtype, int64_t m
   if (x_dtype == XNQ_ACT_OPERAND) return matmul_from_operand(w, x, m, y, y_dtype, ldy, workspace, ws_bytes, static_cast<cudaStream_t>(stream));
   if (x_dtype == XNQ_ACT_IMAGE) return matmul_from_image(w, x, m, y, y_dtype, ldy, workspace, ws_bytes, static_cast<cudaStream_t>(stream));
   int rc = check_activations("matmul_t", x, x_dtype, m, k, ldx);
-  if (rc != XNQ_OK) return rc;
-  if (!is_float_dtype(y_dtype)) return fail(XNQ_ERR_DTYPE, "matmul_t: output dtype %d is not f32/f16/bf16", y_dtype);
-  if (ldy < n) return fail(XNQ_ERR_SHAPE, "matmul_t: ldy = %lld is smaller than n = %lld", (long long)ldy, (long long)n);
-  if (m == 0 || n == 0) return XNQ_OK;
-  if (!y) return fail(XNQ_ERR_NULL, "matmul_t: y is NULL");
-  if (!aligned(y, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "matmul_t: y is not aligned to its element size");
-  if (!aligned(bias, type_size(y_dtype))) return fail(XNQ_ERR_ALIGN, "matmul_t: the bias is not aligned to its element size");
+  if (rc == XNQ_OK) rc = check_result("matmul_t", w, m, bias, y, y_dtype, ldy);
+  if (rc != XNQ_OK || m == 0 || n == 0) return rc;
   const size_t need = least_workspace_bytes(w, m);
   if (!workspace) return fail(XNQ_ERR_NULL, "matmul_t: workspace is NULL (need %zu bytes)", need);
   if (!aligned(workspace, 256)) return fail(XNQ_ERR_ALIGN, "matmul_t: workspace must be 256-byte aligned");

@@ -171,11 +171,6 @@ class QLlama:
         else:
             self._head_img = self._xn_img if c.head_dtype.vec_dot_type == c.linear_dtype.vec_dot_type else None
 
-        for L in self.layers:   # scratch is sized once, before any capture
-            for w in (L.wqkv, L.wo, L.wgu, L.wdown):
-                w.workspace(max(batch, max_prefill_rows))
-        self.lm_head.workspace(batch)
-
     # -- pieces ----------------------------------------------------------------------------------
     def _shard(self, dense: torch.Tensor, dt: GgmlDType) -> QCudaTensor:
         """Quantize and keep this rank's rows of an N-sharded linear (quantization is per row, so slicing first is exact)."""

@@ -202,9 +202,8 @@ class QCudaTensor:
 
     # -- compute --------------------------------------------------------------------------------
     def workspace(self, m: int) -> torch.Tensor:
-        """Scratch for ``m`` activation rows. All weights of a device share one buffer (the reference's device
-        has a single stream, cuda_backend/mod.rs:141-167, so calls never overlap); it only ever grows, and
-        outgrown buffers stay alive because a captured graph may still point at them."""
+        """Scratch for one call of ``m`` activation rows, from torch's caching allocator: calls on several streams, from several threads and in graphs
+        that are replayed side by side each have their own. Keep it until the call has been enqueued."""
         return _lib.native().workspace(self._native, m)
 
     def hint_next(self) -> None:
