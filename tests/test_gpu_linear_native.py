@@ -94,3 +94,16 @@ def test_in_a_captured_graph(weight):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+def test_a_weight_on_a_device_without_an_index(weight):
+    """It refuses rows of a device with an index, with and without `out`; images are taken, on the current device."""
+    from xn_b200 import decoder_ops as ops, quantized as Q
+    w = Q.QCudaTensor.from_qtensor(Q.QTensor(weight.data(), (N, K), D.Q4K), torch.device("cuda"))
+    x = _rows(3, K)
+    for call in (lambda: w.matmul_t(x), lambda: Q.QCudaLinear.new(w).forward(x), lambda: w.matmul_t(x, out=torch.empty(3, N, device=DEV))):
+        with pytest.raises(ValueError, match="input on cuda:0, weight on cuda"):
+            call()
+    image = ops.quantize_act_image(x, ops.ActImage.for_weight(D.Q4K, 3, K, DEV))
+    assert torch.equal(w.matmul_t(image), weight.matmul_t(image))
+    assert w.workspace(3).device == DEV

@@ -33,7 +33,7 @@ PyObject *g_check = nullptr;         // raises the error of a status
 struct Weight { // what a call needs of a weight; owned by the capsule that the Python weight keeps
   const void *handle;
   int64_t n, k;
-  c10::DeviceIndex device;
+  c10::DeviceIndex device; // -1: the weight was put on "cuda", without an index
   int64_t ws_rows; // rows asked for last and the scratch they need: a program calls a linear with the same few row counts
   size_t ws_bytes;
   bool row_without_scratch; // until xnq_matvec has said that it does not serve this weight
@@ -125,7 +125,8 @@ PyObject *workspace(PyObject *, PyObject *args) {
   if (!PyArg_ParseTuple(args, "OL", &capsule, &m)) return nullptr;
   Weight *w = static_cast<Weight *>(PyCapsule_GetPointer(capsule, NAME));
   if (!w) return nullptr;
-  return THPVariable_Wrap(at::Tensor(at::detail::empty_cuda({(int64_t)scratch_bytes(w, m)}, at::kByte, at::Device(at::kCUDA, w->device), std::nullopt)));
+  const at::Device device(at::kCUDA, w->device < 0 ? c10::cuda::current_device() : w->device);
+  return THPVariable_Wrap(at::Tensor(at::detail::empty_cuda({(int64_t)scratch_bytes(w, m)}, at::kByte, device, std::nullopt)));
   END_HANDLE_TH_ERRORS
 }
 

@@ -109,7 +109,8 @@ class QCudaTensor:
         self.n_total, self.n, self.row0, self.k, self.device_bytes = nt.value, nl.value, r0.value, k.value, nb.value
         global _linear
         _linear = _lib.native().linear
-        self._native = _lib.native().weight(handle, self.n, self.k, device.index if device.index is not None else torch.cuda.current_device())
+        # (a device without an index is no tensor's device: rows are refused, in C++ as by the general path)
+        self._native = _lib.native().weight(handle, self.n, self.k, device.index if device.index is not None else -1)
 
     # -- construction ---------------------------------------------------------------------------
     @classmethod
