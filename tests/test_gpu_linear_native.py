@@ -2,6 +2,7 @@
 import pytest
 import torch
 from torch.overrides import TorchFunctionMode
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from xn_b200 import synth
 from xn_b200.dtypes import GgmlDType as D
@@ -107,3 +108,63 @@ def test_a_weight_on_a_device_without_an_index(weight):
     image = ops.quantize_act_image(x, ops.ActImage.for_weight(D.Q4K, 3, K, DEV))
     assert torch.equal(w.matmul_t(image), weight.matmul_t(image))
     assert w.workspace(3).device == DEV
+
+
+class Recorder(TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func.overloadpacket)
+        return func(*args, **(kwargs or {}))
+
+
+class FunctionRecorder(TorchFunctionMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen.append(getattr(func, "__name__", ""))
+        return func(*args, **(kwargs or {}))
+
+
+def test_modes_see_the_addition_of_a_bias(weight):
+    from xn_b200 import quantized as Q
+    x, bias = _rows(3, K), torch.randn(N, device=DEV)
+    layer = Q.QCudaLinear.new(weight, bias)
+    want = layer.forward(x)
+    assert torch.equal(want, weight.matmul_t(x) + bias)
+    with Recorder() as r:
+        assert torch.equal(layer.forward(x), want)
+    assert torch.ops.aten.add_ in r.seen
+    with FunctionRecorder() as r:
+        assert torch.equal(layer.forward(x), want)
+    assert "add_" in r.seen
+    assert torch.equal(layer.forward(x), want)
+
+
+def test_transforms_and_tracers(weight):
+    """What torch wraps has no memory that a kernel could read: such calls are refused, as the results of a call inside `grad` or `jvp` are."""
+    from xn_b200 import quantized as Q
+    x, biases = _rows(3, K), torch.randn(4, N, device=DEV)
+    forward = lambda b: Q.QCudaLinear.new(weight, b).forward(x)
+    want = forward(biases[0])
+    for call in (lambda: torch.func.vmap(forward)(biases), lambda: torch.func.vmap(lambda r: weight.matmul_t(r[None]))(x),
+                 lambda: torch.func.grad(lambda b: forward(b).sum())(biases[0]), lambda: torch.func.jvp(forward, (biases[0],), (biases[1],))):
+        with pytest.raises(RuntimeError):
+            call()
+    assert torch.equal(forward(biases[0]), want)
+    seen = []
+
+    def look(t):
+        seen.append(Q._linear(weight._native, t, None) is None)
+        return forward(biases[0]) + t[0, 0]
+    trace = torch.jit.trace(look, x, check_trace=False)
+    assert seen == [True] and "add_" in str(trace.graph)
+    assert Q._linear(weight._native, x, None) is not None
+    with torch.inference_mode():
+        assert Q._linear(weight._native, x, None) is not None
+    with torch.autocast("cuda"):
+        assert Q._linear(weight._native, x, None) is not None

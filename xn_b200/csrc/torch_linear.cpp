@@ -11,6 +11,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -61,7 +62,14 @@ bool plain(PyObject *o) {
   const c10::DispatchKeySet ks = THPVariable_Unpack(o).key_set();
   return (ks.raw_repr() & ~allowed.raw_repr()) == 0 && ks.has(c10::DispatchKey::CUDA);
 }
-bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set() || at::impl::torch_function_mode_enabled(); }
+// Something of torch looks at operators or replaces them: a function or dispatch mode, a transform of torch.func (whatever tensors it has wrapped), a tracer.
+bool observed() {
+  constexpr c10::DispatchKeySet ordinary({c10::DispatchKey::BackendSelect, c10::DispatchKey::ADInplaceOrView});
+  return (c10::impl::tls_local_dispatch_key_set().included_.raw_repr() & ~ordinary.raw_repr()) != 0 || c10::impl::TorchDispatchModeTLS::any_modes_set() ||
+         at::impl::torch_function_mode_enabled();
+}
+
+PyObject *py_observed(PyObject *, PyObject *) { return PyBool_FromLong(observed()); }
 
 // linear(weight capsule, x, bias or None) -> y, or None where the general code has to take the call
 PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
@@ -72,7 +80,7 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   }
   Weight *w = static_cast<Weight *>(PyCapsule_GetPointer(args[0], NAME));
   if (!w) return nullptr;
-  if (!plain(args[1]) || modes_active()) Py_RETURN_NONE;
+  if (!plain(args[1]) || observed()) Py_RETURN_NONE;
   const at::Tensor &x = THPVariable_Unpack(args[1]);
   const int xt = xnq_dtype(x.scalar_type());
   const int64_t dims = x.dim();
@@ -154,6 +162,7 @@ PyMethodDef methods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(linear)), METH_FASTCALL, "linear(weight, x, bias) -> y or None"},
     {"workspace", workspace, METH_VARARGS, "workspace(weight, rows) -> scratch"},
     {"weight", weight, METH_VARARGS, "weight(handle, n, k, device index) -> capsule"},
+    {"observed", py_observed, METH_NOARGS, "observed() -> whether a mode, a transform or a tracer looks at torch's operators"},
     {"bind", bind, METH_VARARGS, "bind(matmul, matvec, workspace_bytes, check)"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_xnq_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -348,9 +348,9 @@ class QCudaLinear:
             raise ValueError(f"input tensor has only one dimension {tuple(xs.shape)}")  # mod.rs:363-365
         if bias is None:
             return weight.matmul_t(xs)
-        # broadcast_add, q8.rs:172-175: by the matmul's kernel, but for a bias that torch has to see the addition of (gradients, transforms)
-        # or that the kernel cannot read (another device, strides)
-        if type(bias) in _PLAIN_TENSORS and not hasattr(xs, "act_dtype") and bias.device == weight.device and bias.shape == (weight.n,) and not (
+        # broadcast_add, q8.rs:172-175: by the matmul's kernel, but for a bias that torch has to see the addition of (gradients, transforms, modes,
+        # tracers) or that the kernel cannot read (another device, strides)
+        if not _lib.native().observed() and type(bias) in _PLAIN_TENSORS and not hasattr(xs, "act_dtype") and bias.device == weight.device and bias.shape == (weight.n,) and not (
                 bias.requires_grad and torch.is_grad_enabled()) and not torch._C._functorch.is_functorch_wrapped_tensor(bias) and forward_ad._current_level < 0:
             return weight._matmul_float(xs, None, bias.to(xs.dtype).contiguous())
         out = weight.matmul_t(xs)
