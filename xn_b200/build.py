@@ -1,7 +1,7 @@
-"""Builds ``libxnq.so`` (the C-ABI CUDA library) in-tree with nvcc, for sm_100a only, and ``_xnq_torch.so`` (the torch side of a linear's call)
-with the host compiler.
+"""Builds, in-tree, ``libxnq.so`` (the C-ABI CUDA library; nvcc alone, for sm_100a only) and ``_xnq_torch.so`` (the torch side of a linear's call; the host
+compiler, and the headers of the torch that is installed).
 
-Usage: ``python -m xn_b200.build [--force]``.  No other architecture, no PTX fallback.
+Usage: ``python -m xn_b200.build [--force] [--library]``.  No other architecture, no PTX fallback.  ``--library``: ``libxnq.so`` alone.
 """
 from __future__ import annotations
 
@@ -16,6 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libxnq.so")
 TORCH_MODULE = os.path.join(HERE, "_xnq_torch.so")
+TORCH_STAMP = os.path.join(HERE, "build", "torch_module.txt")
 
 EXTRA = os.environ.get("XNQ_EXTRA_NVCC_FLAGS", "").split()
 if os.environ.get("XNQ_LIB_NAME"):
@@ -52,10 +53,27 @@ def is_stale() -> bool:
     return any(os.path.getmtime(p) > t for p in sources() + _deps())
 
 
-def build_torch_module(force: bool = False) -> str:
+def _torch_stamp() -> str:
+    """What the module is compiled against: it uses torch's own layouts, so another torch or Python needs another build."""
+    import torch
+    return f"torch {torch.__version__} {torch.version.git_version} python {sys.version}"
+
+
+def torch_module_is_stale() -> bool:
     src = os.path.join(CSRC, "torch_linear.cpp")
-    if not force and os.path.exists(TORCH_MODULE) and os.path.getmtime(TORCH_MODULE) >= os.path.getmtime(src):
+    if not os.path.exists(TORCH_MODULE) or os.path.getmtime(TORCH_MODULE) < os.path.getmtime(src):
+        return True
+    try:
+        with open(TORCH_STAMP) as f:
+            return f.read() != _torch_stamp()
+    except OSError:
+        return True
+
+
+def build_torch_module(force: bool = False) -> str:
+    if not force and not torch_module_is_stale():
         return TORCH_MODULE
+    src = os.path.join(CSRC, "torch_linear.cpp")
     import sysconfig
 
     import torch
@@ -68,11 +86,13 @@ def build_torch_module(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"the host compiler failed on {src}:\n{r.stdout}\n{r.stderr}")
+    os.makedirs(os.path.dirname(TORCH_STAMP), exist_ok=True)
+    with open(TORCH_STAMP, "w") as f:
+        f.write(_torch_stamp())
     return TORCH_MODULE
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    build_torch_module(force)
     if not force and not is_stale():
         return LIB
     os.makedirs(OBJ, exist_ok=True)
@@ -101,3 +121,5 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
 
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    if "--library" not in sys.argv:
+        print(build_torch_module(force="--force" in sys.argv))
