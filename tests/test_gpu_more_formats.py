@@ -123,3 +123,21 @@ def test_a_rows_bits_do_not_depend_on_the_batch(dt, n, k, ms):
         buf = torch.full((m * n + 64,), 777.0, device=DEV)
         t.matmul_t(x[:m], out=buf[: m * n].view(m, n))
         assert torch.equal(buf[: m * n].view(m, n), alone[:m]) and torch.all(buf[m * n:] == 777.0), (dt.name, n, k, m)
+
+
+# Many activation rows: how many CTAs share a tile's weight rows depends on the number of tiles (1200 rows: 150 tiles of eight; 2376: one more than there are
+# places for CTAs; 2369: the last of one row). Every row has the bits it has alone, and every element is written, once and nowhere else.
+@pytest.mark.parametrize("dt", FORMATS)
+@pytest.mark.parametrize("n,k,m", [(300, 512, 1200), (67, 256, 2376), (1030, 256, 2369), (517, 2048, 600), (4097, 512, 100)])
+def test_many_activation_rows(dt, n, k, m):
+    from xn_b200 import quantized as Q
+    Q.init(DEV)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(synth.make_weight(dt, n, k, seed=n), (n, k), dt), DEV)
+    x = torch.from_numpy(synth.make_activation(m, k, seed=k)).to(DEV)
+    buf = torch.full((m * n + 64,), 777.0, device=DEV)
+    t.matmul_t(x, out=buf[: m * n].view(m, n))
+    assert torch.all(buf[m * n:] == 777.0)
+    got = buf[: m * n].view(m, n)
+    assert torch.equal(got, torch.cat([t.matmul_t(part) for part in x.split(4)]))
+    for i in (0, m // 2, m - 1):
+        assert torch.equal(got[i], t.matmul_t(x[i:i + 1])[0])
