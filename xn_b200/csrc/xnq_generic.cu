@@ -331,21 +331,23 @@ template <>
 struct LaneSum<XNQ_Q2K> { using T = double; };
 __host__ __device__ constexpr int k_splits(int pieces) { return pieces < 64 ? 1 : (pieces < 128 ? 2 : 4); }
 
-// Eight rows: the device's CTAs walk all groups of weight rows, and the first pieces of a CTA's next group are requested while it multiplies
+// Eight rows: the device's CTAs may walk all groups of weight rows, and the first pieces of a CTA's next group are requested while it multiplies
 // the last ones of this (Q5_K 4096 x 4096, 7 rows 16.5 -> 13.9 us; Q4_1 3840 x 576, 62 rows 23.2 -> 17.7). With fewer rows more CTAs in flight do
 // better (Q5_1 26309 x 2752, one row: 21.5 us, walking 31.8), and with Q3_K's 22 words a piece (20256 x 2304, 6 rows: 41.8, walking 43.5): a
-// CTA has one group.
+// CTA has one group. So it has where one tile of activation rows meets weight rows of 32-value blocks whose pieces take a warp three turns or more (Q5_1 6582 x
+// 10496, 8 rows: 40.8, walking 43.9; Q4_1 4096 x 14336, 6 rows: 30.2, walking 32.6; two turns, Q5_0 2048 x 8192, 6 rows: 13.2, walking 12.3; Q5_K
+// 6582 x 10496, 8 rows: 58.3, walking 51.3), and where each has one anyway.
 __host__ __device__ constexpr bool walks(int dt, int mt) { return mt >= 8 && dt != XNQ_Q3K; }
+__host__ __device__ constexpr bool blocks_of_32(int dt) { return dt == XNQ_Q4_1 || dt == XNQ_Q5_0 || dt == XNQ_Q5_1; }
 
 // BIAS: a variant of its own, as in the dp4a kernels. With a test of the pointer beside the store, calls without a bias took, one row, Q5_K 14336 x 4096
 // 26.8 us instead of 26.6, Q3_K 4096 x 4096 8.17 instead of 8.06, and four rows of Q4_1 14336 x 4096 27.3 instead of 26.9.
-template <int DT, int MT, bool BIAS>
+template <int DT, int MT, bool BIAS, bool WALK>
 __global__ void __launch_bounds__(TPB, 2) generic_matmul_kernel(const uint8_t *__restrict__ w, ActView act, int64_t n, int64_t row_bytes, void *y, int y_dtype,
                                                              int64_t ldy, const void *__restrict__ bias, int64_t groups) {
   constexpr int NV = GR * MT;
   constexpr bool K256 = DT == XNQ_Q2K || DT == XNQ_Q3K || DT == XNQ_Q5K;
   using Sum = typename LaneSum<DT>::T;
-  constexpr bool WALK = walks(DT, MT);
   __shared__ Sum red[WALK ? 2 : 1][TPB / 32][NV];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int pieces = (int)(act.k / 32), ks_n = k_splits(pieces);
@@ -495,12 +497,20 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
     if (act.bsum) a.bsum += r0 * (k256 ? w.k / 16 : w.k / QK);
     void *yp = static_cast<char *>(y) + (size_t)r0 * ldy * type_size(y_dtype);
     const int64_t tiles = (a.m + mt - 1) / mt;
-    const dim3 grid((unsigned)(walks(DT, mt) ? walk_parts(groups, tiles) : groups), (unsigned)tiles);
-    const auto launch = [&](auto rows_t, auto bias_t) {
-      return launch_pdl(generic_matmul_kernel<DT, decltype(rows_t)::value, decltype(bias_t)::value>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes, yp, y_dtype, ldy, bias,
-                        groups);
+    const int pieces = (int)(w.k / 32), turns = (pieces + 32 * k_splits(pieces) - 1) / (32 * k_splits(pieces));
+    const bool plain = !walks(DT, mt) || (blocks_of_32(DT) && tiles == 1 && turns >= 3);
+    const int64_t parts = plain ? groups : walk_parts(groups, tiles);
+    const dim3 grid((unsigned)parts, (unsigned)tiles);
+    const auto launch = [&](auto rows_t, auto bias_t, auto walk_t) {
+      return launch_pdl(generic_matmul_kernel<DT, decltype(rows_t)::value, decltype(bias_t)::value, decltype(walk_t)::value>, grid, dim3(TPB), 0, s, w.qs, a, w.n, row_bytes,
+                        yp, y_dtype, ldy, bias, groups);
     };
-    const auto launch_rows = [&](auto rows_t) { return bias ? launch(rows_t, std::true_type{}) : launch(rows_t, std::false_type{}); };
+    const auto launch_rows = [&](auto rows_t) {
+      if constexpr (walks(DT, decltype(rows_t)::value))
+        if (!blocks_of_32(DT) || parts < groups) return bias ? launch(rows_t, std::true_type{}, std::true_type{}) : launch(rows_t, std::false_type{}, std::true_type{});
+      if constexpr (!walks(DT, decltype(rows_t)::value) || blocks_of_32(DT))
+        return bias ? launch(rows_t, std::true_type{}, std::false_type{}) : launch(rows_t, std::false_type{}, std::false_type{});
+    };
     cudaError_t e;
     switch (mt) {
       case 1: e = launch_rows(std::integral_constant<int, 1>{}); break;
@@ -516,8 +526,14 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
 template <int DT, int MT>
 int init_matmul_rows() { // kernels are loaded before any stream capture
   cudaFuncAttributes fa;
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, MT, false>));
-  XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, MT, true>));
+  if constexpr (walks(DT, MT)) {
+    XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, MT, false, true>));
+    XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, MT, true, true>));
+  }
+  if constexpr (!walks(DT, MT) || blocks_of_32(DT)) {
+    XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, MT, false, false>));
+    XNQ_CUDA(cudaFuncGetAttributes(&fa, generic_matmul_kernel<DT, MT, true, false>));
+  }
   return XNQ_OK;
 }
 template <int DT>
