@@ -483,9 +483,13 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
   const int rows_per_cta = TPB / 32 / k_splits((int)(w.k / 32)) * GR;
   const int64_t groups = (w.n + rows_per_cta - 1) / rows_per_cta;
   // Activation rows a warp takes at a time: eight, as far as that leaves the device enough CTAs (Q5_K 384 x 1536, 38 rows: 10.1 us with eight,
-  // 6.4 with four; Q5_1 384 x 512, 10 rows: 5.9, 4.1, 3.3 and 2.9 with eight to one); Q2_K, whose lanes' sums are f64, four (1280 x 6656, 39 rows:
-  // 62 and 49). Sixteen, with spilled registers, were slower everywhere (Q5_K 384 x 1536: 25; Q4_1 3840 x 576, 62 rows: 32.3, eight 23.2).
-  int mt = act.m >= 5 && DT != XNQ_Q2K ? 8 : (act.m >= 3 ? 4 : (int)act.m);
+  // 6.4 with four; Q5_1 384 x 512, 10 rows: 5.9, 4.1, 3.3 and 2.9 with eight to one). Q2_K's lanes' sums are f64: four where the CTAs would not fill
+  // one and a half rounds with eight (476 x 8448, 20 rows: 15.5, with eight 16.9) and for several tiles against weight rows of three turns (4096 x
+  // 14336, 20 rows: 103 and 135), else eight (4096 x 4096, 7 rows: 13.5, with four 18.0; 1200 rows: 1538 and 2308; 1280 x 6656, 39 rows: 35.2 and 48.9).
+  // Sixteen, with spilled registers, were slower everywhere (Q5_K 384 x 1536: 25; Q4_1 3840 x 576, 62 rows: 32.3, eight 23.2).
+  const int pieces = (int)(w.k / 32), turns = (pieces + 32 * k_splits(pieces) - 1) / (32 * k_splits(pieces)); // of a warp along k
+  const bool eight = DT != XNQ_Q2K || (groups * ((act.m + 7) / 8) >= 3 * g_sms && (turns < 3 || act.m <= 8));
+  int mt = act.m >= 5 && eight ? 8 : (act.m >= 3 ? 4 : (int)act.m);
   while (mt > 1 && groups * ((act.m + mt - 1) / mt) < 200) mt /= 2;
   const bool k256 = act.act_dtype == XNQ_Q8K;
   const int64_t pass = (int64_t)mt * 65535; // grid.y is limited to 65535 tiles of activation rows
@@ -497,7 +501,6 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
     if (act.bsum) a.bsum += r0 * (k256 ? w.k / 16 : w.k / QK);
     void *yp = static_cast<char *>(y) + (size_t)r0 * ldy * type_size(y_dtype);
     const int64_t tiles = (a.m + mt - 1) / mt;
-    const int pieces = (int)(w.k / 32), turns = (pieces + 32 * k_splits(pieces) - 1) / (32 * k_splits(pieces));
     const bool plain = !walks(DT, mt) || (blocks_of_32(DT) && tiles == 1 && turns >= 3);
     const int64_t parts = plain ? groups : walk_parts(groups, tiles);
     const dim3 grid((unsigned)parts, (unsigned)tiles);
