@@ -336,7 +336,8 @@ __host__ __device__ constexpr int k_splits(int pieces) { return pieces < 64 ? 1 
 // better (Q5_1 26309 x 2752, one row: 21.5 us, walking 31.8), and with Q3_K's 22 words a piece (20256 x 2304, 6 rows: 41.8, walking 43.5): a
 // CTA has one group. So it has where one tile of activation rows meets weight rows of 32-value blocks whose pieces take a warp three turns or more (Q5_1 6582 x
 // 10496, 8 rows: 40.8, walking 43.9; Q4_1 4096 x 14336, 6 rows: 30.2, walking 32.6; two turns, Q5_0 2048 x 8192, 6 rows: 13.2, walking 12.3; Q5_K
-// 6582 x 10496, 8 rows: 58.3, walking 51.3), and where each has one anyway.
+// 6582 x 10496, 8 rows: 58.3, walking 51.3), and where each has one anyway. Q5_1's one tile walks only over two rounds of groups or more (8192 x 1024, 8
+// rows: walking 1.08 times as long; 4096 x 4096: 0.93), and not where the lanes of a warp part in its last turn (17980 x 2816, 6 rows: 30.6, walking 32.6).
 __host__ __device__ constexpr bool walks(int dt, int mt) { return mt >= 8 && dt != XNQ_Q3K; }
 __host__ __device__ constexpr bool blocks_of_32(int dt) { return dt == XNQ_Q4_1 || dt == XNQ_Q5_0 || dt == XNQ_Q5_1; }
 
@@ -501,7 +502,8 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
     if (act.bsum) a.bsum += r0 * (k256 ? w.k / 16 : w.k / QK);
     void *yp = static_cast<char *>(y) + (size_t)r0 * ldy * type_size(y_dtype);
     const int64_t tiles = (a.m + mt - 1) / mt;
-    const bool plain = !walks(DT, mt) || (blocks_of_32(DT) && tiles == 1 && turns >= 3);
+    const bool plain = !walks(DT, mt) || (blocks_of_32(DT) && tiles == 1 &&
+                                          (turns >= 3 || (DT == XNQ_Q5_1 && (groups < 4 * g_sms || (turns == 2 && pieces % 32 != 0)))));
     const int64_t parts = plain ? groups : walk_parts(groups, tiles);
     const dim3 grid((unsigned)parts, (unsigned)tiles);
     const auto launch = [&](auto rows_t, auto bias_t, auto walk_t) {
