@@ -111,7 +111,7 @@ def test_matmul_row_and_tile_edges(dt, kb):
 # How many activation rows a warp takes, and whether a CTA walks over several groups of weight rows, depends on the shape (one, two and four warps
 # to a row of k; many and few groups; tiles of eight, four, two rows and one): a row's bits do not.
 @pytest.mark.parametrize("dt", FORMATS)
-@pytest.mark.parametrize("n,k,ms", [(9001, 512, (5, 8, 9, 24)), (4097, 2048, (2, 7, 17)), (3001, 4096, (3, 8, 13)), (130, 1024, (2, 3, 4, 5, 10, 40)), (1, 512, (9,)),
+@pytest.mark.parametrize("n,k,ms", [(2710, 1280, (2, 3, 4, 6, 8)), (1430, 1024, (3, 4, 5, 8)), (4500, 1536, (6, 8)), (5000, 2816, (7,)), (9001, 512, (5, 8, 9, 24)), (4097, 2048, (2, 7, 17)), (3001, 4096, (3, 8, 13)), (130, 1024, (2, 3, 4, 5, 10, 40)), (1, 512, (9,)),
                                     (2050, 8448, (5, 8, 9))])
 def test_a_rows_bits_do_not_depend_on_the_batch(dt, n, k, ms):
     from xn_b200 import quantized as Q

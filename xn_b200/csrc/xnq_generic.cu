@@ -484,14 +484,19 @@ int launch_matmul_dt(const WeightView &w, const ActView &act, int64_t row_bytes,
   const int rows_per_cta = TPB / 32 / k_splits((int)(w.k / 32)) * GR;
   const int64_t groups = (w.n + rows_per_cta - 1) / rows_per_cta;
   // Activation rows a warp takes at a time: eight, as far as that leaves the device enough CTAs (Q5_K 384 x 1536, 38 rows: 10.1 us with eight,
-  // 6.4 with four; Q5_1 384 x 512, 10 rows: 5.9, 4.1, 3.3 and 2.9 with eight to one). Q2_K's lanes' sums are f64: four where the CTAs would not fill
+  // 6.4 with four; Q5_1 384 x 512, 10 rows: 5.9, 4.1, 3.3 and 2.9 with eight to one): one to an SM, and a third more for eight and where the last of
+  // several tiles has fewer rows, whose CTAs are done sooner (779 x 8192, Q3_K, 3 rows: four at a time 5.8, two 7.6; 359 x 8192, Q4_1, 6 rows: two 1.3
+  // times as fast as four). Q2_K's lanes' sums are f64: four where the CTAs would not fill
   // one and a half rounds with eight (476 x 8448, 20 rows: 15.5, with eight 16.9) and for several tiles against weight rows of three turns (4096 x
   // 14336, 20 rows: 103 and 135), else eight (4096 x 4096, 7 rows: 13.5, with four 18.0; 1200 rows: 1538 and 2308; 1280 x 6656, 39 rows: 35.2 and 48.9).
   // Sixteen, with spilled registers, were slower everywhere (Q5_K 384 x 1536: 25; Q4_1 3840 x 576, 62 rows: 32.3, eight 23.2).
   const int pieces = (int)(w.k / 32), turns = (pieces + 32 * k_splits(pieces) - 1) / (32 * k_splits(pieces)); // of a warp along k
   const bool eight = DT != XNQ_Q2K || (groups * ((act.m + 7) / 8) >= 3 * g_sms && (turns < 3 || act.m <= 8));
   int mt = act.m >= 5 && eight ? 8 : (act.m >= 3 ? 4 : (int)act.m);
-  while (mt > 1 && groups * ((act.m + mt - 1) / mt) < 200) mt /= 2;
+  for (int64_t tiles = 0; mt > 1; mt /= 2) {
+    tiles = (act.m + mt - 1) / mt;
+    if (groups * tiles >= (mt == 8 || (tiles > 1 && act.m % mt) ? 4 * g_sms / 3 : g_sms)) break;
+  }
   const bool k256 = act.act_dtype == XNQ_Q8K;
   const int64_t pass = (int64_t)mt * 65535; // grid.y is limited to 65535 tiles of activation rows
   for (int64_t r0 = 0; r0 < act.m; r0 += pass) {
