@@ -291,7 +291,7 @@ def test_integer_kernel_parts_of_tiles(Q, O, dt, n, k):
 # 16-bit results take as many tiles of activation rows as finish first: 8 of 192 rows instead of 6 of 256, 10 of 64 instead of 3, 2 of 80 instead of 1, 7 of 256
 # on single CTAs where pairs would take a round more; bits of a tile's sums do not depend on its width, so that f32 results rounded once are the same
 @pytest.mark.parametrize("dt", WEIGHT_TYPES)
-@pytest.mark.parametrize("n,m", [(3584, 1459), (1100, 600), (4100, 150), (2615, 1773)])
+@pytest.mark.parametrize("n,m", [(3584, 1459), (1100, 600), (4100, 150), (2615, 1773), (8910, 165)])
 def test_fp16_kernel_number_of_tiles(Q, O, dt, n, m):
     k = 768 if dt.block_size == 256 else 736
     w = synth.make_weight(dt, n, k, seed=m + n)

@@ -1016,7 +1016,9 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   // 16-bit results, whose tiles are whole: equal tiles of activation rows, in the MMA's steps of 16 columns (pairs: 32, 16 of each CTA), as many as
   // finish first: rounds of the CTAs times a tile's time. Measured for one round (18944 x 1024 and 4096; Q4_K, Q8_0 and Q6_K alike), a k-step takes
   // the same up to 128 rows (what bounds it is the conversion of the weights) and then a 256th more for every further row: 66 rows 0.277 us, 128
-  // 0.290, 192 0.374, 256 0.423; a tile's start and end take two k-steps and another for 64 rows.
+  // 0.290, 192 0.374, 256 0.423; a tile's start and end take two k-steps and another for 64 rows. Where more than half of the SMs are
+  // at work all of it takes 1.4 us longer: 4096 x 1024, 165 rows 9.8 us as two tiles on 64 CTAs, 11.3 as three on 96; 8912 x 1280, 165 rows 12.6 as one on
+  // 70 CTAs, 13.3 as two on 140 (Q8_0 12.9 and 14.6); but 9060 x 4480, 138 rows 28.5 as one on 71, 27.1 as two on 142.
   // Pairs halve the activation operand's traffic, which is what bounds wide tiles: from 224 rows a tile on they are the faster or the equal
   // ones (in a long stream of calls, Q4_K 14336 x 4096: 224 rows 41.8 against 42.6 us, 512 rows 74.5 / 77.5, 1024 rows 128 / 139; but 176 rows
   // 39.0 / 37.0). With few tiles a pair's coarser share of the work costs more than that (Q4_K 1536 x 2048, 2000 rows, 21 k-steps a pair: 35.2 / 33.5).
@@ -1025,11 +1027,13 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
   bool pairs = false;
   a.mt = (int)std::min<int64_t>(MAX_MT, m_pad);
   if (a.whole_tiles) {
-    double best = 0;
+    double best = 0, best_crowded = 0;
     const auto consider = [&](int mt, bool pair) {
       const long long tiles_m = (m_pad + mt - 1) / mt, ctas = pair ? g_num_pairs : sms, count = (pair ? (row_tiles + 1) / 2 : row_tiles) * tiles_m;
-      const double time = (double)((count + ctas - 1) / ctas) * (ksteps * (256. + std::max(0, mt - 128)) * (pair ? 0.95 : 1.) + 512. + 4. * mt);
-      if (best == 0 || time < 0.98 * best) best = time, a.mt = mt, a.tiles_m = (int)tiles_m, pairs = pair; // fewer and wider ones where it makes no difference
+      const double crowded = std::min(count, ctas) * (pair ? 2 : 1) > sms / 2 ? 1300. : 0.;
+      const double time = (double)((count + ctas - 1) / ctas) * (ksteps * (256. + std::max(0, mt - 128)) * (pair ? 0.95 : 1.) + 512. + 4. * mt) + crowded;
+      // fewer and wider ones where it makes no difference (the 1.4 us are allowed for as they are)
+      if (best == 0 || time < (crowded > best_crowded ? 1. : 0.98) * best) best = time, best_crowded = crowded, a.mt = mt, a.tiles_m = (int)tiles_m, pairs = pair;
     };
     const int64_t fewest = a.tiles_m;
     for (int64_t t = fewest, last = 0; t <= std::min(4 * fewest, fewest + 12); t++) {
