@@ -311,3 +311,45 @@ def test_fp16_kernel_number_of_tiles(Q, O, dt, n, m):
 @pytest.mark.parametrize("dt", WEIGHT_TYPES)
 def test_fp16_kernel_keeps_off_sms(Q, O, dt):
     test_fp16_kernel_number_of_tiles(Q, O, dt, 8910, 165)
+
+
+def _status_is_clean():
+    import ctypes
+
+    from xn_b200 import _lib
+    bits = ctypes.c_uint(0)
+    _lib.check(_lib.lib().xnq_device_status(ctypes.byref(bits)))
+    assert bits.value == 0, f"device status {bits.value:#x}"
+
+
+# Rows of a wider buffer: nothing past a row's end is written, between the rows or behind the last one, in 16-byte stores (n and the rows' distance are whole
+# pieces of them) and in single ones
+@pytest.mark.parametrize("dt", WEIGHT_TYPES)
+@pytest.mark.parametrize("n,m,gap", [(515, 700, 7), (512, 700, 8), (516, 528, 12), (1029, 260, 3), (120, 70, 8), (1, 300, 1)])
+def test_fp16_kernel_keeps_inside_its_rows(Q, dt, n, m, gap):
+    k = 512 if dt.block_size == 256 else 352
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(synth.make_weight(dt, n, k, seed=m + n), (n, k), dt), DEV)
+    x = torch.from_numpy(synth.make_activation(m, k, seed=m)).to(DEV)
+    for out in (torch.float32, torch.float16, torch.bfloat16):
+        want = t.matmul_t(x, out=torch.empty(m, n, dtype=out, device=DEV))
+        wide = torch.full((m, n + gap), 777.0, dtype=out, device=DEV)
+        t.matmul_t(x, out=wide[:, :n])
+        assert torch.all(wide[:, n:] == 777.0), (dt.name, out)
+        if out is torch.float32:   # parts of a split tile may meet in another order
+            assert torch.allclose(wide[:, :n], want, rtol=0, atol=1e-5 * float(want.abs().max()))
+        else:
+            assert torch.equal(wide[:, :n], want)
+
+
+# As test_fp16_kernel_missing_steps, each of the calls against the oracle, and no wait ran out
+@pytest.mark.parametrize("dt", [d for d in WEIGHT_TYPES if d.block_size == 32])
+@pytest.mark.parametrize("n,k,m", [(640, 8384, 814), (1029, 8512, 700), (300, 1312, 814), (2048, 96, 1100), (520, 4128, 100)])
+def test_fp16_kernel_missing_steps_in_every_call(Q, O, dt, n, k, m):
+    w = synth.make_weight(dt, n, k, seed=m + n)
+    x = synth.make_activation(m, k, seed=m)
+    t = Q.QCudaTensor.from_qtensor(Q.QTensor(w, (n, k), dt), DEV)
+    xd = torch.from_numpy(x).to(DEV)
+    want = O.matmul(int(dt), x, w, n, threads=O.hw_threads())
+    for i in range(20):
+        _check(t.matmul_t(xd).cpu().numpy(), want, f"{dt.name} m={m} n={n} k={k}, call {i}")
+    _status_is_clean()
