@@ -942,6 +942,24 @@ constexpr size_t SM_SMEM = 228 * 1024, MAX_SPREAD = SM_SMEM / 2;
 static_assert(RowQ4_0::SLOT == RowQ4K::SLOT && RowQ8_0::SLOT == RowQ4K::SLOT, "the raw ring's plan assumes one slot size for these");
 constexpr size_t PREFILL_SMEM = 225 * 1024; // everything an SM offers minus the static barriers and a reserve
 
+// Shared-memory plan: B ring | raw ring | the drain warps' chunks. With up to eight stages a producer warp can be a whole super-step ahead of the MMAs;
+// what is left goes to the raw ring (it covers the memory latency of the weights).
+constexpr uint32_t b_stride_of(int rows) { return ((uint32_t)rows * 128 + 1023) & ~1023u; }
+struct SmemPlan {
+  int nstages, raw_slots;
+};
+constexpr SmemPlan smem_plan(int rows, uint32_t slot) { // rows: a CTA's activation rows of a tile; slot: bytes of a raw super-step
+  const size_t budget = PREFILL_SMEM - 1024 - EPI_WARPS * EPI_SLOT, stride = b_stride_of(rows); // 1024: alignment slack
+  SmemPlan p{0, 0};
+  for (int raw = 3; raw >= 2 && p.nstages < MIN_STAGES; raw--) // at least so many raw slots
+    p.nstages = (int)std::min<size_t>(MAX_STAGES, (budget - raw * slot) / stride);
+  p.raw_slots = (int)std::min<size_t>(MAX_RAW_SLOTS, (budget - p.nstages * stride) / slot);
+  return p;
+}
+constexpr bool plan_is(int rows, uint32_t slot, int stages, int slots) { return smem_plan(rows, slot).nstages == stages && smem_plan(rows, slot).raw_slots == slots; }
+static_assert(plan_is(256, RowQ4K::SLOT, 4, 4) && plan_is(256, RowQ6K::SLOT, 4, 2), "a wide tile of one CTA: four stages");
+static_assert(plan_is(128, RowQ4K::SLOT, 8, 4) && plan_is(128, RowQ6K::SLOT, 7, 3), "and half of it, of a pair's CTA");
+
 template <typename RowT>
 int init_fmt(int *pairs) { // pairs: lowered to what the device holds at a time of this kernel (0: not set yet)
   XNQ_CUDA(cudaFuncSetAttribute(prefill_persistent_kernel<RowT, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREFILL_SMEM));
@@ -1045,18 +1063,12 @@ int launch_prefill(const WeightView &w, float wscale, const void *x, int x_dtype
     }
   }
   const int cg = pairs ? 2 : 1;
-  // Shared-memory plan: B ring | raw ring. With up to eight stages a producer warp can be a whole super-step ahead of the MMAs; what is
-  // left goes to the raw ring (it covers the memory latency of the weights). At 256 activation rows that is five stages and three
-  // raw slots (two for Q6_K), for a pair eight and five (three).
   const uint32_t slot = w.dtype == XNQ_Q6K ? RowQ6K::SLOT : RowQ4K::SLOT;
-  a.b_stride = ((uint32_t)(a.mt / cg) * 128 + 1023) & ~1023u;
-  const size_t budget = PREFILL_SMEM - 1024 - EPI_WARPS * EPI_SLOT; // 1024: alignment slack
-  for (int raw = 3; raw >= 2; raw--) { // at least so many raw slots
-    a.nstages = (int)std::min<size_t>(MAX_STAGES, (budget - raw * slot) / a.b_stride);
-    if (a.nstages >= MIN_STAGES) break;
-  }
-  if (a.nstages < MIN_STAGES) return fail(XNQ_ERR_SIZE, "prefill: shared-memory plan does not fit");
-  a.raw_slots = (int)std::min<size_t>(MAX_RAW_SLOTS, (budget - (size_t)a.nstages * a.b_stride) / slot);
+  a.b_stride = b_stride_of(a.mt / cg);
+  const SmemPlan plan = smem_plan(a.mt / cg, slot);
+  if (plan.nstages < MIN_STAGES) return fail(XNQ_ERR_SIZE, "prefill: shared-memory plan does not fit");
+  a.nstages = plan.nstages;
+  a.raw_slots = plan.raw_slots;
   a.raw_off = a.nstages * a.b_stride;
   a.epi_off = a.raw_off + a.raw_slots * slot;
   const size_t yes = type_size(y_dtype), piece = 16 / yes;
@@ -1091,7 +1103,7 @@ int prefill_init(int device) {
   cudaDeviceProp prop;
   XNQ_CUDA(cudaGetDeviceProperties(&prop, device));
   g_num_sms = prop.multiProcessorCount;
-  // pairs that are resident together: the CTAs of a split tile wait for one another
+  // pairs that are resident together: the rule on the number of tiles counts rounds of them
   int pairs = 0, rc = XNQ_OK;
   if ((rc = init_fmt<RowQ4_0>(&pairs)) != XNQ_OK || (rc = init_fmt<RowQ8_0>(&pairs)) != XNQ_OK || (rc = init_fmt<RowQ4K>(&pairs)) != XNQ_OK ||
       (rc = init_fmt<RowQ6K>(&pairs)) != XNQ_OK)
