@@ -162,8 +162,8 @@ size_t xnq_matmul_workspace_bytes(const xnq_weight *w, int64_t max_m);
  * Enqueues on `stream` only; allocates nothing. */
 int xnq_matmul_t(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, void *y,
                  int y_dtype, int64_t ldy, void *workspace, size_t ws_bytes, void *stream);
-/* The same on float activations with a bias: n_local values of y's type in device memory, added to the f32 sums before they are
- * rounded to y's type (Q8Linear::forward's broadcast_add, q8.rs:172-175); NULL: none. */
+/* The same on float activations with a bias: n_local values of y's type in device memory; NULL: none. The bits are those of an addition of its own in y's
+ * type (Q8Linear::forward's broadcast_add, q8.rs:172-175): the f32 sum is rounded to y's type, the bias is added in f32, the result is rounded again. */
 int xnq_matmul_t_bias(const xnq_weight *w, const void *x, int x_dtype, int64_t m, int64_t ldx, const void *bias, void *y,
                       int y_dtype, int64_t ldy, void *workspace, size_t ws_bytes, void *stream);
 /* xnq_matmul_t_bias of one row where that needs no scratch: Q4_0, Q8_0, Q4_K and Q6_K weights of up to 4096 columns. Others: XNQ_ERR_UNSUPPORTED
