@@ -105,3 +105,34 @@ def test_one_row_without_scratch(dt, n, k, served):
         assert L.xnq_matvec(w._h, x.data_ptr(), Q._XNQ_IDS[act], None, None, Q._XNQ_IDS[act], None) == -1
         assert L.xnq_matvec(w._h, x.data_ptr(), Q._XNQ_IDS[act], None, y.data_ptr(), 2, None) == -2
         assert L.xnq_matvec(w._h, x.data_ptr() + 2, Q._XNQ_IDS[act], None, y.data_ptr(), Q._XNQ_IDS[act], None) == -4
+
+
+def test_many_streams():
+    """More streams than scratch is kept for, again after all weights are gone."""
+    streams = [torch.cuda.Stream(DEV) for _ in range(24)]
+    for _ in range(2):
+        layer, xs, want = _pairs(D.Q5K, 2048, 2048, 7, torch.float32)
+        got = []
+        for _ in range(4):
+            for i, s in enumerate(streams):
+                with torch.cuda.stream(s):
+                    got.append((i % 2, layer.forward(xs[i % 2])))
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want[i]) for i, y in got)
+        del layer, got
+
+
+def test_rows_of_changing_number():
+    """Calls whose scratch differs in size and kind, in turn on one stream, scratch that is kept and scratch that is not."""
+    layer, _, _ = _pairs(D.Q4K, 512, 2048, 2, torch.float32)
+    other, _, _ = _pairs(D.Q5K, 512, 2048, 2, torch.float32)
+    ms = (1, 2, 3, 7, 16, 64, 65, 300, 2000)
+    xs = [torch.from_numpy(synth.make_activation(m, 2048, seed=m)).to(torch.bfloat16).to(DEV) for m in ms]
+    want = []
+    for x in xs:
+        want.append([w.forward(x) for w in (layer, other)])
+        torch.cuda.synchronize()
+    got = [[w.forward(x) for w in (layer, other)] for _ in range(20) for x in xs]
+    torch.cuda.synchronize()
+    for i, ys in enumerate(got):
+        assert all(torch.equal(y, v) for y, v in zip(ys, want[i % len(ms)])), ms[i % len(ms)]

@@ -3,7 +3,8 @@
 //
 // A one-row call is bound by the host, not by its kernel (Q4_0 4096 x 4096: the kernel takes 3.3 us). In Python, with the library called through
 // ctypes, it took 10.5 us: some 25 attribute reads and comparisons, a tensor made through the dispatcher, twelve arguments converted one by one, and
-// the launch. Everything that is not ordinary returns None, and the Python code takes the call; nothing is kept from one call for the next.
+// the launch. Everything that is not ordinary returns None, and the Python code takes the call; nothing is kept from one call for the next but
+// scratch, by stream.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -20,6 +21,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <mutex>
 
 namespace {
 
@@ -41,12 +43,61 @@ struct Weight { // what a call needs of a weight; owned by the capsule that the 
 };
 constexpr int UNSUPPORTED = -8; // XNQ_ERR_UNSUPPORTED
 constexpr const char *NAME = "xnq.weight";
-void free_weight(PyObject *capsule) { delete static_cast<Weight *>(PyCapsule_GetPointer(capsule, NAME)); }
 
-// Scratch (the quantized activations, the tickets and partial sums of split tiles) is a call's own, from torch's caching allocator, which gives a
-// block out again in the order of the stream that it was allocated for, or within the graph that is being captured. One buffer for all calls of a
-// device was overwritten by calls on another stream, by another thread's call between a call's kernels, and by graphs replayed side by side. A block
-// costs 0.35 us of a one-row call (Q4_0 4096 x 4096: 4.1 us instead of 3.75), so that rows that need none get none.
+// Scratch (the quantized activations, the tickets and partial sums of split tiles): one buffer for all calls of a device was overwritten by calls on
+// another stream, by another thread's call between a call's kernels, and by graphs replayed side by side. So a call gets a block of its own from torch's
+// caching allocator, which gives it out again in the order of the stream that it was allocated for, or within the graph that is being captured. That
+// costs a call 0.4 us (one row of Q5_K 384 x 1536, which the host bounds: 5.65 instead of 5.25 us), so that rows that need no scratch get none, and
+// up to a MiB, all that such small calls ask for, is taken from a slab of the stream (5.4 us): whoever enqueues a call's kernels holds the slab's
+// lock, and the stream keeps them in order. Not under capture: a graph may be replayed on another stream. At most SLABS streams have one; the slabs are given
+// back with the last weight. (Not from the caching allocator, whose block might belong to a pool of the program's.)
+struct Slab {
+  c10::DeviceIndex device;
+  cudaStream_t stream;
+  void *p;
+  std::mutex lock;
+};
+constexpr size_t SLAB = 1 << 20;
+constexpr int SLABS = 16;
+Slab g_slabs[SLABS]; // they and the counts: under the interpreter's lock
+int g_num_slabs = 0;
+int64_t g_weights = 0;
+
+struct RelaxedCapture { // (a graph that another thread is capturing does not mind what this one allocates or frees)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// the slab of a stream of the current device, or null: the call takes a block of its own
+Slab *slab_for(c10::DeviceIndex device, cudaStream_t stream, size_t bytes) {
+  if (bytes > SLAB) return nullptr;
+  cudaStreamCaptureStatus capture;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  if (capture != cudaStreamCaptureStatusNone) return nullptr;
+  for (int i = 0; i < g_num_slabs; i++)
+    if (g_slabs[i].stream == stream && g_slabs[i].device == device) return &g_slabs[i];
+  if (g_num_slabs == SLABS) return nullptr;
+  Slab &s = g_slabs[g_num_slabs];
+  const RelaxedCapture relaxed;
+  if (cudaMalloc(&s.p, SLAB) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  s.device = device, s.stream = stream;
+  g_num_slabs++;
+  return &s;
+}
+void free_weight(PyObject *capsule) {
+  delete static_cast<Weight *>(PyCapsule_GetPointer(capsule, NAME));
+  if (--g_weights > 0) return;
+  const RelaxedCapture relaxed;
+  for (; g_num_slabs > 0; g_num_slabs--) (void)cudaFree(g_slabs[g_num_slabs - 1].p); // (waits for the kernels that use it; fails where the process is ending)
+  (void)cudaGetLastError();
+}
+
 size_t scratch_bytes(Weight *w, int64_t rows) {
   if (w->ws_rows != rows) w->ws_rows = rows, w->ws_bytes = std::max<size_t>(g_workspace_bytes(w->handle, rows), 256);
   return w->ws_bytes;
@@ -105,7 +156,7 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   at::Tensor y = at::Tensor(at::detail::empty_cuda(shape, x.scalar_type(), x.device(), std::nullopt));
   void *const yp = y.mutable_data_ptr();
   const void *const xp = x.const_data_ptr();
-  void *const stream = c10::cuda::getCurrentCUDAStream(w->device).stream();
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(w->device).stream();
   int rc = UNSUPPORTED;
   if (m == 1 && w->row_without_scratch) {
     Py_BEGIN_ALLOW_THREADS // a launch may block while the device's queue is full
@@ -115,9 +166,14 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   }
   if (rc == UNSUPPORTED) {
     const size_t wsb = scratch_bytes(w, m);
-    const c10::DataPtr ws = c10::cuda::CUDACachingAllocator::get()->allocate(wsb); // for the current device and stream, where the call launches
+    Slab *const slab = slab_for(w->device, stream, wsb);
+    c10::DataPtr block;
+    if (!slab) block = c10::cuda::CUDACachingAllocator::get()->allocate(wsb); // for the current device and stream, where the call launches
+    void *const ws = slab ? slab->p : block.get();
     Py_BEGIN_ALLOW_THREADS
-    rc = g_matmul(w->handle, xp, xt, m, ldx, bias, yp, xt, w->n, ws.get(), wsb, stream);
+    if (slab) slab->lock.lock();
+    rc = g_matmul(w->handle, xp, xt, m, ldx, bias, yp, xt, w->n, ws, wsb, stream);
+    if (slab) slab->lock.unlock();
     Py_END_ALLOW_THREADS
   }
   if (rc != 0) return PyObject_CallFunction(g_check, "i", rc);
@@ -144,7 +200,9 @@ PyObject *weight(PyObject *, PyObject *args) {
   long long n, k;
   int device;
   if (!PyArg_ParseTuple(args, "KLLi", &handle, &n, &k, &device)) return nullptr;
-  return PyCapsule_New(new Weight{reinterpret_cast<const void *>(handle), n, k, (c10::DeviceIndex)device, -1, 0, true}, NAME, free_weight);
+  PyObject *capsule = PyCapsule_New(new Weight{reinterpret_cast<const void *>(handle), n, k, (c10::DeviceIndex)device, -1, 0, true}, NAME, free_weight);
+  if (capsule) g_weights++;
+  return capsule;
 }
 
 // bind(xnq_matmul_t_bias, xnq_matvec, xnq_matmul_workspace_bytes, check): the library that ctypes has loaded
