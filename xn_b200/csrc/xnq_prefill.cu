@@ -112,8 +112,8 @@ __device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity,
 }
 // Whether the phase has completed, without waiting for it. A wait takes 120 to 250 cycles even when there is nothing to wait for, and with 32 rows every
 // role took a turn of 550 cycles that way. The loops below look at the next turn's barrier while this turn's work is under way and wait only for what was
-// not there yet. With Q6_K's shorter conversion, a stream of calls, best and median clock: Q6_K 128256 x 4096, 32 rows 130 and 139 -> 114 and 129 us; Q4_K
-// 28672 x 4096, 65 rows 38.0 -> 36.2; Q8_0 8192 x 4096, 128 rows 29.4 -> 28.4. (Two k-steps a turn on top: no difference.)
+// not there yet: Q4_K 28672 x 4096, 65 rows 38.0 -> 36.2 us; Q8_0 8192 x 4096, 128 rows 29.4 -> 28.4; with Q6_K's shorter conversion, Q6_K 128256 x 4096, 32
+// rows 142 -> 131 in one run (137 in most; a long stream of calls, under the power limit). (Two k-steps a turn on top: no difference.)
 __device__ __forceinline__ bool mbar_peek(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -704,8 +704,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
     int i = 0;
     for (int seg = 0; i < nsteps && alive; seg++) {
       const int len = min(KT - cur.kt, nsteps - i);
-      const int row_tile = cur.tile_n * CG + (int)rank, tile = row_tile * TM + cur.tile_m; // each CTA of a pair settles its own 128 rows of a split tile
-      const bool whole = (cur.kt == 0 && len == KT) || row_tile >= p.row_tiles;
+      const int row_tile = cur.tile_n * CG + (int)rank, tile = row_tile * TM + cur.tile_m;
+      const bool whole = CG == 2 || (cur.kt == 0 && len == KT); // (pairs take whole tiles of 16-bit results only)
       const int buf = NACC == 2 ? seg & 1 : 0, use = NACC == 2 ? seg >> 1 : seg;
       const int64_t m0 = (int64_t)cur.tile_m * p.mt;
       const int mt = CG == 2 ? p.mt : (int)min((int64_t)p.mt, p.m_pad - m0); // columns
@@ -746,7 +746,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
       if (alive) {
         tc_fence_after();
         const uint32_t lane_addr = tmem_d + (uint32_t)(buf * 128) + ((uint32_t)(32 * q) << 16);
-        const int es = p.y_dtype == XNQ_F32 ? 4 : 2;
+        const bool f32 = CG == 1 && p.y_dtype == XNQ_F32;
+        const int es = f32 ? 4 : 2;
         const int64_t row_bytes = p.ldy * es, row0 = (int64_t)row_tile * TILE_N + 32 * q;
         const int rows = (int)max((int64_t)0, min((int64_t)32, p.w.n - row0)); // of this warp's 32
         char *const y0 = static_cast<char *>(p.y) + m0 * row_bytes + row0 * es;
@@ -771,7 +772,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
             for (int j = 0; j < 16; j++) sts32(slot + (uint32_t)(j * 128) + ((uint32_t)(lane * 4) ^ ((j & 1) << 4)), v[j]);
             if (next < mt) tmem_ld16(lane_addr + next, v); // arrives while the chunk is stored
             __syncwarp();
-            if (p.y_dtype == XNQ_F32) {
+            if (f32) {
               if (ticket == 0) store_turned<STORE_F32>(slot, ru, bias, yp, row_bytes, cols, rows, lane);
               else store_turned<ADD_F32>(slot, ru, bias, yp, row_bytes, cols, rows, lane);
             } else if (p.y_dtype == XNQ_F16) {
@@ -782,7 +783,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) prefill_persistent_kernel(const _
             __syncwarp();
           } else {
             const bool row_ok = lane < rows;
-            if (p.y_dtype == XNQ_F32) {
+            if (f32) {
               if (ticket == 0) store_direct<STORE_F32>(v, ru, bias, yp, row_bytes, cols, row_ok, lane);
               else store_direct<ADD_F32>(v, ru, bias, yp, row_bytes, cols, row_ok, lane);
             } else if (p.y_dtype == XNQ_F16) {
