@@ -9,6 +9,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/GradMode.h>
@@ -48,7 +49,7 @@ constexpr const char *NAME = "xnq.weight";
 // another stream, by another thread's call between a call's kernels, and by graphs replayed side by side. So a call gets a block of its own from torch's
 // caching allocator, which gives it out again in the order of the stream that it was allocated for, or within the graph that is being captured. That
 // costs a call 0.4 us (one row of Q5_K 384 x 1536, which the host bounds: 5.65 instead of 5.25 us), so that rows that need no scratch get none, and
-// up to a MiB, all that such small calls ask for, is taken from a slab of the stream (5.4 us): whoever enqueues a call's kernels holds the slab's
+// up to four MiB, all that such small calls ask for, are taken from a slab of the stream (5.4 us): whoever enqueues a call's kernels holds the slab's
 // lock, and the stream keeps them in order. Not under capture: a graph may be replayed on another stream. At most SLABS streams have one; the slabs are given
 // back with the last weight. (Not from the caching allocator, whose block might belong to a pool of the program's.)
 struct Slab {
@@ -57,7 +58,7 @@ struct Slab {
   void *p;
   std::mutex lock;
 };
-constexpr size_t SLAB = 1 << 20;
+constexpr size_t SLAB = 4 << 20; // the integer kernel's parts of split tiles take 2.4 MB with up to 16 rows
 constexpr int SLABS = 16;
 Slab g_slabs[SLABS]; // they and the counts: under the interpreter's lock
 int g_num_slabs = 0;
@@ -153,7 +154,8 @@ PyObject *linear(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
   }
   c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
   shape[dims - 1] = w->n;
-  at::Tensor y = at::Tensor(at::detail::empty_cuda(shape, x.scalar_type(), x.device(), std::nullopt));
+  // (what empty_cuda does behind its look for the device, which is the current one here)
+  at::Tensor y = at::Tensor(at::detail::empty_generic(shape, c10::cuda::CUDACachingAllocator::get(), c10::DispatchKeySet(c10::DispatchKey::CUDA), x.scalar_type(), std::nullopt));
   void *const yp = y.mutable_data_ptr();
   const void *const xp = x.const_data_ptr();
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(w->device).stream();
