@@ -48,8 +48,8 @@ constexpr const char *NAME = "xnq.weight";
 // Scratch (the quantized activations, the tickets and partial sums of split tiles): one buffer for all calls of a device was overwritten by calls on
 // another stream, by another thread's call between a call's kernels, and by graphs replayed side by side. So a call gets a block of its own from torch's
 // caching allocator, which gives it out again in the order of the stream that it was allocated for, or within the graph that is being captured. That
-// costs a call 0.4 us (one row of Q5_K 384 x 1536, which the host bounds: 5.65 instead of 5.25 us), so that rows that need no scratch get none, and
-// up to four MiB, all that such small calls ask for, are taken from a slab of the stream (5.4 us): whoever enqueues a call's kernels holds the slab's
+// costs a call 0.4 us (two rows of Q4_1 512 x 512, which the host bounds: 6.35 us, with the one buffer 5.85), so that rows that need no scratch get none,
+// and up to four MiB, all that such small calls ask for, are taken from a slab of the stream (5.9 us): whoever enqueues a call's kernels holds the slab's
 // lock, and the stream keeps them in order. Not under capture: a graph may be replayed on another stream. At most SLABS streams have one; the slabs are given
 // back with the last weight. (Not from the caching allocator, whose block might belong to a pool of the program's.)
 struct Slab {

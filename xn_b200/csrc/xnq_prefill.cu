@@ -363,7 +363,8 @@ __device__ __forceinline__ void store_direct(const uint32_t (&v)[16], uint32_t r
 // MMA were what bounded such tiles (28672 x 4096, 2000 rows: 415 -> 390 us at full clock). The leader issues the MMAs; the other CTA's warp
 // of that role tells it when its half of a stage is there, and the commits arrive on both CTAs' barriers. (The relay's arrival and the
 // leader's wait have the default semantics: with .release.cluster and .acquire.cluster each costs a fence of some 1000 cycles and the kernel
-// took 654 us. What they order, tensor-memory stores and bulk copies, has completed before the local barrier lets the relay pass.)
+// took 654 us. PTX promises the order at that scope only; the default suffices because what it orders, tensor-memory stores and bulk copies, has been
+// performed in the memory of the CTA whose half of the MMA reads it before that CTA's own barrier lets the relay pass.)
 // One CTA per SM (or pair per two) walks a contiguous range of the flattened (tile, k-step) space, so all SMs finish
 // together whatever the tile count, and a tile whose k-steps are split between CTAs is summed in
 // global memory: the first CTA to finish its part stores it and raises the tile's flag, the others add
